@@ -49,6 +49,16 @@ __device__ __forceinline__ float diff_shift(float a, float b, int k, float L) {
 // pbcCalc (femmd2D/src/def.h:112)
 __device__ __forceinline__ float wrap_coord(float r, float L) { return r - floorf(r / L) * L; }
 
+// wrap_coord without its division for -L <= r < 2 L, where floor(r / L) is
+// -1, 0 or 1 whatever the quotient's rounding (r < L gives a quotient of at
+// most 1 - 2^-24, r < 2 L one of at most 2 - 2^-23): the same single rounding.
+__device__ __forceinline__ float wrap_near(float r, float L) {
+    if (r >= 0.0f && r < L) return r;
+    if (r < 0.0f && r >= -L) return r + L;
+    if (r >= L && r < 2.0f * L) return r - L;
+    return wrap_coord(r, L);
+}
+
 // cellId (femmd2D/src/nnCuda.cu:9-17): float multiply, IEEE divide, truncate;
 // an index equal to the cell count is moved into the last cell.  Indices
 // outside the grid (only reachable on a non-periodic axis, where the
@@ -102,6 +112,27 @@ __device__ __forceinline__ float own_logf(float x) {
     const float ln2_lo = 1.428606765330187e-06f;
     float fk = (float)k;
     return (fk * ln2_lo + lm) + fk * ln2_hi;
+}
+
+// Packed single precision, each lane rounded as the scalar operation.  A
+// packed product must not feed a packed sum: the assembler contracts the two
+// into a fused multiply-add even with .rn and -fmad=false (measured; the same
+// for __fmul2_rn and __fadd2_rn), so such products are formed by __fmul_rn.
+__device__ __forceinline__ unsigned long long pack2(float2 a) {
+    return (unsigned long long)__float_as_uint(a.y) << 32 | __float_as_uint(a.x);
+}
+__device__ __forceinline__ float2 unpack2(unsigned long long v) {
+    return make_float2(__uint_as_float((unsigned)v), __uint_as_float((unsigned)(v >> 32)));
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+    unsigned long long r;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+    return unpack2(r);
+}
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack2(a)), "l"(pack2(b)));
+    return unpack2(r);
 }
 
 __device__ __forceinline__ float warp_sum_f(float v) {

@@ -208,6 +208,13 @@ struct femmd_ctx {
     // a wait that gave up, which can leave records ahead of the tag base)
     bool smallClean = false;
     bool testExpire = false;  // femmd_test_expire_next_exchange
+    // the whole-run launch (k_coop): exchange words and cell counts, zero
+    // together with their scalars (runClean); coopOff: a cell held more than
+    // kCellCap particles, the plain kernels from then on
+    DBuf<unsigned long long> runRec;
+    DBuf<int> cellFill, cellIds;
+    DBuf<float4> cellCand;
+    bool runClean = false, coopOff = false;
     // profiling
     bool profiling = false;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> forceEvents;
@@ -350,7 +357,7 @@ static void release_device(femmd_ctx *c) {
     c->props.release(); c->propsCk.release(); c->propPart.release(); c->centroid.release();
     c->propsUploaded = false;
     c->perm.release(); c->sPerm.release(); c->fBlockSums.release(); c->ckPerm.release(); c->idType.release();
-    c->newCell.release(); c->blockWin.release(); c->smallRec.release(); c->sPos.release(); c->sVel.release(); c->sAcc.release();
+    c->newCell.release(); c->blockWin.release(); c->smallRec.release(); c->runRec.release(); c->cellFill.release(); c->cellIds.release(); c->cellCand.release(); c->sPos.release(); c->sVel.release(); c->sAcc.release();
     c->cpos0.release(); c->cpos1.release(); c->cslot.release();
     c->idMass.release(); c->idSigma.release(); c->idWallDelta.release(); c->idWallSig.release(); c->xfer1.release();
     auto &a = c->adj;
@@ -492,6 +499,10 @@ static DevSys make_sys(femmd_ctx *c) {
     s.C2 = c->C2;
     s.C3 = c->C3;
     s.sc = c->sc.p;
+    s.runRec = c->runRec.p;
+    s.cellFill = c->cellFill.p;
+    s.cellIds = c->cellIds.p;
+    s.cellCand = c->coopOff ? nullptr : c->cellCand.p;
     s.obs = c->obs.p;
     s.obsCap = c->obsCap;
     s.trace = c->tracing ? c->trace.p : nullptr;
@@ -518,6 +529,7 @@ static DevSys make_sys(femmd_ctx *c) {
     s.posPre = area ? c->posPre.p : nullptr;
     s.nPre = area ? c->nBonded : 0;
     s.fast = c->forceMode == FEMMD_FORCE_FAST;
+    s.imgD = c->nnRadius + c->skin;  // only which loop is tried first depends on it
     if (s.fast) {
         s.imgD = c->imgD;
         s.perm = c->perm.p;
@@ -813,6 +825,7 @@ static femmd_status upload_topology(femmd_ctx *ctx) {
     CK(ctx->cellStart.ensure(ctx->ncells + 8));
     CK(ctx->blockSums.ensure(scan_blocks(ctx->ncells)));
     CK(ctx->sc.ensure(1));
+    ctx->runClean = ctx->coopOff = false;
     cudaStream_t s = ctx->stream;
     if (N > 0) {
         CK(cudaMemcpyAsync(ctx->dmass.p, ctx->mass.data(), N * sizeof(float), cudaMemcpyHostToDevice, s));
@@ -1221,11 +1234,69 @@ static femmd_status small_units(femmd_ctx *ctx, const DevSys &s, int units) {
     return FEMMD_OK;
 }
 
+// A bounded wait gave up inside a run: the exchange records and their tag
+// bases start anew before the next one, and the cell counts of a binning that
+// did not finish are cleared.
+static femmd_status expired(femmd_ctx *ctx, const char *what) {
+    ctx->smallClean = ctx->runClean = false;
+    CK(cudaMemsetAsync(ctx->cellCount.p, 0, sizeof(int) * std::max(ctx->ncells, 1), ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
+    return fail(ctx, FEMMD_TIMEOUT, "a bounded device wait expired (%s)", what);
+}
+
+// Whether runs of the context go to one cooperative launch (k_coop.cu), its
+// buffers allocated on the first of them.
+static bool coop_ready(femmd_ctx *ctx) {
+    if (fast_mode(ctx) || ctx->coopOff || !coop_size_ok((int)ctx->pos.size(), ctx->ncells)) return false;
+    const size_t cells = ctx->ncells;
+    if (ctx->runRec.ensure((3 * 16 + 4 * 4) * (size_t)kCoopMaxBlocks) || ctx->cellFill.ensure(2 * cells) ||
+        ctx->cellIds.ensure(cells * kCellCap) || ctx->cellCand.ensure(cells * kCellCap)) {
+        cudaGetLastError();  // no memory for the cell table: the plain kernels
+        ctx->coopOff = true;
+        return false;
+    }
+    return coop_run_fits(make_sys(ctx));
+}
+
+// A run, or part of one, of a small or medium system in one cooperative
+// launch (k_coop.cu); the parity follows its drifts.
+static femmd_status coop_launch(femmd_ctx *ctx, int begin, int units, int end, float2 *slots) {
+    if (!ctx->runClean) {
+        CK(cudaMemsetAsync(ctx->runRec.p, 0, ctx->runRec.n * sizeof(unsigned long long), ctx->stream));
+        CK(cudaMemsetAsync(ctx->cellFill.p, 0, ctx->cellFill.n * sizeof(int), ctx->stream));
+        CK(cudaMemsetAsync(&ctx->sc.p->runTag, 0, 2 * sizeof(int), ctx->stream));  // runTag, runFill
+        static_assert(offsetof(DevScalars, runFill) == offsetof(DevScalars, runTag) + sizeof(int), "run scalars");
+        ctx->runClean = true;
+    }
+    CoopArgs a = {};
+    a.parity = ctx->cur;
+    a.begin = begin;
+    a.units = units;
+    a.end = end;
+    a.withhold = ctx->testExpire ? 1 : 0;
+    ctx->testExpire = false;
+    a.ckPos = ctx->ckPos.p;
+    a.ckVel = ctx->ckVel.p;
+    a.ckAcc = ctx->ckAcc.p;
+    a.slots = slots;
+    CK(launch_coop_run(ctx->stream, make_sys(ctx), a));
+    ctx->profKernels++;
+    ctx->cur ^= (begin + units) & 1;
+    return FEMMD_OK;
+}
+
+// Whether run(n) is one cooperative launch from its run start to its last
+// step (no trajectory frame inside it, no averaging, no direct launches).
+static bool coop_whole(femmd_ctx *ctx, int n) {
+    return n > 0 && !ctx->profiling && !ctx->propAvg && !(ctx->traj.on && ctx->traj.every > 0) && coop_ready(ctx);
+}
+
 static femmd_status launch_units(femmd_ctx *ctx, int units, bool use_graphs) {
     if (units <= 0) return FEMMD_OK;
     if (use_graphs && !ctx->propAvg) {
         const DevSys s = make_sys(ctx);
         if (small_run_fits(s)) return small_units(ctx, s, units);
+        if (coop_ready(ctx)) return coop_launch(ctx, 0, units, 0, nullptr);
     }
     if (!use_graphs) {
         DevSys s = make_sys(ctx);
@@ -1662,7 +1733,8 @@ static void traj_refresh_meta(femmd_ctx *ctx) {
     frame_meta(ctx, T.meta);
 }
 
-static femmd_status run_once(femmd_ctx *ctx, int n, bool &aborted) {
+static femmd_status run_once(femmd_ctx *ctx, int n, bool whole, bool &aborted) {
+    if (whole) return coop_launch(ctx, 1, n - 1, 1, nullptr);
     DevSys s = make_sys(ctx);
     Launch L;
     L.stream = ctx->stream;
@@ -2283,12 +2355,16 @@ femmd_status femmd_run(femmd_ctx *ctx, int steps) {
     if ((st = ensure_obs(ctx, steps))) return st;
     const int N = (int)ctx->pos.size();
     for (int attempt = 0; attempt < 8; attempt++) {
-        // start checkpoint (positions, velocities, accelerations)
+        // start checkpoint (positions, velocities, accelerations); a run that
+        // is one launch writes its own
         const float2 *pc = ctx->cur ? ctx->dpos1.p : ctx->dpos0.p;
         int cur0 = ctx->cur;
-        CK(cudaMemcpyAsync(ctx->ckPos.p, pc, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
-        CK(cudaMemcpyAsync(ctx->ckVel.p, ctx->dvel.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
-        CK(cudaMemcpyAsync(ctx->ckAcc.p, ctx->dacc.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
+        const bool whole = coop_whole(ctx, steps);
+        if (!whole) {
+            CK(cudaMemcpyAsync(ctx->ckPos.p, pc, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
+            CK(cudaMemcpyAsync(ctx->ckVel.p, ctx->dvel.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
+            CK(cudaMemcpyAsync(ctx->ckAcc.p, ctx->dacc.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
+        }
         if (fast_mode(ctx))
             CK(cudaMemcpyAsync(ctx->ckPerm.p, ctx->perm.p, N * sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
         if (ctx->propAvg)
@@ -2298,14 +2374,12 @@ femmd_status femmd_run(femmd_ctx *ctx, int steps) {
             CK(cudaMemsetAsync(ctx->trace.p, 0, (size_t)ctx->obsCap * kTraceCols * sizeof(unsigned long long),
                                ctx->stream));
         bool aborted = false;
-        if ((st = run_once(ctx, steps, aborted))) return st;
+        if ((st = run_once(ctx, steps, whole, aborted))) return st;
         if ((st = collect_profile(ctx))) return st;
         if ((st = read_scalars(ctx))) return st;
         if (ctx->hsc->overflow & 2) return fail(ctx, FEMMD_CAPACITY_OVERFLOW, "inconsistent cell counts");
         if (ctx->hsc->overflow & 8) {
-            ctx->smallClean = false;
-            return fail(ctx, FEMMD_TIMEOUT,
-                        "a bounded device wait expired (a copy to shared memory or a grid-wide exchange)");
+            return expired(ctx, "a copy to shared memory or a grid-wide exchange");
         }
         if (!ctx->hsc->overflow && !aborted) {
             traj_commit(ctx->traj);
@@ -2336,6 +2410,10 @@ femmd_status femmd_run(femmd_ctx *ctx, int steps) {
         }
         if (ctx->propAvg)
             CK(cudaMemcpyAsync(ctx->props.p, ctx->propsCk.p, sizeof(DevProps), cudaMemcpyDeviceToDevice, ctx->stream));
+        if (ctx->hsc->overflow & 16) {
+            ctx->coopOff = true;  // a crowded cell: the plain kernels
+            if (!(ctx->hsc->overflow & 1)) continue;
+        }
         int need = std::max(ctx->hsc->maxCount, ctx->nbrCap + ctx->nbrCap / 2);
         if ((st = alloc_list(ctx, need + need / 4 + 8))) return st;
     }
@@ -3105,23 +3183,29 @@ static femmd_status adj_recompute(femmd_ctx *ctx, int g, std::vector<int> &rebui
     DevSys s = make_sys(ctx);
     Launch L;
     L.stream = st;
-    CK(cudaMemsetAsync(&ctx->sc.p->overflow, 0, 3 * sizeof(int), st));
-    CK(enqueue_run_start(L, s));
-    CK(enqueue_rebuild(L, s, 0, 1));
-    CK(enqueue_step(L, s, MODE_FIRST, 0, 0, 0));
-    int cur = 1;
-    CK(cudaMemcpyAsync(a.slots.p + N, ctx->dpos1.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, st));
-    for (int u = 1; u < K; u++) {
-        CK(enqueue_step(L, s, MODE_MID, cur, 0, 0));
-        float2 *pout = cur ? ctx->dpos0.p : ctx->dpos1.p;
-        CK(cudaMemcpyAsync(a.slots.p + (size_t)(u + 1) * N, pout, N * sizeof(float2), cudaMemcpyDeviceToDevice, st));
-        // the rebuild kernels only where the forward rebuilt (elsewhere
-        // their check would return at once); a disagreement is caught below
-        if (a.segReb[g][u]) CK(enqueue_rebuild(L, s, 1 - cur, 1));
-        cur ^= 1;
-    }
     femmd_status e;
+    CK(cudaMemsetAsync(&ctx->sc.p->overflow, 0, 3 * sizeof(int), st));
+    if (coop_ready(ctx)) {
+        if ((e = coop_launch(ctx, 1, K - 1, 0, a.slots.p))) return e;
+    } else {
+        CK(enqueue_run_start(L, s));
+        CK(enqueue_rebuild(L, s, 0, 1));
+        CK(enqueue_step(L, s, MODE_FIRST, 0, 0, 0));
+        int cur = 1;
+        CK(cudaMemcpyAsync(a.slots.p + N, ctx->dpos1.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, st));
+        for (int u = 1; u < K; u++) {
+            CK(enqueue_step(L, s, MODE_MID, cur, 0, 0));
+            float2 *pout = cur ? ctx->dpos0.p : ctx->dpos1.p;
+            CK(cudaMemcpyAsync(a.slots.p + (size_t)(u + 1) * N, pout, N * sizeof(float2), cudaMemcpyDeviceToDevice,
+                               st));
+            // the rebuild kernels only where the forward rebuilt (elsewhere
+            // their check would return at once); a disagreement is caught below
+            if (a.segReb[g][u]) CK(enqueue_rebuild(L, s, 1 - cur, 1));
+            cur ^= 1;
+        }
+    }
     if ((e = read_scalars(ctx))) return e;
+    if (ctx->hsc->overflow & 8) return expired(ctx, "a grid-wide exchange");
     if (ctx->hsc->overflow || ctx->hsc->nonfinite)
         return fail(ctx, ctx->hsc->overflow ? FEMMD_CAPACITY_OVERFLOW : FEMMD_NONFINITE,
                     "the recomputed segment differs from the forward pass (overflow or non-finite force)");

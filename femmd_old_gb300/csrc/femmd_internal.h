@@ -35,11 +35,12 @@ constexpr int kTraceCols = 6;      // per-step trace row (ns): tri start/end, st
 // Per type-pair constants, all formed on the host with the reference's float
 // operations (interactionsCuda.cu:43-55, 79-88) so that the kernel's per-pair
 // arithmetic reproduces the reference bit for bit.
-// The four values the pair loop reads first share one aligned 16 bytes.
+// The four values the pair loop reads first share one aligned 16 bytes, the
+// two that it multiplies together (packed) the first 8 of them.
 struct __align__(16) PairEntry {
-    float rcut2;  // (rc*rc)*sigma_ij*sigma_ij      (sigma by type)
     float c;      // 48*eps/(sigma_ij*sigma_ij)     (sigma by type)
     float eps4;   // 4*eps
+    float rcut2;  // (rc*rc)*sigma_ij*sigma_ij      (sigma by type)
     float us;     // uShift
     float sig2;   // sigma_ij*sigma_ij              (sigma by type)
     float rc;     // rc (units of sigma_ij)
@@ -81,7 +82,11 @@ struct DevScalars {
     // the small-system run (k_fsmall): the tag base of its next launch's
     // exchanges, the steps one launch advanced, the steps left and the
     // position parity the next launch starts from (it ends on parity 0)
-    unsigned int gbTag, pad2;
+    unsigned int gbTag;
+    // the whole-run launch (k_coop): the tag base of its next launch's
+    // exchanges, and which of its two cell-count arrays the last rebuild used
+    unsigned int runTag;
+    int runFill, pad2;
     int smallDone, smallLeft, smallPar;
     int testWithhold;  // the next small run's block 0 withholds its first exchange record (a test of the timeout)
 };
@@ -195,6 +200,12 @@ struct DevSys {
     // the small-system run's exchange records: three sets of kSmallMaxTiles
     // records {tag << 32 | max v^2 bits, U, W, K fixed point}
     unsigned long long *smallRec;
+    // the whole-run launch (k_coop): three sets of kCoopMaxBlocks exchange
+    // words and four of energy sums; its cells hold up to kCellCap particles
+    // each (ids, then the candidates in id order; two arrays of counts in turn)
+    unsigned long long *runRec;
+    int *cellFill, *cellIds;
+    float4 *cellCand;
 };
 
 constexpr int kSmallMaxTiles = 128;  // step blocks of the largest system the small-system run takes
@@ -254,6 +265,27 @@ cudaError_t launch_small_run(cudaStream_t st, const DevSys &s);
 cudaError_t enqueue_small_run(Launch &L, const DevSys &s, cudaGraphConditionalHandle hw,
                               cudaGraphConditionalHandle hif);
 cudaError_t enqueue_perm_consts(Launch &L, const DevSys &s);
+
+// A kernel's dynamic shared-memory limit raised to at least 'smem' and its
+// resident blocks on the whole GPU, cached (k_fast.cu).
+cudaError_t kernel_setup(const void *fn, int threads, size_t smem, int *resident);
+
+// ---- whole runs of small and medium systems in one cooperative launch (k_coop.cu)
+constexpr int kCoopMaxBlocks = 256;
+constexpr int kCellCap = 32;  // particles of a cell at most (a fuller one: the plain kernels)
+struct CoopArgs {
+    int parity;   // of the current positions
+    int begin;    // the run start, forced rebuild and first step, and the checkpoint of the start state
+    int units;    // middle steps
+    int end;      // the last step
+    int withhold; // block 0 withholds its first exchange record (a test of the timeout)
+    float2 *ckPos, *ckVel, *ckAcc;
+    float2 *slots;  // positions after drift u also to slots + (u + 1) N, or null
+    int rows, incStaged, triStaged;  // shared memory: list rows, incidences, triangles (the launch sets them)
+};
+bool coop_size_ok(int N, int ncells);
+bool coop_run_fits(const DevSys &s);
+cudaError_t launch_coop_run(cudaStream_t st, const DevSys &s, const CoopArgs &a);
 
 // ---- forces + integration (k_force.cu)
 cudaError_t enqueue_step(Launch &L, const DevSys &s, int mode, int parity, cudaGraphConditionalHandle h, int use_h);

@@ -1,0 +1,76 @@
+// k_coop.cu -- launch of the whole-run kernel (k_coop.cuh), and its variant
+// for one particle type.
+#include <algorithm>
+#include "k_coop.cuh"
+
+namespace femmd {
+
+const void *coop_kernel_one(const DevSys &s) { return coop_image<false, false>(s); }
+
+namespace {
+
+// Particles of the largest system that runs in one launch.  Measured on
+// run(50) against the plain kernels' graph (us): LJ fluid 67,600 particles
+// 1148 / 1539, 160,000 2095 / 1848 (equal near 125,000); disks in solvent
+// 68,288 1512 / 1787, 150,800 2662 / 2111 (96,000); suspension 32,512
+// 650 / 923, 130,048 1336 / 1254 (108,000).
+constexpr int kCoopMaxN = 98304;
+
+const void *coop_kernel(const DevSys &s) {
+    if (!s.sigmaByType) return coop_kernel_sigma(s);
+    return s.numTypes > 1 ? coop_kernel_types(s) : coop_kernel_one(s);
+}
+
+constexpr size_t kCoopSmem = 180 * 1024;  // dynamic shared memory of a block at most
+
+// Blocks of a system (one per tile, at most one per SM) and what their shared
+// memory holds: terms, sums and counts always, then incidences and triangles
+// where they fit, then as many list rows as do.
+// False when the system does not fit.
+bool coop_shape(const DevSys &s, int &grid, size_t &smem, CoopArgs &a) {
+    int sms = 0, dev = 0;
+    if (cudaGetDevice(&dev) || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return false;
+    const int ntiles = (s.N + kStepBlock - 1) / kStepBlock;
+    const int ntt = s.feaForces ? (s.ntri + kTriTile - 1) / kTriTile : 0;
+    grid = std::max(1, std::min(std::min(sms, kCoopMaxBlocks), std::max(ntiles, ntt)));
+    const int per = (ntiles + grid - 1) / grid, tper = (ntt + grid - 1) / grid;
+    if (per > kCoopMaxTiles || tper > kCoopMaxTiles) return false;
+    smem = 4 * (size_t)kTermComp * sizeof(float) + (size_t)per * 4 * kStepBlock * sizeof(int);  // terms, sums, counts
+    const size_t inc = (size_t)per * kIncWords * kStepBlock * sizeof(int), tri = (size_t)tper * kTriTile * sizeof(int4);
+    const size_t row = 4 * (size_t)per * kListRow * sizeof(int);  // four list rows
+    a.incStaged = s.nBonded > 0 && smem + inc + row <= kCoopSmem;
+    if (a.incStaged) smem += inc;
+    a.triStaged = ntt > 0 && smem + tri + row <= kCoopSmem;
+    if (a.triStaged) smem += tri;
+    a.rows = 4 * (int)std::min<size_t>(s.nbrCap / 4, (kCoopSmem - smem) / row);
+    smem += a.rows / 4 * row;
+    return a.rows > 0 || s.nbrCap == 0;
+}
+
+}  // namespace
+
+bool coop_run_fits(const DevSys &s) {
+    if (s.fast || s.areaUnits > 0 || s.trace || !s.cellCand || s.N <= 0) return false;
+    int grid, resident = 0;
+    size_t smem;
+    CoopArgs a = {};
+    if (!coop_shape(s, grid, smem, a)) return false;
+    if (kernel_setup(coop_kernel(s), kCoopThreads, smem, &resident)) return false;
+    return resident >= grid;
+}
+
+// The sizes a whole-run launch is made for: its cell table has kCellCap slots
+// per cell, so that a nearly empty box is left to the plain kernels.
+bool coop_size_ok(int N, int ncells) { return N > 0 && N <= kCoopMaxN && ncells <= 4 * N + 4096; }
+
+cudaError_t launch_coop_run(cudaStream_t st, const DevSys &s, const CoopArgs &a) {
+    int grid;
+    size_t smem;
+    DevSys sa = s;
+    CoopArgs aa = a;
+    if (!coop_shape(s, grid, smem, aa)) return cudaErrorInvalidConfiguration;
+    void *args[] = {&sa, &aa};
+    return cudaLaunchCooperativeKernel(coop_kernel(s), dim3(grid), dim3(kCoopThreads), args, smem, st);
+}
+
+}  // namespace femmd

@@ -1,0 +1,899 @@
+// k_coop.cuh -- a whole run of a small or medium system in one cooperative
+// launch (reference-exact force mode).
+//
+// One graph unit of the plain path (step kernel, conditional rebuild) costs
+// 15-25 us whatever the system's size: launches, the IF node, and the drain
+// of each kernel.  Up to a few hundred thousand particles the arithmetic of a
+// step takes less than that, so k_coop advances the run inside one launch:
+// every block owns fixed tiles of particles and triangles, a step is the
+// triangle pass, a grid-wide exchange, the particle pass and a second
+// exchange (the first one only with triangles), and every block takes the
+// rebuild decision of NeighborList::update (femmd2D/src/nn.cpp:114-134) from
+// the same exchanged maximum.  A system of one tile runs in one block,
+// where an exchange is a block barrier.
+//
+// At these sizes a step is bound by latency: dependent L2 accesses (about
+// 0.4 us each: an exchange invalidates L1) and, with a warp or two per
+// scheduler, dependent instructions (7 cycles each: a thread that works its 20
+// pairs one after another takes 12,000 cycles).  So a particle is worked by
+// four lanes: each gathers and works every fourth list entry and puts the
+// pair's four terms (force x, y, energy, virial) into shared memory, and then
+// each adds up one of the four sums over the entries in list order; lanes 0
+// and 1 integrate one axis each.  The lists, the bond and triangle
+// incidences and the triangles' vertices stay in shared memory for the whole
+// launch, loads that do not depend on each other are issued together, and the
+// energy sums are reduced while the exchange is waited for.
+//
+// Measured against the plain kernels in CUDA graphs (a whole set_state, run,
+// get_state; us): LJ fluid 400 particles run(20) 659 -> 244, 10,201 run(50)
+// 1379 -> 525; 256-disk suspension (32,512) run(100) 1825 -> 1260; adjoint of 64
+// disks over 200 steps 14,315 -> 8390.  A step of the 10,201 particles: 4.1 us in
+// the particle pass, 2.7 us in the exchange; a thread per particle instead of
+// a quad took 7.7 us there.  Exchange words side by side in one line instead
+// of a line each: 3.6 us with 80 blocks, 6 with 152 (against 2.7 and 3.3).
+//
+// The per-particle and per-triangle arithmetic and the list order are those
+// of the plain kernels (step_body.cuh, nn_body.cuh), and so is the grouping
+// of the energy sums: FP32 over the 32 lanes and the 4 (8) warps of a tile of
+// 128 particles (256 triangles), then 64-bit fixed point, which is exact in
+// any order.  Positions, velocities, forces, energies and rebuild steps are
+// therefore the plain path's bit for bit.
+//
+// Exchanges: each block writes a word {tag << 32 | value} into one of three
+// rotating sets with release semantics; warp 0 of every block polls all words
+// (relaxed loads, all of a lane's in flight together, then an acquire fence;
+// bounded: a wait that gives up sets the timeout flag, and the block leaves
+// the kernel).  Tags grow by one per exchange over the life of the context
+// (DevScalars::runTag), so a stale word never matches.  A set is written
+// again three exchanges later, which no block reaches before every block has
+// published two exchanges later.  A step's energy sums go to one of four
+// rotating sets after its exchange is published and are therefore visible to
+// a block that has completed the following one; block 0 adds them up during
+// the exchange after that.
+#pragma once
+#include <cuda_runtime.h>
+#include "femmd_internal.h"
+#include "launch.h"
+#include "device_common.cuh"
+#include "nn_body.cuh"
+#include "step_body.cuh"
+
+namespace femmd {
+
+namespace {
+
+constexpr int kCoopThreads = 512;
+constexpr int kCoopSpin = 1 << 20;  // polls (about 0.5 us each) before an exchange gives up
+constexpr int kCoopTimeout = 8;     // DevScalars::overflow bit: a bounded wait expired
+constexpr int kCoopCrowded = 16;    // DevScalars::overflow bit: a cell holds more than kCellCap particles
+constexpr int kCoopMaxTiles = 32;   // tiles of one block (one lane of a warp sums each)
+constexpr int kTriTile = 256;       // triangles per energy group (k_tri_forces' block)
+constexpr int kListLanes = 8;       // lanes that build one particle's list
+constexpr int kWordQ = kCoopMaxBlocks / 32;  // words per lane of the polling warp
+// Incidences of one bonded particle kept in shared memory: a count word, up
+// to kIncTri triangle entries and kIncBond bond entries of two words.
+constexpr int kIncTri = 8, kIncBond = 6, kIncWords = 1 + kIncTri + 2 * kIncBond;
+constexpr int kQuadPairs = 6;                // list entries per lane and round
+constexpr int kQuadRows = 4 * kQuadPairs;    // entries per particle and round
+// One round's terms in shared memory: component c of entry k of the tile's
+// particle p at c kTermComp + k kTermRow + p.  The pads put the four entries
+// a quad writes together, and the four components it reads together, into
+// different banks.
+constexpr int kTermRow = kStepBlock + 8, kTermComp = kQuadRows * kTermRow + 8;
+constexpr int kListRow = kStepBlock + 8;     // a list row in shared memory (padded as kTermRow)
+constexpr int kWordStride = 16;              // exchange words 128 bytes apart: one L2 line each
+
+__device__ __forceinline__ void st_release(unsigned long long *p, unsigned long long v) {
+    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+// Loads that stay where they are written, ahead of what uses them (a plain
+// load is moved down to its use when registers are short).
+__device__ __forceinline__ float2 ld_early(const float2 *p) {
+    float2 v;
+    asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ float4 ld_early(const float4 *p) {
+    float4 v;
+    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ int ld_early(const int *p) {
+    int v;
+    asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
+
+struct CoopDue {
+    unsigned x;  // the exchange that published the step
+    int mode, row, reb;
+    float vm, d;
+};
+
+struct CoopShared {
+    PairEntry tab[kMaxTypes * kMaxTypes];
+    float vmax[kCoopThreads / 32];    // per warp: its particles' largest v^2
+    float tred[kCoopMaxTiles][8];     // per triangle tile and warp: energy
+    unsigned long long acc[3];        // the step's energy sums of this block (U, W, K)
+    CoopDue due[4];                   // block 0: steps whose totals have still to be added up
+    int wsum[kCoopThreads / 32];
+    unsigned ok, maxBits, before;     // of the last exchange; before: the sum of the earlier blocks' values
+};
+
+// What every block carries through the launch (the same on each).
+struct CoopRun {
+    unsigned base, xi;       // tag base, exchanges so far
+    unsigned dueIn, dueOut;  // entries pushed to and taken from CoopShared::due
+    float dispHi;
+    int row, stepNow, updates;
+    int cnt;  // which of the two cell-count arrays the last rebuild filled
+};
+
+__device__ __forceinline__ unsigned long long *coop_words(const DevSys &s, unsigned x) {
+    return s.runRec + (size_t)(x % 3u) * kCoopMaxBlocks * kWordStride;
+}
+__device__ __forceinline__ unsigned long long *coop_sums(const DevSys &s, unsigned x) {
+    return s.runRec + 3 * kCoopMaxBlocks * kWordStride + (size_t)(x % 4u) * kCoopMaxBlocks * 4;
+}
+
+// One warp: the totals of a step's sums into the scalars and, for the modes
+// that complete a step, its observable row.
+__device__ __noinline__ void coop_totals(const DevSys &s, const CoopDue &d) {
+    const unsigned long long *set = coop_sums(s, d.x);
+    const int lane = threadIdx.x & 31;
+    unsigned long long u = 0ull, w = 0ull, k = 0ull;
+    for (int b = lane; b < (int)gridDim.x; b += 32) {
+        u += __ldcg(set + 4 * (size_t)b);
+        w += __ldcg(set + 4 * (size_t)b + 1);
+        k += __ldcg(set + 4 * (size_t)b + 2);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        u += __shfl_down_sync(0xffffffffu, u, o);
+        w += __shfl_down_sync(0xffffffffu, w, o);
+        k += __shfl_down_sync(0xffffffffu, k, o);
+    }
+    if (lane == 0) {
+        DevScalars *sc = s.sc;
+        const double U = from_fixed(u), W = from_fixed(w), KE = from_fixed(k);
+        sc->U = U;
+        sc->W = W;
+        if (d.mode == MODE_MID || d.mode == MODE_LAST) {
+            sc->KE = KE;
+            sc->vvMax = d.vm;
+            if (s.obs && d.row < s.obsCap) {
+                double *o = s.obs + (size_t)d.row * kObsCols;
+                o[0] = U;
+                o[1] = W;
+                o[2] = KE;
+                o[3] = (double)d.vm;
+                o[4] = (double)d.d;
+                o[5] = (double)d.reb;
+            }
+        }
+    }
+    __syncwarp();
+}
+
+// This block's word, then the wait for every block's: maxBits = the largest
+// value as a float; SUM: before = the sum of the earlier blocks' values.
+// Block 0's warp 2 meanwhile adds up the totals that are due (all: every one
+// left), and 'meanwhile' runs on the warps from 3 on.  withhold: the word is
+// not written (femmd_test_expire_next_exchange).  False when a wait gave up.
+// Call it after a block barrier that follows the block's stores; it ends with
+// one.
+struct Nothing {
+    __device__ void operator()() const {}
+};
+template <bool SUM = false, class Work = Nothing>
+__device__ __forceinline__ bool coop_exchange(const DevSys &s, CoopShared &sh, CoopRun &r, unsigned value,
+                                              bool withhold = false, bool all = false, Work meanwhile = {}) {
+    const unsigned tag = r.base + r.xi + 1u;
+    unsigned long long *set = coop_words(s, r.xi);
+    const bool grid = gridDim.x > 1 || withhold;
+    if (threadIdx.x == 0 && grid && !withhold) st_release(set + blockIdx.x * kWordStride, ((unsigned long long)tag << 32) | value);
+    if (threadIdx.x < 32) {
+        const int lane = threadIdx.x;
+        float m = lane == 0 ? __uint_as_float(value) : 0.0f;
+        unsigned before = 0;
+        int ok = 1;
+        if (grid) {
+            unsigned long long w[kWordQ];
+            bool more = true;
+            for (int it = 0; more && it < kCoopSpin; it++) {
+                if (it > 0) __nanosleep(20);
+                more = false;
+#pragma unroll
+                for (int q = 0; q < kWordQ; q++)
+                    if (q * 32 + lane < (int)gridDim.x) w[q] = ld_relaxed(set + (q * 32 + lane) * kWordStride);
+#pragma unroll
+                for (int q = 0; q < kWordQ; q++)
+                    if (q * 32 + lane < (int)gridDim.x) more = more || (unsigned)(w[q] >> 32) != tag;
+            }
+            ok = __all_sync(0xffffffffu, !more);
+            fence_gpu();
+#pragma unroll
+            for (int q = 0; q < kWordQ; q++)
+                if (q * 32 + lane < (int)gridDim.x) {
+                    m = fmaxf(m, __uint_as_float((unsigned)w[q]));
+                    if (SUM && q * 32 + lane < (int)blockIdx.x) before += (unsigned)w[q];
+                }
+        }
+        m = warp_max(m);
+        if (SUM) before = __reduce_add_sync(0xffffffffu, before);
+        if (lane == 0) {
+            sh.ok = (unsigned)ok;
+            sh.maxBits = __float_as_uint(m);
+            if (SUM) sh.before = before;
+        }
+    }
+    // a step's sums are visible once the exchange after its own is complete
+    while (r.dueOut != r.dueIn && !all) {
+        const CoopDue &d = sh.due[r.dueOut & 3u];
+        if ((int)(r.xi - d.x) < 2) break;
+        if (blockIdx.x == 0 && threadIdx.x >> 5 == 2) coop_totals(s, d);
+        r.dueOut++;
+    }
+    r.xi++;
+    if (threadIdx.x >> 5 >= 3) meanwhile();
+    __syncthreads();
+    if (sh.ok) return true;
+    if (threadIdx.x == 0) atomicOr(&s.sc->overflow, kCoopTimeout);
+    return false;
+}
+
+// Exclusive scan of v over the block (every thread calls it); 'total' is the
+// block's sum.
+__device__ __forceinline__ int block_scan(CoopShared &sh, int v, int &total) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+    int x = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    __syncthreads();  // wsum may still be read
+    if (lane == 31) sh.wsum[warp] = x;
+    __syncthreads();
+    const int w = lane < nw ? sh.wsum[lane] : 0;
+    int z = w;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, z, o);
+        if (lane >= o) z += y;
+    }
+    total = __shfl_sync(0xffffffffu, z, 31);
+    return __shfl_sync(0xffffffffu, z - w, warp) + x - v;
+}
+
+// The launch's shared-memory arrays beside CoopShared.
+struct CoopMem {
+    float *term;  // a round's terms (kTermComp)
+    float *part;  // [tile of the block][3][kStepBlock]: the particles' U, W, m v^2 of the step
+    int *list;    // [tile][rows][kListRow]: the first 'rows' list entries of every particle
+    int rows;     // (a multiple of 4)
+    int *count;  // [tile][kStepBlock]: list lengths
+    int *inc;    // [tile][kIncWords][kStepBlock], or null
+    int4 *tri;   // [triangle tile][kTriTile]: vertices, or null
+};
+
+// The list of particle i (slot 'col' of the block's tile j) by kListLanes
+// lanes: the 3 x 3 cells in the reference's order (dx outer, dy inner, each
+// cell's particles by ascending id, cell indices wrapped as applyCellBC,
+// nnCuda.cu:26-36), kListLanes candidates of a cell at a time, a ballot
+// placing the hits.  FAST: fast_walk_ok, the image shift is the cell's; else
+// the minimum image per pair.  The first candidates of all nine cells are in
+// flight together.  Entries go to shared memory (from entry mem.rows on, to
+// the list itself).  All lanes of the warp call it; returns the list length.
+template <bool FAST>
+__device__ __forceinline__ int coop_list(const DevSys &s, const CoopMem &mem, const int *cnt, const float2 *pos, int i,
+                                         int j, int col, bool valid) {
+    const int lane = threadIdx.x & 31, sub = lane & (kListLanes - 1), shift = lane & ~(kListLanes - 1);
+    const int ncx = s.ncx, ncy = s.ncy, cap = s.nbrCap;
+    const float R2 = s.nnRadiusSq;
+    const float Lx = s.wrapx ? s.Lx : 0.0f, Ly = s.wrapy ? s.Ly : 0.0f;
+    const float2 p = valid ? pos[i] : make_float2(0.0f, 0.0f);
+    const int gi = valid ? s.excl[i] : -1;
+    int ix, iy;
+    cell_xy(p.x, p.y, ncx, ncy, s.Lx, s.Ly, ix, iy);
+    const int cx[3] = {(ix == 0 ? ncx : ix) - 1, ix, ix == ncx - 1 ? 0 : ix + 1};
+    const int cy[3] = {(iy == 0 ? ncy : iy) - 1, iy, iy == ncy - 1 ? 0 : iy + 1};
+    const float sx[3] = {ix == 0 ? -Lx : 0.0f, 0.0f, ix == ncx - 1 ? Lx : 0.0f};
+    const float sy[3] = {iy == 0 ? -Ly : 0.0f, 0.0f, iy == ncy - 1 ? Ly : 0.0f};
+    int n[9];
+    float4 c0[9];
+#pragma unroll
+    for (int q = 0; q < 9; q++) {
+        const int cell = cx[q / 3] * ncy + cy[q % 3];
+        n[q] = ld_early(cnt + cell);
+        c0[q] = ld_early(s.cellCand + (size_t)cell * kCellCap + sub);
+    }
+    int *lst = mem.list + (size_t)j * mem.rows * kListRow + col;
+    int k = 0;
+    auto test = [&](float4 c, bool on, int q) {
+        float dr2;
+        if (FAST) {
+            const float dx = (p.x - c.x) - sx[q / 3], dy = (p.y - c.y) - sy[q % 3];
+            dr2 = dx * dx + dy * dy;
+        } else {
+            float dxr, dxo, dyr, dyo;
+            image_axis(p.x, c.x, s.Lx, s.wrapx, false, dxr, dxo);
+            image_axis(p.y, c.y, s.Ly, s.wrapy, false, dyr, dyo);
+            dr2 = dxr * dxr + dyr * dyr;
+        }
+        const int tag = __float_as_int(c.z);
+        const bool hit = on && dr2 <= R2 && (tag & kIdMask) != i && (gi == -1 || gi != __float_as_int(c.w));
+        const unsigned hits = (__ballot_sync(0xffffffffu, hit) >> shift) & ((1u << kListLanes) - 1u);
+        if (hit) {
+            const int at = k + __popc(hits & ((1u << sub) - 1u));
+            if (at < mem.rows) lst[at * kListRow] = tag;
+            else if (at < cap) s.nbr[nbr_at(at, i, s.Ncap)] = tag;
+        }
+        k += __popc(hits);
+    };
+    bool more = false;
+#pragma unroll
+    for (int q = 0; q < 9; q++) {
+        n[q] = valid ? min(n[q], kCellCap) : 0;
+        more = more || n[q] > kListLanes;
+    }
+    if (!__any_sync(0xffffffffu, more)) {
+#pragma unroll
+        for (int q = 0; q < 9; q++) test(c0[q], sub < n[q], q);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 9; q++) {
+            test(c0[q], sub < n[q], q);
+            const int most = __reduce_max_sync(0xffffffffu, n[q]);
+            const int cell = cx[q / 3] * ncy + cy[q % 3];
+            for (int o = kListLanes; o < most; o += kListLanes) {
+                const bool on = o + sub < n[q];
+                test(s.cellCand[(size_t)cell * kCellCap + (on ? o + sub : 0)], on, q);
+            }
+        }
+    }
+    if (valid && sub == 0) {
+        s.nbrCount[i] = k;
+        mem.count[j * kStepBlock + col] = min(k, cap);
+    }
+    return k;
+}
+
+// NeighborList::update's taken branch for the positions of buffer p: cells of
+// at most kCellCap particles by counting atomics, the in-cell order by id,
+// and the lists of the block's own particles.  Two exchanges.  False when one
+// gave up.
+__device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, const CoopMem &mem, CoopRun &r, int p,
+                                          bool withhold) {
+    const float2 *pos = p ? s.pos1 : s.pos0;
+    DevScalars *sc = s.sc;
+    const int ntiles = (s.N + kStepBlock - 1) / kStepBlock, groups = blockDim.x / kStepBlock;
+    const int grp = threadIdx.x / kStepBlock, gt = threadIdx.x % kStepBlock, lane = threadIdx.x & 31;
+    r.updates += 1;
+    r.dispHi = 0.0f;
+    r.cnt ^= 1;
+    int *cnt = s.cellFill + (size_t)r.cnt * s.ncells, *other = s.cellFill + (size_t)(r.cnt ^ 1) * s.ncells;
+    // 1: cells, and the ids into them in any order
+    for (int j = grp; blockIdx.x + j * gridDim.x < ntiles; j += groups) {
+        const int i = (blockIdx.x + j * gridDim.x) * kStepBlock + gt;
+        if (i >= s.N) continue;
+        const float2 x = pos[i];
+        if (!(isfinite(x.x) && isfinite(x.y))) atomicOr(&sc->nonfinite, 1);
+        if (outside_box(s, x)) atomicOr(&sc->outside, 1);
+        const int c = cell_col(x.x, x.y, s.ncx, s.ncy, s.Lx, s.Ly);
+        s.cellOf[i] = c;
+        const int k = atomicAdd(cnt + c, 1);
+        if (k < kCellCap) s.cellIds[(size_t)c * kCellCap + k] = i;
+        else atomicOr(&sc->overflow, kCoopCrowded);  // the run is repeated by the plain kernels
+    }
+    __syncthreads();
+    if (!coop_exchange(s, sh, r, 0u, withhold)) return false;
+    // a non-finite position or a crowded cell: the rest is skipped (the run
+    // fails or is repeated), the exchange is not
+    const bool skip = __ldcg(&sc->nonfinite) != 0 || (__ldcg(&sc->overflow) & kCoopCrowded);
+    // 2: ascending id inside each cell; the other counts cleared for the next
+    // rebuild (their last readers were the lists before this rebuild)
+    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < s.ncells; c += gridDim.x * blockDim.x) other[c] = 0;
+    if (!skip)
+        for (int j = grp; blockIdx.x + j * gridDim.x < ntiles; j += groups) {
+            const int i = (blockIdx.x + j * gridDim.x) * kStepBlock + gt;
+            if (i >= s.N) continue;
+            const int c = s.cellOf[i], n = min(__ldcg(cnt + c), kCellCap);
+            const int4 *ids = reinterpret_cast<const int4 *>(s.cellIds + (size_t)c * kCellCap);
+            const float2 x = pos[i];
+            const int tag = own_tag(s, i), gi = s.excl[i];
+            int k = 0;
+            for (int q = 0; q < n; q += 8) {
+                const int4 a = __ldcg(ids + q / 4), b = __ldcg(ids + q / 4 + 1);
+                const int id[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+#pragma unroll
+                for (int u = 0; u < 8; u++) k += q + u < n && id[u] < i;
+            }
+            s.cellCand[(size_t)c * kCellCap + k] = make_float4(x.x, x.y, __int_as_float(tag), __int_as_float(gi));
+        }
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        sc->nbrSum = 0ull;
+        sc->maxCount = 0;
+        sc->builds += 1ull;
+    }
+    __syncthreads();
+    if (!coop_exchange(s, sh, r, 0u)) return false;
+    // 3: the lists of the block's own particles
+    if (!skip) {
+        const bool fast = (s.wrapx ? s.ncx >= 5 : s.ncx >= 3) && (s.wrapy ? s.ncy >= 5 : s.ncy >= 3) &&
+                          !__ldcg(&sc->outside);  // fast_walk_ok
+        constexpr int per = 32 / kListLanes;      // particles per warp
+        const int mine = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;  // tiles
+        int kmax = 0, ksum = 0;
+        for (int b = (threadIdx.x >> 5) * per; b < mine * kStepBlock; b += (blockDim.x >> 5) * per) {
+            const int q = b + lane / kListLanes, j = q / kStepBlock, col = q % kStepBlock;
+            const int i = (blockIdx.x + j * gridDim.x) * kStepBlock + col;
+            const int k = fast ? coop_list<true>(s, mem, cnt, pos, i, j, col, i < s.N)
+                               : coop_list<false>(s, mem, cnt, pos, i, j, col, i < s.N);
+            if (i < s.N && (lane & (kListLanes - 1)) == 0) {
+                kmax = max(kmax, k);
+                ksum += k;
+            }
+        }
+        __syncwarp();
+        kmax = __reduce_max_sync(0xffffffffu, kmax);
+        ksum = __reduce_add_sync(0xffffffffu, ksum);
+        if (lane == 0) {
+            if (ksum) atomicAdd(&sc->nbrSum, (unsigned long long)ksum);
+            if (kmax > 0) atomicMax(&sc->maxCount, kmax);
+            if (kmax > s.nbrCap) atomicOr(&sc->overflow, 1);
+        }
+        __syncthreads();
+        // the lists' own copy (getters, the kernels that follow), a 16-byte
+        // group per store; unused words of a particle's last group are zero
+        for (int q = threadIdx.x; q < mine * kStepBlock; q += blockDim.x) {
+            const int j2 = q / kStepBlock, col = q % kStepBlock, i = (blockIdx.x + j2 * gridDim.x) * kStepBlock + col;
+            if (i >= s.N) continue;
+            const int k = min(mem.count[q], mem.rows);
+            const int *lst = mem.list + (size_t)j2 * mem.rows * kListRow + col;
+            for (int g = 0; 4 * g < k; g++) {
+                int v[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) v[u] = 4 * g + u < k ? lst[(4 * g + u) * kListRow] : 0;
+                reinterpret_cast<int4 *>(s.nbr)[(size_t)g * s.Ncap + i] = make_int4(v[0], v[1], v[2], v[3]);
+            }
+        }
+    }
+    __syncthreads();
+    return true;
+}
+
+// The cell arrays of the last rebuild as the plain kernels leave them:
+// cellStart (the exclusive scan of the counts, a contiguous chunk of cells per
+// block), sortedIds and cellSorted.
+__device__ __forceinline__ bool coop_cells(const DevSys &s, CoopShared &sh, CoopRun &r) {
+    const int *cnt = s.cellFill + (size_t)r.cnt * s.ncells;
+    const int chunk = (s.ncells + gridDim.x - 1) / gridDim.x;
+    const int c0 = min((int)blockIdx.x * chunk, s.ncells), c1 = min(c0 + chunk, s.ncells);
+    int sum = 0, tot = 0;
+    for (int cb = c0; cb < c1; cb += blockDim.x) {
+        const int c = cb + threadIdx.x;
+        block_scan(sh, c < c1 ? min(__ldcg(cnt + c), kCellCap) : 0, tot);
+        sum += tot;
+    }
+    __syncthreads();
+    if (!coop_exchange<true>(s, sh, r, (unsigned)sum)) return false;
+    int carry = gridDim.x > 1 ? (int)sh.before : 0;
+    for (int cb = c0; cb < c1; cb += blockDim.x) {
+        const int c = cb + threadIdx.x;
+        const int n = c < c1 ? min(__ldcg(cnt + c), kCellCap) : 0;
+        const int at = carry + block_scan(sh, n, tot);
+        carry += tot;
+        if (c < c1) s.cellStart[c] = at;
+        for (int q = 0; q < n && at + q < s.N; q++) {
+            const float4 e = __ldcg(s.cellCand + (size_t)c * kCellCap + q);
+            s.cellSorted[at + q] = e;
+            s.sortedIds[at + q] = __float_as_int(e.z) & kIdMask;
+        }
+    }
+    if (blockIdx.x == 0 && threadIdx.x == 0) s.cellStart[s.ncells] = s.N;
+    return true;
+}
+
+// The four terms of one pair as lj_pair (step_body.cuh) adds them: force x and
+// y, doubled energy and virial, or zeros outside the cutoff.
+template <bool MT, bool SG, bool WX, bool WY, bool SIG1>
+__device__ __forceinline__ float4 coop_pair(const DevSys &s, const PairEntry *tab, int ti, float si, float sj,
+                                            float2 pi, int tag, float2 pj) {
+    float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    const PairEntry pe0 = tab[0];
+    lj_pair_sig<MT, SG, WX, WY, SIG1>(s, tab, pe0, ti, si, sj, pi, tag, pj, o.x, o.y, o.z, o.w);
+    return o;
+}
+
+// particle_step for one particle by the four lanes of a quad (lane 'q' of 0 ..
+// 3; particle i, slot 'col' of the block's tile j; on: i < N).  All lanes of
+// the warp call it.
+template <bool MT, bool SG, bool WX, bool WY, bool SIG1>
+__device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &mem, const PairEntry *tab, int i, bool on,
+                                              int j, int col, int q, int mode, int stepNow, const float2 *pin,
+                                              float2 *pout, float2 *slot, float &vvm, bool &bad) {
+    const int ic = on ? i : 0;
+    const int cnt = on ? mem.count[j * kStepBlock + col] : 0;
+    const int *lst = mem.list + (size_t)j * mem.rows * kListRow + col;
+    const int most = __reduce_max_sync(0xffffffffu, cnt);
+    // the lane's entries base + q, base + q + 4, ... and their positions
+    int tag[kQuadPairs];
+    float2 pj[kQuadPairs];
+    auto gather = [&](int base) {
+#pragma unroll
+        for (int u = 0; u < kQuadPairs; u++) {
+            const int k = base + 4 * u + q;
+            tag[u] = ic;  // an unused place: the particle itself, no term is taken from it
+            if (k < cnt) tag[u] = k < mem.rows ? lst[k * kListRow] : s.nbr[nbr_at(k, i, s.Ncap)];
+        }
+#pragma unroll
+        for (int u = 0; u < kQuadPairs; u++) pj[u] = ld_early(pin + (tag[u] & kIdMask));
+    };
+    const float2 pi = ld_early(pin + ic);
+    gather(0);
+    const float m = s.mass[ic];
+    const float2 v2 = ld_early(s.vel + ic);
+    const int ti = MT ? s.typeId[ic] : 0;
+    const float si = SG ? s.sigma[ic] : 0.0f;
+    // what comes before the pair forces (bonded_forces), on every lane
+    float ue = 0.0f, utri = 0.0f, uwall = 0.0f, fx = 0.0f, fy = 0.0f;
+    const int *inc = mem.inc ? mem.inc + (size_t)j * kIncWords * kStepBlock + col : nullptr;
+    const int head = (inc && on && i < s.nBonded) ? inc[0] : -1;
+    if (head >= 0) {
+        // with the incidences at hand: the triangles' forces and the first
+        // two partners in flight, then the terms in order
+        const int nT = head & 0xff, nB = head >> 8;
+        auto bond = [&](int k) {
+            return make_int2(inc[(1 + kIncTri + 2 * k) * kStepBlock], inc[(2 + kIncTri + 2 * k) * kStepBlock]);
+        };
+        float2 tf[kIncTri], pb[2];
+#pragma unroll
+        for (int k = 0; k < kIncTri; k++)
+            if (k < nT) tf[k] = ld_early(s.triF + inc[(1 + k) * kStepBlock]);
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+            if (k < nB) pb[k] = ld_early(pin + (bond(k).x & 0x7fffffff));
+        if (s.refWalls) ref_walls(s, i, pi, fx, fy, uwall);
+        if (s.gravity > 0.0f) fy -= m * s.gravity;
+#pragma unroll
+        for (int k = 0; k < 2; k++)
+            if (k < nB) bond_term<WX, WY>(s, bond(k), pi, pb[k], fx, fy, ue);
+        for (int k = 2; k < nB; k++) {
+            const int2 en = bond(k);
+            bond_term<WX, WY>(s, en, pi, pin[en.x & 0x7fffffff], fx, fy, ue);
+        }
+#pragma unroll
+        for (int k = 0; k < kIncTri; k++)
+            if (k < nT) {
+                fx += tf[k].x;
+                fy += tf[k].y;
+            }
+    } else if (on) {
+        bonded_forces<WX, WY, false>(s, i, mode, pin, pi, fx, fy, ue, utri, uwall);
+    }
+    // the pairs: the lane's sum is force x, force y, energy or virial
+    float sum = q == 0 ? fx : (q == 1 ? fy : (q == 2 ? ue : 0.0f));
+    const float *mine = mem.term + q * kTermComp + col;
+    const bool near = __any_sync(0xffffffffu, on && near_edge<WX, WY>(s, pi));
+    for (int base = 0; base < most; base += kQuadRows) {
+        if (base > 0) gather(base);
+        float4 o[kQuadPairs];
+        bool done = false;
+        if (SIG1 && !SG && !near) {
+            float far = 0.0f, close = 1.0f;
+#pragma unroll
+            for (int u = 0; u < kQuadPairs; u++) {
+                const bool in = base + 4 * u + q < cnt;
+                const float4 e = *reinterpret_cast<const float4 *>(
+                    tab + (MT ? ti * s.numTypes + ((unsigned)tag[u] >> kIdBits) : 0));
+                o[u] = lj_terms_x2(pi, pj[u], make_float2(e.x, e.y), e.z, e.w, in, far, close);
+            }
+            done = !__any_sync(0xffffffffu, !lj_sums_ok<WX, WY>(s, far, close));
+        }
+        if (!done) {
+#pragma unroll
+            for (int u = 0; u < kQuadPairs; u++) {
+                o[u] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (base + 4 * u + q < cnt)
+                    o[u] = coop_pair<MT, SG, WX, WY, SIG1>(s, tab, ti, si, SG ? s.sigma[tag[u] & kIdMask] : 0.0f, pi,
+                                                           tag[u], pj[u]);
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < kQuadPairs; u++) {
+            float *w = mem.term + (4 * u + q) * kTermRow + col;
+            w[0] = o[u].x;
+            w[kTermComp] = o[u].y;
+            w[2 * kTermComp] = o[u].z;
+            w[3 * kTermComp] = o[u].w;
+        }
+        __syncwarp();
+        const int rows = min(most - base, kQuadRows);
+#pragma unroll 8
+        for (int k = 0; k < rows; k++) sum += mine[k * kTermRow];
+        __syncwarp();
+    }
+    // finish_particle, an axis per lane (lanes 2 and 3 along with 0 and 1)
+    const bool y = q & 1;
+    float f = sum, e = sum * 0.5f;
+    if (q >= 2) f = 0.0f;
+    if (q == 2) e += uwall;
+    if (s.wallOn && on) {
+        const float yw = wall_y(s, stepNow);
+        const float dl = s.wallDelta[i];
+        const float ht = (pi.y + dl) - yw;
+        if (ht > 0.0f) {
+            if (q == 1) f -= s.wallK * ht;
+            if (q == 2) e += 0.5f * s.wallK * ht * ht;
+        }
+        const float hb = dl - pi.y;
+        if (hb > 0.0f) {
+            if (q == 1) f += s.wallK * hb;
+            if (q == 2) e += 0.5f * s.wallK * hb * hb;
+        }
+    }
+    bad = bad || (on && !isfinite(f));
+    const float a = f / m;
+    float v = y ? v2.y : v2.x, vv = 0.0f;
+    if (mode != MODE_FIRST) {
+        v += s.hdt * a;
+        const float sq = v * v;
+        vv = sq + __shfl_xor_sync(0xffffffffu, sq, 1);
+    }
+    float *part = mem.part + (size_t)j * 3 * kStepBlock + col;
+    if (q == 2) part[0] = on ? e : 0.0f;
+    if (q == 3) part[kStepBlock] = on ? e : 0.0f;
+    if (q == 0) part[2 * kStepBlock] = on ? m * vv : 0.0f;
+    if (on && q < 2) {
+        vvm = fmaxf(vvm, vv);
+        float *vel = reinterpret_cast<float *>(s.vel + i) + q;
+        if (mode == MODE_LAST) {
+            *vel = v;
+            reinterpret_cast<float *>(s.acc + i)[q] = a;
+            reinterpret_cast<float *>(s.forceOut + i)[q] = f;
+        } else {
+            v += s.hdt * a;
+            float x = (y ? pi.y : pi.x) + s.dt * v;
+            if (y ? WY : WX) x = wrap_near(x, y ? s.Ly : s.Lx);
+            reinterpret_cast<float *>(pout + i)[q] = x;
+            *vel = v;
+            if (slot) reinterpret_cast<float *>(slot + i)[q] = x;
+        }
+    }
+}
+
+// One warp: the block's energy sums of a step.  A tile's 128 particles in the
+// plain kernels' grouping: FP32 over 32 lanes (warp_sum_f), over the four
+// warps in order, then fixed point; a triangle tile's eight warp sums alike.
+// Warps 'w0', w0 + 1, ... of the block share the tiles.
+__device__ __forceinline__ void coop_block_sums(const DevSys &s, CoopShared &sh, const CoopMem &mem, int tiles,
+                                                int ttiles, int w0) {
+    const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - w0, nw = (blockDim.x >> 5) - w0;
+    bool ob = false;
+    for (int j = w; j < tiles; j += nw) {
+        const float *part = mem.part + (size_t)j * 3 * kStepBlock + lane;
+        float t[3] = {0.0f, 0.0f, 0.0f};
+#pragma unroll
+        for (int g = 0; g < kStepBlock / 32; g++)
+#pragma unroll
+            for (int c = 0; c < 3; c++) t[c] += warp_sum_f(part[c * kStepBlock + 32 * g]);
+        if (lane == 0)
+#pragma unroll
+            for (int c = 0; c < 3; c++) atomicAdd(&sh.acc[c], to_fixed(t[c], ob));
+    }
+    for (int j = w * 32 + lane; j < ttiles; j += nw * 32) {
+        float x = 0.0f;
+#pragma unroll
+        for (int g = 0; g < kTriTile / 32; g++) x += sh.tred[j][g];
+        atomicAdd(&sh.acc[0], to_fixed(x, ob));
+    }
+    if (ob) atomicOr(&s.sc->nonfinite, 2);
+}
+
+}  // namespace
+
+// A run or part of one: with 'begin', the run start (forced rebuild, first
+// force pass, half kick and drift) and the checkpoint of the start state;
+// then 'units' middle steps, each followed by its rebuild when the half-skin
+// rule calls for one; with 'end', the last step.  slots: when not null, the
+// positions after drift u go to slots + (u + 1) N too.
+template <bool MT, bool SG, bool WX, bool WY, bool SIG1>
+__global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) {
+    extern __shared__ int4 dyn[];
+    __shared__ CoopShared sh;
+    DevScalars *sc = s.sc;
+    const int nt = MT ? s.numTypes * s.numTypes : 1;
+    for (int q = threadIdx.x; q < nt; q += blockDim.x) sh.tab[q] = s.pair[q];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    CoopRun r = {};
+    r.base = sc->runTag;
+    r.dispHi = a.begin ? 0.0f : sc->dispHi;
+    r.row = a.begin ? 0 : sc->obsRow;
+    r.stepNow = a.begin ? s.stepBase : sc->stepNow;
+    r.updates = a.begin ? 0 : sc->totalUpdates;
+    r.cnt = sc->runFill;
+    int p = a.parity;
+    bool withhold = a.withhold && blockIdx.x == 0;
+    // tile j of block b is tile b + j grid: 128 particles, worked by the whole
+    // block, four lanes each
+    static_assert(kCoopThreads == 4 * kStepBlock, "a quad per particle of a tile");
+    const int ntiles = (s.N + kStepBlock - 1) / kStepBlock, groups = blockDim.x / kStepBlock;
+    const int grp = threadIdx.x / kStepBlock, gt = threadIdx.x % kStepBlock;
+    const bool tris = s.feaForces && s.ntri > 0;
+    const int ntt = tris ? (s.ntri + kTriTile - 1) / kTriTile : 0, tgroups = blockDim.x / kTriTile;
+    const int tgrp = threadIdx.x / kTriTile, tgt = threadIdx.x % kTriTile;
+    const int per = (ntiles + gridDim.x - 1) / gridDim.x, tper = (ntt + gridDim.x - 1) / gridDim.x;
+    const int tiles = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int ttiles = (int)blockIdx.x < ntt ? (ntt - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    CoopMem mem;
+    mem.rows = a.rows;
+    mem.tri = a.triStaged ? dyn : nullptr;
+    mem.term = reinterpret_cast<float *>(dyn + (a.triStaged ? tper * kTriTile : 0));
+    mem.part = mem.term + 4 * kTermComp;
+    mem.count = reinterpret_cast<int *>(mem.part + (size_t)per * 3 * kStepBlock);
+    mem.inc = a.incStaged ? mem.count + per * kStepBlock : nullptr;
+    mem.list = mem.count + per * kStepBlock + (a.incStaged ? per * kIncWords * kStepBlock : 0);
+    if (a.begin) {
+        const float2 *x = p ? s.pos1 : s.pos0;
+        for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.N; i += gridDim.x * blockDim.x) {
+            a.ckPos[i] = x[i];
+            a.ckVel[i] = s.vel[i];
+            a.ckAcc[i] = s.acc[i];
+        }
+    }
+    if (mem.tri)
+        for (int j = tgrp; blockIdx.x + j * gridDim.x < ntt; j += tgroups) {
+            const int t = (blockIdx.x + j * gridDim.x) * kTriTile + tgt;
+            if (t < s.ntri) mem.tri[j * kTriTile + tgt] = __ldg(s.triIdx + t);
+        }
+    for (int j = grp; blockIdx.x + j * gridDim.x < ntiles; j += groups) {
+        const int i = (blockIdx.x + j * gridDim.x) * kStepBlock + gt;
+        if (mem.inc && i < min(s.nBonded, s.N)) {
+            int *inc = mem.inc + (size_t)j * kIncWords * kStepBlock + gt;
+            const int tb = s.tStart[i], nT = s.feaForces ? s.tStart[i + 1] - tb : 0;
+            const int bb = s.bStart[i], nB = s.bondForces ? s.bStart[i + 1] - bb : 0;
+            const bool fits = nT <= kIncTri && nB <= kIncBond;
+            inc[0] = fits ? (nT | nB << 8) : -1;
+            for (int k = 0; fits && k < nT; k++) {
+                const int en = __ldg(s.tEnt + tb + k);
+                inc[(1 + k) * kStepBlock] = 3 * (en >> 2) + (en & 3);  // its entry of triF
+            }
+            for (int k = 0; fits && k < nB; k++) {
+                const int2 en = __ldg(s.bEnt + bb + k);
+                inc[(1 + kIncTri + 2 * k) * kStepBlock] = en.x;
+                inc[(2 + kIncTri + 2 * k) * kStepBlock] = en.y;
+            }
+        }
+        if (!a.begin && i < s.N) {
+            // lists from the last rebuild before this launch
+            const int cnt = min(s.nbrCount[i], s.nbrCap);
+            mem.count[j * kStepBlock + gt] = cnt;
+            for (int k = 0; k < min(cnt, mem.rows); k++)
+                mem.list[((size_t)j * mem.rows + k) * kListRow + gt] = s.nbr[nbr_at(k, i, s.Ncap)];
+        }
+    }
+    if (threadIdx.x < 3) sh.acc[threadIdx.x] = 0ull;
+    __syncthreads();
+    bool ok = true;
+    const int updates0 = r.updates;
+    bool rebuild = a.begin != 0;
+    const int total = (a.begin ? 1 : 0) + a.units + (a.end ? 1 : 0);
+    for (int u = 0;; u++) {
+        if (rebuild) {
+            if (!(ok = coop_rebuild(s, sh, mem, r, p, withhold))) break;
+            withhold = false;
+        }
+        if (u >= total) break;
+        const int mode = (a.begin && u == 0) ? MODE_FIRST : ((a.end && u == total - 1) ? MODE_LAST : MODE_MID);
+        const float2 *pin = p ? s.pos1 : s.pos0;
+        float2 *pout = p ? s.pos0 : s.pos1;
+        if (tris) {
+            for (int j = tgrp; blockIdx.x + j * gridDim.x < ntt; j += tgroups) {
+                const int t = (blockIdx.x + j * gridDim.x) * kTriTile + tgt;
+                float e = 0.0f;
+                if (t < s.ntri) e = tri_force(s, pin, t, mem.tri ? mem.tri[j * kTriTile + tgt] : __ldg(s.triIdx + t));
+                e = warp_sum_f(e);
+                if (lane == 0) sh.tred[j][warp % (kTriTile / 32)] = e;
+            }
+            __syncthreads();
+            if (!(ok = coop_exchange(s, sh, r, 0u, withhold))) break;
+            withhold = false;
+        }
+        float vvm = 0.0f;
+        bool bad = false;
+        for (int j = 0; j < tiles; j++) {
+            const int col = threadIdx.x >> 2, i = (blockIdx.x + j * gridDim.x) * kStepBlock + col;
+            coop_particle<MT, SG, WX, WY, SIG1>(s, mem, sh.tab, i, i < s.N, j, col, threadIdx.x & 3, mode, r.stepNow,
+                                                pin, pout, a.slots ? a.slots + (size_t)(u + 1) * s.N : nullptr, vvm,
+                                                bad);
+        }
+        vvm = warp_max(vvm);
+        const unsigned anybad = __ballot_sync(0xffffffffu, bad);
+        if (lane == 0) {
+            sh.vmax[warp] = vvm;
+            if (anybad) atomicOr(&sc->nonfinite, 1);
+        }
+        __syncthreads();
+        const unsigned x = r.xi;
+        float mm = 0.0f;
+        if (warp == 0) mm = warp_max(lane < kCoopThreads / 32 ? sh.vmax[lane] : 0.0f);
+        if (!(ok = coop_exchange(s, sh, r, __float_as_uint(mm), withhold, false,
+                                 [&] { coop_block_sums(s, sh, mem, tiles, ttiles, 3); })))
+            break;
+        withhold = false;
+        if (threadIdx.x < 3) {
+            // visible to the others with this block's next word
+            coop_sums(s, x)[4 * (size_t)blockIdx.x + threadIdx.x] = sh.acc[threadIdx.x];
+            sh.acc[threadIdx.x] = 0ull;
+        }
+        // the rebuild rule (md3dsystem.cpp:177, nn.cpp:118), the same on every block
+        const float vm2 = __uint_as_float(sh.maxBits);
+        int reb = 0;
+        if (mode != MODE_FIRST) {
+            const float d = r.dispHi + sqrtf(vm2) * s.dt;
+            reb = (double)d > s.halfSkin;
+            r.dispHi = d;
+        }
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            CoopDue &d = sh.due[r.dueIn & 3u];
+            d.x = x;
+            d.mode = mode;
+            d.row = r.row;
+            d.reb = reb;
+            d.vm = vm2;
+            d.d = r.dispHi;
+            sc->rebuild = reb;
+        }
+        r.dueIn++;
+        if (mode != MODE_FIRST) r.row++;
+        if (mode != MODE_LAST) {
+            r.stepNow++;
+            p ^= 1;
+        }
+        rebuild = mode == MODE_MID && reb;
+    }
+    // the cell arrays of the last rebuild; then the last sums
+    if (ok && r.updates != updates0) ok = coop_cells(s, sh, r);
+    __syncthreads();
+    if (ok) ok = coop_exchange(s, sh, r, 0u, false, true);
+    if (ok && blockIdx.x == 0 && warp == 2)
+        for (; r.dueOut != r.dueIn; r.dueOut++) coop_totals(s, sh.due[r.dueOut & 3u]);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        sc->dispHi = r.dispHi;
+        sc->obsRow = r.row;
+        sc->stepNow = r.stepNow;
+        sc->totalUpdates = r.updates;
+        sc->runTag = r.base + r.xi;
+        sc->runFill = r.cnt;
+    }
+}
+
+// The kernel of a system with (MT) several types and (SG) a sigma per particle.
+template <bool MT, bool SG, bool WX, bool WY>
+const void *coop_sig(const DevSys &s) {
+    if constexpr (!SG) {
+        if (s.sigmaOne) return (const void *)k_coop<MT, SG, WX, WY, true>;
+    }
+    return (const void *)k_coop<MT, SG, WX, WY, false>;
+}
+
+template <bool MT, bool SG>
+const void *coop_image(const DevSys &s) {
+    if (s.wrapx && s.wrapy) return coop_sig<MT, SG, true, true>(s);
+    if (s.wrapx) return coop_sig<MT, SG, true, false>(s);
+    return coop_sig<MT, SG, false, false>(s);
+}
+
+// one translation unit each
+const void *coop_kernel_one(const DevSys &s);    // k_coop.cu
+const void *coop_kernel_types(const DevSys &s);  // k_coop_types.cu
+const void *coop_kernel_sigma(const DevSys &s);  // k_coop_sigma.cu
+
+}  // namespace femmd

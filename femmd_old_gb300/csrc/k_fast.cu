@@ -51,7 +51,7 @@ constexpr int kPermBlock = 1024;  // cell slots per block of the storage reorder
 // call and the occupancy query would cost host time at every launch
 // otherwise.  The limit only grows (it is one value per kernel, and launches
 // of one kernel take different sizes).
-static cudaError_t kernel_setup(const void *fn, int threads, size_t smem, int *resident) {
+cudaError_t kernel_setup(const void *fn, int threads, size_t smem, int *resident) {
     struct Occ {
         int dev;
         const void *fn;

@@ -18,9 +18,8 @@ namespace femmd {
 
 // calcFeaForcesCPU2 (interactions.cpp:532-689) with Bm and vol0 precomputed
 // from the reference positions by the same float operations.
-__device__ __forceinline__ float tri_neo_hookean(const DevSys &s, const float2 *pos, int t, float2 &f0, float2 &f1,
-                                                 float2 &f2) {
-    int4 q = __ldg(s.triIdx + t);
+__device__ __forceinline__ float tri_neo_hookean(const DevSys &s, const float2 *pos, int t, int4 q, float2 &f0,
+                                                 float2 &f1, float2 &f2) {
     float2 r0 = pos[q.x], r1 = pos[q.y], r2 = pos[q.z];
     float4 bm = __ldg(s.triGeo + 2 * t);
     float vol0 = __ldg(s.triGeo + 2 * t + 1).x;
@@ -89,8 +88,7 @@ __device__ __forceinline__ float tri_neo_hookean(const DevSys &s, const float2 *
 // computeFeaForcesGPU (interactionsCuda.cu:312-451): Green strain, linear C,
 // float arithmetic of the reference kernel; xm rows 1-2 and |area|
 // precomputed from the reference positions.
-__device__ __forceinline__ float tri_green(const DevSys &s, const float2 *pos, int t, float2 *f) {
-    int4 q = __ldg(s.triIdx + t);
+__device__ __forceinline__ float tri_green(const DevSys &s, const float2 *pos, int t, int4 q, float2 *f) {
     int p[3] = {q.x, q.y, q.z};
     float rx[3], ry[3], X[3], Y[3];
 #pragma unroll
@@ -145,19 +143,23 @@ __device__ __forceinline__ float tri_green(const DevSys &s, const float2 *pos, i
     return pesum * tetVol;
 }
 
-// Nodal forces of triangle t into triF, energy returned (law of s.feaLaw).
-__device__ __forceinline__ float tri_force(const DevSys &s, const float2 *pos, int t) {
+// Nodal forces of triangle t (vertices q) into triF, energy returned (law of s.feaLaw).
+__device__ __forceinline__ float tri_force(const DevSys &s, const float2 *pos, int t, int4 q) {
     float2 f[3];
     float e;
     if (s.feaLaw == 0)
-        e = tri_neo_hookean(s, pos, t, f[0], f[1], f[2]);
+        e = tri_neo_hookean(s, pos, t, q, f[0], f[1], f[2]);
     else
-        e = tri_green(s, pos, t, f);
+        e = tri_green(s, pos, t, q, f);
     s.triF[3 * t + 0] = f[0];
     s.triF[3 * t + 1] = f[1];
     s.triF[3 * t + 2] = f[2];
     s.triE[t] = e;
     return e;
+}
+
+__device__ __forceinline__ float tri_force(const DevSys &s, const float2 *pos, int t) {
+    return tri_force(s, pos, t, __ldg(s.triIdx + t));
 }
 
 // ------------------------------------------------------------ particles
@@ -244,8 +246,9 @@ __device__ __forceinline__ float img(float a, float b, float L, bool ex, float &
 // takes the once-rounded value instead (ref + TwoSum error), a branch that
 // only boundary pairs enter.
 template <bool MT, bool SG, bool WX, bool WY, bool SIG1>
-__device__ __forceinline__ void lj_pair(const DevSys &s, const PairEntry *tab, const PairEntry &pe0, int ti, float si,
-                                        float2 pi, int tag, float2 pj, float &fx, float &fy, float &u2, float &w2) {
+__device__ __forceinline__ void lj_pair_sig(const DevSys &s, const PairEntry *tab, const PairEntry &pe0, int ti,
+                                            float si, float sj, float2 pi, int tag, float2 pj, float &fx, float &fy,
+                                            float &u2, float &w2) {
     float dx = pi.x - pj.x, dy = pi.y - pj.y;
     bool wrx = false, wry = false;
     // |d| >= L/2 is rare (boundary pairs): one compare on the common path
@@ -273,7 +276,7 @@ __device__ __forceinline__ void lj_pair(const DevSys &s, const PairEntry *tab, c
     const PairEntry &pe = MT ? tab[ti * s.numTypes + ((unsigned)tag >> kIdBits)] : pe0;
     float rcut2, sig2, c;
     if (SG) {
-        float sij = (si + __ldg(s.sigma + (tag & kIdMask))) / 2.0f;
+        float sij = (si + sj) / 2.0f;
         rcut2 = pe.rc * pe.rc * sij * sij;
         sig2 = sij * sij;
         c = pe.eps48 / sig2;
@@ -301,6 +304,110 @@ __device__ __forceinline__ void lj_pair(const DevSys &s, const PairEntry *tab, c
     }
 }
 
+// calcBondForcesCPU for one incidence en of a particle at pw with its
+// partner at pj: f on the bond's first particle, -f on the second; the
+// energy (doubled like the pair terms) with the first.
+template <bool WX, bool WY>
+__device__ __forceinline__ void bond_term(const DevSys &s, int2 en, float2 pw, float2 pj, float &fx, float &fy,
+                                          float &ue) {
+    const bool second = en.x < 0;
+    const float r0 = __int_as_float(en.y);
+    const float2 a = second ? pj : pw, b = second ? pw : pj;
+    float dxr, dyr;
+    bool wr = false;
+    float dx = img<WX>(a.x, b.x, s.Lx, s.imageExact, dxr, wr);
+    float dy = img<WY>(a.y, b.y, s.Ly, s.imageExact, dyr, wr);
+    float r = sqrtf(dx * dx + dy * dy);
+    float dl = r - r0;
+    float k = s.bondKMode ? s.E / r0 : s.kBond;
+    float kdr = -k * dl / r;
+    float f1 = kdr * dx, f2 = kdr * dy;
+    if (!second) {
+        fx += f1;
+        fy += f2;
+        ue += k * dl * dl;
+    } else {
+        fx -= f1;
+        fy -= f2;
+    }
+}
+
+template <bool MT, bool SG, bool WX, bool WY, bool SIG1>
+__device__ __forceinline__ void lj_pair(const DevSys &s, const PairEntry *tab, const PairEntry &pe0, int ti, float si,
+                                        float2 pi, int tag, float2 pj, float &fx, float &fy, float &u2, float &w2) {
+    lj_pair_sig<MT, SG, WX, WY, SIG1>(s, tab, pe0, ti, si, SG ? __ldg(s.sigma + (tag & kIdMask)) : 0.0f, pi, tag, pj,
+                                      fx, fy, u2, w2);
+}
+
+// Lennard-Jones pairs with unit sigma, added up in packed single precision
+// (add, multiply and fused multiply-add of two floats at a time, each rounded
+// as the scalar operation): lj_pair's values in lj_pair's order, in about a
+// third of its instructions.
+//   * d = p_i - p_j as one fused multiply-add by -1 (one rounding: the same
+//     difference), no image test.  'far' keeps the largest |difference|: if it
+//     reaches half a box length, a pair crossed the boundary and the caller
+//     works the particle again by lj_pair.
+//   * 1/r^2 correctly rounded as __frcp_rn gives it: the approximate
+//     reciprocal and one Newton-Raphson step in fused multiply-adds
+//     (Markstein, "Computation of elementary functions on the IBM RISC
+//     System/6000 processor", 1990).  All floats of [2^-100, 2^100] were
+//     compared with __frcp_rn; 'close' keeps the smallest r^2, and below
+//     kPairClose the caller works the particle again by lj_pair.
+//   * c s6 (s6 - 1/2) and 4 eps s6 (s6 - 1) as one packed product.
+// Measured: the batched kernel 27.2 -> 23.5 ms (128 replicas, run(100)), the
+// large mixed system's run(50) 9.32 -> 8.84 ms.
+//   * outside the cutoff zeros are added: no branch per pair.  (A sum that
+//     starts at +0 never is -0, so +-0 added leaves it as it is.)
+constexpr float kPairClose = 1e-30f;
+
+// The pair's terms: force x and y, doubled energy and virial.
+__device__ __forceinline__ float4 lj_terms_x2(float2 pi, float2 pj, float2 ce, float rcut2, float us, bool on,
+                                              float &far, float &close) {
+    const float2 d = __ffma2_rn(pj, make_float2(-1.0f, -1.0f), pi);
+    const float2 sq = mul2(d, d);
+    const float dr2 = sq.x + sq.y;
+    if (on) {
+        far = fmaxf(far, fmaxf(fabsf(d.x), fabsf(d.y)));
+        close = fminf(close, dr2);
+    }
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(dr2));
+    const float dr2i = __fmaf_rn(y, __fmaf_rn(-dr2, y, 1.0f), y);
+    const float dr6i = dr2i * dr2i * dr2i;
+    const float2 r6 = make_float2(dr6i, dr6i);
+    const float2 g = mul2(mul2(ce, r6), add2(r6, make_float2(-0.5f, -1.0f)));
+    const bool in = on && dr2 < rcut2;
+    const float fc = in ? g.x * dr2i : 0.0f;
+    const float u = in ? g.y + us : 0.0f;
+    return make_float4(__fmul_rn(fc, d.x), __fmul_rn(fc, d.y), u, __fmul_rn(fc, dr2));
+}
+
+struct LjSums {
+    float2 F, UW;  // force; doubled energy and virial
+    float far, close;
+};
+
+__device__ __forceinline__ void lj_pair_x2(float2 pi, float2 pj, float2 ce, float rcut2, float us, bool on,
+                                           LjSums &a) {
+    const float4 t = lj_terms_x2(pi, pj, ce, rcut2, us, on, a.far, a.close);
+    a.F = add2(a.F, make_float2(t.x, t.y));
+    a.UW = add2(a.UW, make_float2(t.z, t.w));
+}
+
+// Whether the terms stand: no pair crossed the boundary, none was too close.
+template <bool WX, bool WY>
+__device__ __forceinline__ bool lj_sums_ok(const DevSys &s, float far, float close) {
+    const float h = WX && WY ? fminf(0.5f * s.Lx, 0.5f * s.Ly) : (WX ? 0.5f * s.Lx : 0.0f);
+    return (!(WX || WY) || far < h) && close >= kPairClose;
+}
+
+// A particle at p within reach of a periodic edge (its listed pairs may cross it).
+template <bool WX, bool WY>
+__device__ __forceinline__ bool near_edge(const DevSys &s, float2 p) {
+    const float D = s.imgD;
+    return (WX && (p.x < D || p.x > s.Lx - D)) || (WY && (p.y < D || p.y > s.Ly - D));
+}
+
 // The forces that come before the pair forces in the reference's CPU order
 // for particle i at position pi: the fixed walls and gravity, then (bonded
 // particles) the bond incidences in bond order and the triangles' nodal forces
@@ -309,7 +416,6 @@ __device__ __forceinline__ void lj_pair(const DevSys &s, const PairEntry *tab, c
 template <bool WX, bool WY, bool RO>
 __device__ __forceinline__ void bonded_forces(const DevSys &s, int i, int mode, const float2 *pin, float2 pi,
                                               float &fx, float &fy, float &ue, float &utri, float &uwall) {
-    const float Lx = s.Lx, Ly = s.Ly;
     // walls and bonds come before the area springs in the reference's force
     // order: they see the positions from before that pass (posPre, for the
     // particles of [0, nPre); pin without area springs)
@@ -317,34 +423,13 @@ __device__ __forceinline__ void bonded_forces(const DevSys &s, int i, int mode, 
     if (s.gravity > 0.0f) fy -= s.mass[i] * s.gravity;
     if (i < s.nBonded) {
         if (s.bondForces) {
-            // calcBondForcesCPU: f on the bond's first particle, -f on the second
             const float2 *pb = s.nPre > 0 ? s.posPre : pin;
             const float2 pw = s.nPre > 0 ? s.posPre[i] : pi;
             const int qb = s.bStart[i], qe = s.bStart[i + 1];
             for (int q = qb; q < qe; q++) {
-                int2 en = __ldg(s.bEnt + q);
-                const bool second = en.x < 0;
+                const int2 en = __ldg(s.bEnt + q);
                 const int j = en.x & 0x7fffffff;
-                const float r0 = __int_as_float(en.y);
-                const float2 pj = RO ? __ldg(pb + j) : pb[j];
-                const float2 a = second ? pj : pw, b = second ? pw : pj;
-                float dxr, dyr;
-                bool wr = false;
-                float dx = img<WX>(a.x, b.x, Lx, s.imageExact, dxr, wr);
-                float dy = img<WY>(a.y, b.y, Ly, s.imageExact, dyr, wr);
-                float r = sqrtf(dx * dx + dy * dy);
-                float dl = r - r0;
-                float k = s.bondKMode ? s.E / r0 : s.kBond;
-                float kdr = -k * dl / r;
-                float f1 = kdr * dx, f2 = kdr * dy;
-                if (!second) {
-                    fx += f1;
-                    fy += f2;
-                    ue += k * dl * dl;  // doubled like the pair terms
-                } else {
-                    fx -= f1;
-                    fy -= f2;
-                }
+                bond_term<WX, WY>(s, en, pw, RO ? __ldg(pb + j) : pb[j], fx, fy, ue);
             }
         }
         if (s.feaForces) {
@@ -364,17 +449,20 @@ __device__ __forceinline__ void bonded_forces(const DevSys &s, int i, int mode, 
 // the doubled energy and virial, add the wall energy and the moving walls,
 // then the integration of the mode (kick, observables, next half kick and
 // drift into pout) and the outputs of MODE_FORCES / MODE_INIT / MODE_LAST.
+// m, v: its mass and velocity; stepIdx: the step the moving walls are at
+// (-1: DevScalars::stepNow).
 template <bool WX, bool WY>
 __device__ __forceinline__ void finish_particle(const DevSys &s, int i, int mode, float2 pi, float2 *pout, float fx,
-                                                float fy, float ue, float we, float utri, float uwall, float &ue_out,
-                                                float &we_out, float &ke, float &vvm, bool &bad) {
+                                                float fy, float ue, float we, float utri, float uwall, float m,
+                                                float2 v, float &ue_out, float &we_out, float &ke, float &vvm,
+                                                bool &bad, int stepIdx = -1) {
     const float Lx = s.Lx, Ly = s.Ly;
     ue *= 0.5f;
     we *= 0.5f;
     ue += uwall;
     if (s.wallOn) {
         // harmonic walls after the pair forces: top wall at y_w(n), bottom at 0
-        const float yw = wall_y(s, s.sc->stepNow);
+        const float yw = wall_y(s, stepIdx >= 0 ? stepIdx : s.sc->stepNow);
         const float dl = s.wallDelta[i];
         const float ht = (pi.y + dl) - yw;
         if (ht > 0.0f) {
@@ -388,7 +476,6 @@ __device__ __forceinline__ void finish_particle(const DevSys &s, int i, int mode
         }
     }
     bad = bad || !(isfinite(fx) && isfinite(fy));
-    const float m = s.mass[i];
     const float ax = fx / m, ay = fy / m;
     const float dt = s.dt, hdt = s.hdt;
     if (mode == MODE_FORCES) {
@@ -398,7 +485,6 @@ __device__ __forceinline__ void finish_particle(const DevSys &s, int i, int mode
         s.acc[i] = make_float2(ax, ay);
         s.forceOut[i] = make_float2(fx, fy);
     } else {
-        float2 v = s.vel[i];
         if (mode == MODE_MID || mode == MODE_LAST) {
             // leapFrogStep2 then evalProps
             v.x += hdt * ax;
@@ -440,14 +526,58 @@ __device__ __forceinline__ void particle_step(const DevSys &s, const PairEntry *
     const float2 pi = pin[i];
     float fx = 0.0f, fy = 0.0f;
     bonded_forces<WX, WY, RO>(s, i, mode, pin, pi, fx, fy, ue, utri, uwall);
-    {
+    const int cnt = min(s.nbrCount[i], s.nbrCap);
+    bool done = false;
+    if constexpr (SIG1 && !SG) {
+        // away from the periodic edges (all lanes of the warp that got here):
+        // the packed sums, four gathers in flight at a time
+        if (!__any_sync(__activemask(), near_edge<WX, WY>(s, pi))) {
+            const int4 *__restrict__ lst = reinterpret_cast<const int4 *>(s.nbr) + i;
+            const size_t row = (size_t)s.Ncap;
+            const int ti = MT ? s.typeId[i] * s.numTypes : 0;
+            const PairEntry pe0 = tab[0];
+            LjSums a = {make_float2(fx, fy), make_float2(ue, we), 0.0f, 1.0f};
+            const int4 zero4 = make_int4(0, 0, 0, 0);
+            int4 g = cnt > 0 ? (RO ? __ldg(lst) : *lst) : zero4;
+            for (int base = 0; base < cnt; base += 4) {
+                lst += row;
+                const int4 gn = base + 4 < cnt ? (RO ? __ldg(lst) : *lst) : zero4;
+                const int tags[4] = {g.x, g.y, g.z, g.w};
+                float2 q[4];
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const int j = tags[u] & kIdMask;
+                    q[u] = base + u < cnt ? (RO ? __ldg(pin + j) : pin[j]) : make_float2(pi.x + 1.0f, pi.y);
+                }
+#pragma unroll
+                for (int u = 0; u < 4; u++) {
+                    const bool on = base + u < cnt;  // (an unused word of the last group may hold anything)
+                    if (MT) {
+                        const float4 e =
+                            *reinterpret_cast<const float4 *>(tab + ti + (on ? (unsigned)tags[u] >> kIdBits : 0u));
+                        lj_pair_x2(pi, q[u], make_float2(e.x, e.y), e.z, e.w, on, a);
+                    } else {
+                        lj_pair_x2(pi, q[u], make_float2(pe0.c, pe0.eps4), pe0.rcut2, pe0.us, on, a);
+                    }
+                }
+                g = gn;
+            }
+            if (lj_sums_ok<WX, WY>(s, a.far, a.close)) {
+                fx = a.F.x;
+                fy = a.F.y;
+                ue = a.UW.x;
+                we = a.UW.y;
+                done = true;
+            }
+        }
+    }
+    if (!done) {
         // pairForce over the Verlet list, in list order.  The list comes in
         // 16-byte groups of four entries (nbr_at); the next group is in
         // flight while the current one is worked.  PIPE > 0: the four
         // neighbour positions of a group are gathered before its pair terms
         // are added in order; otherwise each is gathered at its turn (fewer
         // live registers, for the kernels whose occupancy needs them).
-        const int cnt = min(s.nbrCount[i], s.nbrCap);
         const int4 *__restrict__ lst = reinterpret_cast<const int4 *>(s.nbr) + i;
         const size_t row = (size_t)s.Ncap;
         const int ti = MT ? s.typeId[i] : 0;
@@ -498,7 +628,9 @@ __device__ __forceinline__ void particle_step(const DevSys &s, const PairEntry *
             g = gn;
         }
     }
-    finish_particle<WX, WY>(s, i, mode, pi, pout, fx, fy, ue, we, utri, uwall, ue_out, we_out, ke, vvm, bad);
+    const float2 v = (mode != MODE_FORCES && mode != MODE_INIT) ? s.vel[i] : make_float2(0.0f, 0.0f);
+    finish_particle<WX, WY>(s, i, mode, pi, pout, fx, fy, ue, we, utri, uwall, s.mass[i], v, ue_out, we_out, ke, vvm,
+                            bad);
 }
 
 // End of a step kernel: the block's energy, virial, kinetic and max-speed
