@@ -584,7 +584,7 @@ class Batch:
         self._call("femmd_batch_set_launch", int(threads), int(ctas_per_sm))
 
     def set_split(self, on=True):
-        """Run replicas heavier than a CTA's average share on CTA pairs."""
+        """Run the heaviest replicas on thread-block clusters of up to 8 CTAs each."""
         self._call("femmd_batch_set_split", int(bool(on)))
 
     def launch(self):

@@ -343,13 +343,23 @@ cudaError_t enqueue_props(Launch &L, const DevSys &s, const float2 *pos, int ncl
 // the elastomers, which come first)
 
 // ---- batched replicas (k_batch.cu): one persistent launch over many systems
+constexpr int kBatchMaxCluster = 8;
+// The replicas order[first .. first + count) on clusters of 'cluster' CTAs
+// (1: a CTA each), 'ctas' CTAs in all.
+struct BatchClass {
+    int cluster, first, count, ctas;
+    bool operator==(const BatchClass &o) const {
+        return cluster == o.cluster && first == o.first && count == o.count && ctas == o.ctas;
+    }
+};
 struct BatchLaunch {
     const DevSys *reps;
     const int *order, *parity;
-    int *queue;  // {next work index, finished CTAs, next single-CTA index}, zero before a launch
-    int nwork, minBlocks;
-    int nbig;    // the first nbig replicas of 'order' run on CTA pairs (0: none)
-    int steps, ctas, threads;
+    int *queue;  // per class {next work index, finished CTAs}, zero before a launch
+    int nclass;
+    BatchClass cls[kBatchMaxCluster];
+    int minBlocks;
+    int steps, threads;
     size_t smem;
     bool multiType, sigmaByType, sigmaOne, wrapx, wrapy, exact;
 };

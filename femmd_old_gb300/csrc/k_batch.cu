@@ -2,14 +2,20 @@
 //
 // Each replica is a complete femmd2D system (its own box, cell grid, lists,
 // bonds, triangles and run state), described by the same DevSys block as a
-// single context.  One CTA owns a set of replicas (longest-processing-time
-// assignment by the host) and runs the whole run(n) sequence of each -- the
+// single context.  One CTA, or for the heaviest replicas a thread-block
+// cluster of up to eight (batch_classes in femmd_api.cu), takes the next
+// replica of its queue and runs the whole run(n) sequence of each -- the
 // reference's Integrator::run (femmd2D/src/integrator.cpp:31-57): forced
 // rebuild, first force pass and drift, n-1 steps with the half-skin rebuild
 // rule, last step -- with block-level rebuilds and steps separated only by
 // __syncthreads.  Replicas never exchange data, so there is no grid-wide
-// synchronisation and no per-step launch: one kernel launch covers all
-// replicas and all steps.
+// synchronisation and no per-step launch: one kernel launch per class of
+// cluster size, side by side, covers all replicas and all steps.
+//
+// Bound by instruction issue where every SM is full, else by the largest
+// replicas: 128 replicas of 500 to 20,000 atoms (676,000 in all), run(100) with
+// the states copied in and out: 27.4 ms on one CTA or a pair each, 17.1 ms on
+// clusters by weight (23.5 ms with the packed pair terms alone).
 //
 // The per-particle and per-triangle arithmetic is step_body.cuh /
 // nn_body.cuh, the same code as the single-system kernels, and the list order
@@ -79,24 +85,24 @@ __device__ __forceinline__ void block_reduce_step(float &a, float &b, float &c, 
     }
 }
 
-// The threads that work on one replica: one CTA (Solo), or the two CTAs of
-// a thread-block cluster (Pair).  Loops over particles, triangles and
+// The threads that work on one replica: one CTA (Solo), or the CTAs of a
+// thread-block cluster (Gang).  Loops over particles, triangles and
 // candidates are strided over the team; sync() is __syncthreads or the
 // cluster barrier (release/acquire at cluster scope, so global writes made
-// by either CTA before it are seen by both after it).  Every sync() is
+// by any of its CTAs before it are seen by all after it).  Every sync() is
 // reached by every thread of the team the same number of times: no sync()
-// sits under a condition that could differ between the two CTAs.
+// sits under a condition that could differ between its CTAs.
 struct SoloTeam {
-    static constexpr int size = 1;
+    __device__ int size() const { return 1; }
     __device__ int rank() const { return 0; }
     __device__ void sync() const { __syncthreads(); }
     // combine one float/int partial per CTA in the leader (rank 0)
     __device__ float *slot(float *x, int) const { return x; }
 };
 
-struct PairTeam {
-    static constexpr int size = 2;
-    int r;
+struct GangTeam {
+    int r, n;
+    __device__ int size() const { return n; }
     __device__ int rank() const { return r; }
     __device__ void sync() const { cg::this_cluster().sync(); }
     // the leader's copy of a shared array, at this CTA's entries
@@ -110,7 +116,7 @@ template <class Team>
 __device__ __noinline__ void block_rebuild(const Team team, const DevSys &s, int parity, int *iscr, float *xch) {
     const float2 *pos = parity ? s.pos1 : s.pos0;
     const int lane = threadIdx.x & 31;
-    const int t0 = team.rank() * blockDim.x + threadIdx.x, tstride = Team::size * blockDim.x;
+    const int t0 = team.rank() * blockDim.x + threadIdx.x, tstride = team.size() * blockDim.x;
     const bool lead = team.rank() == 0 && threadIdx.x == 0;
     if (lead && s.sc->rebuild) {
         s.sc->totalUpdates += 1;
@@ -220,7 +226,7 @@ __device__ __noinline__ void block_rebuild(const Team team, const DevSys &s, int
     if (threadIdx.x == 0) *team.slot(xch, 1) = __int_as_float(kmax);
     team.sync();
     if (lead) {
-        for (int q = 1; q < Team::size; q++) kmax = max(kmax, __float_as_int(xch[q]));
+        for (int q = 1; q < team.size(); q++) kmax = max(kmax, __float_as_int(xch[q]));
         s.sc->maxCount = kmax;
         if (kmax > s.nbrCap) s.sc->overflow |= 1;
         s.sc->builds += 1ull;
@@ -234,7 +240,7 @@ __device__ __noinline__ void block_step(const Team team, const DevSys &s, const 
                                         float *fscr, float *xch) {
     const float2 *pin = parity ? s.pos1 : s.pos0;
     float2 *pout = parity ? s.pos0 : s.pos1;
-    const int t0 = team.rank() * blockDim.x + threadIdx.x, tstride = Team::size * blockDim.x;
+    const int t0 = team.rank() * blockDim.x + threadIdx.x, tstride = team.size() * blockDim.x;
     float etri = 0.0f;
     if (s.feaForces && s.ntri > 0) {
         for (int t = t0; t < s.ntri; t += tstride) etri += tri_force(s, pin, t);
@@ -260,7 +266,7 @@ __device__ __noinline__ void block_step(const Team team, const DevSys &s, const 
     if (team.rank() == 0 && threadIdx.x == 0) {
         float te = xch[0], tu = xch[1], tw = xch[2], tk = xch[3], tm = xch[4];
         bool nb = xch[5] != 0.0f;
-        for (int q = 1; q < Team::size; q++) {
+        for (int q = 1; q < team.size(); q++) {
             te += xch[6 * q];
             tu += xch[6 * q + 1];
             tw += xch[6 * q + 2];
@@ -346,18 +352,18 @@ __device__ __forceinline__ void run_replica(const Team team, const DevSys *reps,
 
 }  // namespace
 
-// Replicas are handed out from a queue: 'order' lists them heaviest first,
-// and each CTA takes the next one when it is free (greedy list scheduling,
-// which also balances CTAs that share an SM).  queue[0] is the next index,
-// queue[1] counts finished CTAs; the last CTA to finish resets the queue.
-// MINB: resident CTAs per SM the register allocation must allow.
+// The replicas of one class (order[0 .. nwork), heaviest first) are handed out
+// from a queue: each CTA takes the next one when it is free (greedy list
+// scheduling, which also balances CTAs that share an SM).  queue[0] is the
+// next index, queue[1] counts finished CTAs; the last CTA to finish resets the
+// queue.  MINB: resident CTAs per SM the register allocation must allow.
 template <bool MT, bool SG, bool WX, bool WY, bool SIG1, int MINB>
 __global__ void __launch_bounds__(1024, MINB) k_batch(const DevSys *__restrict__ reps, const int *__restrict__ order,
-                                                      int nwork, int nbig, int *queue, const int *__restrict__ parity0,
+                                                      int nwork, int *queue, const int *__restrict__ parity0,
                                                       int steps) {
     __shared__ DevSys S;
     __shared__ float fscr[6 * 32];
-    __shared__ float xch[6 * 2];
+    __shared__ float xch[6];
     __shared__ int iscr[33];
     __shared__ int next;
     extern __shared__ PairEntry tab[];
@@ -375,67 +381,64 @@ __global__ void __launch_bounds__(1024, MINB) k_batch(const DevSys *__restrict__
         if (atomicAdd(queue + 1, 1) == (int)gridDim.x - 1) {
             queue[0] = 0;
             queue[1] = 0;
-            queue[2] = 0;
         }
     }
 }
 
-// The same with the CTAs in pairs (thread-block clusters of two): first the
-// order's nbig heaviest replicas, each run by a pair (particles, triangles
-// and candidates split between the two CTAs; the leader's pick of the queue
-// shared through its shared memory), then the rest one CTA each, from their
-// own counter queue[2].  A replica much larger than the average work of a
-// CTA then no longer sets the length of the whole launch.
+// The same with a thread-block cluster (of the size the launch gives) on each
+// replica: particles, triangles and candidates split between its CTAs; the
+// leader's pick of the queue is shared through its shared memory.
 template <bool MT, bool SG, bool WX, bool WY, bool SIG1>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(1024, 1)
-    k_batch_pair(const DevSys *__restrict__ reps, const int *__restrict__ order, int nwork, int nbig, int *queue,
+__global__ void __launch_bounds__(1024, 1)
+    k_batch_gang(const DevSys *__restrict__ reps, const int *__restrict__ order, int nwork, int *queue,
                  const int *__restrict__ parity0, int steps) {
     __shared__ DevSys S;
     __shared__ float fscr[6 * 32];
-    __shared__ float xch[6 * 2];
+    __shared__ float xch[6 * kBatchMaxCluster];
     __shared__ int iscr[33];
     __shared__ int next;
     extern __shared__ PairEntry tab[];
-    const PairTeam pair{(int)cg::this_cluster().block_rank()};
+    const GangTeam gang{(int)cg::this_cluster().block_rank(), (int)cg::this_cluster().num_blocks()};
     for (;;) {
-        if (pair.rank() == 0 && threadIdx.x == 0) next = atomicAdd(queue, 1);
-        pair.sync();
+        if (gang.rank() == 0 && threadIdx.x == 0) next = atomicAdd(queue, 1);
+        gang.sync();
         const int q = *cg::this_cluster().map_shared_rank(&next, 0);
-        pair.sync();  // both have read the leader's pick before it changes
-        if (q >= nbig) break;  // the same q in both CTAs
-        run_replica<MT, SG, WX, WY, SIG1>(pair, reps, order[q], parity0, steps, S, tab, fscr, iscr, xch);
-    }
-    const SoloTeam solo;
-    for (;;) {
-        if (threadIdx.x == 0) next = nbig + atomicAdd(queue + 2, 1);
-        __syncthreads();
-        const int q = next;
-        __syncthreads();
-        if (q >= nwork) break;
-        run_replica<MT, SG, WX, WY, SIG1>(solo, reps, order[q], parity0, steps, S, tab, fscr, iscr, xch);
+        gang.sync();  // all have read the leader's pick before it changes
+        if (q >= nwork) break;  // the same q in every CTA
+        run_replica<MT, SG, WX, WY, SIG1>(gang, reps, order[q], parity0, steps, S, tab, fscr, iscr, xch);
     }
     if (threadIdx.x == 0) {
         __threadfence();
         if (atomicAdd(queue + 1, 1) == (int)gridDim.x - 1) {
             queue[0] = 0;
             queue[1] = 0;
-            queue[2] = 0;
         }
     }
 }
 
 namespace {
 
+// One kernel per class, side by side (parallel branches of a graph; one after
+// another in a stream), the largest clusters first.
 template <bool MT, bool SG, bool WX, bool WY, bool SIG1>
 cudaError_t launch_batch(Launch &L, const BatchLaunch &b) {
-    if (b.nbig > 0)
-        return L.kernel(k_batch_pair<MT, SG, WX, WY, SIG1>, dim3(b.ctas), dim3(b.threads), b.smem, b.reps, b.order,
-                        b.nwork, b.nbig, b.queue, b.parity, b.steps);
-    if (b.minBlocks >= 2)
-        return L.kernel(k_batch<MT, SG, WX, WY, SIG1, 2>, dim3(b.ctas), dim3(b.threads), b.smem, b.reps, b.order,
-                        b.nwork, 0, b.queue, b.parity, b.steps);
-    return L.kernel(k_batch<MT, SG, WX, WY, SIG1, 1>, dim3(b.ctas), dim3(b.threads), b.smem, b.reps, b.order,
-                    b.nwork, 0, b.queue, b.parity, b.steps);
+    const std::vector<cudaGraphNode_t> before = L.deps;
+    cudaError_t e = cudaSuccess;
+    for (int k = 0; k < b.nclass && !e; k++) {
+        const BatchClass &c = b.cls[k];
+        int *queue = b.queue + 2 * k;
+        if (L.graph) L.deps = before;
+        if (c.cluster > 1)
+            e = L.kernel_clusters(k_batch_gang<MT, SG, WX, WY, SIG1>, c.cluster, dim3(c.ctas), dim3(b.threads), b.smem,
+                                  b.reps, b.order + c.first, c.count, queue, b.parity, b.steps);
+        else if (b.minBlocks >= 2)
+            e = L.kernel(k_batch<MT, SG, WX, WY, SIG1, 2>, dim3(c.ctas), dim3(b.threads), b.smem, b.reps,
+                         b.order + c.first, c.count, queue, b.parity, b.steps);
+        else
+            e = L.kernel(k_batch<MT, SG, WX, WY, SIG1, 1>, dim3(c.ctas), dim3(b.threads), b.smem, b.reps,
+                         b.order + c.first, c.count, queue, b.parity, b.steps);
+    }
+    return e;
 }
 
 template <bool MT, bool SG, bool WX, bool WY>
