@@ -208,7 +208,7 @@ struct femmd_ctx {
     // a wait that gave up, which can leave records ahead of the tag base)
     bool smallClean = false;
     bool testExpire = false;  // femmd_test_expire_next_exchange
-    // the whole-run launch (k_coop): exchange words and cell counts, zero
+    // the whole-run launch (k_coop): exchange slots and cell counts, zero
     // together with their scalars (runClean); coopOff: a cell held more than
     // kCellCap particles, the plain kernels from then on
     DBuf<unsigned long long> runRec;
@@ -904,7 +904,7 @@ static femmd_status upload_topology(femmd_ctx *ctx) {
         CK(ctx->fBlockSums.ensure((N + 1023) / 1024));
         CK(ctx->newCell.ensure(N));
         CK(ctx->blockWin.ensure(kWinInts * (size_t)((N + kFastBlock - 1) / kFastBlock)));
-        CK(ctx->smallRec.ensure(3 * 4 * (size_t)kSmallMaxTiles));
+        CK(ctx->smallRec.ensure(4 * 16 + 3 * 4 * (size_t)kSmallMaxTiles));
         ctx->smallClean = false;
         if (ctx->nBonded > 0) {
             // the cell-ordered position mirror (slot N: the ghost)
@@ -1249,7 +1249,7 @@ static femmd_status expired(femmd_ctx *ctx, const char *what) {
 static bool coop_ready(femmd_ctx *ctx) {
     if (fast_mode(ctx) || ctx->coopOff || !coop_size_ok((int)ctx->pos.size(), ctx->ncells)) return false;
     const size_t cells = ctx->ncells;
-    if (ctx->runRec.ensure((3 * 16 + 4 * 4) * (size_t)kCoopMaxBlocks) || ctx->cellFill.ensure(2 * cells) ||
+    if (ctx->runRec.ensure(kCoopRecWords) || ctx->cellFill.ensure(2 * cells) ||
         ctx->cellIds.ensure(cells * kCellCap) || ctx->cellCand.ensure(cells * kCellCap)) {
         cudaGetLastError();  // no memory for the cell table: the plain kernels
         ctx->coopOff = true;

@@ -79,12 +79,10 @@ struct DevScalars {
     unsigned long long nbrSum, builds;
     unsigned long long accU, accW, accK;  // fixed-point accumulators (two's complement)
     unsigned int vvMaxBits, pad1;         // max v^2 as float bits (v^2 >= 0)
-    // the small-system run (k_fsmall): the tag base of its next launch's
-    // exchanges, the steps one launch advanced, the steps left and the
+    // the small-system run (k_fsmall): its exchanges so far, the steps one launch advanced, the steps left and the
     // position parity the next launch starts from (it ends on parity 0)
     unsigned int gbTag;
-    // the whole-run launch (k_coop): the tag base of its next launch's
-    // exchanges, and which of its two cell-count arrays the last rebuild used
+    // the whole-run launch (k_coop): the exchanges so far, and which of its two cell-count arrays the last rebuild used
     unsigned int runTag;
     int runFill, pad2;
     int smallDone, smallLeft, smallPar;
@@ -197,11 +195,11 @@ struct DevSys {
     // no bonded particles.  Other blocks keep 32-bit entries (nbr_at).
     int win16;
     int *blockWin;
-    // the small-system run's exchange records: three sets of kSmallMaxTiles
-    // records {tag << 32 | max v^2 bits, U, W, K fixed point}
+    // the small-system run's exchange slots (grid_sync.cuh), then three sets of
+    // kSmallMaxTiles records {-, U, W, K fixed point}
     unsigned long long *smallRec;
-    // the whole-run launch (k_coop): three sets of kCoopMaxBlocks exchange
-    // words and four of energy sums; its cells hold up to kCellCap particles
+    // the whole-run launch (k_coop): its exchange slots (grid_sync.cuh), then
+    // four sets of energy sums per block; its cells hold up to kCellCap particles
     // each (ids, then the candidates in id order; two arrays of counts in turn)
     unsigned long long *runRec;
     int *cellFill, *cellIds;
@@ -272,6 +270,7 @@ cudaError_t kernel_setup(const void *fn, int threads, size_t smem, int *resident
 
 // ---- whole runs of small and medium systems in one cooperative launch (k_coop.cu)
 constexpr int kCoopMaxBlocks = 256;
+constexpr size_t kCoopRecWords = 4 * 16 + 4 * 4 * (size_t)kCoopMaxBlocks;  // exchange slots, then the sums
 constexpr int kCellCap = 32;  // particles of a cell at most (a fuller one: the plain kernels)
 struct CoopArgs {
     int parity;   // of the current positions

@@ -31,7 +31,9 @@ bool coop_shape(const DevSys &s, int &grid, size_t &smem, CoopArgs &a) {
     int sms = 0, dev = 0;
     if (cudaGetDevice(&dev) || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return false;
     const int ntiles = (s.N + kStepBlock - 1) / kStepBlock;
-    const int ntt = s.feaForces ? (s.ntri + kTriTile - 1) / kTriTile : 0;
+    // (the grid depends on the topology alone: the exchanges count blocks over
+    // the life of the context, and the triangle forces can be turned on later)
+    const int ntt = (s.ntri + kTriTile - 1) / kTriTile;
     grid = std::max(1, std::min(std::min(sms, kCoopMaxBlocks), std::max(ntiles, ntt)));
     const int per = (ntiles + grid - 1) / grid, tper = (ntt + grid - 1) / grid;
     if (per > kCoopMaxTiles || tper > kCoopMaxTiles) return false;

@@ -25,12 +25,10 @@
 // energy sums are reduced while the exchange is waited for.
 //
 // Measured against the plain kernels in CUDA graphs (a whole set_state, run,
-// get_state; us): LJ fluid 400 particles run(20) 659 -> 244, 10,201 run(50)
-// 1379 -> 525; 256-disk suspension (32,512) run(100) 1825 -> 1260; adjoint of 64
-// disks over 200 steps 14,315 -> 8390.  A step of the 10,201 particles: 4.1 us in
-// the particle pass, 2.7 us in the exchange; a thread per particle instead of
-// a quad took 7.7 us there.  Exchange words side by side in one line instead
-// of a line each: 3.6 us with 80 blocks, 6 with 152 (against 2.7 and 3.3).
+// get_state; us): LJ fluid 400 particles run(20) 643 -> 216, 10,201 run(50)
+// 1374 -> 454; 256-disk suspension (32,512) run(100) 1837 -> 1000; adjoint of 64
+// disks over 200 steps 14,170 -> 7451.  The particle pass of the 10,201
+// particles takes 4.1 us; a thread per particle instead of a quad took 7.7.
 //
 // The per-particle and per-triangle arithmetic and the list order are those
 // of the plain kernels (step_body.cuh, nn_body.cuh), and so is the grouping
@@ -39,15 +37,10 @@
 // any order.  Positions, velocities, forces, energies and rebuild steps are
 // therefore the plain path's bit for bit.
 //
-// Exchanges: each block writes a word {tag << 32 | value} into one of three
-// rotating sets with release semantics; warp 0 of every block polls all words
-// (relaxed loads, all of a lane's in flight together, then an acquire fence;
-// bounded: a wait that gives up sets the timeout flag, and the block leaves
-// the kernel).  Tags grow by one per exchange over the life of the context
-// (DevScalars::runTag), so a stale word never matches.  A set is written
-// again three exchanges later, which no block reaches before every block has
-// published two exchanges later.  A step's energy sums go to one of four
-// rotating sets after its exchange is published and are therefore visible to
+// Exchanges are grid_exchange's (grid_sync.cuh), bounded: a wait that gives
+// up sets the timeout flag, and the block leaves the kernel.  They are numbered
+// over the life of the context (DevScalars::runTag).  A step's energy sums go
+// to one of four rotating sets after its exchange and are therefore visible to
 // a block that has completed the following one; block 0 adds them up during
 // the exchange after that.
 #pragma once
@@ -55,6 +48,7 @@
 #include "femmd_internal.h"
 #include "launch.h"
 #include "device_common.cuh"
+#include "grid_sync.cuh"
 #include "nn_body.cuh"
 #include "step_body.cuh"
 
@@ -63,13 +57,11 @@ namespace femmd {
 namespace {
 
 constexpr int kCoopThreads = 512;
-constexpr int kCoopSpin = 1 << 20;  // polls (about 0.5 us each) before an exchange gives up
 constexpr int kCoopTimeout = 8;     // DevScalars::overflow bit: a bounded wait expired
 constexpr int kCoopCrowded = 16;    // DevScalars::overflow bit: a cell holds more than kCellCap particles
 constexpr int kCoopMaxTiles = 32;   // tiles of one block (one lane of a warp sums each)
 constexpr int kTriTile = 256;       // triangles per energy group (k_tri_forces' block)
 constexpr int kListLanes = 8;       // lanes that build one particle's list
-constexpr int kWordQ = kCoopMaxBlocks / 32;  // words per lane of the polling warp
 // Incidences of one bonded particle kept in shared memory: a count word, up
 // to kIncTri triangle entries and kIncBond bond entries of two words.
 constexpr int kIncTri = 8, kIncBond = 6, kIncWords = 1 + kIncTri + 2 * kIncBond;
@@ -81,16 +73,7 @@ constexpr int kQuadRows = 4 * kQuadPairs;    // entries per particle and round
 // different banks.
 constexpr int kTermRow = kStepBlock + 8, kTermComp = kQuadRows * kTermRow + 8;
 constexpr int kListRow = kStepBlock + 8;     // a list row in shared memory (padded as kTermRow)
-constexpr int kWordStride = 16;              // exchange words 128 bytes apart: one L2 line each
 
-__device__ __forceinline__ void st_release(unsigned long long *p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long *p) {
-    unsigned long long v;
-    asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
 // Loads that stay where they are written, ahead of what uses them (a plain
 // load is moved down to its use when registers are short).
 __device__ __forceinline__ float2 ld_early(const float2 *p) {
@@ -108,8 +91,6 @@ __device__ __forceinline__ int ld_early(const int *p) {
     asm volatile("ld.global.s32 %0, [%1];" : "=r"(v) : "l"(p));
     return v;
 }
-__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-
 struct CoopDue {
     unsigned x;  // the exchange that published the step
     int mode, row, reb;
@@ -123,23 +104,21 @@ struct CoopShared {
     unsigned long long acc[3];        // the step's energy sums of this block (U, W, K)
     CoopDue due[4];                   // block 0: steps whose totals have still to be added up
     int wsum[kCoopThreads / 32];
-    unsigned ok, maxBits, before;     // of the last exchange; before: the sum of the earlier blocks' values
+    unsigned ok, maxBits;             // of the last exchange
+    int before;                       // particles in the earlier blocks' cells
 };
 
 // What every block carries through the launch (the same on each).
 struct CoopRun {
-    unsigned base, xi;       // tag base, exchanges so far
+    unsigned base, xi;       // exchanges before this launch, and of it
     unsigned dueIn, dueOut;  // entries pushed to and taken from CoopShared::due
     float dispHi;
     int row, stepNow, updates;
     int cnt;  // which of the two cell-count arrays the last rebuild filled
 };
 
-__device__ __forceinline__ unsigned long long *coop_words(const DevSys &s, unsigned x) {
-    return s.runRec + (size_t)(x % 3u) * kCoopMaxBlocks * kWordStride;
-}
 __device__ __forceinline__ unsigned long long *coop_sums(const DevSys &s, unsigned x) {
-    return s.runRec + 3 * kCoopMaxBlocks * kWordStride + (size_t)(x % 4u) * kCoopMaxBlocks * 4;
+    return s.runRec + kGridSlots * kGridSlotWords + (size_t)(x % 4u) * kCoopMaxBlocks * 4;
 }
 
 // One warp: the totals of a step's sums into the scalars and, for the modes
@@ -181,62 +160,28 @@ __device__ __noinline__ void coop_totals(const DevSys &s, const CoopDue &d) {
     __syncwarp();
 }
 
-// This block's word, then the wait for every block's: maxBits = the largest
-// value as a float; SUM: before = the sum of the earlier blocks' values.
+// An exchange: maxBits = the largest value as a float (the values' bits).
 // Block 0's warp 2 meanwhile adds up the totals that are due (all: every one
-// left), and 'meanwhile' runs on the warps from 3 on.  withhold: the word is
-// not written (femmd_test_expire_next_exchange).  False when a wait gave up.
-// Call it after a block barrier that follows the block's stores; it ends with
-// one.
+// left), and 'meanwhile' runs on the warps from 3 on.  withhold: this block
+// does not count (femmd_test_expire_next_exchange).  False when the wait gave
+// up.  Call it after a block barrier that follows the block's stores; it ends
+// with one.
 struct Nothing {
     __device__ void operator()() const {}
 };
-template <bool SUM = false, class Work = Nothing>
+template <class Work = Nothing>
 __device__ __forceinline__ bool coop_exchange(const DevSys &s, CoopShared &sh, CoopRun &r, unsigned value,
                                               bool withhold = false, bool all = false, Work meanwhile = {}) {
-    const unsigned tag = r.base + r.xi + 1u;
-    unsigned long long *set = coop_words(s, r.xi);
-    const bool grid = gridDim.x > 1 || withhold;
-    if (threadIdx.x == 0 && grid && !withhold) st_release(set + blockIdx.x * kWordStride, ((unsigned long long)tag << 32) | value);
-    if (threadIdx.x < 32) {
-        const int lane = threadIdx.x;
-        float m = lane == 0 ? __uint_as_float(value) : 0.0f;
-        unsigned before = 0;
-        int ok = 1;
-        if (grid) {
-            unsigned long long w[kWordQ];
-            bool more = true;
-            for (int it = 0; more && it < kCoopSpin; it++) {
-                if (it > 0) __nanosleep(20);
-                more = false;
-#pragma unroll
-                for (int q = 0; q < kWordQ; q++)
-                    if (q * 32 + lane < (int)gridDim.x) w[q] = ld_relaxed(set + (q * 32 + lane) * kWordStride);
-#pragma unroll
-                for (int q = 0; q < kWordQ; q++)
-                    if (q * 32 + lane < (int)gridDim.x) more = more || (unsigned)(w[q] >> 32) != tag;
-            }
-            ok = __all_sync(0xffffffffu, !more);
-            fence_gpu();
-#pragma unroll
-            for (int q = 0; q < kWordQ; q++)
-                if (q * 32 + lane < (int)gridDim.x) {
-                    m = fmaxf(m, __uint_as_float((unsigned)w[q]));
-                    if (SUM && q * 32 + lane < (int)blockIdx.x) before += (unsigned)w[q];
-                }
-        }
-        m = warp_max(m);
-        if (SUM) before = __reduce_add_sync(0xffffffffu, before);
-        if (lane == 0) {
-            sh.ok = (unsigned)ok;
-            sh.maxBits = __float_as_uint(m);
-            if (SUM) sh.before = before;
-        }
+    if (threadIdx.x == 0) {
+        unsigned m = value, o = 0u;
+        sh.ok = (gridDim.x == 1 && !withhold) ||
+                grid_exchange(s.runRec, r.base + r.xi, gridDim.x, value, 0u, withhold, m, o);
+        sh.maxBits = m;
     }
     // a step's sums are visible once the exchange after its own is complete
     while (r.dueOut != r.dueIn && !all) {
         const CoopDue &d = sh.due[r.dueOut & 3u];
-        if ((int)(r.xi - d.x) < 2) break;
+        if ((int)(r.base + r.xi - d.x) < 2) break;
         if (blockIdx.x == 0 && threadIdx.x >> 5 == 2) coop_totals(s, d);
         r.dueOut++;
     }
@@ -482,9 +427,19 @@ __device__ __forceinline__ bool coop_cells(const DevSys &s, CoopShared &sh, Coop
         block_scan(sh, c < c1 ? min(__ldcg(cnt + c), kCellCap) : 0, tot);
         sum += tot;
     }
+    // every block's count through the set of sums that is not in use
+    unsigned long long *counts = coop_sums(s, r.base + r.xi + 2u);
+    if (threadIdx.x == 0) counts[4 * (size_t)blockIdx.x + 3] = (unsigned long long)sum;
     __syncthreads();
-    if (!coop_exchange<true>(s, sh, r, (unsigned)sum)) return false;
-    int carry = gridDim.x > 1 ? (int)sh.before : 0;
+    if (!coop_exchange(s, sh, r, 0u)) return false;
+    if (threadIdx.x < 32) {
+        int before = 0;
+        for (int b = threadIdx.x; b < (int)blockIdx.x; b += 32) before += (int)__ldcg(counts + 4 * (size_t)b + 3);
+        before = __reduce_add_sync(0xffffffffu, before);
+        if (threadIdx.x == 0) sh.before = before;
+    }
+    __syncthreads();
+    int carry = sh.before;
     for (int cb = c0; cb < c1; cb += blockDim.x) {
         const int c = cb + threadIdx.x;
         const int n = c < c1 ? min(__ldcg(cnt + c), kCellCap) : 0;
@@ -821,7 +776,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
             if (anybad) atomicOr(&sc->nonfinite, 1);
         }
         __syncthreads();
-        const unsigned x = r.xi;
+        const unsigned x = r.base + r.xi;
         float mm = 0.0f;
         if (warp == 0) mm = warp_max(lane < kCoopThreads / 32 ? sh.vmax[lane] : 0.0f);
         if (!(ok = coop_exchange(s, sh, r, __float_as_uint(mm), withhold, false,

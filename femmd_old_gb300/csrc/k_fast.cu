@@ -38,6 +38,7 @@
 #include "femmd_internal.h"
 #include "launch.h"
 #include "device_common.cuh"
+#include "grid_sync.cuh"
 #include "nn_body.cuh"
 #include "step_body.cuh"
 
@@ -2116,81 +2117,41 @@ static cudaError_t fstep_image(Launch &L, const DevSys &s, int mode, int parity,
 // or a non-finite position ends it too (the run is then repeated or fails).
 // The number of steps done goes to DevScalars::smallDone.
 //
-// The exchange: each block writes a record {tag << 32 | word, U, W, K} (word:
-// its max v^2 bits after a step, flag bits during a rebuild; U, W, K: its
-// fixed-point energy sums) into one of three record sets, the tag word last
-// with release semantics, and warp 0 of every block waits until all tag
-// words carry the exchange's tag (acquire), taking the largest word as a
-// float and the OR of the words.  Block 0 sums a step's fixed-point records
-// (exact integer sums: the same totals as the step kernels' atomics) during
-// the next exchange, while it waits.  Set j is written again at exchange
-// j + 3, which no block reaches before block 0 has published exchange j + 2,
-// after those sums.  Tags grow by one per exchange (DevScalars::gbTag holds
-// the next launch's base).
-constexpr int kGridSpin = 1 << 20;  // polls of one record (about 0.5 us each) before an exchange gives up
+// The exchange (grid_sync.cuh): a step's carries the largest v^2, a rebuild's
+// the OR of flag bits.  Before a step's exchange each block writes a record
+// {U, W, K} (its fixed-point energy sums) into one of three record sets;
+// block 0 sums a step's records (exact integer sums: the same totals as the
+// step kernels' atomics) during the next exchange, while it waits.  Set j is
+// written again at exchange j + 3, which no block reaches before block 0 has
+// counted in exchange j + 2, after those sums.  Exchanges are numbered over the
+// life of the context (DevScalars::gbTag holds the next launch's first).
 
-__device__ __forceinline__ void st_release_u64(unsigned long long *p, unsigned long long v) {
-    asm volatile("st.release.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long *p) {
-    unsigned long long v;
-    asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-    return v;
-}
-
-// This block's record of exchange 'tag' (record set par), then the wait of
-// warp 0 for every block's: xsh[0] = 1 (0 when a wait gave up), xsh[1] = the
-// OR of the words, xsh[2] = their maximum as a float.  withhold: the record
-// is not written (femmd_test_expire_next_exchange: every wait gives up).
+// This block's record of exchange x (record set par), then the wait for every
+// block: xsh[0] = 1 (0 when the wait gave up), xsh[1] = the OR of the blocks'
+// words (flags) or xsh[2] = their maximum as a float (a step).  withhold: this
+// block does not count (femmd_test_expire_next_exchange: every wait gives up).
 // Call after a __syncthreads that follows the block's stores.
-__device__ __forceinline__ void small_exchange(const DevSys &s, unsigned tag, int par, unsigned long long qu,
-                                               unsigned long long qw, unsigned long long qk, unsigned word,
+__device__ __forceinline__ void small_exchange(const DevSys &s, unsigned x, int par, unsigned long long qu,
+                                               unsigned long long qw, unsigned long long qk, unsigned word, bool flags,
                                                unsigned *xsh, bool withhold) {
-    unsigned long long *set = s.smallRec + (size_t)par * kSmallMaxTiles * 4;
-    const int lane = threadIdx.x & 31;
-    if (threadIdx.x == 0 && !withhold) {
-        unsigned long long *r = set + 4 * (size_t)blockIdx.x;
-        r[1] = qu;
-        r[2] = qw;
-        r[3] = qk;
-        st_release_u64(r, ((unsigned long long)tag << 32) | word);
-    }
-    if (threadIdx.x < 32) {
-        float m = 0.0f;
-        unsigned orw = 0u;
-        int ok = 1;
-        for (int b = lane; b < (int)gridDim.x && ok; b += 32) {
-            const unsigned long long *w = set + 4 * (size_t)b;
-            unsigned long long x = ld_acquire_u64(w);
-            int it = 0;
-            while ((unsigned)(x >> 32) != tag) {
-                if (++it > kGridSpin) {
-                    ok = 0;
-                    break;
-                }
-                __nanosleep(32);
-                x = ld_acquire_u64(w);
-            }
-            if (ok) {
-                m = fmaxf(m, __uint_as_float((unsigned)x));
-                orw |= (unsigned)x;
-            }
+    if (threadIdx.x == 0) {
+        unsigned long long *r = s.smallRec + kGridSlots * kGridSlotWords + 4 * ((size_t)par * kSmallMaxTiles + blockIdx.x);
+        if (!flags) {
+            r[1] = qu;
+            r[2] = qw;
+            r[3] = qk;
         }
-        ok = __all_sync(0xffffffffu, ok);
-        m = warp_max(m);
-        orw = __reduce_or_sync(0xffffffffu, orw);
-        if (lane == 0) {
-            xsh[0] = (unsigned)ok;
-            xsh[1] = orw;
-            xsh[2] = __float_as_uint(m);
-        }
+        unsigned m, o;
+        xsh[0] = grid_exchange(s.smallRec, x, gridDim.x, flags ? 0u : word, flags ? word : 0u, withhold, m, o);
+        xsh[1] = o;
+        xsh[2] = m;
     }
 }
 
 // Block 0, warp 1: the totals of an earlier step's records (set par), into
 // the scalars and the observable row of that step.
 __device__ __forceinline__ void small_totals(const DevSys &s, int par, float vm2, float d, int r, int row) {
-    const unsigned long long *set = s.smallRec + (size_t)par * kSmallMaxTiles * 4;
+    const unsigned long long *set = s.smallRec + kGridSlots * kGridSlotWords + (size_t)par * kSmallMaxTiles * 4;
     const int lane = threadIdx.x & 31;
     unsigned long long su = 0ull, sw = 0ull, sk = 0ull;
     for (int b = lane; b < (int)gridDim.x; b += 32) {
@@ -2337,8 +2298,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_fsmall(DevSys s, int rows,
     bool pending = false, stop = false, failed = false;
     __syncthreads();
     // one exchange: true unless a wait gave up
-    auto xchg = [&](unsigned long long qa, unsigned long long qb, unsigned long long qc, unsigned word) {
-        small_exchange(s, base + xi + 1u, (int)(xi % 3u), qa, qb, qc, word, xsh,
+    auto xchg = [&](unsigned long long qa, unsigned long long qb, unsigned long long qc, unsigned word,
+                    bool flags = true) {
+        small_exchange(s, base + xi, (int)(xi % 3u), qa, qb, qc, word, flags, xsh,
                        withhold && xi == 0 && blockIdx.x == 0);
         if (blockIdx.x == 0 && warp == 1 && pset >= 0) small_totals(s, pset, pvm, pd, pr, prow);
         __syncthreads();
@@ -2699,7 +2661,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_fsmall(DevSys s, int rows,
             if (ob) atomicOr(&sc->nonfinite, 2);
         }
         const int stepSet = (int)(xi % 3u);
-        if (!xchg(qa, qb, qc, __float_as_uint(mm))) break;
+        if (!xchg(qa, qb, qc, __float_as_uint(mm), false)) break;
         // the step's totals, the same on every block: the rebuild rule of
         // evalProps / NeighborList::update (md3dsystem.cpp:177, nn.cpp:118)
         const float vm2 = __uint_as_float(xsh[2]);
