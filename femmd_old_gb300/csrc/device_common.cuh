@@ -53,10 +53,8 @@ __device__ __forceinline__ float wrap_coord(float r, float L) { return r - floor
 // -1, 0 or 1 whatever the quotient's rounding (r < L gives a quotient of at
 // most 1 - 2^-24, r < 2 L one of at most 2 - 2^-23): the same single rounding.
 __device__ __forceinline__ float wrap_near(float r, float L) {
-    if (r >= 0.0f && r < L) return r;
-    if (r < 0.0f && r >= -L) return r + L;
-    if (r >= L && r < 2.0f * L) return r - L;
-    return wrap_coord(r, L);
+    const float w = r < 0.0f ? r + L : (r >= L ? r - L : r);
+    return (r >= -L && r < 2.0f * L) ? w : wrap_coord(r, L);
 }
 
 // cellId (femmd2D/src/nnCuda.cu:9-17): float multiply, IEEE divide, truncate;

@@ -446,6 +446,8 @@ static DevSys make_sys(femmd_ctx *c) {
     s.dt = c->dt;
     s.hdt = 0.5f * c->dt;
     s.halfSkin = 0.5 * (double)c->skin;
+    s.halfSkinF = (float)s.halfSkin;
+    if ((double)s.halfSkinF > s.halfSkin) s.halfSkinF = std::nextafterf(s.halfSkinF, -INFINITY);
     s.ncx = c->ncx;
     s.ncy = c->ncy;
     s.ncells = c->ncells;

@@ -96,6 +96,7 @@ struct DevSys {
     int wrapx, wrapy;
     float Lx, Ly, dt, hdt;
     double halfSkin;
+    float halfSkinF;  // halfSkin rounded down: d > halfSkinF is (double)d > halfSkin for every float d
     int ncx, ncy, ncells;
     float nnRadiusSq;
     int imageExact;

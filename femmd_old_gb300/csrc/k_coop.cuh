@@ -45,6 +45,7 @@
 // the exchange after that.
 #pragma once
 #include <cuda_runtime.h>
+#include <type_traits>
 #include "femmd_internal.h"
 #include "launch.h"
 #include "device_common.cuh"
@@ -235,7 +236,7 @@ struct CoopMem {
 // placing the hits.  FAST: fast_walk_ok, the image shift is the cell's; else
 // the minimum image per pair.  The first candidates of all nine cells are in
 // flight together.  Entries go to shared memory (from entry mem.rows on, to
-// the list itself).  All lanes of the warp call it; returns the list length.
+// the list itself; the others are copied there at the end of the launch).  All lanes of the warp call it; returns the list length.
 template <bool FAST>
 __device__ __forceinline__ int coop_list(const DevSys &s, const CoopMem &mem, const int *cnt, const float2 *pos, int i,
                                          int j, int col, bool valid) {
@@ -394,24 +395,27 @@ __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, co
             if (kmax > 0) atomicMax(&sc->maxCount, kmax);
             if (kmax > s.nbrCap) atomicOr(&sc->overflow, 1);
         }
-        __syncthreads();
-        // the lists' own copy (getters, the kernels that follow), a 16-byte
-        // group per store; unused words of a particle's last group are zero
-        for (int q = threadIdx.x; q < mine * kStepBlock; q += blockDim.x) {
-            const int j2 = q / kStepBlock, col = q % kStepBlock, i = (blockIdx.x + j2 * gridDim.x) * kStepBlock + col;
-            if (i >= s.N) continue;
-            const int k = min(mem.count[q], mem.rows);
-            const int *lst = mem.list + (size_t)j2 * mem.rows * kListRow + col;
-            for (int g = 0; 4 * g < k; g++) {
-                int v[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) v[u] = 4 * g + u < k ? lst[(4 * g + u) * kListRow] : 0;
-                reinterpret_cast<int4 *>(s.nbr)[(size_t)g * s.Ncap + i] = make_int4(v[0], v[1], v[2], v[3]);
-            }
-        }
     }
     __syncthreads();
     return true;
+}
+
+// The lists of the last rebuild where the getters and the kernels that follow
+// read them, a 16-byte group per store; unused words of a particle's last group
+// are zero.
+__device__ __forceinline__ void coop_write_lists(const DevSys &s, const CoopMem &mem, int tiles) {
+    for (int q = threadIdx.x; q < tiles * kStepBlock; q += blockDim.x) {
+        const int j = q / kStepBlock, col = q % kStepBlock, i = (blockIdx.x + j * gridDim.x) * kStepBlock + col;
+        if (i >= s.N) continue;
+        const int k = min(mem.count[q], mem.rows);
+        const int *lst = mem.list + (size_t)j * mem.rows * kListRow + col;
+        for (int g = 0; 4 * g < k; g++) {
+            int v[4];
+#pragma unroll
+            for (int u = 0; u < 4; u++) v[u] = 4 * g + u < k ? lst[(4 * g + u) * kListRow] : 0;
+            reinterpret_cast<int4 *>(s.nbr)[(size_t)g * s.Ncap + i] = make_int4(v[0], v[1], v[2], v[3]);
+        }
+    }
 }
 
 // The cell arrays of the last rebuild as the plain kernels leave them:
@@ -541,15 +545,22 @@ __device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &me
         if (base > 0) gather(base);
         float4 o[kQuadPairs];
         bool done = false;
-        if (SIG1 && !SG && !near) {
+        if (SIG1 && !SG) {
+            // the packed terms, with the images where a lane of the warp is
+            // near an edge; the scalar ones where they do not stand
             float far = 0.0f, close = 1.0f;
+            auto packed = [&](auto edge) {
 #pragma unroll
-            for (int u = 0; u < kQuadPairs; u++) {
-                const bool in = base + 4 * u + q < cnt;
-                const float4 e = *reinterpret_cast<const float4 *>(
-                    tab + (MT ? ti * s.numTypes + ((unsigned)tag[u] >> kIdBits) : 0));
-                o[u] = lj_terms_x2(pi, pj[u], make_float2(e.x, e.y), e.z, e.w, in, far, close);
-            }
+                for (int u = 0; u < kQuadPairs; u++) {
+                    const bool in = base + 4 * u + q < cnt;
+                    const float4 e = *reinterpret_cast<const float4 *>(
+                        tab + (MT ? ti * s.numTypes + ((unsigned)tag[u] >> kIdBits) : 0));
+                    o[u] = lj_terms_x2<decltype(edge)::value, WX, WY>(s, pi, pj[u], make_float2(e.x, e.y), e.z, e.w,
+                                                                     in, far, close);
+                }
+            };
+            if (near) packed(std::true_type{});
+            else packed(std::false_type{});
             done = !__any_sync(0xffffffffu, !lj_sums_ok<WX, WY>(s, far, close));
         }
         if (!done) {
@@ -793,7 +804,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
         int reb = 0;
         if (mode != MODE_FIRST) {
             const float d = r.dispHi + sqrtf(vm2) * s.dt;
-            reb = (double)d > s.halfSkin;
+            reb = d > s.halfSkinF;  // (double)d > halfSkin
             r.dispHi = d;
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -815,7 +826,10 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
         rebuild = mode == MODE_MID && reb;
     }
     // the cell arrays of the last rebuild; then the last sums
-    if (ok && r.updates != updates0) ok = coop_cells(s, sh, r);
+    if (ok && r.updates != updates0) {
+        coop_write_lists(s, mem, tiles);
+        ok = coop_cells(s, sh, r);
+    }
     __syncthreads();
     if (ok) ok = coop_exchange(s, sh, r, 0u, false, true);
     if (ok && blockIdx.x == 0 && warp == 2)

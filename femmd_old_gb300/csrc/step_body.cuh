@@ -360,14 +360,34 @@ __device__ __forceinline__ void lj_pair(const DevSys &s, const PairEntry *tab, c
 //     starts at +0 never is -0, so +-0 added leaves it as it is.)
 constexpr float kPairClose = 1e-30f;
 
-// The pair's terms: force x and y, doubled energy and virial.
-__device__ __forceinline__ float4 lj_terms_x2(float2 pi, float2 pj, float2 ce, float rcut2, float us, bool on,
-                                              float &far, float &close) {
-    const float2 d = __ffma2_rn(pj, make_float2(-1.0f, -1.0f), pi);
-    const float2 sq = mul2(d, d);
-    const float dr2 = sq.x + sq.y;
+// The pair's terms: force x and y, doubled energy and virial.  EDGE: the
+// minimum image is taken (lj_pair's: the reference's float one decides, and
+// inside the cutoff a crossing difference is rounded once in exact-image mode),
+// by selections; 'far' is not used.
+template <bool EDGE, bool WX, bool WY>
+__device__ __forceinline__ float4 lj_terms_x2(const DevSys &s, float2 pi, float2 pj, float2 ce, float rcut2, float us,
+                                              bool on, float &far, float &close) {
+    const float2 raw = __ffma2_rn(pj, make_float2(-1.0f, -1.0f), pi);
+    float2 d = raw;
+    if (EDGE) {
+        const float hx = 0.5f * s.Lx, hy = 0.5f * s.Ly;
+        if (WX) d.x = raw.x - (raw.x >= hx ? s.Lx : (raw.x < -hx ? -s.Lx : 0.0f));
+        if (WY) d.y = raw.y - (raw.y >= hy ? s.Ly : (raw.y < -hy ? -s.Ly : 0.0f));
+    }
+    float2 sq = mul2(d, d);
+    float dr2 = sq.x + sq.y;
+    const bool in = on && dr2 < rcut2;
+    if (EDGE && s.imageExact) {
+        // two_sum_err of p_i - p_j, added where the difference crossed
+        const bool cx = WX && (raw.x >= 0.5f * s.Lx || raw.x < -0.5f * s.Lx);
+        const bool cy = WY && (raw.y >= 0.5f * s.Ly || raw.y < -0.5f * s.Ly);
+        d.x += cx ? two_sum_err(pi.x, -pj.x, raw.x) : 0.0f;
+        d.y += cy ? two_sum_err(pi.y, -pj.y, raw.y) : 0.0f;
+        sq = mul2(d, d);
+        dr2 = sq.x + sq.y;
+    }
     if (on) {
-        far = fmaxf(far, fmaxf(fabsf(d.x), fabsf(d.y)));
+        if (!EDGE) far = fmaxf(far, fmaxf(fabsf(d.x), fabsf(d.y)));
         close = fminf(close, dr2);
     }
     float y;
@@ -376,7 +396,6 @@ __device__ __forceinline__ float4 lj_terms_x2(float2 pi, float2 pj, float2 ce, f
     const float dr6i = dr2i * dr2i * dr2i;
     const float2 r6 = make_float2(dr6i, dr6i);
     const float2 g = mul2(mul2(ce, r6), add2(r6, make_float2(-0.5f, -1.0f)));
-    const bool in = on && dr2 < rcut2;
     const float fc = in ? g.x * dr2i : 0.0f;
     const float u = in ? g.y + us : 0.0f;
     return make_float4(__fmul_rn(fc, d.x), __fmul_rn(fc, d.y), u, __fmul_rn(fc, dr2));
@@ -387,9 +406,9 @@ struct LjSums {
     float far, close;
 };
 
-__device__ __forceinline__ void lj_pair_x2(float2 pi, float2 pj, float2 ce, float rcut2, float us, bool on,
-                                           LjSums &a) {
-    const float4 t = lj_terms_x2(pi, pj, ce, rcut2, us, on, a.far, a.close);
+__device__ __forceinline__ void lj_pair_x2(const DevSys &s, float2 pi, float2 pj, float2 ce, float rcut2, float us,
+                                           bool on, LjSums &a) {
+    const float4 t = lj_terms_x2<false, false, false>(s, pi, pj, ce, rcut2, us, on, a.far, a.close);
     a.F = add2(a.F, make_float2(t.x, t.y));
     a.UW = add2(a.UW, make_float2(t.z, t.w));
 }
@@ -555,9 +574,9 @@ __device__ __forceinline__ void particle_step(const DevSys &s, const PairEntry *
                     if (MT) {
                         const float4 e =
                             *reinterpret_cast<const float4 *>(tab + ti + (on ? (unsigned)tags[u] >> kIdBits : 0u));
-                        lj_pair_x2(pi, q[u], make_float2(e.x, e.y), e.z, e.w, on, a);
+                        lj_pair_x2(s, pi, q[u], make_float2(e.x, e.y), e.z, e.w, on, a);
                     } else {
-                        lj_pair_x2(pi, q[u], make_float2(pe0.c, pe0.eps4), pe0.rcut2, pe0.us, on, a);
+                        lj_pair_x2(s, pi, q[u], make_float2(pe0.c, pe0.eps4), pe0.rcut2, pe0.us, on, a);
                     }
                 }
                 g = gn;
