@@ -215,6 +215,7 @@ struct femmd_ctx {
     DBuf<int> cellFill, cellIds;
     DBuf<float4> cellCand;
     bool runClean = false, coopOff = false;
+    bool permIdent = false;  // fast mode: the storage order is the id order
     // profiling
     bool profiling = false;
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> forceEvents;
@@ -958,6 +959,7 @@ static femmd_status upload_state(femmd_ctx *ctx) {
             Launch L;
             L.stream = s;
             CK(enqueue_perm_identity(L, ds));
+            ctx->permIdent = true;
         }
     }
     ctx->cur = 0;
@@ -1029,6 +1031,7 @@ static femmd_status size_list(femmd_ctx *ctx, int min_cap) {
     L.stream = ctx->stream;
     CK(cudaMemsetAsync(&ctx->sc.p->overflow, 0, 3 * sizeof(int), ctx->stream));
     CK(enqueue_rebuild(L, s, ctx->cur, 0));
+    ctx->permIdent = false;
     femmd_status st;
     if ((st = read_scalars(ctx))) return st;
     if (ctx->hsc->nonfinite) return fail(ctx, FEMMD_NONFINITE, "a position is NaN or infinite");
@@ -1249,7 +1252,7 @@ static femmd_status expired(femmd_ctx *ctx, const char *what) {
 // Whether runs of the context go to one cooperative launch (k_coop.cu), its
 // buffers allocated on the first of them.
 static bool coop_ready(femmd_ctx *ctx) {
-    if (fast_mode(ctx) || ctx->coopOff || !coop_size_ok((int)ctx->pos.size(), ctx->ncells)) return false;
+    if (ctx->coopOff || !coop_size_ok((int)ctx->pos.size(), ctx->ncells)) return false;
     const size_t cells = ctx->ncells;
     if (ctx->runRec.ensure(kCoopRecWords) || ctx->cellFill.ensure(2 * cells) ||
         ctx->cellIds.ensure(cells * kCellCap) || ctx->cellCand.ensure(cells * kCellCap)) {
@@ -1288,9 +1291,29 @@ static femmd_status coop_launch(femmd_ctx *ctx, int begin, int units, int end, f
 }
 
 // Whether run(n) is one cooperative launch from its run start to its last
-// step (no trajectory frame inside it, no averaging, no direct launches).
+// step (no trajectory frame inside it, no averaging, no direct launches; in
+// the fast mode, not a system of the small-system run).
 static bool coop_whole(femmd_ctx *ctx, int n) {
-    return n > 0 && !ctx->profiling && !ctx->propAvg && !(ctx->traj.on && ctx->traj.every > 0) && coop_ready(ctx);
+    if (n <= 0 || ctx->profiling || ctx->propAvg || (ctx->traj.on && ctx->traj.every > 0)) return false;
+    if (fast_mode(ctx) && small_run_fits(make_sys(ctx))) return false;
+    return coop_ready(ctx);
+}
+
+// Fast mode: the state back in id order (the whole-run launch keeps it so).
+static femmd_status to_id_order(femmd_ctx *ctx) {
+    if (!fast_mode(ctx) || ctx->permIdent) return FEMMD_OK;
+    const size_t bytes = ctx->pos.size() * sizeof(float2);
+    DevSys s = make_sys(ctx);
+    Launch L;
+    L.stream = ctx->stream;
+    float2 *state[3] = {ctx->cur ? ctx->dpos1.p : ctx->dpos0.p, ctx->dvel.p, ctx->dacc.p};
+    for (float2 *a : state) {
+        CK(enqueue_unpermute2(L, s, a, ctx->sPos.p));
+        CK(cudaMemcpyAsync(a, ctx->sPos.p, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    }
+    CK(enqueue_perm_identity(L, s));
+    ctx->permIdent = true;
+    return FEMMD_OK;
 }
 
 static femmd_status launch_units(femmd_ctx *ctx, int units, bool use_graphs) {
@@ -1298,7 +1321,7 @@ static femmd_status launch_units(femmd_ctx *ctx, int units, bool use_graphs) {
     if (use_graphs && !ctx->propAvg) {
         const DevSys s = make_sys(ctx);
         if (small_run_fits(s)) return small_units(ctx, s, units);
-        if (coop_ready(ctx)) return coop_launch(ctx, 0, units, 0, nullptr);
+        if (!fast_mode(ctx) && coop_ready(ctx)) return coop_launch(ctx, 0, units, 0, nullptr);
     }
     if (!use_graphs) {
         DevSys s = make_sys(ctx);
@@ -2362,12 +2385,14 @@ femmd_status femmd_run(femmd_ctx *ctx, int steps) {
         const float2 *pc = ctx->cur ? ctx->dpos1.p : ctx->dpos0.p;
         int cur0 = ctx->cur;
         const bool whole = coop_whole(ctx, steps);
+        if (whole && (st = to_id_order(ctx))) return st;
+        ctx->permIdent = whole;
         if (!whole) {
             CK(cudaMemcpyAsync(ctx->ckPos.p, pc, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
             CK(cudaMemcpyAsync(ctx->ckVel.p, ctx->dvel.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
             CK(cudaMemcpyAsync(ctx->ckAcc.p, ctx->dacc.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
         }
-        if (fast_mode(ctx))
+        if (fast_mode(ctx) && !whole)
             CK(cudaMemcpyAsync(ctx->ckPerm.p, ctx->perm.p, N * sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
         if (ctx->propAvg)
             CK(cudaMemcpyAsync(ctx->propsCk.p, ctx->props.p, sizeof(DevProps), cudaMemcpyDeviceToDevice, ctx->stream));
@@ -2402,7 +2427,7 @@ femmd_status femmd_run(femmd_ctx *ctx, int steps) {
         CK(cudaMemcpyAsync(pd, ctx->ckPos.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
         CK(cudaMemcpyAsync(ctx->dvel.p, ctx->ckVel.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
         CK(cudaMemcpyAsync(ctx->dacc.p, ctx->ckAcc.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, ctx->stream));
-        if (fast_mode(ctx)) {
+        if (fast_mode(ctx) && !whole) {
             // the checkpoint's storage order and the constants in that order
             CK(cudaMemcpyAsync(ctx->perm.p, ctx->ckPerm.p, N * sizeof(int), cudaMemcpyDeviceToDevice, ctx->stream));
             DevSys ds = make_sys(ctx);
@@ -2434,6 +2459,7 @@ femmd_status femmd_do_step(femmd_ctx *ctx) {
     CK(cudaMemsetAsync(&ctx->sc.p->overflow, 0, 3 * sizeof(int), ctx->stream));
     CK(enqueue_drift(L, s, ctx->cur));
     ctx->cur ^= 1;
+    ctx->permIdent = false;
     CK(enqueue_rebuild(L, s, ctx->cur, 1));
     CK(enqueue_step(L, s, MODE_LAST, ctx->cur, 0, 0));
     if (ctx->propAvg) CK(enqueue_step_props(ctx, L, s, ctx->cur));
@@ -2457,6 +2483,7 @@ femmd_status femmd_build_neighbor_list(femmd_ctx *ctx) {
         Launch L;
         L.stream = ctx->stream;
         CK(cudaMemsetAsync(&ctx->sc.p->overflow, 0, 3 * sizeof(int), ctx->stream));  // overflow, nonfinite, outside
+        ctx->permIdent = false;
         CK(enqueue_rebuild(L, s, ctx->cur, 0));
         if ((st = read_scalars(ctx))) return st;
         if (ctx->hsc->nonfinite) return fail(ctx, FEMMD_NONFINITE, "a position is NaN or infinite");

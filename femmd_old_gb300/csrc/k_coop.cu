@@ -17,6 +17,7 @@ namespace {
 constexpr int kCoopMaxN = 98304;
 
 const void *coop_kernel(const DevSys &s) {
+    if (s.fast) return coop_kernel_fast(s);
     if (!s.sigmaByType) return coop_kernel_sigma(s);
     return s.numTypes > 1 ? coop_kernel_types(s) : coop_kernel_one(s);
 }
@@ -37,7 +38,7 @@ bool coop_shape(const DevSys &s, int &grid, size_t &smem, CoopArgs &a) {
     grid = std::max(1, std::min(std::min(sms, kCoopMaxBlocks), std::max(ntiles, ntt)));
     const int per = (ntiles + grid - 1) / grid, tper = (ntt + grid - 1) / grid;
     if (per > kCoopMaxTiles || tper > kCoopMaxTiles) return false;
-    smem = 4 * (size_t)kTermComp * sizeof(float) + (size_t)per * 4 * kStepBlock * sizeof(int);  // terms, sums, counts
+    smem = coop_terms(s.fast) * (size_t)kTermComp * sizeof(float) + (size_t)per * 4 * kStepBlock * sizeof(int);  // terms, sums, counts
     const size_t inc = (size_t)per * kIncWords * kStepBlock * sizeof(int), tri = (size_t)tper * kTriTile * sizeof(int4);
     const size_t row = 4 * (size_t)per * kListRow * sizeof(int);  // four list rows
     a.incStaged = s.nBonded > 0 && smem + inc + row <= kCoopSmem;
@@ -52,7 +53,7 @@ bool coop_shape(const DevSys &s, int &grid, size_t &smem, CoopArgs &a) {
 }  // namespace
 
 bool coop_run_fits(const DevSys &s) {
-    if (s.fast || s.areaUnits > 0 || s.trace || !s.cellCand || s.N <= 0) return false;
+    if ((s.fast && !s.sigmaByType) || s.areaUnits > 0 || s.trace || !s.cellCand || s.N <= 0) return false;
     int grid, resident = 0;
     size_t smem;
     CoopArgs a = {};

@@ -1,5 +1,5 @@
 // k_coop.cuh -- a whole run of a small or medium system in one cooperative
-// launch (reference-exact force mode).
+// launch (both force modes).
 //
 // One graph unit of the plain path (step kernel, conditional rebuild) costs
 // 15-25 us whatever the system's size: launches, the IF node, and the drain
@@ -37,6 +37,15 @@
 // any order.  Positions, velocities, forces, energies and rebuild steps are
 // therefore the plain path's bit for bit.
 //
+// FAST: the fast force mode's arithmetic (k_fast.cu) instead, bit for bit as
+// to positions, velocities and forces.  Its pair sums run over the even and the
+// odd list entries apart (one type: the two lanes of fast_pairs_x2) or in list
+// order (several types: fast_pairs) by fused multiply-adds, so a lane puts a
+// pair's factors into shared memory and the sums are formed there.  The
+// launch keeps the particles in id order: the lists' order does not depend on
+// the storage order, and it leaves lists without windows behind (storage
+// slots, padded with the ghost's).
+//
 // Exchanges are grid_exchange's (grid_sync.cuh), bounded: a wait that gives
 // up sets the timeout flag, and the block leaves the kernel.  They are numbered
 // over the life of the context (DevScalars::runTag).  A step's energy sums go
@@ -49,6 +58,7 @@
 #include "femmd_internal.h"
 #include "launch.h"
 #include "device_common.cuh"
+#include "fast_body.cuh"
 #include "grid_sync.cuh"
 #include "nn_body.cuh"
 #include "step_body.cuh"
@@ -73,6 +83,8 @@ constexpr int kQuadRows = 4 * kQuadPairs;    // entries per particle and round
 // a quad writes together, and the four components it reads together, into
 // different banks.
 constexpr int kTermRow = kStepBlock + 8, kTermComp = kQuadRows * kTermRow + 8;
+// components of a term: the four sums' own, or the fast mode's factors
+__host__ __device__ constexpr int coop_terms(bool fast) { return fast ? 6 : 4; }
 constexpr int kListRow = kStepBlock + 8;     // a list row in shared memory (padded as kTermRow)
 
 // Loads that stay where they are written, ahead of what uses them (a plain
@@ -402,7 +414,10 @@ __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, co
 
 // The lists of the last rebuild where the getters and the kernels that follow
 // read them, a 16-byte group per store; unused words of a particle's last group
-// are zero.
+// are zero (FAST: the ghost slot's number; and the records of the step blocks,
+// which are kStepBlock slots each, say that they have no window and how many
+// groups their longest list has).
+template <bool FAST>
 __device__ __forceinline__ void coop_write_lists(const DevSys &s, const CoopMem &mem, int tiles) {
     for (int q = threadIdx.x; q < tiles * kStepBlock; q += blockDim.x) {
         const int j = q / kStepBlock, col = q % kStepBlock, i = (blockIdx.x + j * gridDim.x) * kStepBlock + col;
@@ -412,8 +427,24 @@ __device__ __forceinline__ void coop_write_lists(const DevSys &s, const CoopMem 
         for (int g = 0; 4 * g < k; g++) {
             int v[4];
 #pragma unroll
-            for (int u = 0; u < 4; u++) v[u] = 4 * g + u < k ? lst[(4 * g + u) * kListRow] : 0;
+            for (int u = 0; u < 4; u++) v[u] = 4 * g + u < k ? lst[(4 * g + u) * kListRow] : (FAST ? s.N : 0);
             reinterpret_cast<int4 *>(s.nbr)[(size_t)g * s.Ncap + i] = make_int4(v[0], v[1], v[2], v[3]);
+        }
+        const int all = mem.count[q];
+        if (FAST && all > mem.rows)
+            for (int e = all; e & 3; e++) s.nbr[nbr_at(e, i, s.Ncap)] = s.N;
+    }
+    if (FAST) {
+        static_assert(kStepBlock == kFastBlock, "a tile is a step block");
+        const int lane = threadIdx.x & 31;
+        for (int j = threadIdx.x >> 5; j < tiles; j += blockDim.x >> 5) {
+            const int b = blockIdx.x + j * gridDim.x;
+            int most = 0;
+            for (int c = lane; c < kStepBlock; c += 32)
+                if (b * kStepBlock + c < s.N) most = max(most, mem.count[j * kStepBlock + c]);
+            most = __reduce_max_sync(0xffffffffu, most);
+            int *w = s.blockWin + kWinInts * (size_t)b;
+            for (int c = lane; c < kWinInts; c += 32) w[c] = c == kWLen ? -1 : (c == kWGroups ? (most + 3) >> 2 : 0);
         }
     }
 }
@@ -471,10 +502,150 @@ __device__ __forceinline__ float4 coop_pair(const DevSys &s, const PairEntry *ta
     return o;
 }
 
+// finish_particle (FAST: fast_finish), an axis per lane (lanes 2 and 3 along
+// with 0 and 1).  f: lanes 0 and 1, the axis' force; e2: lanes 2 and 3, the
+// doubled energy and virial.
+template <bool WX, bool WY, bool FAST>
+__device__ __forceinline__ void coop_finish(const DevSys &s, const CoopMem &mem, int i, bool on, int j, int col, int q,
+                                            int mode, int stepNow, float2 pi, float m, float2 v2, float f, float e2,
+                                            float uwall, float2 *pout, float2 *slot, float &vvm, bool &bad) {
+    const bool y = q & 1;
+    float e = e2 * 0.5f;
+    if (q == 2) e += uwall;
+    if (s.wallOn && on) {
+        const float yw = wall_y(s, stepNow);
+        const float dl = s.wallDelta[i];
+        const float ht = (pi.y + dl) - yw;
+        if (ht > 0.0f) {
+            if (q == 1) f -= s.wallK * ht;
+            if (q == 2) e += 0.5f * s.wallK * ht * ht;
+        }
+        const float hb = dl - pi.y;
+        if (hb > 0.0f) {
+            if (q == 1) f += s.wallK * hb;
+            if (q == 2) e += 0.5f * s.wallK * hb * hb;
+        }
+    }
+    bad = bad || (on && !isfinite(f));
+    const float a = FAST ? f * rcp_approx(m) : f / m;
+    float v = y ? v2.y : v2.x, vv = 0.0f;
+    if (mode != MODE_FIRST) {
+        v = FAST ? __fmaf_rn(s.hdt, a, v) : v + s.hdt * a;
+        const float sq = v * v, other = __shfl_xor_sync(0xffffffffu, sq, 1);
+        vv = sq + other;
+        if (FAST) {
+            vv = __fmaf_rn(v, v, other);  // on the lanes of the x axis
+            vv = __shfl_sync(0xffffffffu, vv, threadIdx.x & 30);
+        }
+    }
+    float *part = mem.part + (size_t)j * 3 * kStepBlock + col;
+    if (q == 2) part[0] = on ? e : 0.0f;
+    if (q == 3) part[kStepBlock] = on ? e : 0.0f;
+    if (q == 0) part[2 * kStepBlock] = on ? m * vv : 0.0f;
+    if (on && q < 2) {
+        vvm = fmaxf(vvm, vv);
+        float *vel = reinterpret_cast<float *>(s.vel + i) + q;
+        if (mode == MODE_LAST) {
+            *vel = v;
+            reinterpret_cast<float *>(s.acc + i)[q] = a;
+            reinterpret_cast<float *>(s.forceOut + i)[q] = f;
+        } else {
+            const float p = y ? pi.y : pi.x, L = y ? s.Ly : s.Lx;
+            v = FAST ? __fmaf_rn(s.hdt, a, v) : v + s.hdt * a;
+            float x = FAST ? __fmaf_rn(s.dt, v, p) : p + s.dt * v;
+            if (y ? WY : WX) x = FAST ? fast_wrap(x, L) : wrap_near(x, L);
+            reinterpret_cast<float *>(pout + i)[q] = x;
+            *vel = v;
+            if (slot) reinterpret_cast<float *>(slot + i)[q] = x;
+        }
+    }
+}
+
+// The pair sums of the fast mode and the rest of the step.  Components of the
+// terms: one type fc, dx, dy, ir6, ir2, r2; several types fc, dx, dy, u, r2.
+// Lane 0 forms sum fc dx, lane 1 sum fc dy; one type: lane 2 sum ir6^2 and sum
+// ir6, lane 3 sum ir2 r2 (the pairs inside the cutoff), each over the even and
+// the odd entries apart; several types: lane 2 sum u, lane 3 sum fc r2.
+template <bool MT, bool WX, bool WY, bool SIG1, class Gather>
+__device__ __forceinline__ void fast_sums(const DevSys &s, const CoopMem &mem, const PairEntry *tab, Gather &gather,
+                                          int most, int cnt, int q, int col, int ti, const int *tag, const float2 *pj,
+                                          float2 pi, bool near, float fx, float fy, float ue, float uwall, float m,
+                                          float2 v2, int i, bool on, int j, int mode, int stepNow, float2 *pout,
+                                          float2 *slot, float &vvm, bool &bad) {
+    const int ca = MT ? (q == 2 ? 3 : 0) : (q < 2 ? 0 : q + 1);
+    const int cb = q < 2 ? q + 1 : (MT ? 4 : (q == 2 ? 3 : 5));
+    const float *pa = mem.term + ca * kTermComp + col, *pb = mem.term + cb * kTermComp + col;
+    float s0 = MT ? (q == 0 ? fx : (q == 1 ? fy : 0.0f)) : 0.0f, s1 = 0.0f, t0 = 0.0f, t1 = 0.0f;
+    const PairEntry pe0 = tab[0];
+    for (int base = 0; base < most; base += kQuadRows) {
+        if (base > 0) gather(base);
+#pragma unroll
+        for (int u = 0; u < kQuadPairs; u++) {
+            const PairEntry pe = MT ? tab[ti * s.numTypes + ((unsigned)tag[u] >> kIdBits)] : pe0;
+            float dx, dy;
+            if (near) {
+                dx = fdiff<WX, true>(pi.x, pj[u].x, s.Lx);
+                dy = fdiff<WY, true>(pi.y, pj[u].y, s.Ly);
+            } else {
+                dx = pi.x - pj[u].x;
+                dy = pi.y - pj[u].y;
+            }
+            const float r2 = __fmaf_rn(dx, dx, __fmul_rn(dy, dy));
+            const bool in = base + 4 * u + q < cnt && r2 < pe.rcut2;
+            const float ir2 = in ? ((SIG1 && !MT) ? rcp_approx(r2) : pe.sig2 * rcp_approx(r2)) : 0.0f;
+            const float ir4 = ir2 * ir2, ir6 = ir4 * ir2, ir8 = ir4 * ir4;
+            const float fc = ir8 * __fmaf_rn(pe.c, ir6, -0.5f * pe.c);
+            float *w = mem.term + (4 * u + q) * kTermRow + col;
+            w[0] = fc;
+            w[kTermComp] = dx;
+            w[2 * kTermComp] = dy;
+            if (MT) {
+                w[3 * kTermComp] = in ? __fmaf_rn(pe.eps4, __fmaf_rn(ir6, ir6, -ir6), pe.us) : 0.0f;
+                w[4 * kTermComp] = r2;
+            } else {
+                w[3 * kTermComp] = ir6;
+                w[4 * kTermComp] = ir2;
+                w[5 * kTermComp] = r2;
+            }
+        }
+        __syncwarp();
+        const int rows = (min(most - base, kQuadRows) + 1) & ~1;
+        if (MT) {
+#pragma unroll 4
+            for (int k = 0; k < rows; k++) s0 = __fmaf_rn(pa[k * kTermRow], q == 2 ? 1.0f : pb[k * kTermRow], s0);
+        } else {
+#pragma unroll 4
+            for (int k = 0; k < rows; k += 2) {
+                const float a0 = pa[k * kTermRow], a1 = pa[(k + 1) * kTermRow];
+                s0 = __fmaf_rn(a0, pb[k * kTermRow], s0);
+                s1 = __fmaf_rn(a1, pb[(k + 1) * kTermRow], s1);
+                t0 += a0;
+                t1 += a1;
+            }
+        }
+        __syncwarp();
+    }
+    float f = 0.0f, e2;
+    if (MT) {
+        if (q < 2) f = s0;
+        e2 = q == 2 ? ue + s0 : s0;
+    } else {
+        const float S = s0 + s1, T = t0 + t1;
+        const int lane = threadIdx.x & 31, l2 = (lane & ~3) + 2;
+        const float A = __shfl_sync(0xffffffffu, S, l2), B = __shfl_sync(0xffffffffu, T, l2);
+        float n = __shfl_sync(0xffffffffu, S, l2 + 1);
+        if (!SIG1) n = n / pe0.sig2;
+        if (q == 0) f = fx + S;
+        if (q == 1) f = fy + S;
+        e2 = q == 2 ? ue + __fmaf_rn(pe0.eps4, A - B, pe0.us * n) : pe0.eps48 * __fmaf_rn(-0.5f, B, A);
+    }
+    coop_finish<WX, WY, true>(s, mem, i, on, j, col, q, mode, stepNow, pi, m, v2, f, e2, uwall, pout, slot, vvm, bad);
+}
+
 // particle_step for one particle by the four lanes of a quad (lane 'q' of 0 ..
 // 3; particle i, slot 'col' of the block's tile j; on: i < N).  All lanes of
 // the warp call it.
-template <bool MT, bool SG, bool WX, bool WY, bool SIG1>
+template <bool MT, bool SG, bool WX, bool WY, bool SIG1, bool FAST>
 __device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &mem, const PairEntry *tab, int i, bool on,
                                               int j, int col, int q, int mode, int stepNow, const float2 *pin,
                                               float2 *pout, float2 *slot, float &vvm, bool &bad) {
@@ -537,10 +708,15 @@ __device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &me
     } else if (on) {
         bonded_forces<WX, WY, false>(s, i, mode, pin, pi, fx, fy, ue, utri, uwall);
     }
+    const bool near = __any_sync(0xffffffffu, on && near_edge<WX, WY>(s, pi));
+    if constexpr (FAST) {
+        fast_sums<MT, WX, WY, SIG1>(s, mem, tab, gather, most, cnt, q, col, ti, tag, pj, pi, near, fx, fy, ue, uwall,
+                                    m, v2, i, on, j, mode, stepNow, pout, slot, vvm, bad);
+        return;
+    }
     // the pairs: the lane's sum is force x, force y, energy or virial
     float sum = q == 0 ? fx : (q == 1 ? fy : (q == 2 ? ue : 0.0f));
     const float *mine = mem.term + q * kTermComp + col;
-    const bool near = __any_sync(0xffffffffu, on && near_edge<WX, WY>(s, pi));
     for (int base = 0; base < most; base += kQuadRows) {
         if (base > 0) gather(base);
         float4 o[kQuadPairs];
@@ -586,53 +762,8 @@ __device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &me
         for (int k = 0; k < rows; k++) sum += mine[k * kTermRow];
         __syncwarp();
     }
-    // finish_particle, an axis per lane (lanes 2 and 3 along with 0 and 1)
-    const bool y = q & 1;
-    float f = sum, e = sum * 0.5f;
-    if (q >= 2) f = 0.0f;
-    if (q == 2) e += uwall;
-    if (s.wallOn && on) {
-        const float yw = wall_y(s, stepNow);
-        const float dl = s.wallDelta[i];
-        const float ht = (pi.y + dl) - yw;
-        if (ht > 0.0f) {
-            if (q == 1) f -= s.wallK * ht;
-            if (q == 2) e += 0.5f * s.wallK * ht * ht;
-        }
-        const float hb = dl - pi.y;
-        if (hb > 0.0f) {
-            if (q == 1) f += s.wallK * hb;
-            if (q == 2) e += 0.5f * s.wallK * hb * hb;
-        }
-    }
-    bad = bad || (on && !isfinite(f));
-    const float a = f / m;
-    float v = y ? v2.y : v2.x, vv = 0.0f;
-    if (mode != MODE_FIRST) {
-        v += s.hdt * a;
-        const float sq = v * v;
-        vv = sq + __shfl_xor_sync(0xffffffffu, sq, 1);
-    }
-    float *part = mem.part + (size_t)j * 3 * kStepBlock + col;
-    if (q == 2) part[0] = on ? e : 0.0f;
-    if (q == 3) part[kStepBlock] = on ? e : 0.0f;
-    if (q == 0) part[2 * kStepBlock] = on ? m * vv : 0.0f;
-    if (on && q < 2) {
-        vvm = fmaxf(vvm, vv);
-        float *vel = reinterpret_cast<float *>(s.vel + i) + q;
-        if (mode == MODE_LAST) {
-            *vel = v;
-            reinterpret_cast<float *>(s.acc + i)[q] = a;
-            reinterpret_cast<float *>(s.forceOut + i)[q] = f;
-        } else {
-            v += s.hdt * a;
-            float x = (y ? pi.y : pi.x) + s.dt * v;
-            if (y ? WY : WX) x = wrap_near(x, y ? s.Ly : s.Lx);
-            reinterpret_cast<float *>(pout + i)[q] = x;
-            *vel = v;
-            if (slot) reinterpret_cast<float *>(slot + i)[q] = x;
-        }
-    }
+    coop_finish<WX, WY, false>(s, mem, i, on, j, col, q, mode, stepNow, pi, m, v2, q < 2 ? sum : 0.0f, sum, uwall, pout,
+                               slot, vvm, bad);
 }
 
 // One warp: the block's energy sums of a step.  A tile's 128 particles in the
@@ -670,7 +801,7 @@ __device__ __forceinline__ void coop_block_sums(const DevSys &s, CoopShared &sh,
 // then 'units' middle steps, each followed by its rebuild when the half-skin
 // rule calls for one; with 'end', the last step.  slots: when not null, the
 // positions after drift u go to slots + (u + 1) N too.
-template <bool MT, bool SG, bool WX, bool WY, bool SIG1>
+template <bool MT, bool SG, bool WX, bool WY, bool SIG1, bool FAST>
 __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) {
     extern __shared__ int4 dyn[];
     __shared__ CoopShared sh;
@@ -702,7 +833,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
     mem.rows = a.rows;
     mem.tri = a.triStaged ? dyn : nullptr;
     mem.term = reinterpret_cast<float *>(dyn + (a.triStaged ? tper * kTriTile : 0));
-    mem.part = mem.term + 4 * kTermComp;
+    mem.part = mem.term + coop_terms(FAST) * kTermComp;
     mem.count = reinterpret_cast<int *>(mem.part + (size_t)per * 3 * kStepBlock);
     mem.inc = a.incStaged ? mem.count + per * kStepBlock : nullptr;
     mem.list = mem.count + per * kStepBlock + (a.incStaged ? per * kIncWords * kStepBlock : 0);
@@ -776,7 +907,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
         bool bad = false;
         for (int j = 0; j < tiles; j++) {
             const int col = threadIdx.x >> 2, i = (blockIdx.x + j * gridDim.x) * kStepBlock + col;
-            coop_particle<MT, SG, WX, WY, SIG1>(s, mem, sh.tab, i, i < s.N, j, col, threadIdx.x & 3, mode, r.stepNow,
+            coop_particle<MT, SG, WX, WY, SIG1, FAST>(s, mem, sh.tab, i, i < s.N, j, col, threadIdx.x & 3, mode, r.stepNow,
                                                 pin, pout, a.slots ? a.slots + (size_t)(u + 1) * s.N : nullptr, vvm,
                                                 bad);
         }
@@ -827,7 +958,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
     }
     // the cell arrays of the last rebuild; then the last sums
     if (ok && r.updates != updates0) {
-        coop_write_lists(s, mem, tiles);
+        coop_write_lists<FAST>(s, mem, tiles);
         ok = coop_cells(s, sh, r);
     }
     __syncthreads();
@@ -844,25 +975,27 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
     }
 }
 
-// The kernel of a system with (MT) several types and (SG) a sigma per particle.
-template <bool MT, bool SG, bool WX, bool WY>
+// The kernel of a system with (MT) several types and (SG) a sigma per
+// particle, in the fast mode or not.
+template <bool MT, bool SG, bool WX, bool WY, bool FAST>
 const void *coop_sig(const DevSys &s) {
-    if constexpr (!SG) {
-        if (s.sigmaOne) return (const void *)k_coop<MT, SG, WX, WY, true>;
+    if constexpr (!SG && !(FAST && MT)) {
+        if (s.sigmaOne) return (const void *)k_coop<MT, SG, WX, WY, true, FAST>;
     }
-    return (const void *)k_coop<MT, SG, WX, WY, false>;
+    return (const void *)k_coop<MT, SG, WX, WY, false, FAST>;
 }
 
-template <bool MT, bool SG>
+template <bool MT, bool SG, bool FAST = false>
 const void *coop_image(const DevSys &s) {
-    if (s.wrapx && s.wrapy) return coop_sig<MT, SG, true, true>(s);
-    if (s.wrapx) return coop_sig<MT, SG, true, false>(s);
-    return coop_sig<MT, SG, false, false>(s);
+    if (s.wrapx && s.wrapy) return coop_sig<MT, SG, true, true, FAST>(s);
+    if (s.wrapx) return coop_sig<MT, SG, true, false, FAST>(s);
+    return coop_sig<MT, SG, false, false, FAST>(s);
 }
 
 // one translation unit each
 const void *coop_kernel_one(const DevSys &s);    // k_coop.cu
 const void *coop_kernel_types(const DevSys &s);  // k_coop_types.cu
 const void *coop_kernel_sigma(const DevSys &s);  // k_coop_sigma.cu
+const void *coop_kernel_fast(const DevSys &s);   // k_coop_fast.cu
 
 }  // namespace femmd

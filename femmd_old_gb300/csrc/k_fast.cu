@@ -38,6 +38,7 @@
 #include "femmd_internal.h"
 #include "launch.h"
 #include "device_common.cuh"
+#include "fast_body.cuh"
 #include "grid_sync.cuh"
 #include "nn_body.cuh"
 #include "step_body.cuh"
@@ -866,26 +867,6 @@ cudaError_t enqueue_rebuild_fast(Launch &L, const DevSys &s, int parity, int che
 
 // ============================================================ step kernel
 
-__device__ __forceinline__ float rcp_approx(float x) {
-    float r;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
-// The pair difference on one axis.  IMG: the particle lies within imgD of
-// a periodic edge, so an interacting pair may cross it: a difference of
-// more than half the box is moved by one box length, rounded once from its
-// exact value.
-template <bool WRAP, bool IMG>
-__device__ __forceinline__ float fdiff(float a, float b, float L) {
-    float d = a - b;
-    if (WRAP && IMG && fabsf(d) > 0.5f * L) {
-        const float sh = d > 0.0f ? L : -L;
-        d = (d - sh) + two_sum_err(a, -b, d);
-    }
-    return d;
-}
-
 // One Lennard-Jones pair of particle i (type ti, sigma si) with neighbour
 // position q, tag/type tj and sigma sj, added into the running sums.  The
 // cutoff test selects the terms (no branch per pair).  One type with sigma
@@ -1100,16 +1081,6 @@ __device__ __forceinline__ void fast_pairs_x2(const DevSys &s, const PairEntry &
     const float n = SIG1 ? Nv.x + Nv.y : (Nv.x + Nv.y) / pe.sig2;
     ue2 += __fmaf_rn(pe.eps4, A - B, pe.us * n);
     we2 += pe.eps48 * __fmaf_rn(-0.5f, B, A);
-}
-
-// x wrapped into [0, L): one box length added or taken away, the reference's
-// r - floor(r/L) L for every |r| < 2L (the same single rounding), the full
-// expression beyond.
-__device__ __forceinline__ float fast_wrap(float x, float L) {
-    if (x < 0.0f) x += L;
-    else if (x >= L) x -= L;
-    if (!(x >= 0.0f && x < L)) x = wrap_coord(x, L);
-    return x;
 }
 
 // The rest of particle i's step in the fast mode: finish_particle with the

@@ -77,6 +77,68 @@ def test_one_launch_equals_plain_kernels(name):
         assert np.array_equal(np.ascontiguousarray(a).view(np.uint8), np.ascontiguousarray(b).view(np.uint8))
 
 
+def rows_as_sets(start, lst):
+    rows = np.repeat(np.arange(len(start) - 1), np.diff(start))
+    return lst[np.lexsort((lst, rows))]
+
+
+FAST_SCENES = {
+    "one_type": lambda: ragged_fluid(16385),
+    "one_type_sigma": lambda: resized(ragged_fluid(17003, density=0.75), 1.1),
+    "x_periodic": lambda: ragged_fluid(1500, density=0.6, pbc=1),
+    "walls": lambda: ragged_fluid(700, density=0.6, pbc=0),
+    "two_types": lambda: ragged_fluid(2300, types=2),
+    "disks": lambda: S.suspension(n_side=9, T=0.5),
+    "mixed": lambda: S.large_mixed(n_side=5, n_solvent=7001),
+}
+
+
+def resized(sc, sigma):
+    """Every sigma and length of a scene's fluid scaled by 'sigma'."""
+    def call(name, a):
+        if name == "init":
+            return name, (a[0] * sigma, a[1] * sigma)
+        if name == "add_particles":
+            return name, (a[0] * sigma, a[1] * sigma, *a[2:5], a[5] * sigma, a[6])
+        return name, a
+    sc.calls = [call(n, a) for n, a in sc.calls]
+    return sc
+
+
+@pytest.mark.parametrize("name", FAST_SCENES)
+def test_fast_mode_one_launch_equals_its_kernels(name):
+    """The fast mode's whole-run launch against its step and rebuild kernels:
+    state, forces, largest speeds, rebuilds and cells bit for bit, neighbour
+    sets equal.  The energies are sums of the same single-precision terms in
+    other groups: each group adds at most 128 terms one by one or 64 sums of
+    such groups, so a total is within 192 * 2^-24 = 1.2e-5 of the sum of its
+    terms' magnitudes, for which the particles' own |energy| bound stands in."""
+    sc = FAST_SCENES[name]()
+    systems = []
+    for direct in (False, True):
+        s = F.System()
+        s.set_force_mode(1)
+        sc.replay(s)
+        s.set_profiling(direct)
+        systems.append(s)
+    for n in (1, 2, 33, 20):
+        got = []
+        for s in systems:
+            s.run(n)
+            st, lst = s.neighbors()
+            got.append(dict(exact=[*s.get_state(), s.forces(), s.step_observables()[:, 3:], *s.cells(), st,
+                                   rows_as_sets(st, lst)], obs=s.step_observables(), updates=s.total_updates()))
+        for a, b in zip(got[0]["exact"], got[1]["exact"]):
+            assert np.array_equal(np.ascontiguousarray(a).view(np.uint8), np.ascontiguousarray(b).view(np.uint8))
+        assert got[0]["updates"] == got[1]["updates"]
+        for s in systems:
+            s.calc_forces()  # over the lists that the run left behind
+        fa, fb = (s.forces() for s in systems)
+        assert np.array_equal(fa.view(np.uint32), fb.view(np.uint32))
+        scale = max(np.abs(systems[0].particle_energies()).sum(), np.abs(got[0]["obs"][:, :3]).max())
+        assert np.abs(got[0]["obs"][:, :3] - got[1]["obs"][:, :3]).max() <= 1.2e-5 * scale
+
+
 def test_list_overflow_repeats_the_run():
     """Lists outgrown inside the launch: the run is rolled back and repeated."""
     sc = ragged_fluid(3000)
