@@ -167,7 +167,7 @@ struct femmd_ctx {
     int cur = 0;
     int nbrCap = 0, Ncap = 0, nBonded = 0, sigmaByType = 1, sigmaOne = 0;
     DBuf<float2> dpos0, dpos1, dvel, dacc, dforce, dref, ckPos, ckVel, ckAcc, triF, triLame;
-    DBuf<float> dmass, dsigma, denergy, triE, wallDelta, wallSig;
+    DBuf<float> dmass, dsigma, denergy, triE, triTmp, wallDelta, wallSig;
     bool ownMaterial = false, materialDirty = false;
     // area springs: kept positions and the per-mesh work list
     DBuf<float2> posPre;
@@ -190,7 +190,7 @@ struct femmd_ctx {
     DBuf<DevProps> props, propsCk;
     DBuf<double> propPart;
     DBuf<int> dtype, dexcl, cellOf, rank, cellCount, cellStart, blockSums, unsorted, sortedIds, nbr, nbrCount, bStart, tStart,
-        tEnt;
+        tEnt, triOfs, triOwn, triLoc;
     DBuf<int2> bEnt;
     DBuf<int4> triIdx;
     DBuf<float4> triGeo, cellSorted;
@@ -215,6 +215,7 @@ struct femmd_ctx {
     DBuf<int> cellFill, cellIds;
     DBuf<float4> cellCand;
     bool runClean = false, coopOff = false;
+    int triGrid = 0, triMost = 0;  // coop_plan: made for this many blocks (0: not made), CoopArgs::triMost
     bool permIdent = false;  // fast mode: the storage order is the id order
     // profiling
     bool profiling = false;
@@ -345,6 +346,7 @@ static void release_device(femmd_ctx *c) {
     c->dpos0.release(); c->dpos1.release(); c->dvel.release(); c->dacc.release(); c->dforce.release();
     c->dref.release(); c->ckPos.release(); c->ckVel.release(); c->ckAcc.release(); c->triF.release();
     c->dmass.release(); c->dsigma.release(); c->denergy.release(); c->triE.release();
+    c->triTmp.release(); c->triOfs.release(); c->triOwn.release(); c->triLoc.release();
     c->dtype.release(); c->dexcl.release(); c->cellOf.release(); c->rank.release(); c->cellCount.release();
     c->cellStart.release(); c->blockSums.release(); c->sortedIds.release(); c->unsorted.release(); c->nbr.release();
     c->nbrCount.release(); c->bStart.release(); c->tStart.release(); c->tEnt.release(); c->bEnt.release();
@@ -829,6 +831,7 @@ static femmd_status upload_topology(femmd_ctx *ctx) {
     CK(ctx->blockSums.ensure(scan_blocks(ctx->ncells)));
     CK(ctx->sc.ensure(1));
     ctx->runClean = ctx->coopOff = false;
+    ctx->triGrid = 0;
     cudaStream_t s = ctx->stream;
     if (N > 0) {
         CK(cudaMemcpyAsync(ctx->dmass.p, ctx->mass.data(), N * sizeof(float), cudaMemcpyHostToDevice, s));
@@ -1249,6 +1252,62 @@ static femmd_status expired(femmd_ctx *ctx, const char *what) {
     return fail(ctx, FEMMD_TIMEOUT, "a bounded device wait expired (%s)", what);
 }
 
+// The triangles by block of the whole-run launch (CoopArgs), laid out once per
+// topology; without where a particle has more incidences than the launch keeps
+// at hand (then, and where they do not fit its shared memory, the triangle pass
+// is a phase of its own with an exchange after it).
+static CoopArgs coop_plan(femmd_ctx *ctx, const DevSys &s) {
+    CoopArgs a = {};
+    const int nt = (int)ctx->refVol.size(), N = (int)ctx->pos.size(), grid = coop_grid(s);
+    if (nt == 0 || grid == 0) return a;
+    if (ctx->triGrid != grid) {
+        ctx->triGrid = grid;
+        ctx->triMost = 0;
+        const int ntiles = (N + kStepBlock - 1) / kStepBlock, nbd = ctx->nBonded;
+        std::vector<int> start(nbd + 1, 0), bonds(nbd, 0);
+        for (int v : ctx->tri) start[v + 1]++;
+        for (int v : ctx->bond) bonds[v]++;
+        for (int v = 0; v < nbd; v++) {
+            if (start[v + 1] > kCoopIncTri || bonds[v] > kCoopIncBond) return a;
+            start[v + 1] += start[v];
+        }
+        std::vector<std::vector<int>> own(grid);
+        std::vector<int> loc(3 * (size_t)nt), fill(start.begin(), start.end() - 1);
+        for (int t = 0; t < nt; t++) {
+            for (int k = 0; k < 3; k++) {
+                const int v = ctx->tri[3 * t + k];
+                std::vector<int> &o = own[coop_block(ntiles, grid, v / kStepBlock)];
+                if (o.empty() || (o.back() & 0x7fffffff) != t) o.push_back(k == 0 ? (int)((unsigned)t | 0x80000000u) : t);
+                loc[fill[v]++] = 3 * ((int)o.size() - 1) + k;
+            }
+        }
+        std::vector<int> ofs(grid + 1, 0), all;
+        size_t most = 0;
+        for (int b = 0; b < grid; b++) {
+            all.insert(all.end(), own[b].begin(), own[b].end());
+            ofs[b + 1] = (int)all.size();
+            most = std::max(most, own[b].size());
+        }
+        cudaStream_t st = ctx->stream;
+        if (ctx->triOfs.ensure(ofs.size()) || ctx->triOwn.ensure(all.size()) || ctx->triLoc.ensure(loc.size()) ||
+            ctx->triTmp.ensure(3 * (size_t)nt) ||
+            cudaMemcpyAsync(ctx->triOfs.p, ofs.data(), ofs.size() * sizeof(int), cudaMemcpyHostToDevice, st) ||
+            cudaMemcpyAsync(ctx->triOwn.p, all.data(), all.size() * sizeof(int), cudaMemcpyHostToDevice, st) ||
+            cudaMemcpyAsync(ctx->triLoc.p, loc.data(), loc.size() * sizeof(int), cudaMemcpyHostToDevice, st) ||
+            cudaStreamSynchronize(st)) {
+            cudaGetLastError();  // no memory: the triangle pass apart
+            return a;
+        }
+        ctx->triMost = (int)((most + 1) & ~(size_t)1);  // (even: what follows in shared memory is 16-byte aligned)
+    }
+    a.triOfs = ctx->triOfs.p;
+    a.triOwn = ctx->triOwn.p;
+    a.triLoc = ctx->triLoc.p;
+    a.triTmp = ctx->triTmp.p;
+    a.triMost = ctx->triMost;
+    return a;
+}
+
 // Whether runs of the context go to one cooperative launch (k_coop.cu), its
 // buffers allocated on the first of them.
 static bool coop_ready(femmd_ctx *ctx) {
@@ -1260,7 +1319,8 @@ static bool coop_ready(femmd_ctx *ctx) {
         ctx->coopOff = true;
         return false;
     }
-    return coop_run_fits(make_sys(ctx));
+    const DevSys s = make_sys(ctx);
+    return coop_run_fits(s, coop_plan(ctx, s));
 }
 
 // A run, or part of one, of a small or medium system in one cooperative
@@ -1273,7 +1333,8 @@ static femmd_status coop_launch(femmd_ctx *ctx, int begin, int units, int end, f
         static_assert(offsetof(DevScalars, runFill) == offsetof(DevScalars, runTag) + sizeof(int), "run scalars");
         ctx->runClean = true;
     }
-    CoopArgs a = {};
+    const DevSys s = make_sys(ctx);
+    CoopArgs a = coop_plan(ctx, s);
     a.parity = ctx->cur;
     a.begin = begin;
     a.units = units;
@@ -1284,7 +1345,7 @@ static femmd_status coop_launch(femmd_ctx *ctx, int begin, int units, int end, f
     a.ckVel = ctx->ckVel.p;
     a.ckAcc = ctx->ckAcc.p;
     a.slots = slots;
-    CK(launch_coop_run(ctx->stream, make_sys(ctx), a));
+    CK(launch_coop_run(ctx->stream, s, a));
     ctx->profKernels++;
     ctx->cur ^= (begin + units) & 1;
     return FEMMD_OK;

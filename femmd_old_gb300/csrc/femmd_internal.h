@@ -271,7 +271,8 @@ cudaError_t kernel_setup(const void *fn, int threads, size_t smem, int *resident
 
 // ---- whole runs of small and medium systems in one cooperative launch (k_coop.cu)
 constexpr int kCoopMaxBlocks = 256;
-constexpr size_t kCoopRecWords = 4 * 16 + 4 * 4 * (size_t)kCoopMaxBlocks;  // exchange slots, then the sums
+// exchange slots, four sets of sums, a word per block
+constexpr size_t kCoopRecWords = 4 * 16 + 4 * 4 + (size_t)kCoopMaxBlocks;
 constexpr int kCellCap = 32;  // particles of a cell at most (a fuller one: the plain kernels)
 struct CoopArgs {
     int parity;   // of the current positions
@@ -282,9 +283,21 @@ struct CoopArgs {
     float2 *ckPos, *ckVel, *ckAcc;
     float2 *slots;  // positions after drift u also to slots + (u + 1) N, or null
     int rows, incStaged, triStaged;  // shared memory: list rows, incidences, triangles (the launch sets them)
+    // Triangles by block (every block works all the triangles of its own
+    // particles): block b's are triOwn[triOfs[b] ..), a number and, in bit 31, whether
+    // the triangle's energy is this block's to add; triLoc: tEnt's entries as the
+    // place of the triangle's force in the particle's block.  triMost: the most of one
+    // block, 0 without.  triTmp: three sets of the triangles' energies.
+    const int *triOfs, *triOwn, *triLoc;
+    float *triTmp;
+    int triMost, triLocal;  // triLocal: they are used (the launch sets it)
 };
 bool coop_size_ok(int N, int ncells);
-bool coop_run_fits(const DevSys &s);
+bool coop_run_fits(const DevSys &s, const CoopArgs &plan);
+// The blocks of a system; with triangles by block, the block of a tile of 128 particles.
+int coop_grid(const DevSys &s);
+int coop_block(int ntiles, int grid, int tile);
+constexpr int kCoopIncTri = 8, kCoopIncBond = 6;  // most incidences of a particle that triangles by block allow
 cudaError_t launch_coop_run(cudaStream_t st, const DevSys &s, const CoopArgs &a);
 
 // ---- forces + integration (k_force.cu)

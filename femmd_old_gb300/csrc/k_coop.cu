@@ -29,22 +29,20 @@ constexpr size_t kCoopSmem = 180 * 1024;  // dynamic shared memory of a block at
 // where they fit, then as many list rows as do.
 // False when the system does not fit.
 bool coop_shape(const DevSys &s, int &grid, size_t &smem, CoopArgs &a) {
-    int sms = 0, dev = 0;
-    if (cudaGetDevice(&dev) || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return false;
-    const int ntiles = (s.N + kStepBlock - 1) / kStepBlock;
-    // (the grid depends on the topology alone: the exchanges count blocks over
-    // the life of the context, and the triangle forces can be turned on later)
-    const int ntt = (s.ntri + kTriTile - 1) / kTriTile;
-    grid = std::max(1, std::min(std::min(sms, kCoopMaxBlocks), std::max(ntiles, ntt)));
+    const int ntiles = (s.N + kStepBlock - 1) / kStepBlock, ntt = (s.ntri + kTriTile - 1) / kTriTile;
+    if (!(grid = coop_grid(s))) return false;
     const int per = (ntiles + grid - 1) / grid, tper = (ntt + grid - 1) / grid;
     if (per > kCoopMaxTiles || tper > kCoopMaxTiles) return false;
+    const size_t own = (size_t)a.triMost * (sizeof(int4) + 3 * sizeof(float2));
     smem = coop_terms(s.fast) * (size_t)kTermComp * sizeof(float) + (size_t)per * 4 * kStepBlock * sizeof(int);  // terms, sums, counts
     const size_t inc = (size_t)per * kIncWords * kStepBlock * sizeof(int), tri = (size_t)tper * kTriTile * sizeof(int4);
     const size_t row = 4 * (size_t)per * kListRow * sizeof(int);  // four list rows
     a.incStaged = s.nBonded > 0 && smem + inc + row <= kCoopSmem;
     if (a.incStaged) smem += inc;
-    a.triStaged = ntt > 0 && smem + tri + row <= kCoopSmem;
+    a.triLocal = a.triMost > 0 && a.incStaged && smem + own + row <= kCoopSmem;
+    a.triStaged = ntt > 0 && !a.triLocal && smem + tri + row <= kCoopSmem;
     if (a.triStaged) smem += tri;
+    if (a.triLocal) smem += own;
     a.rows = 4 * (int)std::min<size_t>(s.nbrCap / 4, (kCoopSmem - smem) / row);
     smem += a.rows / 4 * row;
     return a.rows > 0 || s.nbrCap == 0;
@@ -52,11 +50,23 @@ bool coop_shape(const DevSys &s, int &grid, size_t &smem, CoopArgs &a) {
 
 }  // namespace
 
-bool coop_run_fits(const DevSys &s) {
+// The blocks of a system: one per tile, at most one per SM (0: no device).  They
+// depend on the topology alone: the exchanges count blocks over the life of the
+// context, and the triangle forces can be turned on later.
+int coop_grid(const DevSys &s) {
+    int sms = 0, dev = 0;
+    if (cudaGetDevice(&dev) || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev)) return 0;
+    const int ntiles = (s.N + kStepBlock - 1) / kStepBlock, ntt = (s.ntri + kTriTile - 1) / kTriTile;
+    return std::max(1, std::min(std::min(sms, kCoopMaxBlocks), std::max(ntiles, ntt)));
+}
+
+int coop_block(int ntiles, int grid, int tile) { return coop_pairs(ntiles, grid) ? tile / 2 : tile % grid; }
+
+bool coop_run_fits(const DevSys &s, const CoopArgs &plan) {
     if ((s.fast && !s.sigmaByType) || s.areaUnits > 0 || s.trace || !s.cellCand || s.N <= 0) return false;
     int grid, resident = 0;
     size_t smem;
-    CoopArgs a = {};
+    CoopArgs a = plan;
     if (!coop_shape(s, grid, smem, a)) return false;
     if (kernel_setup(coop_kernel(s), kCoopThreads, smem, &resident)) return false;
     return resident >= grid;

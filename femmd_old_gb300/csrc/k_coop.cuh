@@ -5,12 +5,20 @@
 // 15-25 us whatever the system's size: launches, the IF node, and the drain
 // of each kernel.  Up to a few hundred thousand particles the arithmetic of a
 // step takes less than that, so k_coop advances the run inside one launch:
-// every block owns fixed tiles of particles and triangles, a step is the
-// triangle pass, a grid-wide exchange, the particle pass and a second
-// exchange (the first one only with triangles), and every block takes the
-// rebuild decision of NeighborList::update (femmd2D/src/nn.cpp:114-134) from
-// the same exchanged maximum.  A system of one tile runs in one block,
-// where an exchange is a block barrier.
+// every block owns fixed tiles of particles, a step is the triangle pass, the
+// particle pass and a grid-wide exchange, and every block takes the rebuild
+// decision of NeighborList::update (femmd2D/src/nn.cpp:114-134) from the same
+// exchanged maximum.  A system of one tile runs in one block, where an
+// exchange is a block barrier.
+//
+// Every block works all the triangles of its own particles (CoopArgs::triOwn)
+// and keeps their forces in shared memory: the few with particles of two blocks
+// are worked twice, and the particle pass needs no exchange before it.  Of a
+// triangle's blocks one stores its energy, which is added up a step later.
+// Where a particle has too many incidences or shared memory is short, the
+// triangles are shared out and an exchange follows the triangle pass: 256 disks
+// run(100) 1034 us against 849, 144 disks in solvent (fast mode) run(50) 1211
+// against 1137, the adjoint of 64 disks 7729 against 7034.
 //
 // At these sizes a step is bound by latency: dependent L2 accesses (about
 // 0.4 us each: an exchange invalidates L1) and, with a warp or two per
@@ -25,9 +33,10 @@
 // energy sums are reduced while the exchange is waited for.
 //
 // Measured against the plain kernels in CUDA graphs (a whole set_state, run,
-// get_state; us): LJ fluid 400 particles run(20) 643 -> 216, 10,201 run(50)
-// 1374 -> 454; 256-disk suspension (32,512) run(100) 1837 -> 1000; adjoint of 64
-// disks over 200 steps 14,170 -> 7451.  The particle pass of the 10,201
+// get_state; us): LJ fluid 400 particles run(20) 659 -> 207, 10,201 run(50)
+// 1390 -> 407; 256-disk suspension (32,512) run(100) 1842 -> 849; adjoint of 64
+// disks over 200 steps 14,260 -> 7034; fast mode, run(50): LJ fluid 90,000 1408
+// -> 1112, 144 disks in solvent (68,288) 1778 -> 1137.  The particle pass of the 10,201
 // particles takes 4.1 us; a thread per particle instead of a quad took 7.7.
 //
 // The per-particle and per-triangle arithmetic and the list order are those
@@ -48,10 +57,11 @@
 //
 // Exchanges are grid_exchange's (grid_sync.cuh), bounded: a wait that gives
 // up sets the timeout flag, and the block leaves the kernel.  They are numbered
-// over the life of the context (DevScalars::runTag).  A step's energy sums go
-// to one of four rotating sets after its exchange and are therefore visible to
-// a block that has completed the following one; block 0 adds them up during
-// the exchange after that.
+// over the life of the context (DevScalars::runTag).  A step's energy sums are
+// added into one of four rotating sets after its exchange (the triangles' by
+// block after the next step's) and are therefore complete to a block that has
+// completed the following one; block 0 takes them during the exchange after
+// that.
 #pragma once
 #include <cuda_runtime.h>
 #include <type_traits>
@@ -75,7 +85,7 @@ constexpr int kTriTile = 256;       // triangles per energy group (k_tri_forces'
 constexpr int kListLanes = 8;       // lanes that build one particle's list
 // Incidences of one bonded particle kept in shared memory: a count word, up
 // to kIncTri triangle entries and kIncBond bond entries of two words.
-constexpr int kIncTri = 8, kIncBond = 6, kIncWords = 1 + kIncTri + 2 * kIncBond;
+constexpr int kIncTri = kCoopIncTri, kIncBond = kCoopIncBond, kIncWords = 1 + kIncTri + 2 * kIncBond;
 constexpr int kQuadPairs = 6;                // list entries per lane and round
 constexpr int kQuadRows = 4 * kQuadPairs;    // entries per particle and round
 // One round's terms in shared memory: component c of entry k of the tile's
@@ -105,7 +115,8 @@ __device__ __forceinline__ int ld_early(const int *p) {
     return v;
 }
 struct CoopDue {
-    unsigned x;  // the exchange that published the step
+    unsigned x;  // the exchange after which the last of the step's sums were stored
+    unsigned set;  // their set
     int mode, row, reb;
     float vm, d;
 };
@@ -115,6 +126,7 @@ struct CoopShared {
     float vmax[kCoopThreads / 32];    // per warp: its particles' largest v^2
     float tred[kCoopMaxTiles][8];     // per triangle tile and warp: energy
     unsigned long long acc[3];        // the step's energy sums of this block (U, W, K)
+    unsigned long long accTri;        // triangles by block: the previous step's triangle energy
     CoopDue due[4];                   // block 0: steps whose totals have still to be added up
     int wsum[kCoopThreads / 32];
     unsigned ok, maxBits;             // of the last exchange
@@ -124,34 +136,32 @@ struct CoopShared {
 // What every block carries through the launch (the same on each).
 struct CoopRun {
     unsigned base, xi;       // exchanges before this launch, and of it
-    unsigned dueIn, dueOut;  // entries pushed to and taken from CoopShared::due
+    unsigned dueIn, dueOut;  // entries pushed to and taken from CoopShared::due (one per step)
+    unsigned dueOk;          // entries whose sums are all stored
     float dispHi;
     int row, stepNow, updates;
     int cnt;  // which of the two cell-count arrays the last rebuild filled
 };
 
-__device__ __forceinline__ unsigned long long *coop_sums(const DevSys &s, unsigned x) {
-    return s.runRec + kGridSlots * kGridSlotWords + (size_t)(x % 4u) * kCoopMaxBlocks * 4;
+// Step 'n' of a launch adds its energies (U, W, K as fixed point, every block by
+// integer atomics: exact in any order) into set n mod 4; zero when it starts.
+__device__ __forceinline__ unsigned long long *coop_sums(const DevSys &s, unsigned n) {
+    return s.runRec + kGridSlots * kGridSlotWords + 4 * (size_t)(n % 4u);
+}
+// a word per block
+__device__ __forceinline__ unsigned long long *coop_words(const DevSys &s) {
+    return s.runRec + kGridSlots * kGridSlotWords + 16;
 }
 
-// One warp: the totals of a step's sums into the scalars and, for the modes
-// that complete a step, its observable row.
+// One thread: the totals of a step into the scalars and, for the modes that
+// complete a step, its observable row; the set is zero again.  (Summed up by
+// block 0 from a record per block instead, this took longer than the exchange
+// beside it: 256 disks on 152 blocks, 1053 us a run(100), 849 so.)
 __device__ __noinline__ void coop_totals(const DevSys &s, const CoopDue &d) {
-    const unsigned long long *set = coop_sums(s, d.x);
-    const int lane = threadIdx.x & 31;
-    unsigned long long u = 0ull, w = 0ull, k = 0ull;
-    for (int b = lane; b < (int)gridDim.x; b += 32) {
-        u += __ldcg(set + 4 * (size_t)b);
-        w += __ldcg(set + 4 * (size_t)b + 1);
-        k += __ldcg(set + 4 * (size_t)b + 2);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        u += __shfl_down_sync(0xffffffffu, u, o);
-        w += __shfl_down_sync(0xffffffffu, w, o);
-        k += __shfl_down_sync(0xffffffffu, k, o);
-    }
-    if (lane == 0) {
+    unsigned long long *set = coop_sums(s, d.set);
+    const unsigned long long u = __ldcg(set), w = __ldcg(set + 1), k = __ldcg(set + 2);
+    set[0] = set[1] = set[2] = 0ull;
+    {
         DevScalars *sc = s.sc;
         const double U = from_fixed(u), W = from_fixed(w), KE = from_fixed(k);
         sc->U = U;
@@ -170,7 +180,6 @@ __device__ __noinline__ void coop_totals(const DevSys &s, const CoopDue &d) {
             }
         }
     }
-    __syncwarp();
 }
 
 // An exchange: maxBits = the largest value as a float (the values' bits).
@@ -192,10 +201,10 @@ __device__ __forceinline__ bool coop_exchange(const DevSys &s, CoopShared &sh, C
         sh.maxBits = m;
     }
     // a step's sums are visible once the exchange after its own is complete
-    while (r.dueOut != r.dueIn && !all) {
+    while (r.dueOut != r.dueOk && !all) {
         const CoopDue &d = sh.due[r.dueOut & 3u];
         if ((int)(r.base + r.xi - d.x) < 2) break;
-        if (blockIdx.x == 0 && threadIdx.x >> 5 == 2) coop_totals(s, d);
+        if (blockIdx.x == 0 && threadIdx.x == 64) coop_totals(s, d);
         r.dueOut++;
     }
     r.xi++;
@@ -238,8 +247,26 @@ struct CoopMem {
     int rows;     // (a multiple of 4)
     int *count;  // [tile][kStepBlock]: list lengths
     int *inc;    // [tile][kIncWords][kStepBlock], or null
-    int4 *tri;   // [triangle tile][kTriTile]: vertices, or null
+    // triangles by tile: [triangle tile][kTriTile], the vertices, or null; by
+    // block: the block's, vertices and CoopArgs::triOwn's word, and their forces
+    int4 *tri;
+    float2 *triF;
+    int tiles, first, stride;  // the block's tiles of particles: first, first + stride, ...
 };
+
+// The tiles of block b.  Tile j is b + j grid, so that bonded and free particles
+// (and their rebuilds) are shared out.  With triangles by block and two tiles a
+// block (pair), they are neighbours: fewer triangles have particles of two
+// blocks (256 disks of 216 triangles on 152 blocks: at most 504 a block, 562
+// with tiles apart, where 512 threads want at most 512).
+__host__ __device__ inline bool coop_pairs(int ntiles, int grid) { return (ntiles + grid - 1) / grid == 2; }
+__host__ __device__ inline int coop_tiles(int ntiles, int grid, int b, bool pair, int &first, int &stride) {
+    pair = pair && coop_pairs(ntiles, grid);
+    first = pair ? 2 * b : b;
+    stride = pair ? 1 : grid;
+    if (first >= ntiles) return 0;
+    return pair ? (ntiles - first < 2 ? ntiles - first : 2) : (ntiles - 1 - first) / stride + 1;
+}
 
 // The list of particle i (slot 'col' of the block's tile j) by kListLanes
 // lanes: the 3 x 3 cells in the reference's order (dx outer, dy inner, each
@@ -331,15 +358,15 @@ __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, co
                                           bool withhold) {
     const float2 *pos = p ? s.pos1 : s.pos0;
     DevScalars *sc = s.sc;
-    const int ntiles = (s.N + kStepBlock - 1) / kStepBlock, groups = blockDim.x / kStepBlock;
+    const int groups = blockDim.x / kStepBlock;
     const int grp = threadIdx.x / kStepBlock, gt = threadIdx.x % kStepBlock, lane = threadIdx.x & 31;
     r.updates += 1;
     r.dispHi = 0.0f;
     r.cnt ^= 1;
     int *cnt = s.cellFill + (size_t)r.cnt * s.ncells, *other = s.cellFill + (size_t)(r.cnt ^ 1) * s.ncells;
     // 1: cells, and the ids into them in any order
-    for (int j = grp; blockIdx.x + j * gridDim.x < ntiles; j += groups) {
-        const int i = (blockIdx.x + j * gridDim.x) * kStepBlock + gt;
+    for (int j = grp; j < mem.tiles; j += groups) {
+        const int i = (mem.first + j * mem.stride) * kStepBlock + gt;
         if (i >= s.N) continue;
         const float2 x = pos[i];
         if (!(isfinite(x.x) && isfinite(x.y))) atomicOr(&sc->nonfinite, 1);
@@ -359,8 +386,8 @@ __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, co
     // rebuild (their last readers were the lists before this rebuild)
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < s.ncells; c += gridDim.x * blockDim.x) other[c] = 0;
     if (!skip)
-        for (int j = grp; blockIdx.x + j * gridDim.x < ntiles; j += groups) {
-            const int i = (blockIdx.x + j * gridDim.x) * kStepBlock + gt;
+        for (int j = grp; j < mem.tiles; j += groups) {
+            const int i = (mem.first + j * mem.stride) * kStepBlock + gt;
             if (i >= s.N) continue;
             const int c = s.cellOf[i], n = min(__ldcg(cnt + c), kCellCap);
             const int4 *ids = reinterpret_cast<const int4 *>(s.cellIds + (size_t)c * kCellCap);
@@ -387,11 +414,10 @@ __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, co
         const bool fast = (s.wrapx ? s.ncx >= 5 : s.ncx >= 3) && (s.wrapy ? s.ncy >= 5 : s.ncy >= 3) &&
                           !__ldcg(&sc->outside);  // fast_walk_ok
         constexpr int per = 32 / kListLanes;      // particles per warp
-        const int mine = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;  // tiles
         int kmax = 0, ksum = 0;
-        for (int b = (threadIdx.x >> 5) * per; b < mine * kStepBlock; b += (blockDim.x >> 5) * per) {
+        for (int b = (threadIdx.x >> 5) * per; b < mem.tiles * kStepBlock; b += (blockDim.x >> 5) * per) {
             const int q = b + lane / kListLanes, j = q / kStepBlock, col = q % kStepBlock;
-            const int i = (blockIdx.x + j * gridDim.x) * kStepBlock + col;
+            const int i = (mem.first + j * mem.stride) * kStepBlock + col;
             const int k = fast ? coop_list<true>(s, mem, cnt, pos, i, j, col, i < s.N)
                                : coop_list<false>(s, mem, cnt, pos, i, j, col, i < s.N);
             if (i < s.N && (lane & (kListLanes - 1)) == 0) {
@@ -418,9 +444,10 @@ __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, co
 // which are kStepBlock slots each, say that they have no window and how many
 // groups their longest list has).
 template <bool FAST>
-__device__ __forceinline__ void coop_write_lists(const DevSys &s, const CoopMem &mem, int tiles) {
+__device__ __forceinline__ void coop_write_lists(const DevSys &s, const CoopMem &mem) {
+    const int tiles = mem.tiles;
     for (int q = threadIdx.x; q < tiles * kStepBlock; q += blockDim.x) {
-        const int j = q / kStepBlock, col = q % kStepBlock, i = (blockIdx.x + j * gridDim.x) * kStepBlock + col;
+        const int j = q / kStepBlock, col = q % kStepBlock, i = (mem.first + j * mem.stride) * kStepBlock + col;
         if (i >= s.N) continue;
         const int k = min(mem.count[q], mem.rows);
         const int *lst = mem.list + (size_t)j * mem.rows * kListRow + col;
@@ -438,7 +465,7 @@ __device__ __forceinline__ void coop_write_lists(const DevSys &s, const CoopMem 
         static_assert(kStepBlock == kFastBlock, "a tile is a step block");
         const int lane = threadIdx.x & 31;
         for (int j = threadIdx.x >> 5; j < tiles; j += blockDim.x >> 5) {
-            const int b = blockIdx.x + j * gridDim.x;
+            const int b = mem.first + j * mem.stride;
             int most = 0;
             for (int c = lane; c < kStepBlock; c += 32)
                 if (b * kStepBlock + c < s.N) most = max(most, mem.count[j * kStepBlock + c]);
@@ -462,14 +489,13 @@ __device__ __forceinline__ bool coop_cells(const DevSys &s, CoopShared &sh, Coop
         block_scan(sh, c < c1 ? min(__ldcg(cnt + c), kCellCap) : 0, tot);
         sum += tot;
     }
-    // every block's count through the set of sums that is not in use
-    unsigned long long *counts = coop_sums(s, r.base + r.xi + 2u);
-    if (threadIdx.x == 0) counts[4 * (size_t)blockIdx.x + 3] = (unsigned long long)sum;
+    unsigned long long *counts = coop_words(s);
+    if (threadIdx.x == 0) counts[blockIdx.x] = (unsigned long long)sum;
     __syncthreads();
     if (!coop_exchange(s, sh, r, 0u)) return false;
     if (threadIdx.x < 32) {
         int before = 0;
-        for (int b = threadIdx.x; b < (int)blockIdx.x; b += 32) before += (int)__ldcg(counts + 4 * (size_t)b + 3);
+        for (int b = threadIdx.x; b < (int)blockIdx.x; b += 32) before += (int)__ldcg(counts + b);
         before = __reduce_add_sync(0xffffffffu, before);
         if (threadIdx.x == 0) sh.before = before;
     }
@@ -686,7 +712,10 @@ __device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &me
         float2 tf[kIncTri], pb[2];
 #pragma unroll
         for (int k = 0; k < kIncTri; k++)
-            if (k < nT) tf[k] = ld_early(s.triF + inc[(1 + k) * kStepBlock]);
+            if (k < nT) {
+                const int e = inc[(1 + k) * kStepBlock];
+                tf[k] = mem.triF ? mem.triF[e] : ld_early(s.triF + e);
+            }
 #pragma unroll
         for (int k = 0; k < 2; k++)
             if (k < nB) pb[k] = ld_early(pin + (bond(k).x & 0x7fffffff));
@@ -770,8 +799,9 @@ __device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &me
 // plain kernels' grouping: FP32 over 32 lanes (warp_sum_f), over the four
 // warps in order, then fixed point; a triangle tile's eight warp sums alike.
 // Warps 'w0', w0 + 1, ... of the block share the tiles.
-__device__ __forceinline__ void coop_block_sums(const DevSys &s, CoopShared &sh, const CoopMem &mem, int tiles,
-                                                int ttiles, int w0) {
+__device__ __forceinline__ void coop_block_sums(const DevSys &s, CoopShared &sh, const CoopMem &mem, int ttiles,
+                                                int w0) {
+    const int tiles = mem.tiles;
     const int lane = threadIdx.x & 31, w = (threadIdx.x >> 5) - w0, nw = (blockDim.x >> 5) - w0;
     bool ob = false;
     for (int j = w; j < tiles; j += nw) {
@@ -790,6 +820,24 @@ __device__ __forceinline__ void coop_block_sums(const DevSys &s, CoopShared &sh,
 #pragma unroll
         for (int g = 0; g < kTriTile / 32; g++) x += sh.tred[j][g];
         atomicAdd(&sh.acc[0], to_fixed(x, ob));
+    }
+    if (ob) atomicOr(&s.sc->nonfinite, 2);
+}
+
+// Triangles by block: the energies 'e' of all the triangles, summed over the block's
+// triangle tiles as coop_block_sums does.  Warps w0, w0 + 1, ... share
+// the tiles, the last one first.
+__device__ __forceinline__ void coop_tri_block_sums(const DevSys &s, CoopShared &sh, const float *e, int ttiles, int w0) {
+    const int lane = threadIdx.x & 31, nw = (blockDim.x >> 5) - w0, w = nw - 1 - ((int)(threadIdx.x >> 5) - w0);
+    bool ob = false;
+    for (int j = w; j < ttiles; j += nw) {
+        const int t = (blockIdx.x + j * gridDim.x) * kTriTile + lane;
+        float v[kTriTile / 32], x = 0.0f;
+#pragma unroll
+        for (int g = 0; g < kTriTile / 32; g++) v[g] = t + 32 * g < s.ntri ? __ldcg(e + t + 32 * g) : 0.0f;
+#pragma unroll
+        for (int g = 0; g < kTriTile / 32; g++) x += warp_sum_f(v[g]);
+        if (lane == 0) atomicAdd(&sh.accTri, to_fixed(x, ob));
     }
     if (ob) atomicOr(&s.sc->nonfinite, 2);
 }
@@ -827,12 +875,16 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
     const int ntt = tris ? (s.ntri + kTriTile - 1) / kTriTile : 0, tgroups = blockDim.x / kTriTile;
     const int tgrp = threadIdx.x / kTriTile, tgt = threadIdx.x % kTriTile;
     const int per = (ntiles + gridDim.x - 1) / gridDim.x, tper = (ntt + gridDim.x - 1) / gridDim.x;
-    const int tiles = (int)blockIdx.x < ntiles ? (ntiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     const int ttiles = (int)blockIdx.x < ntt ? (ntt - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
     CoopMem mem;
     mem.rows = a.rows;
-    mem.tri = a.triStaged ? dyn : nullptr;
-    mem.term = reinterpret_cast<float *>(dyn + (a.triStaged ? tper * kTriTile : 0));
+    mem.tiles = coop_tiles(ntiles, gridDim.x, blockIdx.x, a.triLocal, mem.first, mem.stride);
+    const bool local = tris && a.triLocal;
+    const int nown = local ? a.triOfs[blockIdx.x + 1] - a.triOfs[blockIdx.x] : 0;
+    mem.tri = a.triStaged || local ? dyn : nullptr;
+    mem.triF = local ? reinterpret_cast<float2 *>(dyn + a.triMost) : nullptr;
+    mem.term = reinterpret_cast<float *>(dyn + (a.triStaged ? tper * kTriTile : (a.triLocal ? a.triMost : 0)));
+    if (a.triLocal) mem.term += 6 * a.triMost;
     mem.part = mem.term + coop_terms(FAST) * kTermComp;
     mem.count = reinterpret_cast<int *>(mem.part + (size_t)per * 3 * kStepBlock);
     mem.inc = a.incStaged ? mem.count + per * kStepBlock : nullptr;
@@ -845,13 +897,20 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
             a.ckAcc[i] = s.acc[i];
         }
     }
-    if (mem.tri)
+    if (local) {
+        const int *own = a.triOwn + a.triOfs[blockIdx.x];
+        for (int k = threadIdx.x; k < nown; k += blockDim.x) {
+            int4 q = __ldg(s.triIdx + (own[k] & 0x7fffffff));
+            q.w = own[k];
+            dyn[k] = q;
+        }
+    } else if (mem.tri)
         for (int j = tgrp; blockIdx.x + j * gridDim.x < ntt; j += tgroups) {
             const int t = (blockIdx.x + j * gridDim.x) * kTriTile + tgt;
             if (t < s.ntri) mem.tri[j * kTriTile + tgt] = __ldg(s.triIdx + t);
         }
-    for (int j = grp; blockIdx.x + j * gridDim.x < ntiles; j += groups) {
-        const int i = (blockIdx.x + j * gridDim.x) * kStepBlock + gt;
+    for (int j = grp; j < mem.tiles; j += groups) {
+        const int i = (mem.first + j * mem.stride) * kStepBlock + gt;
         if (mem.inc && i < min(s.nBonded, s.N)) {
             int *inc = mem.inc + (size_t)j * kIncWords * kStepBlock + gt;
             const int tb = s.tStart[i], nT = s.feaForces ? s.tStart[i + 1] - tb : 0;
@@ -860,7 +919,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
             inc[0] = fits ? (nT | nB << 8) : -1;
             for (int k = 0; fits && k < nT; k++) {
                 const int en = __ldg(s.tEnt + tb + k);
-                inc[(1 + k) * kStepBlock] = 3 * (en >> 2) + (en & 3);  // its entry of triF
+                inc[(1 + k) * kStepBlock] = local ? __ldg(a.triLoc + tb + k) : 3 * (en >> 2) + (en & 3);  // its force
             }
             for (int k = 0; fits && k < nB; k++) {
                 const int2 en = __ldg(s.bEnt + bb + k);
@@ -877,6 +936,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
         }
     }
     if (threadIdx.x < 3) sh.acc[threadIdx.x] = 0ull;
+    if (threadIdx.x == 3) sh.accTri = 0ull;
     __syncthreads();
     bool ok = true;
     const int updates0 = r.updates;
@@ -891,7 +951,26 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
         const int mode = (a.begin && u == 0) ? MODE_FIRST : ((a.end && u == total - 1) ? MODE_LAST : MODE_MID);
         const float2 *pin = p ? s.pos1 : s.pos0;
         float2 *pout = p ? s.pos0 : s.pos1;
-        if (tris) {
+        if (local) {
+            // every triangle of the block's particles: the forces stay here
+            float *te = a.triTmp + (size_t)(r.dueIn % 3u) * s.ntri;
+            for (int k = threadIdx.x; k < nown; k += blockDim.x) {
+                const int4 q = dyn[k];
+                const int t = q.w & 0x7fffffff;
+                float2 f[3];
+                const float e = tri_eval(s, pin, t, q, f);
+#pragma unroll
+                for (int c = 0; c < 3; c++) mem.triF[3 * k + c] = f[c];
+                if (q.w >= 0) continue;
+                te[t] = e;
+                if (u == total - 1) {  // as the last force evaluation of the plain kernels leaves them
+                    s.triE[t] = e;
+#pragma unroll
+                    for (int c = 0; c < 3; c++) s.triF[3 * t + c] = f[c];
+                }
+            }
+            __syncthreads();
+        } else if (tris) {
             for (int j = tgrp; blockIdx.x + j * gridDim.x < ntt; j += tgroups) {
                 const int t = (blockIdx.x + j * gridDim.x) * kTriTile + tgt;
                 float e = 0.0f;
@@ -905,8 +984,8 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
         }
         float vvm = 0.0f;
         bool bad = false;
-        for (int j = 0; j < tiles; j++) {
-            const int col = threadIdx.x >> 2, i = (blockIdx.x + j * gridDim.x) * kStepBlock + col;
+        for (int j = 0; j < mem.tiles; j++) {
+            const int col = threadIdx.x >> 2, i = (mem.first + j * mem.stride) * kStepBlock + col;
             coop_particle<MT, SG, WX, WY, SIG1, FAST>(s, mem, sh.tab, i, i < s.N, j, col, threadIdx.x & 3, mode, r.stepNow,
                                                 pin, pout, a.slots ? a.slots + (size_t)(u + 1) * s.N : nullptr, vvm,
                                                 bad);
@@ -922,13 +1001,26 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
         float mm = 0.0f;
         if (warp == 0) mm = warp_max(lane < kCoopThreads / 32 ? sh.vmax[lane] : 0.0f);
         if (!(ok = coop_exchange(s, sh, r, __float_as_uint(mm), withhold, false,
-                                 [&] { coop_block_sums(s, sh, mem, tiles, ttiles, 3); })))
+                                 [&] {
+                                     coop_block_sums(s, sh, mem, local ? 0 : ttiles, 3);
+                                     if (local && r.dueIn > 0)
+                                         coop_tri_block_sums(s, sh, a.triTmp + (size_t)((r.dueIn - 1) % 3u) * s.ntri,
+                                                             ttiles, 3);
+                                 })))
             break;
         withhold = false;
         if (threadIdx.x < 3) {
-            // visible to the others with this block's next word
-            coop_sums(s, x)[4 * (size_t)blockIdx.x + threadIdx.x] = sh.acc[threadIdx.x];
+            // visible to the others with this block's next exchange
+            atomicAdd(coop_sums(s, r.dueIn) + threadIdx.x, sh.acc[threadIdx.x]);
             sh.acc[threadIdx.x] = 0ull;
+        }
+        if (local && r.dueIn > 0) {
+            if (threadIdx.x == 3) {
+                atomicAdd(coop_sums(s, r.dueIn - 1), sh.accTri);
+                sh.accTri = 0ull;
+            }
+            if (blockIdx.x == 0 && threadIdx.x == 0) sh.due[(r.dueIn - 1) & 3u].x = x;
+            r.dueOk = r.dueIn;
         }
         // the rebuild rule (md3dsystem.cpp:177, nn.cpp:118), the same on every block
         const float vm2 = __uint_as_float(sh.maxBits);
@@ -941,6 +1033,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             CoopDue &d = sh.due[r.dueIn & 3u];
             d.x = x;
+            d.set = r.dueIn;
             d.mode = mode;
             d.row = r.row;
             d.reb = reb;
@@ -949,6 +1042,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
             sc->rebuild = reb;
         }
         r.dueIn++;
+        if (!local) r.dueOk = r.dueIn;
         if (mode != MODE_FIRST) r.row++;
         if (mode != MODE_LAST) {
             r.stepNow++;
@@ -956,14 +1050,20 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
         }
         rebuild = mode == MODE_MID && reb;
     }
+    if (ok && local && r.dueIn > 0) {
+        // the last step's triangle energies
+        coop_tri_block_sums(s, sh, a.triTmp + (size_t)((r.dueIn - 1) % 3u) * s.ntri, ttiles, 0);
+        __syncthreads();
+        if (threadIdx.x == 3) atomicAdd(coop_sums(s, r.dueIn - 1), sh.accTri);
+    }
     // the cell arrays of the last rebuild; then the last sums
     if (ok && r.updates != updates0) {
-        coop_write_lists<FAST>(s, mem, tiles);
+        coop_write_lists<FAST>(s, mem);
         ok = coop_cells(s, sh, r);
     }
     __syncthreads();
     if (ok) ok = coop_exchange(s, sh, r, 0u, false, true);
-    if (ok && blockIdx.x == 0 && warp == 2)
+    if (ok && blockIdx.x == 0 && threadIdx.x == 64)
         for (; r.dueOut != r.dueIn; r.dueOut++) coop_totals(s, sh.due[r.dueOut & 3u]);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sc->dispHi = r.dispHi;

@@ -143,14 +143,15 @@ __device__ __forceinline__ float tri_green(const DevSys &s, const float2 *pos, i
     return pesum * tetVol;
 }
 
-// Nodal forces of triangle t (vertices q) into triF, energy returned (law of s.feaLaw).
+// Nodal forces of triangle t (vertices q), energy returned (law of s.feaLaw).
+__device__ __forceinline__ float tri_eval(const DevSys &s, const float2 *pos, int t, int4 q, float2 *f) {
+    return s.feaLaw == 0 ? tri_neo_hookean(s, pos, t, q, f[0], f[1], f[2]) : tri_green(s, pos, t, q, f);
+}
+
+// tri_eval with the forces into triF, the energy into triE.
 __device__ __forceinline__ float tri_force(const DevSys &s, const float2 *pos, int t, int4 q) {
     float2 f[3];
-    float e;
-    if (s.feaLaw == 0)
-        e = tri_neo_hookean(s, pos, t, q, f[0], f[1], f[2]);
-    else
-        e = tri_green(s, pos, t, q, f);
+    const float e = tri_eval(s, pos, t, q, f);
     s.triF[3 * t + 0] = f[0];
     s.triF[3 * t + 1] = f[1];
     s.triF[3 * t + 2] = f[2];
