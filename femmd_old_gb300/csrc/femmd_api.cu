@@ -3366,31 +3366,67 @@ femmd_status femmd_adjoint_backward(femmd_ctx *ctx, double c_wall, double c_fea,
     }
     const float dt = ctx->dt, h = 0.5f * ctx->dt;
     std::vector<int> rebuilt;
+    // one cooperative launch per list where the whole-run launch is used too,
+    // else (and while profiling) two kernels a step
+    bool sweep = !ctx->profiling && coop_ready(ctx);
+    if (sweep) {
+        const DevSys s = make_sys(ctx);
+        sweep = adj_sweep_fits(s, coop_plan(ctx, s));
+        CK(cudaMemsetAsync(&ctx->sc.p->sweepLost, 0, sizeof(int), sm));
+    }
     for (int g = nseg - 1; g >= 0; g--) {
         if ((st = adj_recompute(ctx, g, rebuilt))) return st;
         const int K = a.segLen[g], s0 = a.segStart[g];
         DevSys s = make_sys(ctx);
         Launch L;
         L.stream = sm;
-        int listFrom = -1;
-        for (int k = K; k >= (g == 0 ? 0 : 1); k--) {
+        const int lo = g == 0 ? 0 : 1;
+        int listFrom = rebuilt.back();  // the recomputation's last list is still there
+        for (int k = K; k >= lo;) {
             int r = 0;
             for (int v : rebuilt)
                 if (v <= k) r = std::max(r, v);
-            const float2 *pk = a.slots.p + (size_t)k * N;
             if (r != listFrom) {
                 DevSys sb = s;
-                sb.pos0 = const_cast<float2 *>(a.slots.p + (size_t)r * N);
+                sb.pos0 = a.slots.p + (size_t)r * N;
                 CK(enqueue_rebuild(L, sb, 0, 0));
                 listFrom = r;
             }
-            const int n = s0 + k;
-            const int update = k >= 1;
-            const float cNext = (n - 1 == a.segStart[0]) ? h : dt;
-            CK(enqueue_adj_step(L, s, pk, wc, a.triD.p, a.gMu.p, a.gLam.p, a.xbar.p, a.vbar.p, wn, cNext, update,
-                                wall_y_host(ctx, n), a.epsAcc.p, a.sigAcc.p));
-            if (update) std::swap(wc, wn);
+            // the steps of this list
+            const int to = std::max(r, lo);
+            if (sweep) {
+                AdjSweep w = {};
+                w.slots = a.slots.p;
+                w.w0 = wc;
+                w.w1 = wn;
+                w.xbar = a.xbar.p;
+                w.vbar = a.vbar.p;
+                w.gMu = a.gMu.p;
+                w.gLam = a.gLam.p;
+                w.epsAcc = a.epsAcc.p;
+                w.sigAcc = a.sigAcc.p;
+                w.kHi = k;
+                w.kLo = to;
+                w.segStart = s0;
+                w.start = a.segStart[0];
+                CK(launch_adj_sweep(sm, s, coop_plan(ctx, s), w));
+                if ((k - std::max(to, 1) + 1) & 1) std::swap(wc, wn);
+                k = to - 1;
+                continue;
+            }
+            for (; k >= to; k--) {
+                const int n = s0 + k;
+                const int update = k >= 1;
+                const float cNext = (n - 1 == a.segStart[0]) ? h : dt;
+                CK(enqueue_adj_step(L, s, a.slots.p + (size_t)k * N, wc, a.triD.p, a.gMu.p, a.gLam.p, a.xbar.p,
+                                    a.vbar.p, wn, cNext, update, wall_y_host(ctx, n), a.epsAcc.p, a.sigAcc.p));
+                if (update) std::swap(wc, wn);
+            }
         }
+    }
+    if (sweep) {
+        if ((st = read_scalars(ctx))) return st;
+        if (ctx->hsc->sweepLost) return expired(ctx, "a grid-wide exchange");
     }
     // outputs
     if (xbar_init) CK(cudaMemcpyAsync(xbar_init, a.xbar.p, N * sizeof(float2), cudaMemcpyDeviceToHost, sm));

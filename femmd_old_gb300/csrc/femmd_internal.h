@@ -78,7 +78,8 @@ struct DevScalars {
     int obsRow, stepNow;  // stepNow: index n of the positions x_n the next force evaluation sees
     unsigned long long nbrSum, builds;
     unsigned long long accU, accW, accK;  // fixed-point accumulators (two's complement)
-    unsigned int vvMaxBits, pad1;         // max v^2 as float bits (v^2 >= 0)
+    unsigned int vvMaxBits;               // max v^2 as float bits (v^2 >= 0)
+    int sweepLost;                        // a bounded wait of k_adj_sweep expired
     // the small-system run (k_fsmall): its exchanges so far, the steps one launch advanced, the steps left and the
     // position parity the next launch starts from (it ends on parity 0)
     unsigned int gbTag;
@@ -323,6 +324,20 @@ cudaError_t enqueue_adj_seed(Launch &L, const DevSys &s, const float2 *pos, floa
                              double *gLam);
 // One reverse step at positions pos with weights w: xbar += (df/dx)^T w,
 // parameter terms; with update, vbar += dt xbar and wOut = cNext vbar / m.
+// Reverse steps kHi, kHi - 1, ... kLo of one segment (positions slots + k N,
+// lists as built) in one cooperative launch; the weights start in w0 and change
+// buffers with every step but k = 0.
+struct AdjSweep {
+    const float2 *slots;
+    float2 *w0, *w1, *xbar, *vbar;
+    double *gMu, *gLam, *epsAcc, *sigAcc;
+    int kHi, kLo, segStart, start;    // step numbers of the segment's slot 0 and of the run's start
+    int rows, incStaged;              // shared memory (the launch sets them)
+};
+// plan: the triangles by block of the whole-run launch, whose grid it has.
+bool adj_sweep_fits(const DevSys &s, const CoopArgs &plan);
+cudaError_t launch_adj_sweep(cudaStream_t st, const DevSys &s, const CoopArgs &plan, const AdjSweep &a);
+
 cudaError_t enqueue_adj_step(Launch &L, const DevSys &s, const float2 *pos, const float2 *w, float2 *triD,
                              double *gMu, double *gLam, float2 *xbar, float2 *vbar, float2 *wOut, float cNext,
                              int update, float yw, double *epsAcc, double *sigAcc);

@@ -18,7 +18,8 @@
 // Where a particle has too many incidences or shared memory is short, the
 // triangles are shared out and an exchange follows the triangle pass: 256 disks
 // run(100) 1034 us against 849, 144 disks in solvent (fast mode) run(50) 1211
-// against 1137, the adjoint of 64 disks 7729 against 7034.
+// against 1137, the adjoint of 64 disks 7729 against 7034 (its reverse steps by two
+// kernels each).
 //
 // At these sizes a step is bound by latency: dependent L2 accesses (about
 // 0.4 us each: an exchange invalidates L1) and, with a warp or two per
@@ -35,7 +36,7 @@
 // Measured against the plain kernels in CUDA graphs (a whole set_state, run,
 // get_state; us): LJ fluid 400 particles run(20) 659 -> 207, 10,201 run(50)
 // 1390 -> 407; 256-disk suspension (32,512) run(100) 1842 -> 849; adjoint of 64
-// disks over 200 steps 14,260 -> 7034; fast mode, run(50): LJ fluid 90,000 1408
+// disks over 200 steps 14,260 -> 5200; fast mode, run(50): LJ fluid 90,000 1408
 // -> 1112, 144 disks in solvent (68,288) 1778 -> 1137.  The particle pass of the 10,201
 // particles takes 4.1 us; a thread per particle instead of a quad took 7.7.
 //
