@@ -3490,11 +3490,15 @@ struct femmd_batch {
     std::vector<femmd_ctx *> reps;
     int threads = 512, ctasPerSm = 2;
     DBuf<DevSys> dreps;
-    DBuf<int> order, queue, parity;
+    DBuf<BatchRep> state;
+    DBuf<DevScalars> out;
+    DevScalars *hout = nullptr;  // pinned
+    size_t houtN = 0;
+    DBuf<int> order, queue;
     cudaEvent_t ev[64] = {};
     GraphSet graph;
     int graphSteps = -1, graphThreads = 0, graphMinBlocks = 0;
-    const void *graphReps = nullptr, *graphOrder = nullptr;
+    const void *graphReps = nullptr, *graphOrder = nullptr, *graphState = nullptr;
     std::vector<BatchClass> graphCls;
     bool splitLarge = true;  // femmd_batch_set_split
     int graphVariant = -1;
@@ -3590,10 +3594,20 @@ static femmd_status batch_prepare(femmd_batch *b, int steps, BatchLaunch &bl, st
         BCK(cudaStreamSynchronize(c->stream));
     }
     sys.resize(R);
-    std::vector<int> par(R);
+    BCK(b->state.ensure(R));
+    BCK(b->out.ensure(R));
+    if (b->houtN < (size_t)R) {
+        if (b->hout) cudaFreeHost(b->hout);
+        b->hout = nullptr;
+        b->houtN = 0;
+        BCK(cudaMallocHost(&b->hout, R * sizeof(DevScalars)));
+        b->houtN = R;
+    }
+    std::vector<BatchRep> state(R);
     for (int r = 0; r < R; r++) {
-        sys[r] = make_sys(b->reps[r]);
-        par[r] = b->reps[r]->cur;
+        femmd_ctx *c = b->reps[r];
+        sys[r] = make_sys(c);
+        state[r] = {c->ckPos.p, c->ckVel.p, c->ckAcc.p, b->out.p + r, c->cur};
     }
     const DevSys &a = sys[0];
     for (int r = 1; r < R; r++) {
@@ -3628,16 +3642,15 @@ static femmd_status batch_prepare(femmd_batch *b, int steps, BatchLaunch &bl, st
         BCK(b->queue.ensure(2 * kBatchMaxCluster));
         BCK(cudaMemsetAsync(b->queue.p, 0, 2 * kBatchMaxCluster * sizeof(int), b->stream));
     }
-    BCK(b->parity.ensure(R));
     BCK(cudaMemcpyAsync(b->dreps.p, sys.data(), R * sizeof(DevSys), cudaMemcpyHostToDevice, b->stream));
     if (!ord.empty())
         BCK(cudaMemcpyAsync(b->order.p, ord.data(), ord.size() * sizeof(int), cudaMemcpyHostToDevice, b->stream));
-    BCK(cudaMemcpyAsync(b->parity.p, par.data(), R * sizeof(int), cudaMemcpyHostToDevice, b->stream));
+    BCK(cudaMemcpyAsync(b->state.p, state.data(), R * sizeof(BatchRep), cudaMemcpyHostToDevice, b->stream));
     bl.reps = b->dreps.p;
     bl.order = b->order.p;
     bl.queue = b->queue.p;
     bl.minBlocks = b->ctasPerSm >= 2 && b->threads > 512 ? 2 : 1;
-    bl.parity = b->parity.p;
+    bl.state = b->state.p;
     bl.steps = steps;
     bl.threads = b->threads;
     bl.smem = sizeof(PairEntry) * (size_t)(a.numTypes > 1 ? a.numTypes * a.numTypes : 1);
@@ -3657,7 +3670,7 @@ static femmd_status batch_launch(femmd_batch *b, const BatchLaunch &bl) {
     const int variant = bl.multiType | bl.sigmaByType << 1 | bl.sigmaOne << 2 | bl.wrapx << 3 | bl.wrapy << 4;
     const std::vector<BatchClass> cls(bl.cls, bl.cls + bl.nclass);
     const bool rebuild = !b->graph.x || b->graphSteps != bl.steps || b->graphThreads != bl.threads ||
-                         b->graphReps != (const void *)bl.reps || b->graphOrder != (const void *)bl.order ||
+                         b->graphReps != (const void *)bl.reps || b->graphState != (const void *)bl.state || b->graphOrder != (const void *)bl.order ||
                          b->graphVariant != variant || b->graphSmem != bl.smem || b->graphMinBlocks != bl.minBlocks ||
                          !(b->graphCls == cls);
     if (rebuild) {
@@ -3671,6 +3684,7 @@ static femmd_status batch_launch(femmd_batch *b, const BatchLaunch &bl) {
         b->graphSteps = bl.steps;
         b->graphThreads = bl.threads;
         b->graphReps = bl.reps;
+        b->graphState = bl.state;
         b->graphOrder = bl.order;
         b->graphVariant = variant;
         b->graphSmem = bl.smem;
@@ -3727,7 +3741,9 @@ void femmd_batch_destroy(femmd_batch *b) {
     b->dreps.release();
     b->order.release();
     b->queue.release();
-    b->parity.release();
+    b->state.release();
+    b->out.release();
+    if (b->hout) cudaFreeHost(b->hout);
     for (auto e : b->ev)
         if (e) cudaEventDestroy(e);
     if (b->stream) cudaStreamDestroy(b->stream);
@@ -3786,9 +3802,12 @@ femmd_status femmd_batch_run(femmd_batch *b, int steps) {
         BatchLaunch bl;
         std::vector<DevSys> sys;
         if ((st = batch_prepare(b, steps, bl, sys))) return st;
-        if ((st = batch_checkpoint(b, false))) return st;
         if ((st = batch_launch(b, bl))) return st;
-        if ((st = batch_read(b))) return st;
+        const size_t R = b->reps.size();
+        BCK(cudaMemcpyAsync(b->hout, b->out.p, R * sizeof(DevScalars), cudaMemcpyDeviceToHost, b->stream));
+        BCK(cudaStreamSynchronize(b->stream));
+        for (size_t r = 0; r < R; r++)
+            if (!b->reps[r]->pos.empty()) *b->reps[r]->hsc = b->hout[r];
         bool over = false;
         for (femmd_ctx *c : b->reps) {
             if (c->pos.empty()) continue;

@@ -380,9 +380,17 @@ struct BatchClass {
         return cluster == o.cluster && first == o.first && count == o.count && ctas == o.ctas;
     }
 };
+// A replica's part in a launch: the parity of its positions, where its start
+// state is kept (for a repeat after an overflow) and where its scalars go.
+struct BatchRep {
+    float2 *ckPos, *ckVel, *ckAcc;
+    DevScalars *out;
+    int parity;
+};
 struct BatchLaunch {
     const DevSys *reps;
-    const int *order, *parity;
+    const BatchRep *state;
+    const int *order;
     int *queue;  // per class {next work index, finished CTAs}, zero before a launch
     int nclass;
     BatchClass cls[kBatchMaxCluster];

@@ -15,7 +15,8 @@
 // Bound by instruction issue where every SM is full, else by the largest
 // replicas: 128 replicas of 500 to 20,000 atoms (676,000 in all), run(100) with
 // the states copied in and out: 27.4 ms on one CTA or a pair each, 17.1 ms on
-// clusters by weight (23.5 ms with the packed pair terms alone).
+// clusters by weight (23.5 ms with the packed pair terms alone), 13.1 ms with the
+// start states kept and the scalars gathered by the launch.
 //
 // The per-particle and per-triangle arithmetic is step_body.cuh /
 // nn_body.cuh, the same code as the single-system kernels, and the list order
@@ -310,8 +311,8 @@ __device__ __noinline__ void block_step(const Team team, const DevSys &s, const 
 // team: descriptor and pair table into shared memory, run start, forced
 // rebuild, first force pass, steps with the half-skin rule, last step.
 template <bool MT, bool SG, bool WX, bool WY, bool SIG1, class Team>
-__device__ __forceinline__ void run_replica(const Team team, const DevSys *reps, int r, const int *parity0, int steps,
-                                            DevSys &S, PairEntry *tab, float *fscr, int *iscr, float *xch) {
+__device__ __forceinline__ void run_replica(const Team team, const DevSys *reps, int r, const BatchRep *state,
+                                            int steps, DevSys &S, PairEntry *tab, float *fscr, int *iscr, float *xch) {
     {
         const int *src = (const int *)(reps + r);
         int *dst = (int *)&S;
@@ -320,9 +321,20 @@ __device__ __forceinline__ void run_replica(const Team team, const DevSys *reps,
     __syncthreads();
     const int nt = S.numTypes > 1 ? S.numTypes * S.numTypes : 1;
     for (int w = threadIdx.x; w < nt; w += blockDim.x) tab[w] = S.pair[w];
+    const BatchRep rep = state[r];
+    int cur = rep.parity;
+    {
+        const float2 *x = cur ? S.pos1 : S.pos0;
+        for (int i = team.rank() * blockDim.x + threadIdx.x; i < S.N; i += team.size() * blockDim.x) {
+            rep.ckPos[i] = x[i];
+            rep.ckVel[i] = S.vel[i];
+            rep.ckAcc[i] = S.acc[i];
+        }
+    }
     if (team.rank() == 0 && threadIdx.x == 0) {
         // run start: NeighborList::update(1)
         DevScalars *c = S.sc;
+        c->overflow = c->nonfinite = c->outside = 0;
         c->rebuild = 1;
         c->dispHi = 0.0f;
         c->totalUpdates = 0;
@@ -330,7 +342,6 @@ __device__ __forceinline__ void run_replica(const Team team, const DevSys *reps,
         c->stepNow = S.stepBase;
     }
     team.sync();
-    int cur = parity0[r];
     block_rebuild(team, S, cur, iscr, xch);
     if (steps == 0) {
         block_step<MT, SG, WX, WY, SIG1>(team, S, tab, MODE_INIT, cur, fscr, xch);
@@ -348,6 +359,9 @@ __device__ __forceinline__ void run_replica(const Team team, const DevSys *reps,
         block_step<MT, SG, WX, WY, SIG1>(team, S, tab, MODE_LAST, cur, fscr, xch);
     }
     team.sync();
+    if (team.rank() == 0)
+        for (int w = threadIdx.x; w < (int)(sizeof(DevScalars) / sizeof(int)); w += blockDim.x)
+            reinterpret_cast<int *>(rep.out)[w] = __ldcg(reinterpret_cast<const int *>(S.sc) + w);
 }
 
 }  // namespace
@@ -359,7 +373,7 @@ __device__ __forceinline__ void run_replica(const Team team, const DevSys *reps,
 // queue.  MINB: resident CTAs per SM the register allocation must allow.
 template <bool MT, bool SG, bool WX, bool WY, bool SIG1, int MINB>
 __global__ void __launch_bounds__(1024, MINB) k_batch(const DevSys *__restrict__ reps, const int *__restrict__ order,
-                                                      int nwork, int *queue, const int *__restrict__ parity0,
+                                                      int nwork, int *queue, const BatchRep *__restrict__ state,
                                                       int steps) {
     __shared__ DevSys S;
     __shared__ float fscr[6 * 32];
@@ -374,7 +388,7 @@ __global__ void __launch_bounds__(1024, MINB) k_batch(const DevSys *__restrict__
         const int q = next;
         __syncthreads();
         if (q >= nwork) break;
-        run_replica<MT, SG, WX, WY, SIG1>(team, reps, order[q], parity0, steps, S, tab, fscr, iscr, xch);
+        run_replica<MT, SG, WX, WY, SIG1>(team, reps, order[q], state, steps, S, tab, fscr, iscr, xch);
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -391,7 +405,7 @@ __global__ void __launch_bounds__(1024, MINB) k_batch(const DevSys *__restrict__
 template <bool MT, bool SG, bool WX, bool WY, bool SIG1>
 __global__ void __launch_bounds__(1024, 1)
     k_batch_gang(const DevSys *__restrict__ reps, const int *__restrict__ order, int nwork, int *queue,
-                 const int *__restrict__ parity0, int steps) {
+                 const BatchRep *__restrict__ state, int steps) {
     __shared__ DevSys S;
     __shared__ float fscr[6 * 32];
     __shared__ float xch[6 * kBatchMaxCluster];
@@ -405,7 +419,7 @@ __global__ void __launch_bounds__(1024, 1)
         const int q = *cg::this_cluster().map_shared_rank(&next, 0);
         gang.sync();  // all have read the leader's pick before it changes
         if (q >= nwork) break;  // the same q in every CTA
-        run_replica<MT, SG, WX, WY, SIG1>(gang, reps, order[q], parity0, steps, S, tab, fscr, iscr, xch);
+        run_replica<MT, SG, WX, WY, SIG1>(gang, reps, order[q], state, steps, S, tab, fscr, iscr, xch);
     }
     if (threadIdx.x == 0) {
         __threadfence();
@@ -430,13 +444,13 @@ cudaError_t launch_batch(Launch &L, const BatchLaunch &b) {
         if (L.graph) L.deps = before;
         if (c.cluster > 1)
             e = L.kernel_clusters(k_batch_gang<MT, SG, WX, WY, SIG1>, c.cluster, dim3(c.ctas), dim3(b.threads), b.smem,
-                                  b.reps, b.order + c.first, c.count, queue, b.parity, b.steps);
+                                  b.reps, b.order + c.first, c.count, queue, b.state, b.steps);
         else if (b.minBlocks >= 2)
             e = L.kernel(k_batch<MT, SG, WX, WY, SIG1, 2>, dim3(c.ctas), dim3(b.threads), b.smem, b.reps,
-                         b.order + c.first, c.count, queue, b.parity, b.steps);
+                         b.order + c.first, c.count, queue, b.state, b.steps);
         else
             e = L.kernel(k_batch<MT, SG, WX, WY, SIG1, 1>, dim3(c.ctas), dim3(b.threads), b.smem, b.reps,
-                         b.order + c.first, c.count, queue, b.parity, b.steps);
+                         b.order + c.first, c.count, queue, b.state, b.steps);
     }
     return e;
 }
