@@ -16,7 +16,8 @@
 // replicas: 128 replicas of 500 to 20,000 atoms (676,000 in all), run(100) with
 // the states copied in and out: 27.4 ms on one CTA or a pair each, 17.1 ms on
 // clusters by weight (23.5 ms with the packed pair terms alone), 13.1 ms with the
-// start states kept and the scalars gathered by the launch.
+// start states kept and the scalars gathered by the launch, 12.7 ms with the
+// packed terms near the periodic edges too (the run alone 6.87 -> 6.47).
 //
 // The per-particle and per-triangle arithmetic is step_body.cuh /
 // nn_body.cuh, the same code as the single-system kernels, and the list order

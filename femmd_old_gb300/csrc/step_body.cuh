@@ -407,9 +407,10 @@ struct LjSums {
     float far, close;
 };
 
+template <bool EDGE, bool WX, bool WY>
 __device__ __forceinline__ void lj_pair_x2(const DevSys &s, float2 pi, float2 pj, float2 ce, float rcut2, float us,
                                            bool on, LjSums &a) {
-    const float4 t = lj_terms_x2<false, false, false>(s, pi, pj, ce, rcut2, us, on, a.far, a.close);
+    const float4 t = lj_terms_x2<EDGE, WX, WY>(s, pi, pj, ce, rcut2, us, on, a.far, a.close);
     a.F = add2(a.F, make_float2(t.x, t.y));
     a.UW = add2(a.UW, make_float2(t.z, t.w));
 }
@@ -532,6 +533,41 @@ __device__ __forceinline__ void finish_particle(const DevSys &s, int i, int mode
     we_out += we;
 }
 
+// Particle i's list by lj_pair_x2, four gathers in flight at a time.
+template <bool MT, bool EDGE, bool WX, bool WY, bool RO>
+__device__ __forceinline__ void lj_list_x2(const DevSys &s, const PairEntry *tab, int i, int cnt, float2 pi,
+                                           const float2 *pin, LjSums &a) {
+    const int4 *__restrict__ lst = reinterpret_cast<const int4 *>(s.nbr) + i;
+    const size_t row = (size_t)s.Ncap;
+    const int ti = MT ? s.typeId[i] * s.numTypes : 0;
+    const PairEntry pe0 = tab[0];
+    const int4 zero4 = make_int4(0, 0, 0, 0);
+    int4 g = cnt > 0 ? (RO ? __ldg(lst) : *lst) : zero4;
+    for (int base = 0; base < cnt; base += 4) {
+        lst += row;
+        const int4 gn = base + 4 < cnt ? (RO ? __ldg(lst) : *lst) : zero4;
+        const int tags[4] = {g.x, g.y, g.z, g.w};
+        float2 q[4];
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const int j = tags[u] & kIdMask;
+            q[u] = base + u < cnt ? (RO ? __ldg(pin + j) : pin[j]) : make_float2(pi.x + 1.0f, pi.y);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; u++) {
+            const bool on = base + u < cnt;  // (an unused word of the last group may hold anything)
+            if (MT) {
+                const float4 e =
+                    *reinterpret_cast<const float4 *>(tab + ti + (on ? (unsigned)tags[u] >> kIdBits : 0u));
+                lj_pair_x2<EDGE, WX, WY>(s, pi, q[u], make_float2(e.x, e.y), e.z, e.w, on, a);
+            } else {
+                lj_pair_x2<EDGE, WX, WY>(s, pi, q[u], make_float2(pe0.c, pe0.eps4), pe0.rcut2, pe0.us, on, a);
+            }
+        }
+        g = gn;
+    }
+}
+
 // One particle's step: bond, triangle and pair forces gathered in the order the
 // reference's CPU path adds them into force[i], then the mode's integration.
 // ue/we (doubled energy and virial), ke and vvm are accumulated by the caller.
@@ -549,39 +585,18 @@ __device__ __forceinline__ void particle_step(const DevSys &s, const PairEntry *
     const int cnt = min(s.nbrCount[i], s.nbrCap);
     bool done = false;
     if constexpr (SIG1 && !SG) {
-        // away from the periodic edges (all lanes of the warp that got here):
-        // the packed sums, four gathers in flight at a time
-        if (!__any_sync(__activemask(), near_edge<WX, WY>(s, pi))) {
-            const int4 *__restrict__ lst = reinterpret_cast<const int4 *>(s.nbr) + i;
-            const size_t row = (size_t)s.Ncap;
-            const int ti = MT ? s.typeId[i] * s.numTypes : 0;
-            const PairEntry pe0 = tab[0];
+        // the packed sums; the minimum image is taken where a lane of the warp
+        // is near a periodic edge.  There the read-only kernels take the pairs
+        // below (few of a large system's warps, and the second loop would cost
+        // them registers); in the batched kernel most warps are near an edge (a
+        // warp is a third of a lattice row of 10,000 particles).
+        const bool edge = __any_sync(__activemask(), near_edge<WX, WY>(s, pi));
+        if (!edge || !RO) {
             LjSums a = {make_float2(fx, fy), make_float2(ue, we), 0.0f, 1.0f};
-            const int4 zero4 = make_int4(0, 0, 0, 0);
-            int4 g = cnt > 0 ? (RO ? __ldg(lst) : *lst) : zero4;
-            for (int base = 0; base < cnt; base += 4) {
-                lst += row;
-                const int4 gn = base + 4 < cnt ? (RO ? __ldg(lst) : *lst) : zero4;
-                const int tags[4] = {g.x, g.y, g.z, g.w};
-                float2 q[4];
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const int j = tags[u] & kIdMask;
-                    q[u] = base + u < cnt ? (RO ? __ldg(pin + j) : pin[j]) : make_float2(pi.x + 1.0f, pi.y);
-                }
-#pragma unroll
-                for (int u = 0; u < 4; u++) {
-                    const bool on = base + u < cnt;  // (an unused word of the last group may hold anything)
-                    if (MT) {
-                        const float4 e =
-                            *reinterpret_cast<const float4 *>(tab + ti + (on ? (unsigned)tags[u] >> kIdBits : 0u));
-                        lj_pair_x2(s, pi, q[u], make_float2(e.x, e.y), e.z, e.w, on, a);
-                    } else {
-                        lj_pair_x2(s, pi, q[u], make_float2(pe0.c, pe0.eps4), pe0.rcut2, pe0.us, on, a);
-                    }
-                }
-                g = gn;
-            }
+            if (!RO && edge)
+                lj_list_x2<MT, !RO, WX, WY, RO>(s, tab, i, cnt, pi, pin, a);
+            else
+                lj_list_x2<MT, false, WX, WY, RO>(s, tab, i, cnt, pi, pin, a);
             if (lj_sums_ok<WX, WY>(s, a.far, a.close)) {
                 fx = a.F.x;
                 fy = a.F.y;
