@@ -284,14 +284,21 @@ def step_kernel_bytes(s, sc):
     return contract, minimum, st
 
 
-SMALL_RUN_MAX_ATOMS = 128 * 128  # 128 step blocks of 128 slots
+WHOLE_RUN_MAX_ATOMS = 98304  # kCoopMaxN (k_coop.cu)
+SMALL_RUN_MAX_ATOMS = 128 * 128  # 128 tiles of 128
+
+
+def whole_run_path(sc, n):
+    """Whether run() is one cooperative launch (k_coop; the library's
+    coop_whole, as far as a scene shows it)."""
+    return n <= WHOLE_RUN_MAX_ATOMS and "set_kArea" not in {nm for nm, a in sc.calls}
 
 
 def small_run_path(sc, n, bonded):
-    """Whether run() advances its middle steps in the cooperative small-system
-    run (k_fsmall) in the fast mode: one particle kind, no bonded particles,
-    walls, gravity or area springs, an XY-periodic box, at most 128 step
-    blocks (the library's small_run_fits, as far as a scene shows it)."""
+    """Whether the whole-run launch of a fast-mode system groups the energies by
+    storage slot and its rebuild kernel bins in one block: one particle kind, no
+    bonded particles, walls, gravity or area springs, an XY-periodic box, at
+    most 128 tiles."""
     names = {nm for nm, a in sc.calls}
     pbc = [a[0] for nm, a in sc.calls if nm == "PBC"]
     return (not bonded and n <= SMALL_RUN_MAX_ATOMS and sc.meta.get("types", 1) == 1 and pbc and pbc[-1] == 2
@@ -349,19 +356,17 @@ def ours(args, dist):
     # kernel launches inside the timed region
     has_tri = 1 if s.counts()["triangles"] else 0
     bonded = s._vertex_count() > 0
-    small = mode == "fast" and small_run_path(sc, n, bonded)
+    whole = whole_run_path(sc, n)
     if mode != "fast":
         rebuild_kernels = 7  # k_rebuild_begin, count, scan x2, scatter, cell sort, list build
-    elif not bonded and n <= SMALL_RUN_MAX_ATOMS:
+    elif small_run_path(sc, n, bonded):
         rebuild_kernels = 2  # k_fbin_small (binning and placement in one block), k_flist_p
     elif not bonded:
         rebuild_kernels = 7  # k_rebuild_begin, count, scan x2, scatter, k_fplace, k_flist_p
     else:
         rebuild_kernels = 10  # + k_ffree_count, k_fperm, k_fwindows, k_flist in place of k_flist_p
-    if small:
-        # run start, its forced rebuild, the first step, one k_fsmall (the
-        # middle steps and their rebuilds in one cooperative launch), the last step
-        launches = args.steps * (1 + rebuild_kernels + 3)
+    if whole:
+        launches = args.steps  # k_coop
     else:
         launches = args.steps * (1 + rebuild_kernels + (md + 1) * (1 + has_tri)) + rebuild_kernels * rebuilds
 
@@ -407,9 +412,9 @@ def ours(args, dist):
             "reciprocal" + ("" if bonded else "; persistent, a producer warp stages list rows and windows by "
                             "bulk asynchronous copies, packed float2 pair arithmetic")
             if fast else "reference-exact arithmetic and list order")
-    if small:
-        what += ("; timed by its own direct launches: inside run() the middle steps and their rebuilds run in "
-                 "k_fsmall, one cooperative launch with the same pair arithmetic")
+    if whole:
+        what += ("; timed by its own direct launches: a run() is one cooperative launch (k_coop) with the same "
+                 "pair arithmetic")
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": traffic,
                 "kernel": f"{kname} (fused LJ+bond+triangle gather, leapfrog, fixed-point energy sums; {what})",

@@ -360,8 +360,8 @@ class System:
         self._call("femmd_set_profiling", int(bool(on)))
 
     def test_expire_next_exchange(self):
-        """Tests of the failure path: the next small-system run's first
-        grid-wide exchange is left to time out (run() raises FEMMD_TIMEOUT)."""
+        """Tests of the failure path: the first grid-wide exchange of the
+        next run that is one cooperative launch is left to time out (run() raises FEMMD_TIMEOUT)."""
         self._call("femmd_test_expire_next_exchange")
 
     def counts(self):

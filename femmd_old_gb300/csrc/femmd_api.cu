@@ -167,7 +167,7 @@ struct femmd_ctx {
     int cur = 0;
     int nbrCap = 0, Ncap = 0, nBonded = 0, sigmaByType = 1, sigmaOne = 0;
     DBuf<float2> dpos0, dpos1, dvel, dacc, dforce, dref, ckPos, ckVel, ckAcc, triF, triLame;
-    DBuf<float> dmass, dsigma, denergy, triE, triTmp, wallDelta, wallSig;
+    DBuf<float> dmass, dsigma, denergy, triE, triTmp, engTmp, wallDelta, wallSig;
     bool ownMaterial = false, materialDirty = false;
     // area springs: kept positions and the per-mesh work list
     DBuf<float2> posPre;
@@ -202,11 +202,6 @@ struct femmd_ctx {
     DevScalars *hsc = nullptr;  // pinned mirror
     int obsCap = 0, obsRows = 0;
     GraphSet graphs[2][2];      // [parity][0: kGraphUnits units, 1: one unit]
-    GraphSet smallGraph;        // the small-system run's WHILE graph (fast mode)
-    bool smallGraphFailed = false;
-    // the small run's exchange records and tag base are zero (set again after
-    // a wait that gave up, which can leave records ahead of the tag base)
-    bool smallClean = false;
     bool testExpire = false;  // femmd_test_expire_next_exchange
     // the whole-run launch (k_coop): exchange slots and cell counts, zero
     // together with their scalars (runClean); coopOff: a cell held more than
@@ -244,7 +239,6 @@ struct femmd_ctx {
     int forceMode = FEMMD_FORCE_REFERENCE;
     DBuf<int> perm, sPerm, fBlockSums, ckPerm, idType, newCell;
     DBuf<int> blockWin;
-    DBuf<unsigned long long> smallRec;
     DBuf<float2> sPos, sVel, sAcc, cpos0, cpos1;
     DBuf<int> cslot;
     DBuf<float> idMass, idSigma, idWallDelta, idWallSig, xfer1;
@@ -338,7 +332,6 @@ static void mark_topology(femmd_ctx *c) {
 static void release_graphs(femmd_ctx *c) {
     for (auto &p : c->graphs)
         for (auto &g : p) g.release();
-    c->smallGraph.release();
 }
 
 static void release_device(femmd_ctx *c) {
@@ -346,7 +339,7 @@ static void release_device(femmd_ctx *c) {
     c->dpos0.release(); c->dpos1.release(); c->dvel.release(); c->dacc.release(); c->dforce.release();
     c->dref.release(); c->ckPos.release(); c->ckVel.release(); c->ckAcc.release(); c->triF.release();
     c->dmass.release(); c->dsigma.release(); c->denergy.release(); c->triE.release();
-    c->triTmp.release(); c->triOfs.release(); c->triOwn.release(); c->triLoc.release();
+    c->triTmp.release(); c->engTmp.release(); c->triOfs.release(); c->triOwn.release(); c->triLoc.release();
     c->dtype.release(); c->dexcl.release(); c->cellOf.release(); c->rank.release(); c->cellCount.release();
     c->cellStart.release(); c->blockSums.release(); c->sortedIds.release(); c->unsorted.release(); c->nbr.release();
     c->nbrCount.release(); c->bStart.release(); c->tStart.release(); c->tEnt.release(); c->bEnt.release();
@@ -360,7 +353,7 @@ static void release_device(femmd_ctx *c) {
     c->props.release(); c->propsCk.release(); c->propPart.release(); c->centroid.release();
     c->propsUploaded = false;
     c->perm.release(); c->sPerm.release(); c->fBlockSums.release(); c->ckPerm.release(); c->idType.release();
-    c->newCell.release(); c->blockWin.release(); c->smallRec.release(); c->runRec.release(); c->cellFill.release(); c->cellIds.release(); c->cellCand.release(); c->sPos.release(); c->sVel.release(); c->sAcc.release();
+    c->newCell.release(); c->blockWin.release(); c->runRec.release(); c->cellFill.release(); c->cellIds.release(); c->cellCand.release(); c->sPos.release(); c->sVel.release(); c->sAcc.release();
     c->cpos0.release(); c->cpos1.release(); c->cslot.release();
     c->idMass.release(); c->idSigma.release(); c->idWallDelta.release(); c->idWallSig.release(); c->xfer1.release();
     auto &a = c->adj;
@@ -550,7 +543,6 @@ static DevSys make_sys(femmd_ctx *c) {
         s.idWallSig = s.wallSig ? c->idWallSig.p : nullptr;
         s.newCell = c->newCell.p;
         s.blockWin = c->blockWin.p;
-        s.smallRec = c->smallRec.p;
         s.win16 = (c->nBonded == 0 && s.numTypes == 1 && s.sigmaByType) ? 1 : 0;
         if (c->cslot.p) {
             s.cpos0 = c->cpos0.p;
@@ -910,8 +902,6 @@ static femmd_status upload_topology(femmd_ctx *ctx) {
         CK(ctx->fBlockSums.ensure((N + 1023) / 1024));
         CK(ctx->newCell.ensure(N));
         CK(ctx->blockWin.ensure(kWinInts * (size_t)((N + kFastBlock - 1) / kFastBlock)));
-        CK(ctx->smallRec.ensure(4 * 16 + 3 * 4 * (size_t)kSmallMaxTiles));
-        ctx->smallClean = false;
         if (ctx->nBonded > 0) {
             // the cell-ordered position mirror (slot N: the ghost)
             CK(ctx->cpos0.ensure(N + 1)); CK(ctx->cpos1.ensure(N + 1)); CK(ctx->cslot.ensure(N));
@@ -1171,82 +1161,11 @@ static femmd_status build_graph(femmd_ctx *ctx, GraphSet &gs, int parity, int un
     return FEMMD_OK;
 }
 
-// The run graph of a small fast-mode system: WHILE (steps left) { the
-// cooperative small run; IF (rebuild) { the rebuild on parity 0 } }.
-static femmd_status build_small_graph(femmd_ctx *ctx, const DevSys &s) {
-    GraphSet &gs = ctx->smallGraph;
-    gs.release();
-    CK(cudaGraphCreate(&gs.g, 0));
-    Launch L;
-    L.stream = ctx->stream;
-    L.graph = gs.g;
-    cudaGraphConditionalHandle hw;
-    CK(cudaGraphConditionalHandleCreate(&hw, gs.g, 1, cudaGraphCondAssignDefault));
-    Launch body;
-    CK(L.begin_while(hw, body));
-    cudaGraphConditionalHandle hif;
-    CK(cudaGraphConditionalHandleCreate(&hif, body.graph, 0, cudaGraphCondAssignDefault));
-    CK(enqueue_small_run(body, s, hw, hif));
-    Launch rb;
-    CK(body.begin_if(hif, rb));
-    CK(enqueue_rebuild(rb, s, 0, 1));
-    CK(cudaGraphInstantiate(&gs.x, gs.g, 0));
-    return FEMMD_OK;
-}
-
-// A run's middle steps of a small fast-mode system (small_run_fits): one
-// graph launch whose WHILE loop runs the cooperative small run (each launch
-// up to the step that calls for a rebuild) and the rebuild kernels between
-// them, with no host round trip.  Without that graph (not instantiable here)
-// the host loops over direct cooperative launches, waiting once per launch.
-static femmd_status small_units(femmd_ctx *ctx, const DevSys &s, int units) {
-    DevScalars *d = ctx->sc.p;
-    // the small run starts from the current parity and ends on parity 0
-    ctx->hsc->smallLeft = units;
-    ctx->hsc->smallPar = ctx->cur;
-    ctx->hsc->testWithhold = ctx->testExpire ? 1 : 0;
-    ctx->testExpire = false;
-    static_assert(offsetof(DevScalars, smallPar) == offsetof(DevScalars, smallLeft) + sizeof(int) &&
-                      offsetof(DevScalars, testWithhold) == offsetof(DevScalars, smallLeft) + 2 * sizeof(int),
-                  "small-run scalars");
-    CK(cudaMemcpyAsync(&d->smallLeft, &ctx->hsc->smallLeft, 3 * sizeof(int), cudaMemcpyHostToDevice, ctx->stream));
-    ctx->cur = 0;
-    if (!ctx->smallClean) {
-        CK(cudaMemsetAsync(ctx->smallRec.p, 0, ctx->smallRec.n * sizeof(unsigned long long), ctx->stream));
-        CK(cudaMemsetAsync(&d->gbTag, 0, sizeof(unsigned), ctx->stream));
-        ctx->smallClean = true;
-    }
-    if (!ctx->smallGraphFailed && !ctx->smallGraph.x && build_small_graph(ctx, s) != FEMMD_OK) {
-        ctx->smallGraph.release();
-        ctx->smallGraphFailed = true;
-        cudaGetLastError();
-    }
-    if (ctx->smallGraph.x) {
-        CK(cudaGraphLaunch(ctx->smallGraph.x, ctx->stream));
-        return FEMMD_OK;
-    }
-    Launch L;
-    L.stream = ctx->stream;
-    for (int left = units; left > 0;) {
-        CK(launch_small_run(ctx->stream, s));
-        femmd_status st;
-        if ((st = read_scalars(ctx))) return st;
-        const int k = ctx->hsc->smallDone;
-        if (k <= 0 || ctx->hsc->smallLeft <= 0) {
-            if (ctx->hsc->rebuild) CK(enqueue_rebuild(L, s, 0, 1));
-            break;
-        }
-        left = ctx->hsc->smallLeft;
-        if (ctx->hsc->rebuild) CK(enqueue_rebuild(L, s, 0, 1));
-    }
-    return FEMMD_OK;
-}
-
 // A bounded wait gave up inside a run: the exchange records and their tag
 // bases start anew before the next one, and the cell counts of a binning that
 // did not finish are cleared.
 static femmd_status expired(femmd_ctx *ctx, const char *what) {
-    ctx->smallClean = ctx->runClean = false;
+    ctx->runClean = false;
     CK(cudaMemsetAsync(ctx->cellCount.p, 0, sizeof(int) * std::max(ctx->ncells, 1), ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return fail(ctx, FEMMD_TIMEOUT, "a bounded device wait expired (%s)", what);
@@ -1258,6 +1177,7 @@ static femmd_status expired(femmd_ctx *ctx, const char *what) {
 // is a phase of its own with an exchange after it).
 static CoopArgs coop_plan(femmd_ctx *ctx, const DevSys &s) {
     CoopArgs a = {};
+    if (coop_by_slot(s) && !ctx->engTmp.ensure(9 * (size_t)(s.N + kStepBlock))) a.eng = ctx->engTmp.p;
     const int nt = (int)ctx->refVol.size(), N = (int)ctx->pos.size(), grid = coop_grid(s);
     if (nt == 0 || grid == 0) return a;
     if (ctx->triGrid != grid) {
@@ -1325,7 +1245,7 @@ static bool coop_ready(femmd_ctx *ctx) {
 
 // A run, or part of one, of a small or medium system in one cooperative
 // launch (k_coop.cu); the parity follows its drifts.
-static femmd_status coop_launch(femmd_ctx *ctx, int begin, int units, int end, float2 *slots) {
+static femmd_status coop_launch(femmd_ctx *ctx, int begin, int units, int end, float2 *slots, int check = 0) {
     if (!ctx->runClean) {
         CK(cudaMemsetAsync(ctx->runRec.p, 0, ctx->runRec.n * sizeof(unsigned long long), ctx->stream));
         CK(cudaMemsetAsync(ctx->cellFill.p, 0, ctx->cellFill.n * sizeof(int), ctx->stream));
@@ -1337,6 +1257,7 @@ static femmd_status coop_launch(femmd_ctx *ctx, int begin, int units, int end, f
     CoopArgs a = coop_plan(ctx, s);
     a.parity = ctx->cur;
     a.begin = begin;
+    a.check = check;
     a.units = units;
     a.end = end;
     a.withhold = ctx->testExpire ? 1 : 0;
@@ -1351,13 +1272,10 @@ static femmd_status coop_launch(femmd_ctx *ctx, int begin, int units, int end, f
     return FEMMD_OK;
 }
 
-// Whether run(n) is one cooperative launch from its run start to its last
-// step (no trajectory frame inside it, no averaging, no direct launches; in
-// the fast mode, not a system of the small-system run).
+// Whether run(n) is a cooperative launch from its run start to its last step (or
+// from one trajectory frame to the next): no averaging, no direct launches.
 static bool coop_whole(femmd_ctx *ctx, int n) {
-    if (n <= 0 || ctx->profiling || ctx->propAvg || (ctx->traj.on && ctx->traj.every > 0)) return false;
-    if (fast_mode(ctx) && small_run_fits(make_sys(ctx))) return false;
-    return coop_ready(ctx);
+    return n > 0 && !ctx->profiling && !ctx->propAvg && coop_ready(ctx);
 }
 
 // Fast mode: the state back in id order (the whole-run launch keeps it so).
@@ -1379,11 +1297,6 @@ static femmd_status to_id_order(femmd_ctx *ctx) {
 
 static femmd_status launch_units(femmd_ctx *ctx, int units, bool use_graphs) {
     if (units <= 0) return FEMMD_OK;
-    if (use_graphs && !ctx->propAvg) {
-        const DevSys s = make_sys(ctx);
-        if (small_run_fits(s)) return small_units(ctx, s, units);
-        if (!fast_mode(ctx) && coop_ready(ctx)) return coop_launch(ctx, 0, units, 0, nullptr);
-    }
     if (!use_graphs) {
         DevSys s = make_sys(ctx);
         Launch L;
@@ -1819,8 +1732,47 @@ static void traj_refresh_meta(femmd_ctx *ctx) {
     frame_meta(ctx, T.meta);
 }
 
+// Trajectory frames of a run of n steps: the steps m in (s0, s0 + n] that are
+// multiples of 'every' (the reference's steps % trajectorySteps == 0).  Unit u
+// of the run computes the forces at x_{s0+u}; a frame inside the run replaces
+// its unit by LAST (completes v_m, keeps a_m), the copy, and the drift (half kick
+// with a_m, drift, wrap) followed by the rebuild check, which is the unit's work.
+static std::vector<int> run_frames(const femmd_ctx *ctx, int n) {
+    std::vector<int> frames;
+    const Trajectory &T = ctx->traj;
+    const int s0 = ctx->steps;
+    if (T.on && T.every > 0)
+        for (long long m = ((long long)s0 / T.every + 1) * T.every; m <= (long long)s0 + n; m += T.every)
+            if (m > T.lastCommitted) frames.push_back((int)m);
+    return frames;
+}
+
+// run_once in cooperative launches, one from a frame to the next.
+static femmd_status run_coop(femmd_ctx *ctx, int n, bool &aborted) {
+    const std::vector<int> frames = run_frames(ctx, n);
+    const int s0 = ctx->steps;
+    femmd_status st;
+    int u = 1, begin = 1;
+    for (int m : frames) {
+        const int upto = m - s0;
+        if (upto >= n) break;
+        if ((st = coop_launch(ctx, begin, upto - u, 1, nullptr, !begin))) return st;
+        if ((st = traj_snapshot(ctx, m, aborted))) return st;
+        if (aborted) return FEMMD_OK;
+        Launch D;
+        D.stream = ctx->stream;
+        CK(enqueue_drift_in_run(D, make_sys(ctx), ctx->cur));  // the next launch makes the rebuild check
+        ctx->cur ^= 1;
+        ctx->profKernels += D.kernels;
+        u = upto + 1;
+        begin = 0;
+    }
+    if ((st = coop_launch(ctx, begin, n - u, 1, nullptr, !begin))) return st;
+    return !frames.empty() && frames.back() == s0 + n ? traj_snapshot(ctx, s0 + n, aborted) : FEMMD_OK;
+}
+
 static femmd_status run_once(femmd_ctx *ctx, int n, bool whole, bool &aborted) {
-    if (whole) return coop_launch(ctx, 1, n - 1, 1, nullptr);
+    if (whole) return run_coop(ctx, n, aborted);
     DevSys s = make_sys(ctx);
     Launch L;
     L.stream = ctx->stream;
@@ -1839,18 +1791,8 @@ static femmd_status run_once(femmd_ctx *ctx, int n, bool whole, bool &aborted) {
     CK(enqueue_step(L, s, MODE_FIRST, ctx->cur, 0, 0));
     ctx->cur ^= 1;
     femmd_status st;
-    // trajectory frames at the steps m in (s0, s0 + n] that are multiples of
-    // 'every' (the reference's steps % trajectorySteps == 0).  Unit u of the
-    // run computes the forces at x_{s0+u}; a frame inside the run replaces
-    // its unit by LAST (completes v_m, keeps a_m), the copy, and the drift
-    // (half kick with a_m, drift, wrap) followed by the rebuild check, which
-    // is the unit's work bit for bit.
     const int s0 = ctx->steps;
-    std::vector<int> frames;
-    Trajectory &T = ctx->traj;
-    if (T.on && T.every > 0)
-        for (long long m = ((long long)s0 / T.every + 1) * T.every; m <= (long long)s0 + n; m += T.every)
-            if (m > T.lastCommitted) frames.push_back((int)m);
+    const std::vector<int> frames = run_frames(ctx, n);
     int u = 1;
     for (int m : frames) {
         const int upto = m - s0;

@@ -80,14 +80,9 @@ struct DevScalars {
     unsigned long long accU, accW, accK;  // fixed-point accumulators (two's complement)
     unsigned int vvMaxBits;               // max v^2 as float bits (v^2 >= 0)
     int sweepLost;                        // a bounded wait of k_adj_sweep expired
-    // the small-system run (k_fsmall): its exchanges so far, the steps one launch advanced, the steps left and the
-    // position parity the next launch starts from (it ends on parity 0)
-    unsigned int gbTag;
     // the whole-run launch (k_coop): the exchanges so far, and which of its two cell-count arrays the last rebuild used
     unsigned int runTag;
-    int runFill, pad2;
-    int smallDone, smallLeft, smallPar;
-    int testWithhold;  // the next small run's block 0 withholds its first exchange record (a test of the timeout)
+    int runFill;
 };
 
 enum StepMode { MODE_FORCES = 0, MODE_FIRST = 1, MODE_MID = 2, MODE_LAST = 3, MODE_INIT = 4 };
@@ -197,18 +192,14 @@ struct DevSys {
     // no bonded particles.  Other blocks keep 32-bit entries (nbr_at).
     int win16;
     int *blockWin;
-    // the small-system run's exchange slots (grid_sync.cuh), then three sets of
-    // kSmallMaxTiles records {-, U, W, K fixed point}
-    unsigned long long *smallRec;
     // the whole-run launch (k_coop): its exchange slots (grid_sync.cuh), then
-    // four sets of energy sums per block; its cells hold up to kCellCap particles
+    // four sets of energy sums and a word per block; its cells hold up to kCellCap particles
     // each (ids, then the candidates in id order; two arrays of counts in turn)
     unsigned long long *runRec;
     int *cellFill, *cellIds;
     float4 *cellCand;
 };
 
-constexpr int kSmallMaxTiles = 128;  // step blocks of the largest system the small-system run takes
 
 constexpr int kFastBlock = 128;  // storage slots per block of the fast step kernel
 constexpr int kWinMax = 768;     // window entries per block (the ghost included)
@@ -256,14 +247,6 @@ cudaError_t enqueue_unpermute1(Launch &L, const DevSys &s, const float *in, floa
 cudaError_t enqueue_permute2(Launch &L, const DevSys &s, const float2 *in, float2 *out);
 cudaError_t enqueue_perm_identity(Launch &L, const DevSys &s);
 cudaError_t enqueue_cpos_refresh(Launch &L, const DevSys &s, int parity);
-// The small-system run (k_fsmall): whether a system qualifies (fast mode, one
-// kind, no bonded particles, walls or gravity, XY-periodic, few step blocks,
-// every block resident), and one cooperative launch of up to 'steps' middle
-// steps, ending after a step that calls for a rebuild.
-bool small_run_fits(const DevSys &s);
-cudaError_t launch_small_run(cudaStream_t st, const DevSys &s);
-cudaError_t enqueue_small_run(Launch &L, const DevSys &s, cudaGraphConditionalHandle hw,
-                              cudaGraphConditionalHandle hif);
 cudaError_t enqueue_perm_consts(Launch &L, const DevSys &s);
 
 // A kernel's dynamic shared-memory limit raised to at least 'smem' and its
@@ -278,6 +261,7 @@ constexpr int kCellCap = 32;  // particles of a cell at most (a fuller one: the 
 struct CoopArgs {
     int parity;   // of the current positions
     int begin;    // the run start, forced rebuild and first step, and the checkpoint of the start state
+    int check;    // without 'begin': a rebuild first when the last step called for one (DevScalars::rebuild)
     int units;    // middle steps
     int end;      // the last step
     int withhold; // block 0 withholds its first exchange record (a test of the timeout)
@@ -292,7 +276,11 @@ struct CoopArgs {
     const int *triOfs, *triOwn, *triLoc;
     float *triTmp;
     int triMost, triLocal;  // triLocal: they are used (the launch sets it)
+    float *eng;  // coop_by_slot: three sets of the particles' U, W, m v^2 in slot order, else null
 };
+// Whether a launch groups the particles' energies by storage slot, as the fast
+// mode's step kernels do (small systems of one type without bonded particles).
+bool coop_by_slot(const DevSys &s);
 bool coop_size_ok(int N, int ncells);
 bool coop_run_fits(const DevSys &s, const CoopArgs &plan);
 // The blocks of a system; with triangles by block, the block of a tile of 128 particles.

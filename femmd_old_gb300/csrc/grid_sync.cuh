@@ -1,5 +1,5 @@
-// grid_sync.cuh -- the grid-wide exchange of the cooperative run kernels
-// (k_coop.cuh, k_fsmall in k_fast.cu).
+// grid_sync.cuh -- the grid-wide exchange of the cooperative kernels
+// (k_coop in k_coop.cuh, k_adj_sweep in k_adjoint.cu).
 //
 // An exchange is a barrier over the grid that carries the maximum of one
 // unsigned value per block and the OR of another.  Each block's thread 0 adds

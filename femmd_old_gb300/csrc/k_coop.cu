@@ -13,11 +13,12 @@ namespace {
 // run(50) against the plain kernels' graph (us): LJ fluid 67,600 particles
 // 1148 / 1539, 160,000 2095 / 1848 (equal near 125,000); disks in solvent
 // 68,288 1512 / 1787, 150,800 2662 / 2111 (96,000); suspension 32,512
-// 650 / 923, 130,048 1336 / 1254 (108,000).
+// 650 / 923, 130,048 1336 / 1254 (108,000).  In the fast mode (LJ fluid) 90,000
+// particles 1131 / 1420.
 constexpr int kCoopMaxN = 98304;
 
-const void *coop_kernel(const DevSys &s) {
-    if (s.fast) return coop_kernel_fast(s);
+const void *coop_kernel(const DevSys &s, bool bySlot) {
+    if (s.fast) return bySlot ? coop_kernel_slot(s) : coop_kernel_fast(s);
     if (!s.sigmaByType) return coop_kernel_sigma(s);
     return s.numTypes > 1 ? coop_kernel_types(s) : coop_kernel_one(s);
 }
@@ -37,6 +38,7 @@ bool coop_shape(const DevSys &s, int &grid, size_t &smem, CoopArgs &a) {
     smem = coop_terms(s.fast) * (size_t)kTermComp * sizeof(float) + (size_t)per * 4 * kStepBlock * sizeof(int);  // terms, sums, counts
     const size_t inc = (size_t)per * kIncWords * kStepBlock * sizeof(int), tri = (size_t)tper * kTriTile * sizeof(int4);
     const size_t row = 4 * (size_t)per * kListRow * sizeof(int);  // four list rows
+    if (a.eng) smem += (size_t)per * kStepBlock * sizeof(int);  // slots
     a.incStaged = s.nBonded > 0 && smem + inc + row <= kCoopSmem;
     if (a.incStaged) smem += inc;
     a.triLocal = a.triMost > 0 && a.incStaged && smem + own + row <= kCoopSmem;
@@ -60,6 +62,15 @@ int coop_grid(const DevSys &s) {
     return std::max(1, std::min(std::min(sms, kCoopMaxBlocks), std::max(ntiles, ntt)));
 }
 
+// Up to 128 tiles (a block has one then), cells whose starts fit the terms' place.
+// The step kernels' per-step energies differ from sums in id order by float
+// rounding; larger systems' sums are in id order (a slot of every particle after
+// every rebuild would cost them a scan of all cells per block).
+bool coop_by_slot(const DevSys &s) {
+    return s.fast && s.numTypes <= 1 && s.nBonded == 0 && s.N <= 128 * kStepBlock &&
+           s.ncells <= coop_terms(true) * kTermComp;
+}
+
 int coop_block(int ntiles, int grid, int tile) { return coop_pairs(ntiles, grid) ? tile / 2 : tile % grid; }
 
 bool coop_run_fits(const DevSys &s, const CoopArgs &plan) {
@@ -68,7 +79,7 @@ bool coop_run_fits(const DevSys &s, const CoopArgs &plan) {
     size_t smem;
     CoopArgs a = plan;
     if (!coop_shape(s, grid, smem, a)) return false;
-    if (kernel_setup(coop_kernel(s), kCoopThreads, smem, &resident)) return false;
+    if (kernel_setup(coop_kernel(s, a.eng), kCoopThreads, smem, &resident)) return false;
     return resident >= grid;
 }
 
@@ -83,7 +94,7 @@ cudaError_t launch_coop_run(cudaStream_t st, const DevSys &s, const CoopArgs &a)
     CoopArgs aa = a;
     if (!coop_shape(s, grid, smem, aa)) return cudaErrorInvalidConfiguration;
     void *args[] = {&sa, &aa};
-    return cudaLaunchCooperativeKernel(coop_kernel(s), dim3(grid), dim3(kCoopThreads), args, smem, st);
+    return cudaLaunchCooperativeKernel(coop_kernel(s, a.eng), dim3(grid), dim3(kCoopThreads), args, smem, st);
 }
 
 }  // namespace femmd

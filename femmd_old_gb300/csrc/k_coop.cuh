@@ -37,7 +37,9 @@
 // get_state; us): LJ fluid 400 particles run(20) 659 -> 207, 10,201 run(50)
 // 1390 -> 407; 256-disk suspension (32,512) run(100) 1842 -> 849; adjoint of 64
 // disks over 200 steps 14,260 -> 5200; fast mode, run(50): LJ fluid 90,000 1408
-// -> 1112, 144 disks in solvent (68,288) 1778 -> 1137.  The particle pass of the 10,201
+// -> 1112, 144 disks in solvent (68,288) 1778 -> 1137, run(100) of 4096 1275 -> 749
+// (1060 by a kernel of its own for small fluids, a thread per particle, with
+// five launches around it).  The particle pass of the 10,201
 // particles takes 4.1 us; a thread per particle instead of a quad took 7.7.
 //
 // The per-particle and per-triangle arithmetic and the list order are those
@@ -54,7 +56,9 @@
 // pair's factors into shared memory and the sums are formed there.  The
 // launch keeps the particles in id order: the lists' order does not depend on
 // the storage order, and it leaves lists without windows behind (storage
-// slots, padded with the ghost's).
+// slots, padded with the ghost's).  Small systems' energies are grouped by the
+// storage slot the step kernels would have the particle in (coop_by_slot): a
+// particle's go to its slot in memory and are added up a step later.
 //
 // Exchanges are grid_exchange's (grid_sync.cuh), bounded: a wait that gives
 // up sets the timeout flag, and the block leaves the kernel.  They are numbered
@@ -253,6 +257,10 @@ struct CoopMem {
     int4 *tri;
     float2 *triF;
     int tiles, first, stride;  // the block's tiles of particles: first, first + stride, ...
+    // by slot: the storage slot of the block's particles [tile][kStepBlock], and where the step's U, W, m v^2 go ([3][engRow], by slot)
+    int *slot;
+    float *eng;
+    size_t engRow;
 };
 
 // The tiles of block b.  Tile j is b + j grid, so that bonded and free particles
@@ -355,6 +363,7 @@ __device__ __forceinline__ int coop_list(const DevSys &s, const CoopMem &mem, co
 // at most kCellCap particles by counting atomics, the in-cell order by id,
 // and the lists of the block's own particles.  Two exchanges.  False when one
 // gave up.
+template <bool SLOT>
 __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, const CoopMem &mem, CoopRun &r, int p,
                                           bool withhold) {
     const float2 *pos = p ? s.pos1 : s.pos0;
@@ -386,6 +395,24 @@ __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, co
     // 2: ascending id inside each cell; the other counts cleared for the next
     // rebuild (their last readers were the lists before this rebuild)
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < s.ncells; c += gridDim.x * blockDim.x) other[c] = 0;
+    [[maybe_unused]] int *start = reinterpret_cast<int *>(mem.term);  // by slot: the cells' starts (no terms there now)
+    if constexpr (SLOT) {
+        const int chunk = (s.ncells + blockDim.x - 1) / blockDim.x;
+        const int c0 = min((int)threadIdx.x * chunk, s.ncells), c1 = min(c0 + chunk, s.ncells);
+        int sum = 0, tot;
+        for (int c = c0; c < c1; c++) {
+            const int n = min(__ldcg(cnt + c), kCellCap);
+            start[c] = n;
+            sum += n;
+        }
+        int at = block_scan(sh, sum, tot);
+        for (int c = c0; c < c1; c++) {
+            const int n = start[c];
+            start[c] = at;
+            at += n;
+        }
+        __syncthreads();
+    }
     if (!skip)
         for (int j = grp; j < mem.tiles; j += groups) {
             const int i = (mem.first + j * mem.stride) * kStepBlock + gt;
@@ -401,6 +428,7 @@ __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, co
 #pragma unroll
                 for (int u = 0; u < 8; u++) k += q + u < n && id[u] < i;
             }
+            if constexpr (SLOT) mem.slot[j * kStepBlock + gt] = min(start[c] + k, s.N - 1);
             s.cellCand[(size_t)c * kCellCap + k] = make_float4(x.x, x.y, __int_as_float(tag), __int_as_float(gi));
         }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
@@ -532,7 +560,7 @@ __device__ __forceinline__ float4 coop_pair(const DevSys &s, const PairEntry *ta
 // finish_particle (FAST: fast_finish), an axis per lane (lanes 2 and 3 along
 // with 0 and 1).  f: lanes 0 and 1, the axis' force; e2: lanes 2 and 3, the
 // doubled energy and virial.
-template <bool WX, bool WY, bool FAST>
+template <bool WX, bool WY, bool FAST, bool SLOT>
 __device__ __forceinline__ void coop_finish(const DevSys &s, const CoopMem &mem, int i, bool on, int j, int col, int q,
                                             int mode, int stepNow, float2 pi, float m, float2 v2, float f, float e2,
                                             float uwall, float2 *pout, float2 *slot, float &vvm, bool &bad) {
@@ -565,10 +593,17 @@ __device__ __forceinline__ void coop_finish(const DevSys &s, const CoopMem &mem,
             vv = __shfl_sync(0xffffffffu, vv, threadIdx.x & 30);
         }
     }
-    float *part = mem.part + (size_t)j * 3 * kStepBlock + col;
-    if (q == 2) part[0] = on ? e : 0.0f;
-    if (q == 3) part[kStepBlock] = on ? e : 0.0f;
-    if (q == 0) part[2 * kStepBlock] = on ? m * vv : 0.0f;
+    if constexpr (SLOT) {
+        if (on && q != 1) {
+            const int at = mem.slot[j * kStepBlock + col];
+            mem.eng[(q == 0 ? 2 : q - 2) * mem.engRow + at] = q == 0 ? m * vv : e;
+        }
+    } else {
+        float *part = mem.part + (size_t)j * 3 * kStepBlock + col;
+        if (q == 2) part[0] = on ? e : 0.0f;
+        if (q == 3) part[kStepBlock] = on ? e : 0.0f;
+        if (q == 0) part[2 * kStepBlock] = on ? m * vv : 0.0f;
+    }
     if (on && q < 2) {
         vvm = fmaxf(vvm, vv);
         float *vel = reinterpret_cast<float *>(s.vel + i) + q;
@@ -593,7 +628,7 @@ __device__ __forceinline__ void coop_finish(const DevSys &s, const CoopMem &mem,
 // Lane 0 forms sum fc dx, lane 1 sum fc dy; one type: lane 2 sum ir6^2 and sum
 // ir6, lane 3 sum ir2 r2 (the pairs inside the cutoff), each over the even and
 // the odd entries apart; several types: lane 2 sum u, lane 3 sum fc r2.
-template <bool MT, bool WX, bool WY, bool SIG1, class Gather>
+template <bool MT, bool WX, bool WY, bool SIG1, bool SLOT, class Gather>
 __device__ __forceinline__ void fast_sums(const DevSys &s, const CoopMem &mem, const PairEntry *tab, Gather &gather,
                                           int most, int cnt, int q, int col, int ti, const int *tag, const float2 *pj,
                                           float2 pi, bool near, float fx, float fy, float ue, float uwall, float m,
@@ -666,13 +701,13 @@ __device__ __forceinline__ void fast_sums(const DevSys &s, const CoopMem &mem, c
         if (q == 1) f = fy + S;
         e2 = q == 2 ? ue + __fmaf_rn(pe0.eps4, A - B, pe0.us * n) : pe0.eps48 * __fmaf_rn(-0.5f, B, A);
     }
-    coop_finish<WX, WY, true>(s, mem, i, on, j, col, q, mode, stepNow, pi, m, v2, f, e2, uwall, pout, slot, vvm, bad);
+    coop_finish<WX, WY, true, SLOT>(s, mem, i, on, j, col, q, mode, stepNow, pi, m, v2, f, e2, uwall, pout, slot, vvm, bad);
 }
 
 // particle_step for one particle by the four lanes of a quad (lane 'q' of 0 ..
 // 3; particle i, slot 'col' of the block's tile j; on: i < N).  All lanes of
 // the warp call it.
-template <bool MT, bool SG, bool WX, bool WY, bool SIG1, bool FAST>
+template <bool MT, bool SG, bool WX, bool WY, bool SIG1, bool FAST, bool SLOT>
 __device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &mem, const PairEntry *tab, int i, bool on,
                                               int j, int col, int q, int mode, int stepNow, const float2 *pin,
                                               float2 *pout, float2 *slot, float &vvm, bool &bad) {
@@ -740,7 +775,7 @@ __device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &me
     }
     const bool near = __any_sync(0xffffffffu, on && near_edge<WX, WY>(s, pi));
     if constexpr (FAST) {
-        fast_sums<MT, WX, WY, SIG1>(s, mem, tab, gather, most, cnt, q, col, ti, tag, pj, pi, near, fx, fy, ue, uwall,
+        fast_sums<MT, WX, WY, SIG1, SLOT>(s, mem, tab, gather, most, cnt, q, col, ti, tag, pj, pi, near, fx, fy, ue, uwall,
                                     m, v2, i, on, j, mode, stepNow, pout, slot, vvm, bad);
         return;
     }
@@ -792,7 +827,7 @@ __device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &me
         for (int k = 0; k < rows; k++) sum += mine[k * kTermRow];
         __syncwarp();
     }
-    coop_finish<WX, WY, false>(s, mem, i, on, j, col, q, mode, stepNow, pi, m, v2, q < 2 ? sum : 0.0f, sum, uwall, pout,
+    coop_finish<WX, WY, false, false>(s, mem, i, on, j, col, q, mode, stepNow, pi, m, v2, q < 2 ? sum : 0.0f, sum, uwall, pout,
                                slot, vvm, bad);
 }
 
@@ -825,6 +860,24 @@ __device__ __forceinline__ void coop_block_sums(const DevSys &s, CoopShared &sh,
     if (ob) atomicOr(&s.sc->nonfinite, 2);
 }
 
+// By slot: the energies of a step (e) over the block's tiles of slots, as
+// coop_block_sums.  Warps w0, w0 + 1, w0 + 2 take U, W, K.
+__device__ __forceinline__ void coop_slot_sums(const DevSys &s, CoopShared &sh, const CoopMem &mem, const float *e, int w0) {
+    const int lane = threadIdx.x & 31, c = (int)(threadIdx.x >> 5) - w0;
+    if (c < 0 || c >= 3) return;
+    bool ob = false;
+    for (int j = 0; j < mem.tiles; j++) {
+        const int t = (mem.first + j * mem.stride) * kStepBlock + lane;
+        float v[kStepBlock / 32], x = 0.0f;
+#pragma unroll
+        for (int g = 0; g < kStepBlock / 32; g++) v[g] = t + 32 * g < s.N ? __ldcg(e + c * mem.engRow + t + 32 * g) : 0.0f;
+#pragma unroll
+        for (int g = 0; g < kStepBlock / 32; g++) x += warp_sum_f(v[g]);
+        if (lane == 0) atomicAdd(&sh.acc[c], to_fixed(x, ob));
+    }
+    if (ob) atomicOr(&s.sc->nonfinite, 2);
+}
+
 // Triangles by block: the energies 'e' of all the triangles, summed over the block's
 // triangle tiles as coop_block_sums does.  Warps w0, w0 + 1, ... share
 // the tiles, the last one first.
@@ -849,9 +902,11 @@ __device__ __forceinline__ void coop_tri_block_sums(const DevSys &s, CoopShared 
 // force pass, half kick and drift) and the checkpoint of the start state;
 // then 'units' middle steps, each followed by its rebuild when the half-skin
 // rule calls for one; with 'end', the last step.  slots: when not null, the
-// positions after drift u go to slots + (u + 1) N too.
-template <bool MT, bool SG, bool WX, bool WY, bool SIG1, bool FAST>
-__global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) {
+// positions after drift u go to slots + (u + 1) N too.  The parameters are grid
+// constants: one whose address a function takes would be copied to local memory
+// (256 disks, run(100): 825 us with the copy, 780 without).
+template <bool MT, bool SG, bool WX, bool WY, bool SIG1, bool FAST, bool SLOT>
+__global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant__ DevSys s, const __grid_constant__ CoopArgs a) {
     extern __shared__ int4 dyn[];
     __shared__ CoopShared sh;
     DevScalars *sc = s.sc;
@@ -890,6 +945,21 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
     mem.count = reinterpret_cast<int *>(mem.part + (size_t)per * 3 * kStepBlock);
     mem.inc = a.incStaged ? mem.count + per * kStepBlock : nullptr;
     mem.list = mem.count + per * kStepBlock + (a.incStaged ? per * kIncWords * kStepBlock : 0);
+    if constexpr (SLOT) {
+        mem.engRow = s.N;
+        mem.eng = nullptr;
+        mem.slot = mem.list;
+        mem.list += per * kStepBlock;
+        for (int q = threadIdx.x; q < per * kStepBlock; q += blockDim.x) mem.slot[q] = 0;  // (a rebuild that is cut short)
+        __syncthreads();
+        if (!a.begin)  // as the last rebuild left it
+            for (int t = threadIdx.x; t < s.N; t += blockDim.x) {
+                const int i = s.sortedIds[t], k = i / kStepBlock - mem.first;
+                if (k >= 0 && k % mem.stride == 0 && k / mem.stride < mem.tiles)
+                    mem.slot[k / mem.stride * kStepBlock + i % kStepBlock] = t;
+            }
+    }
+    const bool late = local || SLOT;  // a step's last sums are added after the next step's exchange
     if (a.begin) {
         const float2 *x = p ? s.pos1 : s.pos0;
         for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < s.N; i += gridDim.x * blockDim.x) {
@@ -941,11 +1011,11 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
     __syncthreads();
     bool ok = true;
     const int updates0 = r.updates;
-    bool rebuild = a.begin != 0;
+    bool rebuild = a.begin || (a.check && __ldcg(&sc->rebuild));
     const int total = (a.begin ? 1 : 0) + a.units + (a.end ? 1 : 0);
     for (int u = 0;; u++) {
         if (rebuild) {
-            if (!(ok = coop_rebuild(s, sh, mem, r, p, withhold))) break;
+            if (!(ok = coop_rebuild<SLOT>(s, sh, mem, r, p, withhold))) break;
             withhold = false;
         }
         if (u >= total) break;
@@ -983,11 +1053,16 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
             if (!(ok = coop_exchange(s, sh, r, 0u, withhold))) break;
             withhold = false;
         }
+        [[maybe_unused]] const float *lastEng = nullptr;
+        if constexpr (SLOT) {
+            lastEng = mem.eng;
+            mem.eng = a.eng + (size_t)(r.dueIn % 3u) * 3 * mem.engRow;
+        }
         float vvm = 0.0f;
         bool bad = false;
         for (int j = 0; j < mem.tiles; j++) {
             const int col = threadIdx.x >> 2, i = (mem.first + j * mem.stride) * kStepBlock + col;
-            coop_particle<MT, SG, WX, WY, SIG1, FAST>(s, mem, sh.tab, i, i < s.N, j, col, threadIdx.x & 3, mode, r.stepNow,
+            coop_particle<MT, SG, WX, WY, SIG1, FAST, SLOT>(s, mem, sh.tab, i, i < s.N, j, col, threadIdx.x & 3, mode, r.stepNow,
                                                 pin, pout, a.slots ? a.slots + (size_t)(u + 1) * s.N : nullptr, vvm,
                                                 bad);
         }
@@ -1003,7 +1078,8 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
         if (warp == 0) mm = warp_max(lane < kCoopThreads / 32 ? sh.vmax[lane] : 0.0f);
         if (!(ok = coop_exchange(s, sh, r, __float_as_uint(mm), withhold, false,
                                  [&] {
-                                     coop_block_sums(s, sh, mem, local ? 0 : ttiles, 3);
+                                     if constexpr (!SLOT) coop_block_sums(s, sh, mem, local ? 0 : ttiles, 3);
+                                     else if (r.dueIn > 0) coop_slot_sums(s, sh, mem, lastEng, 3);
                                      if (local && r.dueIn > 0)
                                          coop_tri_block_sums(s, sh, a.triTmp + (size_t)((r.dueIn - 1) % 3u) * s.ntri,
                                                              ttiles, 3);
@@ -1011,12 +1087,13 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
             break;
         withhold = false;
         if (threadIdx.x < 3) {
-            // visible to the others with this block's next exchange
-            atomicAdd(coop_sums(s, r.dueIn) + threadIdx.x, sh.acc[threadIdx.x]);
+            // visible to the others with this block's next exchange (by slot: the
+            // previous step's; none, zeros, after the first)
+            atomicAdd(coop_sums(s, SLOT ? r.dueIn - 1 : r.dueIn) + threadIdx.x, sh.acc[threadIdx.x]);
             sh.acc[threadIdx.x] = 0ull;
         }
-        if (local && r.dueIn > 0) {
-            if (threadIdx.x == 3) {
+        if (late && r.dueIn > 0) {
+            if (local && threadIdx.x == 3) {
                 atomicAdd(coop_sums(s, r.dueIn - 1), sh.accTri);
                 sh.accTri = 0ull;
             }
@@ -1043,13 +1120,18 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
             sc->rebuild = reb;
         }
         r.dueIn++;
-        if (!local) r.dueOk = r.dueIn;
+        if (!late) r.dueOk = r.dueIn;
         if (mode != MODE_FIRST) r.row++;
         if (mode != MODE_LAST) {
             r.stepNow++;
             p ^= 1;
         }
         rebuild = mode == MODE_MID && reb;
+    }
+    if constexpr (SLOT) if (ok && r.dueIn > 0) {
+        coop_slot_sums(s, sh, mem, mem.eng, 0);
+        __syncthreads();
+        if (threadIdx.x < 3) atomicAdd(coop_sums(s, r.dueIn - 1) + threadIdx.x, sh.acc[threadIdx.x]);
     }
     if (ok && local && r.dueIn > 0) {
         // the last step's triangle energies
@@ -1078,19 +1160,19 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(DevSys s, CoopArgs a) 
 
 // The kernel of a system with (MT) several types and (SG) a sigma per
 // particle, in the fast mode or not.
-template <bool MT, bool SG, bool WX, bool WY, bool FAST>
+template <bool MT, bool SG, bool WX, bool WY, bool FAST, bool SLOT>
 const void *coop_sig(const DevSys &s) {
     if constexpr (!SG && !(FAST && MT)) {
-        if (s.sigmaOne) return (const void *)k_coop<MT, SG, WX, WY, true, FAST>;
+        if (s.sigmaOne) return (const void *)k_coop<MT, SG, WX, WY, true, FAST, SLOT>;
     }
-    return (const void *)k_coop<MT, SG, WX, WY, false, FAST>;
+    return (const void *)k_coop<MT, SG, WX, WY, false, FAST, SLOT>;
 }
 
-template <bool MT, bool SG, bool FAST = false>
+template <bool MT, bool SG, bool FAST = false, bool SLOT = false>
 const void *coop_image(const DevSys &s) {
-    if (s.wrapx && s.wrapy) return coop_sig<MT, SG, true, true, FAST>(s);
-    if (s.wrapx) return coop_sig<MT, SG, true, false, FAST>(s);
-    return coop_sig<MT, SG, false, false, FAST>(s);
+    if (s.wrapx && s.wrapy) return coop_sig<MT, SG, true, true, FAST, SLOT>(s);
+    if (s.wrapx) return coop_sig<MT, SG, true, false, FAST, SLOT>(s);
+    return coop_sig<MT, SG, false, false, FAST, SLOT>(s);
 }
 
 // one translation unit each
@@ -1098,5 +1180,6 @@ const void *coop_kernel_one(const DevSys &s);    // k_coop.cu
 const void *coop_kernel_types(const DevSys &s);  // k_coop_types.cu
 const void *coop_kernel_sigma(const DevSys &s);  // k_coop_sigma.cu
 const void *coop_kernel_fast(const DevSys &s);   // k_coop_fast.cu
+const void *coop_kernel_slot(const DevSys &s);   // k_coop_slot.cu
 
 }  // namespace femmd

@@ -141,7 +141,7 @@ __global__ void __launch_bounds__(kBlock) k_fplace(DevSys s, int parity, int che
 // new order in the scratch arrays); the placement inside a cell is by id, so
 // the order of the counting atomics leaves no trace.
 constexpr int kSmallBinThreads = 1024;
-constexpr int kSmallBinMaxN = kSmallMaxTiles * kFastBlock;
+constexpr int kSmallBinMaxN = 128 * kFastBlock;
 constexpr int kSmallBinPer = kSmallBinMaxN / kSmallBinThreads;  // particles per thread at most
 constexpr size_t kSmallBinMaxSmem = 200 * 1024;
 
@@ -920,10 +920,7 @@ __device__ __forceinline__ void fpair(const DevSys &s, const PairEntry *tab, con
 // pin.  Unused words of the last group name the ghost, so no entry needs a
 // count test.  Energy and virial come back doubled (per ordered pair), as
 // the reference-exact kernel's.
-// NC: the positions stay unchanged for the whole launch, so their gathers
-// may take the non-coherent path; otherwise (the small-system run, where
-// other blocks write them between steps) they are read from L2.
-template <bool MT, bool SG, bool SIG1, bool WX, bool WY, bool IMG, bool WIN, bool NC = true>
+template <bool MT, bool SG, bool SIG1, bool WX, bool WY, bool IMG, bool WIN>
 __device__ __forceinline__ void fast_pairs(const DevSys &s, const PairEntry *tab, int i, float2 pi, int cnt,
                                            const int4 *slist, int srows, const float2 *__restrict__ pin,
                                            const float2 *wpos,
@@ -968,7 +965,7 @@ __device__ __forceinline__ void fast_pairs(const DevSys &s, const PairEntry *tab
                 if (SG) sj[u] = wsig[w];
             } else {
                 const int j = MT ? (e[u] & kIdMask) : e[u];
-                q[u] = NC ? __ldg(pin + j) : __ldcg(pin + j);
+                q[u] = __ldg(pin + j);
                 if (MT) tj[u] = (unsigned)e[u] >> kIdBits;
                 if (SG) sj[u] = __ldg(s.sigma + j);
             }
@@ -1014,7 +1011,7 @@ __device__ __forceinline__ float2 img2(float2 d, float2 q, float2 a, float L) {
 }
 
 // IMG: a warp at a periodic edge (WX, WY): the packed exact image per pair.
-template <bool SIG1, bool WIN, bool W16, bool NC = true, bool IMG = false, bool WX = false, bool WY = false>
+template <bool SIG1, bool WIN, bool W16, bool IMG = false, bool WX = false, bool WY = false>
 __device__ __forceinline__ void fast_pairs_x2(const DevSys &s, const PairEntry &pe, int i, float2 pi, int cnt,
                                               const int4 *slist, int srows, const float2 *__restrict__ pin,
                                               const float2 *wpos, float &fx, float &fy, float &ue2, float &we2) {
@@ -1071,7 +1068,7 @@ __device__ __forceinline__ void fast_pairs_x2(const DevSys &s, const PairEntry &
 #pragma unroll
             for (int u = 0; u < 4; u++)
                 q[u] = WIN ? wpos[min((unsigned)e[u], (unsigned)kWinGhost)]
-                           : (NC ? __ldg(pin + e[u]) : __ldcg(pin + e[u]));
+                           : __ldg(pin + e[u]);
             quad(q);
         }
     }
@@ -1091,7 +1088,7 @@ __device__ __forceinline__ void fast_finish(const DevSys &s, int i, int mode, fl
                                             float2 *pout, float2 *cpout, float fx, float fy, float ue, float we,
                                             float utri,
                                             float uwall, float &ue_out, float &we_out, float &ke, float &vvm,
-                                            bool &bad, float2 *xo = nullptr, float2 *vo = nullptr) {
+                                            bool &bad) {
     ue *= 0.5f;
     we *= 0.5f;
     ue += uwall;
@@ -1140,8 +1137,6 @@ __device__ __forceinline__ void fast_finish(const DevSys &s, int i, int mode, fl
             pout[i] = x;
             if (cpout) cpout[s.cslot[i]] = x;  // the cell-ordered mirror
             s.vel[i] = v;
-            if (xo) *xo = x;
-            if (vo) *vo = v;
         }
     }
     ue_out += ue;
@@ -1590,7 +1585,7 @@ __global__ void __launch_bounds__(kPBlock, kPMinBlocks) k_fstep_p(DevSys s, int 
                     }
                 } else if (cur.len >= 0 && s.win16) {
                     if (img)
-                        fast_pairs_x2<SIG1, true, true, true, true, WX, WY>(s, tab[0], i, cur.p, cur.cnt,
+                        fast_pairs_x2<SIG1, true, true, true, WX, WY>(s, tab[0], i, cur.p, cur.cnt,
                                                                             slist_of(st), rows, pin, wpos_of(st), fx,
                                                                             fy, ue2, we2);
                     else
@@ -1598,7 +1593,7 @@ __global__ void __launch_bounds__(kPBlock, kPMinBlocks) k_fstep_p(DevSys s, int 
                                                         wpos_of(st), fx, fy, ue2, we2);
                 } else if (cur.len >= 0) {
                     if (img)
-                        fast_pairs_x2<SIG1, true, false, true, true, WX, WY>(s, tab[0], i, cur.p, cur.cnt,
+                        fast_pairs_x2<SIG1, true, false, true, WX, WY>(s, tab[0], i, cur.p, cur.cnt,
                                                                              slist_of(st), rows, pin, wpos_of(st), fx,
                                                                              fy, ue2, we2);
                     else
@@ -1606,7 +1601,7 @@ __global__ void __launch_bounds__(kPBlock, kPMinBlocks) k_fstep_p(DevSys s, int 
                                                          wpos_of(st), fx, fy, ue2, we2);
                 } else {
                     if (img)
-                        fast_pairs_x2<SIG1, false, false, true, true, WX, WY>(s, tab[0], i, cur.p, cur.cnt,
+                        fast_pairs_x2<SIG1, false, false, true, WX, WY>(s, tab[0], i, cur.p, cur.cnt,
                                                                               slist_of(st), rows, pin, wpos_of(st),
                                                                               fx, fy, ue2, we2);
                     else
@@ -2070,682 +2065,6 @@ static cudaError_t fstep_image(Launch &L, const DevSys &s, int mode, int parity,
     if (s.wrapx && s.wrapy) return launch_fstep<MT, SG, SIG1, true, true>(L, s, mode, parity, h, use_h);
     if (s.wrapx) return launch_fstep<MT, SG, SIG1, true, false>(L, s, mode, parity, h, use_h);
     return launch_fstep<MT, SG, SIG1, false, false>(L, s, mode, parity, h, use_h);
-}
-
-// ---- the small-system run (one particle kind, sigma by type, no bonded
-// particles, walls, gravity or area springs; a few step blocks).  At this
-// size a step kernel lasts a few microseconds and a graph node or a launch
-// costs as much again, so k_fsmall advances a run's middle steps in one
-// cooperative launch: one block per step block (tile), the tile's list rows
-// kept in shared memory, per step the window copied in, the pair terms and
-// the leapfrog of k_fstep_p, then a bounded grid-wide exchange after which
-// every block takes the same rebuild decision from the same maximum.  A
-// rebuild happens inside the launch too (small_rebuild: the binning, the
-// in-cell placement, the window records and the lists of k_fbin_small and
-// k_flist_p, in four exchanges).  Where that cannot be done (a tile without
-// a window, or one whose cell starts overflow a stage) the launch ends with
-// the rebuild pending and the rebuild kernels run; a neighbour-list overflow
-// or a non-finite position ends it too (the run is then repeated or fails).
-// The number of steps done goes to DevScalars::smallDone.
-//
-// The exchange (grid_sync.cuh): a step's carries the largest v^2, a rebuild's
-// the OR of flag bits.  Before a step's exchange each block writes a record
-// {U, W, K} (its fixed-point energy sums) into one of three record sets;
-// block 0 sums a step's records (exact integer sums: the same totals as the
-// step kernels' atomics) during the next exchange, while it waits.  Set j is
-// written again at exchange j + 3, which no block reaches before block 0 has
-// counted in exchange j + 2, after those sums.  Exchanges are numbered over the
-// life of the context (DevScalars::gbTag holds the next launch's first).
-
-// This block's record of exchange x (record set par), then the wait for every
-// block: xsh[0] = 1 (0 when the wait gave up), xsh[1] = the OR of the blocks'
-// words (flags) or xsh[2] = their maximum as a float (a step).  withhold: this
-// block does not count (femmd_test_expire_next_exchange: every wait gives up).
-// Call after a __syncthreads that follows the block's stores.
-__device__ __forceinline__ void small_exchange(const DevSys &s, unsigned x, int par, unsigned long long qu,
-                                               unsigned long long qw, unsigned long long qk, unsigned word, bool flags,
-                                               unsigned *xsh, bool withhold) {
-    if (threadIdx.x == 0) {
-        unsigned long long *r = s.smallRec + kGridSlots * kGridSlotWords + 4 * ((size_t)par * kSmallMaxTiles + blockIdx.x);
-        if (!flags) {
-            r[1] = qu;
-            r[2] = qw;
-            r[3] = qk;
-        }
-        unsigned m, o;
-        xsh[0] = grid_exchange(s.smallRec, x, gridDim.x, flags ? 0u : word, flags ? word : 0u, withhold, m, o);
-        xsh[1] = o;
-        xsh[2] = m;
-    }
-}
-
-// Block 0, warp 1: the totals of an earlier step's records (set par), into
-// the scalars and the observable row of that step.
-__device__ __forceinline__ void small_totals(const DevSys &s, int par, float vm2, float d, int r, int row) {
-    const unsigned long long *set = s.smallRec + kGridSlots * kGridSlotWords + (size_t)par * kSmallMaxTiles * 4;
-    const int lane = threadIdx.x & 31;
-    unsigned long long su = 0ull, sw = 0ull, sk = 0ull;
-    for (int b = lane; b < (int)gridDim.x; b += 32) {
-        su += __ldcg(set + 4 * (size_t)b + 1);
-        sw += __ldcg(set + 4 * (size_t)b + 2);
-        sk += __ldcg(set + 4 * (size_t)b + 3);
-    }
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        su += __shfl_down_sync(0xffffffffu, su, o);
-        sw += __shfl_down_sync(0xffffffffu, sw, o);
-        sk += __shfl_down_sync(0xffffffffu, sk, o);
-    }
-    if (lane == 0) {
-        DevScalars *sc = s.sc;
-        const double U = from_fixed(su), W = from_fixed(sw), KE = from_fixed(sk);
-        sc->U = U;
-        sc->W = W;
-        sc->KE = KE;
-        sc->vvMax = vm2;
-        if (s.obs && row < s.obsCap) {
-            double *o = s.obs + (size_t)row * kObsCols;
-            o[0] = U;
-            o[1] = W;
-            o[2] = KE;
-            o[3] = (double)vm2;
-            o[4] = (double)d;
-            o[5] = (double)r;
-        }
-    }
-}
-
-// k_fsmall's threads: one per storage slot of the tile for the steps; three
-// per slot (one per stencil column) for the list walk of a rebuild
-constexpr int kSmallThreads = 3 * kFastBlock;
-
-// Shared memory of k_fsmall: scalars, the list rows, the step window, the
-// list build's stage (header, cell starts, window of cellSorted), an entry
-// stage and a count per stencil column, and the cell starts of the binning.
-constexpr size_t kSmHdr = 512;
-__host__ __device__ constexpr size_t small_smem(int rows, int ncells) {
-    return kSmHdr + (size_t)rows * kFastBlock * sizeof(int4) + (size_t)kWinMax * sizeof(float2) +
-           lp_stage_bytes() + 3 * (size_t)(kLStage + 1) * kFastBlock * sizeof(unsigned short) +
-           3 * (size_t)kFastBlock * sizeof(int) + (((size_t)ncells + 1 + 3) & ~(size_t)3) * sizeof(int);
-}
-
-// Rebuild outcomes inside the small run
-constexpr int kSmallRebuilt = 0, kSmallStop = 1, kSmallPending = 2;
-
-// The state a thread of k_fsmall carries between steps and rebuilds.
-struct SmallSlot {
-    float2 pi, v;   // position and velocity of the thread's storage slot
-    float m;        // its mass
-    int id, excl;   // its particle id and exclusion group
-    int cnt;        // its list length
-};
-
-// The tile's list rows and window record (from the global list and
-// blockWin; the L2 copy, since this launch may have written them).
-__device__ __forceinline__ void small_load_tile(const DevSys &s, int rows, int4 *slist, int *wrec, int &G) {
-    const int t = blockIdx.x;
-    const int *bw = s.blockWin + kWinInts * (size_t)t;
-    for (int q = threadIdx.x; q < kWinInts; q += blockDim.x) wrec[q] = __ldcg(bw + q);
-    __syncthreads();
-    G = min(wrec[kWGroups], rows);
-    const int i = t * kFastBlock + threadIdx.x;
-    const int4 *lrow = reinterpret_cast<const int4 *>(s.nbr) + (size_t)t * kFastBlock + threadIdx.x;
-    if (threadIdx.x < kFastBlock && i < s.Ncap)
-        for (int g = 0; g < G; g++) slist[g * kFastBlock + threadIdx.x] = __ldcg(lrow + (size_t)g * s.Ncap);
-}
-
-// Window bytes a step copies (16-byte spans of the record's pieces).
-__device__ __forceinline__ unsigned small_win_bytes(const int *wrec) {
-    unsigned b = 0;
-    if (wrec[kWLen] >= 0)
-        for (int q = 0; q < kWinPieces; q++) {
-            const int a = wrec[kWStart + q], c = wrec[kWCount + q];
-            if (c > 0) b += (unsigned)(((a + c + 1) & ~1) - (a & ~1)) * 8u;
-        }
-    return b;
-}
-
-// Steps come from DevScalars::smallLeft and the start parity from
-// DevScalars::smallPar; a launch ends with the positions in pos0 (parity 0),
-// so that a rebuild that may follow it has a fixed parity.  use_h: inside the run graph, set its WHILE (steps left) and
-// IF (rebuild pending) conditions.
-template <bool SIG1, bool WX, bool WY>
-__global__ void __launch_bounds__(kSmallThreads, 1) k_fsmall(DevSys s, int rows, cudaGraphConditionalHandle hw,
-                                                             cudaGraphConditionalHandle hif, int use_h) {
-    extern __shared__ float4 smem_f4[];
-    unsigned char *sm = reinterpret_cast<unsigned char *>(smem_f4);
-    PairEntry *tab = reinterpret_cast<PairEntry *>(sm);
-    unsigned *xsh = reinterpret_cast<unsigned *>(sm + 32);  // the exchange's ok, OR, max
-    int *bsh = reinterpret_cast<int *>(sm + 44);             // [0] block flags, [1] block max groups
-    float *red = reinterpret_cast<float *>(sm + 52);         // [warp][4]
-    unsigned long long *bar = reinterpret_cast<unsigned long long *>(sm + 120);  // the window copies
-    unsigned long long *lbar = bar + 1;                                          // the list build's copies
-    int *wrec = reinterpret_cast<int *>(sm + 136);                               // the tile's window record
-    int *hd = wrec + kWinInts;                                                   // the list build's header
-    int4 *slist = reinterpret_cast<int4 *>(sm + kSmHdr);
-    float2 *wpos = reinterpret_cast<float2 *>(slist + (size_t)rows * kFastBlock);
-    int *csm = reinterpret_cast<int *>(wpos + kWinMax);
-    float4 *wc = reinterpret_cast<float4 *>(csm + kLPCs);
-    unsigned short(*ost)[kFastBlock] = reinterpret_cast<unsigned short(*)[kFastBlock]>(wc + kWinMax);
-    int *kcol = reinterpret_cast<int *>(ost + 3 * (kLStage + 1));  // [stencil column][slot] entry counts
-    int *cst = kcol + 3 * kFastBlock;
-    static_assert(136 + (kWinInts + kLPHdr) * 4 <= kSmHdr, "small-run shared header");
-    DevScalars *sc = s.sc;
-    const int t = blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    // threads below kFastBlock own the tile's storage slots
-    const bool worker = threadIdx.x < kFastBlock;
-    const int i = t * kFastBlock + (threadIdx.x & (kFastBlock - 1));
-    const bool act = worker && i < s.N;
-    const int ic = act ? i : 0;
-    if (threadIdx.x == 0) {
-        tab[0] = s.pair[0];
-        mbar_init(bar, 1);
-        mbar_init(lbar, 1);
-        wpos[kWinGhost] = s.pos0[s.N];  // the ghost slot's far position, never moved
-    }
-    int G = 0;
-    small_load_tile(s, rows, slist, wrec, G);
-    unsigned wbytes = small_win_bytes(wrec);
-    int p = sc->smallPar;  // the parity of the current positions
-    SmallSlot me;
-    me.pi = (p ? s.pos1 : s.pos0)[ic];
-    me.v = s.vel[ic];
-    me.m = s.mass[ic];
-    me.id = s.perm[ic];
-    me.excl = s.excl[ic];
-    me.cnt = act ? min(s.nbrCount[ic], s.nbrCap) : 0;
-    const float D = s.imgD;
-    const bool outside0 = sc->outside != 0;
-    float dispHi = sc->dispHi;  // every block follows the same recurrence
-    int row = sc->obsRow, stepNow = sc->stepNow;
-    const int steps = sc->smallLeft;
-    const unsigned base = sc->gbTag;
-    const bool withhold = sc->testWithhold != 0;
-    unsigned xi = 0, wuse = 0, luse = 0;  // exchanges, window copies and list-build copies so far
-    // a step's totals that block 0 has still to sum (record set pset)
-    int pset = -1, prow = 0, pr = 0;
-    float pvm = 0.0f, pd = 0.0f;
-    int k = 0;
-    bool pending = false, stop = false, failed = false;
-    __syncthreads();
-    // one exchange: true unless a wait gave up
-    auto xchg = [&](unsigned long long qa, unsigned long long qb, unsigned long long qc, unsigned word,
-                    bool flags = true) {
-        small_exchange(s, base + xi, (int)(xi % 3u), qa, qb, qc, word, flags, xsh,
-                       withhold && xi == 0 && blockIdx.x == 0);
-        if (blockIdx.x == 0 && warp == 1 && pset >= 0) small_totals(s, pset, pvm, pd, pr, prow);
-        __syncthreads();
-        pset = -1;
-        xi++;
-        if (xsh[0]) return true;
-        if (threadIdx.x == 0) atomicOr(&sc->overflow, kFlagTimeout);
-        failed = true;
-        return false;
-    };
-    // a bounded wait for a copy phase, the same verdict on every thread; a
-    // copy that never completed is reported and given one more bounded wait
-    auto copies_done = [&](unsigned long long *b, unsigned par) {
-        const bool ok = mbar_wait_bounded(b, par, kWaitLimit);
-        if (!__syncthreads_or(!ok)) return true;
-        if (threadIdx.x == 0) atomicOr(&sc->overflow, kFlagTimeout);
-        mbar_wait_bounded(b, par, kWaitLimit);
-        failed = true;
-        return false;
-    };
-    // block 0 clears the cell counts for the next binning (every block has
-    // added to them or read them)
-    auto clear_counts = [&]() {
-        if (blockIdx.x == 0)
-            for (int q = threadIdx.x; q < s.ncells; q += kSmallThreads) s.cellCount[q] = 0;
-    };
-    // the rebuild of the positions in pos (parity p), inside the launch
-    auto small_rebuild = [&](float2 *pos) -> int {
-        // 1: cells and ranks among the cell's particles (counting atomics)
-        int c = 0, rk = 0;
-        unsigned fl = 0;
-        if (act) {
-            if (!(isfinite(me.pi.x) && isfinite(me.pi.y))) {
-                atomicOr(&sc->nonfinite, 1);
-                fl |= 1u;
-            }
-            if (outside_box(s, me.pi)) {
-                atomicOr(&sc->outside, 1);
-                fl |= 2u;
-            }
-            c = cell_col(me.pi.x, me.pi.y, s.ncx, s.ncy, s.Lx, s.Ly);
-            rk = atomicAdd(&s.cellCount[c], 1);
-        }
-        fl = (__syncthreads_or(fl & 1u) ? 1u : 0u) | (__syncthreads_or(fl & 2u) ? 2u : 0u);
-        if (!xchg(0ull, 0ull, 0ull, fl)) return kSmallStop;
-        const unsigned f1 = xsh[1];
-        if (f1 & 1u) {  // a non-finite position: the run fails
-            clear_counts();
-            return kSmallStop;
-        }
-        const bool walk_ok = (s.wrapx ? s.ncx >= 5 : s.ncx >= 3) && (s.wrapy ? s.ncy >= 5 : s.ncy >= 3) &&
-                             !outside0 && !(f1 & 2u);
-        // 2: every block scans the counts into cell starts (block 0 also
-        // writes them out), then the ids go to their cells
-        const int nc = s.ncells;
-        for (int q = threadIdx.x; q < nc; q += kSmallThreads) cst[q] = __ldcg(s.cellCount + q);
-        __syncthreads();
-        {
-            // a run of cells per slot thread: its total, the scan of the
-            // totals (warps, then the kFastBlock / 32 warp sums), its run
-            const int per = (nc + kFastBlock - 1) / kFastBlock;
-            const int c0 = worker ? min((int)threadIdx.x * per, nc) : nc, c1 = min(c0 + per, nc);
-            int tot = 0;
-            for (int q = c0; q < c1; q++) tot += cst[q];
-            int x = tot;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            int *ws = reinterpret_cast<int *>(red);  // the slot warps' totals
-            if (worker && lane == 31) ws[warp] = x;
-            __syncthreads();
-            int before = 0;
-            if (worker)
-                for (int w = 0; w < warp; w++) before += ws[w];
-            int run = before + x - tot;
-            for (int q = c0; q < c1; q++) {
-                const int v = cst[q];
-                cst[q] = run;
-                run += v;
-            }
-            if (threadIdx.x == 0) cst[nc] = s.N;
-        }
-        __syncthreads();
-        if (blockIdx.x == 0) {
-            for (int q = threadIdx.x; q <= nc; q += kSmallThreads) s.cellStart[q] = cst[q];
-            if (threadIdx.x == 0) {
-                sc->nbrSum = 0ull;
-                sc->maxCount = 0;
-            }
-        }
-        unsigned f2 = 0;
-        if (act) {
-            const int slot0 = cst[c] + rk;
-            if (slot0 >= 0 && slot0 < s.N) s.unsorted[slot0] = me.id;
-            else f2 = 1u;  // inconsistent counts: never write outside the array
-        }
-        f2 = __syncthreads_or(f2) ? 1u : 0u;
-        if (f2 && threadIdx.x == 0) atomicOr(&sc->overflow, 2);
-        if (!xchg(0ull, 0ull, 0ull, f2)) return kSmallStop;
-        clear_counts();
-        if (xsh[1]) return kSmallStop;
-        // 3: the placement inside the cell by id (k_fplace), and the tile's
-        // window record from the cell starts here
-        unsigned f3 = 0;
-        if (act) {
-            const int b = cst[c], e = cst[c + 1];
-            int r = 0;
-            for (int q = b; q < e; q++) r += __ldcg(s.unsorted + q) < me.id;
-            const int ns = b + r;
-            if (ns < e) {
-                s.cellSorted[ns] = make_float4(me.pi.x, me.pi.y, __int_as_float(ns), __int_as_float(me.excl));
-                s.sortedIds[ns] = ns;
-                s.newCell[ns] = c;
-                s.sPos[ns] = me.pi;
-                s.sVel[ns] = me.v;
-                s.sAcc[ns] = s.acc[i];
-                s.sPerm[ns] = me.id;
-            } else {
-                f3 |= 1u;
-            }
-        }
-        if (threadIdx.x == 0) {
-            auto cell_of = [&](int q) {
-                int lo = 0, hi = nc - 1;
-                while (lo < hi) {
-                    const int mid = (lo + hi + 1) >> 1;
-                    if (cst[mid] <= q) lo = mid;
-                    else hi = mid - 1;
-                }
-                return lo;
-            };
-            fwindow_record_t(s, t, walk_ok, [&](int q) { return cst[q]; }, cell_of);
-            bsh[0] = 0;
-        }
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            // the record just written (this thread's own stores)
-            const int *bw = s.blockWin + kWinInts * (size_t)t;
-            for (int q = 0; q < kWinInts; q++) wrec[q] = bw[q];
-            if (wrec[kWLen] < 0 || lp_cs_words(s, wrec) > kLPCs) bsh[0] = 2;  // no stage for this tile
-        }
-        __syncthreads();
-        f3 = (__syncthreads_or(f3) ? 1u : 0u) | (unsigned)bsh[0];
-        if ((f3 & 1u) && threadIdx.x == 0) atomicOr(&sc->overflow, 2);
-        if (!xchg(0ull, 0ull, 0ull, f3)) return kSmallStop;
-        if (xsh[1] & 1u) return kSmallStop;
-        if (xsh[1] & 2u) return kSmallPending;  // a tile without a stage: the rebuild kernels
-        // 4: the tile's lists (k_flist_p's walk), then the slot's new
-        // particle from the scratch arrays
-        if (threadIdx.x == 0) {
-            if (blockIdx.x == 0) {
-                sc->totalUpdates += 1;  // k_rebuild_begin
-                atomicAdd(&sc->builds, 1ull);
-            }
-            hd[kHT] = t;
-            hd[kHLen] = wrec[kWLen];
-            asm volatile("fence.proxy.async.global;" ::: "memory");
-            lp_issue(s, wrec, hd, csm, wc, lbar);
-        }
-        __syncthreads();
-        if (!copies_done(lbar, luse & 1u)) return kSmallStop;
-        luse++;
-        const int cap = s.nbrCap;
-        const int slot = i;
-        // three threads per slot walk the three stencil columns, each into
-        // its own entry stage; the slot's thread then joins them in column
-        // order (the order of k_flist_p's walk)
-        const int sub = threadIdx.x / kFastBlock;
-        int kd = 0, ix = 0, iy = 0, j = 0, self = 0;
-        float2 q = make_float2(0.0f, 0.0f);
-        if (slot < s.N) {
-            const bool two = hd[kHTwo] != 0;
-            if (two) {
-                const int bnd = csm[min(max(hd[kHCsb + 4] + hd[kHColp + 4], 0), kLPCs - 1)];
-                j = slot >= bnd ? 1 : 0;
-            }
-            const int pown = !two ? 2 : (j == 0 ? 3 : 4);
-            self = min(max(slot + hd[kHDelta + pown], 0), kWinMax - 1);
-            const float4 e = wc[self];
-            cell_xy(e.x, e.y, s.ncx, s.ncy, s.Lx, s.Ly, ix, iy);
-            q = make_float2(e.x, e.y);
-            TileStagePut sp;
-            sp.st = ost + sub * (kLStage + 1);
-            sp.col = threadIdx.x & (kFastBlock - 1);
-            lp_stencil_col(s, hd, csm, wc, ix, iy, j, q, self, sub, sp, kd);
-        }
-        kcol[threadIdx.x] = kd;
-        __syncthreads();
-        int k0 = 0, k1 = 0, kk = 0;
-        if (act) {
-            k0 = kcol[threadIdx.x];
-            k1 = kcol[kFastBlock + threadIdx.x];
-            kk = k0 + k1 + kcol[2 * kFastBlock + threadIdx.x];
-            if (kk > kLStage && cap > kLStage) {
-                // entries past the stage: the whole walk again, straight to the list
-                int k2 = 0;
-                DirectPut16 dp;
-                dp.nbr16 = reinterpret_cast<unsigned short *>(s.nbr);
-                dp.slot = slot;
-                dp.cap = cap;
-                dp.Ncap = s.Ncap;
-                lp_stencil(s, hd, csm, wc, ix, iy, j, q, self, dp, k2);
-            }
-        }
-        // entry k of the joined list (k < kLStage: every column's first kLStage entries are staged)
-        auto entry = [&](int k) -> unsigned {
-            const int d = k < k0 ? 0 : (k < k0 + k1 ? 1 : 2);
-            const int r = k - (d == 0 ? 0 : (d == 1 ? k0 : k0 + k1));
-            return ost[d * (kLStage + 1) + r][threadIdx.x];
-        };
-        const int kc = act ? min(kk, cap) : 0;
-        const int ng = (kc + 7) >> 3;
-        if (worker) {
-            const int ngs = min(ng, kLStage / 8);
-            const int gmax = __reduce_max_sync(0xffffffffu, ngs);
-            int4 *out = reinterpret_cast<int4 *>(s.nbr) + slot;
-            for (int g = 0; g < gmax; g++) {
-                if (g < ngs) {
-                    int v[4];
-#pragma unroll
-                    for (int u = 0; u < 4; u++) {
-                        const int e0 = 8 * g + 2 * u;
-                        const unsigned lo = e0 < kc ? entry(e0) : kWinGhost;
-                        const unsigned hi = e0 + 1 < kc ? entry(e0 + 1) : kWinGhost;
-                        v[u] = (int)(lo | hi << 16);
-                    }
-                    out[(size_t)g * s.Ncap] = make_int4(v[0], v[1], v[2], v[3]);
-                }
-            }
-            if (act && kc > kLStage && (kc & 7)) {
-                unsigned short *n16 = reinterpret_cast<unsigned short *>(s.nbr);
-                for (int q = kc; q < 8 * ng; q++) n16[nbr16_at(q, slot, s.Ncap)] = (unsigned short)kWinGhost;
-            }
-        }
-        if (act) {
-            const int id = __ldcg(s.sPerm + slot);
-            me.pi = __ldcg(s.sPos + slot);
-            me.v = __ldcg(s.sVel + slot);
-            const float2 na = __ldcg(s.sAcc + slot);
-            me.id = id;
-            me.m = __ldg(s.idMass + id);
-            me.cnt = kc;
-            s.nbrCount[slot] = kk;
-            pos[slot] = me.pi;
-            s.vel[slot] = me.v;
-            s.acc[slot] = na;
-            s.perm[slot] = id;
-            const_cast<float *>(s.mass)[slot] = me.m;
-        }
-        const int gm = __reduce_max_sync(0xffffffffu, ng);
-        const int kmax = __reduce_max_sync(0xffffffffu, act ? kk : 0);
-        const int ksum = __reduce_add_sync(0xffffffffu, act ? kk : 0);
-        if (threadIdx.x == 0) bsh[1] = 0;
-        __syncthreads();
-        unsigned f4 = 0;
-        if (lane == 0) {
-            atomicMax(&bsh[1], gm);
-            if (ksum) atomicAdd(&sc->nbrSum, (unsigned long long)ksum);
-            if (kmax > 0) atomicMax(&sc->maxCount, kmax);
-            if (kmax > cap) {
-                atomicOr(&sc->overflow, 1);
-                f4 = 1u;
-            }
-        }
-        f4 = __syncthreads_or(f4) ? 1u : 0u;
-        if (threadIdx.x == 0) {
-            s.blockWin[kWinInts * (size_t)t + kWGroups] = bsh[1];
-            wrec[kWGroups] = bsh[1];
-        }
-        __syncthreads();
-        // the tile's rows into shared memory (this block wrote them)
-        G = min(wrec[kWGroups], rows);
-        if (worker && i < s.Ncap)
-            for (int g = 0; g < G; g++)
-                slist[g * kFastBlock + threadIdx.x] =
-                    __ldcg(reinterpret_cast<const int4 *>(s.nbr) + (size_t)g * s.Ncap + i);
-        wbytes = small_win_bytes(wrec);
-        if (!xchg(0ull, 0ull, 0ull, f4)) return kSmallStop;
-        if (xsh[1]) return kSmallStop;  // a list overflow: the run is repeated with longer lists
-        return kSmallRebuilt;
-    };
-    for (; k < steps;) {
-        const float2 *pin = p ? s.pos1 : s.pos0;
-        float2 *pout = p ? s.pos0 : s.pos1;
-        const int len = wrec[kWLen];
-        // the window by bulk copies (other blocks wrote it before the last
-        // exchange; the proxy fence orders their release before the copies)
-        if (len >= 0) {
-            if (threadIdx.x == 0) {
-                asm volatile("fence.proxy.async.global;" ::: "memory");
-                mbar_expect_tx(bar, wbytes);
-                for (int q = 0; q < kWinPieces; q++) {
-                    const int a = wrec[kWStart + q], c = wrec[kWCount + q];
-                    if (c > 0) {
-                        const int a0 = a & ~1, e0 = (a + c + 1) & ~1;
-                        bulk_copy_g2s(wpos + wrec[kWOff + q] - (a & 1), pin + a0, (unsigned)(e0 - a0) * 8u, bar);
-                    }
-                }
-            }
-            if (!copies_done(bar, wuse & 1u)) break;
-            wuse++;
-        }
-        const float2 pi = me.pi;
-        const int cnt = me.cnt;
-        float fx = 0.0f, fy = 0.0f, ue2 = 0.0f, we2 = 0.0f;
-        const bool near = act && ((WX && (pi.x < D || pi.x > s.Lx - D)) || (WY && (pi.y < D || pi.y > s.Ly - D)));
-        const bool img = __any_sync(0xffffffffu, near);
-        if (act) {
-            if (len >= 0 && s.win16) {
-                if (img) fast_pairs_x2<SIG1, true, true, false, true, WX, WY>(s, tab[0], i, pi, cnt, slist, rows, pin,
-                                                                            wpos, fx, fy, ue2, we2);
-                else fast_pairs_x2<SIG1, true, true, false>(s, tab[0], i, pi, cnt, slist, rows, pin, wpos, fx, fy,
-                                                            ue2, we2);
-            } else if (len >= 0) {
-                if (img) fast_pairs_x2<SIG1, true, false, false, true, WX, WY>(s, tab[0], i, pi, cnt, slist, rows, pin,
-                                                                             wpos, fx, fy, ue2, we2);
-                else fast_pairs_x2<SIG1, true, false, false>(s, tab[0], i, pi, cnt, slist, rows, pin, wpos, fx, fy,
-                                                             ue2, we2);
-            } else {
-                if (img) fast_pairs_x2<SIG1, false, false, false, true, WX, WY>(s, tab[0], i, pi, cnt, slist, rows,
-                                                                              pin, wpos, fx, fy, ue2, we2);
-                else fast_pairs_x2<SIG1, false, false, false>(s, tab[0], i, pi, cnt, slist, rows, pin, wpos, fx, fy,
-                                                              ue2, we2);
-            }
-        }
-        float ue = 0.0f, we = 0.0f, ke = 0.0f, vvm = 0.0f;
-        bool bad = false;
-        if (act)
-            fast_finish<WX, WY>(s, i, MODE_MID, pi, me.m, me.v, pout, nullptr, fx, fy, ue2, we2, 0.0f, 0.0f, ue, we,
-                                ke, vvm, bad, &me.pi, &me.v);
-        // the block's sums
-        const float su = warp_sum_f(ue), sw = warp_sum_f(we), sk = warp_sum_f(ke), mx = warp_max(vvm);
-        const unsigned anybad = __ballot_sync(0xffffffffu, bad);
-        if (worker && lane == 0) {
-            red[4 * warp + 0] = su;
-            red[4 * warp + 1] = sw;
-            red[4 * warp + 2] = sk;
-            red[4 * warp + 3] = mx;
-            if (anybad) atomicOr(&sc->nonfinite, 1);
-        }
-        __syncthreads();
-        unsigned long long qa = 0ull, qb = 0ull, qc = 0ull;
-        float mm = 0.0f;
-        if (threadIdx.x == 0) {
-            float a = 0.0f, b = 0.0f, c = 0.0f;
-            for (int w = 0; w < kFastBlock / 32; w++) {
-                a += red[4 * w];
-                b += red[4 * w + 1];
-                c += red[4 * w + 2];
-                mm = fmaxf(mm, red[4 * w + 3]);
-            }
-            bool ob = false;
-            qa = to_fixed(a, ob);
-            qb = to_fixed(b, ob);
-            qc = to_fixed(c, ob);
-            if (ob) atomicOr(&sc->nonfinite, 2);
-        }
-        const int stepSet = (int)(xi % 3u);
-        if (!xchg(qa, qb, qc, __float_as_uint(mm), false)) break;
-        // the step's totals, the same on every block: the rebuild rule of
-        // evalProps / NeighborList::update (md3dsystem.cpp:177, nn.cpp:118)
-        const float vm2 = __uint_as_float(xsh[2]);
-        const float d = dispHi + sqrtf(vm2) * s.dt;
-        const int r = (double)d > s.halfSkin;
-        pset = stepSet;
-        pvm = vm2;
-        pd = d;
-        pr = r;
-        prow = row;
-        dispHi = d;
-        row++;
-        stepNow++;
-        p ^= 1;
-        k++;
-        if (r) {
-            const int o = small_rebuild(p ? s.pos1 : s.pos0);
-            if (o == kSmallRebuilt) {
-                dispHi = 0.0f;  // k_rebuild_begin
-                continue;
-            }
-            if (o == kSmallPending) pending = true;
-            else stop = true;
-            break;
-        }
-    }
-    // back to parity 0 (each thread its own slot), then one more exchange so
-    // that every block has finished before the rebuild kernels or the next
-    // launch read the positions
-    if (p == 1 && act) s.pos0[i] = me.pi;
-    __syncthreads();
-    bool fin = false;
-    if (!failed) fin = xchg(0ull, 0ull, 0ull, 0u);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        if (!fin) atomicOr(&sc->overflow, kFlagTimeout);
-        // an exchange that gave up, a non-finite position or a list
-        // overflow ends the run's loop
-        const int left = (k > 0 && fin && !stop) ? steps - k : 0;
-        sc->dispHi = dispHi;
-        sc->rebuild = pending ? 1 : 0;
-        sc->obsRow = row;
-        sc->stepNow = stepNow;
-        sc->smallDone = k;
-        sc->smallLeft = left;
-        sc->smallPar = 0;
-        sc->testWithhold = 0;
-        sc->gbTag = base + xi;
-        if (use_h) {
-            cudaGraphSetConditional(hif, pending ? 1u : 0u);
-            cudaGraphSetConditional(hw, left > 0 ? 1u : 0u);
-        }
-    }
-}
-
-// Launch of the small-system run (cooperative: every block resident); the
-// caller has checked small_run_fits.
-template <bool SIG1, bool WX, bool WY>
-static cudaError_t launch_fsmall_t(cudaStream_t st, const DevSys &s, int rows) {
-    const int ntiles = (s.N + kFastBlock - 1) / kFastBlock;
-    const size_t smem = small_smem(rows, s.ncells);
-    auto kern = k_fsmall<SIG1, WX, WY>;
-    int resident = 0;
-    cudaError_t e = kernel_setup((const void *)kern, kSmallThreads, smem, &resident);
-    if (e) return e;
-    DevSys a = s;
-    int ra = rows, ua = 0;
-    cudaGraphConditionalHandle h0 = 0, h1 = 0;
-    void *args[] = {&a, &ra, &h0, &h1, &ua};
-    return cudaLaunchCooperativeKernel((const void *)kern, dim3(ntiles), dim3(kSmallThreads), args, smem, st);
-}
-
-constexpr size_t kSmallMaxSmem = 200 * 1024;
-
-bool small_run_fits(const DevSys &s) {
-    if (!s.fast || !s.win16 || !s.smallRec || s.nBonded != 0 || s.wallOn || s.gravity > 0.0f || s.refWalls ||
-        s.areaUnits > 0 || s.trace || s.N <= 0)
-        return false;
-    const int ntiles = (s.N + kFastBlock - 1) / kFastBlock;
-    if (ntiles > kSmallMaxTiles) return false;
-    const int rows = std::max(1, (s.nbrCap + 7) / 8);
-    const size_t smem = small_smem(rows, s.ncells);
-    if (smem > kSmallMaxSmem) return false;
-    auto kern = s.sigmaOne ? (s.wrapx && s.wrapy ? k_fsmall<true, true, true> : nullptr)
-                           : (s.wrapx && s.wrapy ? k_fsmall<false, true, true> : nullptr);
-    if (!kern) return false;  // the small run is built for XY-periodic boxes
-    int resident = 0;
-    if (kernel_setup((const void *)kern, kSmallThreads, smem, &resident)) return false;
-    return resident >= ntiles;
-}
-
-cudaError_t launch_small_run(cudaStream_t st, const DevSys &s) {
-    const int rows = std::max(1, (s.nbrCap + 7) / 8);
-    return s.sigmaOne ? launch_fsmall_t<true, true, true>(st, s, rows) : launch_fsmall_t<false, true, true>(st, s, rows);
-}
-
-// The small-system run as a graph node (cooperative), with the WHILE and IF
-// handles it sets.
-cudaError_t enqueue_small_run(Launch &L, const DevSys &s, cudaGraphConditionalHandle hw,
-                              cudaGraphConditionalHandle hif) {
-    const int rows = std::max(1, (s.nbrCap + 7) / 8);
-    const int ntiles = (s.N + kFastBlock - 1) / kFastBlock;
-    const size_t smem = small_smem(rows, s.ncells);
-    cudaError_t e;
-    int resident = 0;
-    if (s.sigmaOne) {
-        if ((e = kernel_setup((const void *)k_fsmall<true, true, true>, kSmallThreads, smem, &resident))) return e;
-        e = L.kernel(k_fsmall<true, true, true>, dim3(ntiles), dim3(kSmallThreads), smem, s, rows, hw, hif, 1);
-    } else {
-        if ((e = kernel_setup((const void *)k_fsmall<false, true, true>, kSmallThreads, smem, &resident))) return e;
-        e = L.kernel(k_fsmall<false, true, true>, dim3(ntiles), dim3(kSmallThreads), smem, s, rows, hw, hif, 1);
-    }
-    if (e) return e;
-    return L.cooperative_last();
 }
 
 // The persistent kernel wherever every window can be one bulk copy (no

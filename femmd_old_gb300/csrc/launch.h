@@ -96,14 +96,6 @@ struct Launch {
         return cudaSuccess;
     }
 
-    // Mark the last kernel node cooperative (all its blocks co-resident).
-    cudaError_t cooperative_last() {
-        if (!graph || deps.empty()) return cudaErrorInvalidValue;
-        cudaLaunchAttributeValue v = {};
-        v.cooperative = 1;
-        return cudaGraphKernelNodeSetAttribute(deps.back(), cudaLaunchAttributeCooperative, &v);
-    }
-
     // kernel() with the grid in clusters of n blocks.
     template <typename... KArgs, typename... Args>
     cudaError_t kernel_clusters(void (*k)(KArgs...), int n, dim3 g, dim3 b, size_t smem, Args &&...args) {

@@ -36,8 +36,8 @@ typedef enum {
     FEMMD_CAPACITY_OVERFLOW = 2,  /* a capacity could not be grown */
     FEMMD_NONFINITE = 3,          /* a force or energy became NaN/inf */
     FEMMD_CUDA_ERROR = 4,         /* a CUDA call failed (no GPU, OOM, ...) */
-    FEMMD_TIMEOUT = 5,            /* a bounded device wait expired (the fast step's copies, the small-system
-                                     run's grid-wide exchanges) */
+    FEMMD_TIMEOUT = 5,            /* a bounded device wait expired (the fast step's copies, the grid-wide
+                                     exchanges of the cooperative launches) */
     FEMMD_NOT_READY = 6,          /* call order: e.g. run before init_neighbor_list */
     FEMMD_UNSUPPORTED = 7         /* feature of the reference outside this path */
 } femmd_status;
@@ -248,8 +248,8 @@ femmd_status femmd_event_elapsed(femmd_ctx *ctx, int slot_a, int slot_b, float *
 femmd_status femmd_set_profiling(femmd_ctx *ctx, int profile);
 femmd_status femmd_get_profile(femmd_ctx *ctx, double *force_kernel_ms, long long *force_kernel_launches,
                                double *rebuild_ms, long long *rebuilds, long long *kernel_launches);
-/* For tests of the failure path: in the next run that takes the small-system
- * run (the fast mode's cooperative launch), block 0 withholds its record of
+/* For tests of the failure path: in the next run that is one cooperative
+ * launch (small and medium systems, both force modes), block 0 withholds its record of
  * the first grid-wide exchange, so every block's bounded wait gives up
  * (about a second) and femmd_run returns FEMMD_TIMEOUT with the context
  * still usable.  No GPU fault, trap or endless wait is involved. */
