@@ -13,8 +13,8 @@ namespace {
 // run(50) against the plain kernels' graph (us): LJ fluid 67,600 particles
 // 1148 / 1539, 160,000 2095 / 1848 (equal near 125,000); disks in solvent
 // 68,288 1512 / 1787, 150,800 2662 / 2111 (96,000); suspension 32,512
-// 650 / 923, 130,048 1336 / 1254 (108,000).  In the fast mode (LJ fluid) 90,000
-// particles 1131 / 1420.
+// 650 / 923, 130,048 1336 / 1254 (108,000).  Fast mode: LJ 97,969 1220 / 1419,
+// disks in solvent 97,512 1717 / 2117, suspension 92,583 932 / 1262.
 constexpr int kCoopMaxN = 98304;
 
 const void *coop_kernel(const DevSys &s, bool bySlot) {
