@@ -2124,10 +2124,14 @@ __global__ void __launch_bounds__(kBlock) k_perm_consts(DevSys s, int ident) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= s.N) return;
     int id = i;
-    if (ident)
+    if (ident) {
         s.perm[i] = i;
-    else
+        // the mirror's places, until a rebuild gives others: a drift before one
+        // (after a whole-run launch, which keeps no mirror) writes them
+        if (s.cslot) s.cslot[i] = i;
+    } else {
         id = s.perm[i];
+    }
     const_cast<float *>(s.mass)[i] = s.idMass[id];
     if (s.numTypes > 1) const_cast<int *>(s.typeId)[i] = s.idType[id];
     if (!s.sigmaByType) const_cast<float *>(s.sigma)[i] = s.idSigma[id];
