@@ -75,7 +75,13 @@ struct GraphSet {
     }
 };
 
-constexpr int kGraphUnits = 32;  // [step -> IF rebuild] units per cached graph
+// [step -> IF rebuild] units per cached graph (even); a run's rest is single units,
+// each with a graph launch of its own (4 us).  Measured against 32 (us, LJ 1M fast /
+// 1.5M mixed): run(50) 3576 / 3603, 8274 / 8378; run(300) 19,889 / 19,984, 51,146 /
+// 51,190; the first run of a context 4634 / 5245, 9091 / 9809 (half the nodes to
+// instantiate).  8 units: the LJ fluid's run(50) 3499, the mixed system's
+// run(300) 51,282.
+constexpr int kGraphUnits = 16;
 constexpr unsigned kPos = 1, kVel = 2, kAcc = 4, kForce = 8, kEnergy = 16, kAll = 31;
 
 }  // namespace
