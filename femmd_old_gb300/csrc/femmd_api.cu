@@ -1017,6 +1017,9 @@ static femmd_status alloc_list(femmd_ctx *ctx, int cap) {
     // at least two groups of storage: the fast step kernel loads a
     // particle's first two groups before it knows the list's length
     CK(ctx->nbr.ensure((size_t)std::max(cap, 8) * ctx->Ncap));
+    // a rebuild that meets a non-finite position leaves the lists as they are:
+    // every entry is in range from the start
+    CK(cudaMemsetAsync(ctx->nbr.p, 0, (size_t)std::max(cap, 8) * ctx->Ncap * sizeof(int), ctx->stream));
     ctx->nbrCap = cap;
     release_graphs(ctx);
     return FEMMD_OK;
@@ -1175,6 +1178,15 @@ static femmd_status expired(femmd_ctx *ctx, const char *what) {
     CK(cudaMemsetAsync(ctx->cellCount.p, 0, sizeof(int) * std::max(ctx->ncells, 1), ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return fail(ctx, FEMMD_TIMEOUT, "a bounded device wait expired (%s)", what);
+}
+
+// A whole-run launch was left at a rebuild that it could not make (overflow bit
+// 32): a non-finite position, for which the run is repeated by the plain kernels, or a
+// cell of more than kCellCap particles (bit 16), from which on all runs are theirs.
+// The cell counts of the binning are cleared before the next launch.
+static void coop_left(femmd_ctx *ctx) {
+    ctx->runClean = false;
+    if (ctx->hsc->overflow & 16) ctx->coopOff = true;
 }
 
 // The triangles by block of the whole-run launch (CoopArgs), laid out once per
@@ -2388,12 +2400,13 @@ femmd_status femmd_run(femmd_ctx *ctx, int steps) {
     }
     if ((st = ensure_obs(ctx, steps))) return st;
     const int N = (int)ctx->pos.size();
+    bool plain = false;  // a whole-run launch met a state that it cannot list
     for (int attempt = 0; attempt < 8; attempt++) {
         // start checkpoint (positions, velocities, accelerations); a run that
         // is one launch writes its own
         const float2 *pc = ctx->cur ? ctx->dpos1.p : ctx->dpos0.p;
         int cur0 = ctx->cur;
-        const bool whole = coop_whole(ctx, steps);
+        const bool whole = !plain && coop_whole(ctx, steps);
         if (whole && (st = to_id_order(ctx))) return st;
         ctx->permIdent = whole;
         if (!whole) {
@@ -2446,8 +2459,9 @@ femmd_status femmd_run(femmd_ctx *ctx, int steps) {
         }
         if (ctx->propAvg)
             CK(cudaMemcpyAsync(ctx->props.p, ctx->propsCk.p, sizeof(DevProps), cudaMemcpyDeviceToDevice, ctx->stream));
-        if (ctx->hsc->overflow & 16) {
-            ctx->coopOff = true;  // a crowded cell: the plain kernels
+        if (ctx->hsc->overflow & 32) {
+            plain = true;
+            coop_left(ctx);
             if (!(ctx->hsc->overflow & 1)) continue;
         }
         int need = std::max(ctx->hsc->maxCount, ctx->nbrCap + ctx->nbrCap / 2);
@@ -3244,6 +3258,7 @@ static femmd_status adj_recompute(femmd_ctx *ctx, int g, std::vector<int> &rebui
     }
     if ((e = read_scalars(ctx))) return e;
     if (ctx->hsc->overflow & 8) return expired(ctx, "a grid-wide exchange");
+    if (ctx->hsc->overflow & 32) coop_left(ctx);
     if (ctx->hsc->overflow || ctx->hsc->nonfinite)
         return fail(ctx, ctx->hsc->overflow ? FEMMD_CAPACITY_OVERFLOW : FEMMD_NONFINITE,
                     "the recomputed segment differs from the forward pass (overflow or non-finite force)");

@@ -83,6 +83,7 @@ struct DevScalars {
     // the whole-run launch (k_coop): the exchanges so far, and which of its two cell-count arrays the last rebuild used
     unsigned int runTag;
     int runFill;
+    int runStop;  // its last launch was cut short: the run's later ones return at once
 };
 
 enum StepMode { MODE_FORCES = 0, MODE_FIRST = 1, MODE_MID = 2, MODE_LAST = 3, MODE_INIT = 4 };

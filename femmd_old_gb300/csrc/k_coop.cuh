@@ -85,6 +85,7 @@ namespace {
 constexpr int kCoopThreads = 512;
 constexpr int kCoopTimeout = 8;     // DevScalars::overflow bit: a bounded wait expired
 constexpr int kCoopCrowded = 16;    // DevScalars::overflow bit: a cell holds more than kCellCap particles
+constexpr int kCoopLeft = 32;       // DevScalars::overflow bit: a rebuild could not be made (kRebuildLeft)
 constexpr int kCoopMaxTiles = 32;   // tiles of one block (one lane of a warp sums each)
 constexpr int kTriTile = 256;       // triangles per energy group (k_tri_forces' block)
 constexpr int kListLanes = 8;       // lanes that build one particle's list
@@ -361,11 +362,15 @@ __device__ __forceinline__ int coop_list(const DevSys &s, const CoopMem &mem, co
 
 // NeighborList::update's taken branch for the positions of buffer p: cells of
 // at most kCellCap particles by counting atomics, the in-cell order by id,
-// and the lists of the block's own particles.  Two exchanges.  False when one
-// gave up.
+// and the lists of the block's own particles.  Two exchanges.  A non-finite
+// position or a crowded cell ends the launch here, on every block alike
+// (kRebuildLeft): there are no lists to go on with (before a run's first rebuild
+// not even old ones), and the host repeats the run from its start by the plain kernels.
+enum CoopRebuild { kRebuildLost, kRebuildLeft, kRebuildDone };  // lost: an exchange gave up
+
 template <bool SLOT>
-__device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, const CoopMem &mem, CoopRun &r, int p,
-                                          bool withhold) {
+__device__ __forceinline__ CoopRebuild coop_rebuild(const DevSys &s, CoopShared &sh, const CoopMem &mem, CoopRun &r,
+                                                    int p, bool withhold) {
     const float2 *pos = p ? s.pos1 : s.pos0;
     DevScalars *sc = s.sc;
     const int groups = blockDim.x / kStepBlock;
@@ -385,13 +390,17 @@ __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, co
         s.cellOf[i] = c;
         const int k = atomicAdd(cnt + c, 1);
         if (k < kCellCap) s.cellIds[(size_t)c * kCellCap + k] = i;
-        else atomicOr(&sc->overflow, kCoopCrowded);  // the run is repeated by the plain kernels
+        else atomicOr(&sc->overflow, kCoopCrowded);
     }
     __syncthreads();
-    if (!coop_exchange(s, sh, r, 0u, withhold)) return false;
-    // a non-finite position or a crowded cell: the rest is skipped (the run
-    // fails or is repeated), the exchange is not
-    const bool skip = __ldcg(&sc->nonfinite) != 0 || (__ldcg(&sc->overflow) & kCoopCrowded);
+    if (!coop_exchange(s, sh, r, 0u, withhold)) return kRebuildLost;
+    // the same on every block: what is tested was stored before its block's part
+    // of the exchange above, and nothing sets it again before the next one, which no
+    // block completes without this one
+    if (__ldcg(&sc->nonfinite) != 0 || (__ldcg(&sc->overflow) & kCoopCrowded)) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&sc->overflow, kCoopLeft);
+        return kRebuildLeft;
+    }
     // 2: ascending id inside each cell; the other counts cleared for the next
     // rebuild (their last readers were the lists before this rebuild)
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < s.ncells; c += gridDim.x * blockDim.x) other[c] = 0;
@@ -413,33 +422,32 @@ __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, co
         }
         __syncthreads();
     }
-    if (!skip)
-        for (int j = grp; j < mem.tiles; j += groups) {
-            const int i = (mem.first + j * mem.stride) * kStepBlock + gt;
-            if (i >= s.N) continue;
-            const int c = s.cellOf[i], n = min(__ldcg(cnt + c), kCellCap);
-            const int4 *ids = reinterpret_cast<const int4 *>(s.cellIds + (size_t)c * kCellCap);
-            const float2 x = pos[i];
-            const int tag = own_tag(s, i), gi = s.excl[i];
-            int k = 0;
-            for (int q = 0; q < n; q += 8) {
-                const int4 a = __ldcg(ids + q / 4), b = __ldcg(ids + q / 4 + 1);
-                const int id[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    for (int j = grp; j < mem.tiles; j += groups) {
+        const int i = (mem.first + j * mem.stride) * kStepBlock + gt;
+        if (i >= s.N) continue;
+        const int c = s.cellOf[i], n = min(__ldcg(cnt + c), kCellCap);
+        const int4 *ids = reinterpret_cast<const int4 *>(s.cellIds + (size_t)c * kCellCap);
+        const float2 x = pos[i];
+        const int tag = own_tag(s, i), gi = s.excl[i];
+        int k = 0;
+        for (int q = 0; q < n; q += 8) {
+            const int4 a = __ldcg(ids + q / 4), b = __ldcg(ids + q / 4 + 1);
+            const int id[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
-                for (int u = 0; u < 8; u++) k += q + u < n && id[u] < i;
-            }
-            if constexpr (SLOT) mem.slot[j * kStepBlock + gt] = min(start[c] + k, s.N - 1);
-            s.cellCand[(size_t)c * kCellCap + k] = make_float4(x.x, x.y, __int_as_float(tag), __int_as_float(gi));
+            for (int u = 0; u < 8; u++) k += q + u < n && id[u] < i;
         }
+        if constexpr (SLOT) mem.slot[j * kStepBlock + gt] = min(start[c] + k, s.N - 1);
+        s.cellCand[(size_t)c * kCellCap + k] = make_float4(x.x, x.y, __int_as_float(tag), __int_as_float(gi));
+    }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sc->nbrSum = 0ull;
         sc->maxCount = 0;
         sc->builds += 1ull;
     }
     __syncthreads();
-    if (!coop_exchange(s, sh, r, 0u)) return false;
+    if (!coop_exchange(s, sh, r, 0u)) return kRebuildLost;
     // 3: the lists of the block's own particles
-    if (!skip) {
+    {
         const bool fast = (s.wrapx ? s.ncx >= 5 : s.ncx >= 3) && (s.wrapy ? s.ncy >= 5 : s.ncy >= 3) &&
                           !__ldcg(&sc->outside);  // fast_walk_ok
         constexpr int per = 32 / kListLanes;      // particles per warp
@@ -464,7 +472,7 @@ __device__ __forceinline__ bool coop_rebuild(const DevSys &s, CoopShared &sh, co
         }
     }
     __syncthreads();
-    return true;
+    return kRebuildDone;
 }
 
 // The lists of the last rebuild where the getters and the kernels that follow
@@ -910,6 +918,9 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
     extern __shared__ int4 dyn[];
     __shared__ CoopShared sh;
     DevScalars *sc = s.sc;
+    // a launch of this run before this one was cut short (block 0 sets the word only
+    // after an exchange that every block took part in, or one that gave up)
+    if (!a.begin && __ldcg(&sc->runStop)) return;
     const int nt = MT ? s.numTypes * s.numTypes : 1;
     for (int q = threadIdx.x; q < nt; q += blockDim.x) sh.tab[q] = s.pair[q];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -950,8 +961,6 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
         mem.eng = nullptr;
         mem.slot = mem.list;
         mem.list += per * kStepBlock;
-        for (int q = threadIdx.x; q < per * kStepBlock; q += blockDim.x) mem.slot[q] = 0;  // (a rebuild that is cut short)
-        __syncthreads();
         if (!a.begin)  // as the last rebuild left it
             for (int t = threadIdx.x; t < s.N; t += blockDim.x) {
                 const int i = s.sortedIds[t], k = i / kStepBlock - mem.first;
@@ -1015,7 +1024,9 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
     const int total = (a.begin ? 1 : 0) + a.units + (a.end ? 1 : 0);
     for (int u = 0;; u++) {
         if (rebuild) {
-            if (!(ok = coop_rebuild<SLOT>(s, sh, mem, r, p, withhold))) break;
+            // (neither lists nor their lengths are read before a rebuild that was
+            // made, or the lists of the launch before, loaded above)
+            if (!(ok = coop_rebuild<SLOT>(s, sh, mem, r, p, withhold) == kRebuildDone)) break;
             withhold = false;
         }
         if (u >= total) break;
@@ -1155,6 +1166,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
         sc->totalUpdates = r.updates;
         sc->runTag = r.base + r.xi;
         sc->runFill = r.cnt;
+        sc->runStop = !ok;
     }
 }
 
