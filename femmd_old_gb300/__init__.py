@@ -364,6 +364,10 @@ class System:
         next run that is one cooperative launch is left to time out (run() raises FEMMD_TIMEOUT)."""
         self._call("femmd_test_expire_next_exchange")
 
+    def test_set_exchanges(self, made):
+        """Tests of long-lived contexts: as if 'made' grid-wide exchanges had been made."""
+        self._call("femmd_test_set_exchanges", int(made))
+
     def counts(self):
         return dict(bonds=self._L.femmd_get_num_bonds(self._h), triangles=self._L.femmd_get_num_triangles(self._h),
                     elastomers=self._L.femmd_get_num_elastomers(self._h))

@@ -33,6 +33,7 @@
 
 #include "femmd.h"
 #include "femmd_internal.h"
+#include "grid_sync.cuh"
 #include "launch.h"
 
 using namespace femmd;
@@ -1261,16 +1262,23 @@ static bool coop_ready(femmd_ctx *ctx) {
     return coop_run_fits(s, coop_plan(ctx, s));
 }
 
+// The whole-run launch's exchanges and cell counts, zero before the first and
+// after a launch that was cut short.
+static femmd_status coop_clean(femmd_ctx *ctx) {
+    if (ctx->runClean) return FEMMD_OK;
+    CK(cudaMemsetAsync(ctx->runRec.p, 0, ctx->runRec.n * sizeof(unsigned long long), ctx->stream));
+    CK(cudaMemsetAsync(ctx->cellFill.p, 0, ctx->cellFill.n * sizeof(int), ctx->stream));
+    CK(cudaMemsetAsync(&ctx->sc.p->runTag, 0, sizeof(DevScalars::runTag), ctx->stream));
+    CK(cudaMemsetAsync(&ctx->sc.p->runFill, 0, sizeof(int), ctx->stream));
+    ctx->runClean = true;
+    return FEMMD_OK;
+}
+
 // A run, or part of one, of a small or medium system in one cooperative
 // launch (k_coop.cu); the parity follows its drifts.
 static femmd_status coop_launch(femmd_ctx *ctx, int begin, int units, int end, float2 *slots, int check = 0) {
-    if (!ctx->runClean) {
-        CK(cudaMemsetAsync(ctx->runRec.p, 0, ctx->runRec.n * sizeof(unsigned long long), ctx->stream));
-        CK(cudaMemsetAsync(ctx->cellFill.p, 0, ctx->cellFill.n * sizeof(int), ctx->stream));
-        CK(cudaMemsetAsync(&ctx->sc.p->runTag, 0, 2 * sizeof(int), ctx->stream));  // runTag, runFill
-        static_assert(offsetof(DevScalars, runFill) == offsetof(DevScalars, runTag) + sizeof(int), "run scalars");
-        ctx->runClean = true;
-    }
+    femmd_status st;
+    if ((st = coop_clean(ctx))) return st;
     const DevSys s = make_sys(ctx);
     CoopArgs a = coop_plan(ctx, s);
     a.parity = ctx->cur;
@@ -2919,6 +2927,24 @@ femmd_status femmd_set_profiling(femmd_ctx *ctx, int profile) {
     ctx->profiling = profile != 0;
     ctx->profForceMs = ctx->profRebuildMs = 0;
     ctx->profForceLaunches = ctx->profRebuilds = ctx->profKernels = 0;
+    return FEMMD_OK;
+}
+
+femmd_status femmd_test_set_exchanges(femmd_ctx *ctx, unsigned long long made) {
+    NEED(ctx);
+    femmd_status st;
+    if ((st = prepare(ctx))) return st;
+    if (!coop_ready(ctx)) return fail(ctx, FEMMD_UNSUPPORTED, "runs of this system are not one cooperative launch");
+    if ((st = coop_clean(ctx))) return st;
+    // a slot's count is the grid's blocks for each of its exchanges so far; its
+    // maximum is cleared
+    const unsigned long long blocks = (unsigned long long)coop_grid(make_sys(ctx));
+    std::vector<unsigned long long> slots((size_t)kGridSlots * kGridSlotWords, 0ull);
+    for (int j = 0; j < kGridSlots; j++)
+        slots[(size_t)j * kGridSlotWords + 1] = (made + kGridSlots - 1 - j) / kGridSlots * blocks;
+    CK(cudaMemcpyAsync(ctx->runRec.p, slots.data(), slots.size() * sizeof(slots[0]), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaMemcpyAsync(&ctx->sc.p->runTag, &made, sizeof(made), cudaMemcpyHostToDevice, ctx->stream));
+    CK(cudaStreamSynchronize(ctx->stream));
     return FEMMD_OK;
 }
 

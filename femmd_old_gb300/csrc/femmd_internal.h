@@ -81,7 +81,7 @@ struct DevScalars {
     unsigned int vvMaxBits;               // max v^2 as float bits (v^2 >= 0)
     int sweepLost;                        // a bounded wait of k_adj_sweep expired
     // the whole-run launch (k_coop): the exchanges so far, and which of its two cell-count arrays the last rebuild used
-    unsigned int runTag;
+    unsigned long long runTag;
     int runFill;
     int runStop;  // its last launch was cut short: the run's later ones return at once
 };

@@ -12,7 +12,8 @@
 // away from all pollers), a two-level tree 9600 and 11,200, clusters of eight
 // with one polling CTA each 5400 (32 to 104 blocks).
 //
-// Four slots take turns, exchange X (counted over the life of the context)
+// Four slots take turns, exchange X (counted over the life of the context, in 64
+// bits: a small system makes 2^32 of them in hours)
 // using slot X & 3; a slot's count grows by the grid size with every use, and
 // its max and or are cleared for exchange X + 2 by block 0 after exchange X:
 // every block that used them last (X - 2) has read them before it counted in
@@ -26,7 +27,7 @@ constexpr int kGridSlotWords = 16;  // 8-byte words from one slot to the next (a
 constexpr int kGridSlots = 4;
 constexpr int kGridPolls = 1 << 20;  // polls (about 0.4 us each) before an exchange gives up
 
-__device__ __forceinline__ unsigned long long *grid_slot(unsigned long long *base, unsigned x) {
+__device__ __forceinline__ unsigned long long *grid_slot(unsigned long long *base, unsigned long long x) {
     return base + (size_t)(x & (kGridSlots - 1)) * kGridSlotWords;
 }
 
@@ -35,8 +36,9 @@ __device__ __forceinline__ unsigned long long *grid_slot(unsigned long long *bas
 // this block does not count (a test of the bounded wait).  After a block
 // barrier that follows it, every store made by any block before its call is
 // visible to the whole block.
-__device__ __forceinline__ bool grid_exchange(unsigned long long *base, unsigned x, int blocks, unsigned value,
-                                              unsigned flags, bool withhold, unsigned &maxv, unsigned &orv) {
+__device__ __forceinline__ bool grid_exchange(unsigned long long *base, unsigned long long x, int blocks,
+                                              unsigned value, unsigned flags, bool withhold, unsigned &maxv,
+                                              unsigned &orv) {
     unsigned long long *slot = grid_slot(base, x);
     if (value) asm volatile("red.relaxed.gpu.global.max.u32 [%0], %1;" ::"l"(slot), "r"(value) : "memory");
     if (flags)
@@ -44,7 +46,7 @@ __device__ __forceinline__ bool grid_exchange(unsigned long long *base, unsigned
                      : "memory");
     asm volatile("fence.acq_rel.gpu;" ::: "memory");
     if (!withhold) asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(slot + 1), "l"(1ull) : "memory");
-    const unsigned long long want = ((unsigned long long)(x / kGridSlots) + 1ull) * (unsigned long long)blocks;
+    const unsigned long long want = (x / kGridSlots + 1ull) * (unsigned long long)blocks;
     unsigned long long lo = 0ull, hi = 0ull;
     int it = 0;
     do {

@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_adj_sweep(DevSys s, CoopArg
     __shared__ unsigned okay;
     const int nt = s.numTypes > 1 ? s.numTypes * s.numTypes : 1;
     for (int q = threadIdx.x; q < nt; q += blockDim.x) tab[q] = s.pair[q];
-    const unsigned base = s.sc->runTag;
+    const unsigned long long base = s.sc->runTag;
     unsigned xi = 0;
     const int ntiles = (s.N + kStepBlock - 1) / kStepBlock;
     const bool tris = s.feaForces && s.ntri > 0;

@@ -121,7 +121,7 @@ __device__ __forceinline__ int ld_early(const int *p) {
     return v;
 }
 struct CoopDue {
-    unsigned x;  // the exchange after which the last of the step's sums were stored
+    unsigned long long x;  // the exchange after which the last of the step's sums were stored
     unsigned set;  // their set
     int mode, row, reb;
     float vm, d;
@@ -141,7 +141,8 @@ struct CoopShared {
 
 // What every block carries through the launch (the same on each).
 struct CoopRun {
-    unsigned base, xi;       // exchanges before this launch, and of it
+    unsigned long long base;  // exchanges before this launch
+    unsigned xi;              // and of it
     unsigned dueIn, dueOut;  // entries pushed to and taken from CoopShared::due (one per step)
     unsigned dueOk;          // entries whose sums are all stored
     float dispHi;
@@ -209,7 +210,7 @@ __device__ __forceinline__ bool coop_exchange(const DevSys &s, CoopShared &sh, C
     // a step's sums are visible once the exchange after its own is complete
     while (r.dueOut != r.dueOk && !all) {
         const CoopDue &d = sh.due[r.dueOut & 3u];
-        if ((int)(r.base + r.xi - d.x) < 2) break;
+        if (r.base + r.xi < d.x + 2) break;
         if (blockIdx.x == 0 && threadIdx.x == 64) coop_totals(s, d);
         r.dueOut++;
     }
@@ -1084,7 +1085,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
             if (anybad) atomicOr(&sc->nonfinite, 1);
         }
         __syncthreads();
-        const unsigned x = r.base + r.xi;
+        const unsigned long long x = r.base + r.xi;
         float mm = 0.0f;
         if (warp == 0) mm = warp_max(lane < kCoopThreads / 32 ? sh.vmax[lane] : 0.0f);
         if (!(ok = coop_exchange(s, sh, r, __float_as_uint(mm), withhold, false,

@@ -254,6 +254,10 @@ femmd_status femmd_get_profile(femmd_ctx *ctx, double *force_kernel_ms, long lon
  * (about a second) and femmd_run returns FEMMD_TIMEOUT with the context
  * still usable.  No GPU fault, trap or endless wait is involved. */
 femmd_status femmd_test_expire_next_exchange(femmd_ctx *ctx);
+/* For tests of long-lived contexts: from here on as if 'made' grid-wide
+ * exchanges had been made (FEMMD_UNSUPPORTED where runs are not one
+ * cooperative launch). */
+femmd_status femmd_test_set_exchanges(femmd_ctx *ctx, unsigned long long made);
 
 /* ------------------------------------------------------- batched replicas */
 /* Many independent systems advanced in one persistent launch: each replica
