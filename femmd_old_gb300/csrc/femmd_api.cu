@@ -3253,38 +3253,43 @@ static femmd_status adj_recompute(femmd_ctx *ctx, int g, std::vector<int> &rebui
     auto &a = ctx->adj;
     const int N = (int)ctx->pos.size(), K = a.segLen[g];
     cudaStream_t st = ctx->stream;
-    CK(cudaMemcpyAsync(ctx->dpos0.p, a.ckX.p + (size_t)g * N, N * sizeof(float2), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(ctx->dvel.p, a.ckV.p + (size_t)g * N, N * sizeof(float2), cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(a.slots.p, ctx->dpos0.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, st));
-    ctx->cur = 0;
-    ctx->steps = a.segStart[g];
-    DevSys s = make_sys(ctx);
-    Launch L;
-    L.stream = st;
     femmd_status e;
-    CK(cudaMemsetAsync(&ctx->sc.p->overflow, 0, 3 * sizeof(int), st));
-    if (coop_ready(ctx)) {
-        if ((e = coop_launch(ctx, 1, K - 1, 0, a.slots.p))) return e;
-    } else {
-        CK(enqueue_run_start(L, s));
-        CK(enqueue_rebuild(L, s, 0, 1));
-        CK(enqueue_step(L, s, MODE_FIRST, 0, 0, 0));
-        int cur = 1;
-        CK(cudaMemcpyAsync(a.slots.p + N, ctx->dpos1.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, st));
-        for (int u = 1; u < K; u++) {
-            CK(enqueue_step(L, s, MODE_MID, cur, 0, 0));
-            float2 *pout = cur ? ctx->dpos0.p : ctx->dpos1.p;
-            CK(cudaMemcpyAsync(a.slots.p + (size_t)(u + 1) * N, pout, N * sizeof(float2), cudaMemcpyDeviceToDevice,
-                               st));
-            // the rebuild kernels only where the forward rebuilt (elsewhere
-            // their check would return at once); a disagreement is caught below
-            if (a.segReb[g][u]) CK(enqueue_rebuild(L, s, 1 - cur, 1));
-            cur ^= 1;
+    // as the forward's runs: one launch where they are, the plain kernels else and
+    // where that launch meets a state that it cannot list
+    for (bool whole = coop_whole(ctx, K);; whole = false) {
+        CK(cudaMemcpyAsync(ctx->dpos0.p, a.ckX.p + (size_t)g * N, N * sizeof(float2), cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(ctx->dvel.p, a.ckV.p + (size_t)g * N, N * sizeof(float2), cudaMemcpyDeviceToDevice, st));
+        CK(cudaMemcpyAsync(a.slots.p, ctx->dpos0.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, st));
+        ctx->cur = 0;
+        ctx->steps = a.segStart[g];
+        DevSys s = make_sys(ctx);
+        Launch L;
+        L.stream = st;
+        CK(cudaMemsetAsync(&ctx->sc.p->overflow, 0, 3 * sizeof(int), st));
+        if (whole) {
+            if ((e = coop_launch(ctx, 1, K - 1, 0, a.slots.p))) return e;
+        } else {
+            CK(enqueue_run_start(L, s));
+            CK(enqueue_rebuild(L, s, 0, 1));
+            CK(enqueue_step(L, s, MODE_FIRST, 0, 0, 0));
+            int cur = 1;
+            CK(cudaMemcpyAsync(a.slots.p + N, ctx->dpos1.p, N * sizeof(float2), cudaMemcpyDeviceToDevice, st));
+            for (int u = 1; u < K; u++) {
+                CK(enqueue_step(L, s, MODE_MID, cur, 0, 0));
+                float2 *pout = cur ? ctx->dpos0.p : ctx->dpos1.p;
+                CK(cudaMemcpyAsync(a.slots.p + (size_t)(u + 1) * N, pout, N * sizeof(float2), cudaMemcpyDeviceToDevice,
+                                   st));
+                // the rebuild kernels only where the forward rebuilt (elsewhere
+                // their check would return at once); a disagreement is caught below
+                if (a.segReb[g][u]) CK(enqueue_rebuild(L, s, 1 - cur, 1));
+                cur ^= 1;
+            }
         }
+        if ((e = read_scalars(ctx))) return e;
+        if (ctx->hsc->overflow & 8) return expired(ctx, "a grid-wide exchange");
+        if (!(ctx->hsc->overflow & 32)) break;
+        coop_left(ctx);
     }
-    if ((e = read_scalars(ctx))) return e;
-    if (ctx->hsc->overflow & 8) return expired(ctx, "a grid-wide exchange");
-    if (ctx->hsc->overflow & 32) coop_left(ctx);
     if (ctx->hsc->overflow || ctx->hsc->nonfinite)
         return fail(ctx, ctx->hsc->overflow ? FEMMD_CAPACITY_OVERFLOW : FEMMD_NONFINITE,
                     "the recomputed segment differs from the forward pass (overflow or non-finite force)");
@@ -3398,6 +3403,7 @@ femmd_status femmd_adjoint_backward(femmd_ctx *ctx, double c_wall, double c_fea,
                 w.kLo = to;
                 w.segStart = s0;
                 w.start = a.segStart[0];
+                if ((st = coop_clean(ctx))) return st;
                 CK(launch_adj_sweep(sm, s, coop_plan(ctx, s), w));
                 if ((k - std::max(to, 1) + 1) & 1) std::swap(wc, wn);
                 k = to - 1;
