@@ -3661,7 +3661,9 @@ static femmd_status batch_prepare(femmd_batch *b, int steps, BatchLaunch &bl, st
     return FEMMD_OK;
 }
 
-static femmd_status batch_launch(femmd_batch *b, const BatchLaunch &bl) {
+// The launch as a graph (kept until something that it holds changes): the
+// kernels of its cluster sizes are parallel branches.
+static femmd_status batch_graph(femmd_batch *b, const BatchLaunch &bl) {
     const int variant = bl.multiType | bl.sigmaByType << 1 | bl.sigmaOne << 2 | bl.wrapx << 3 | bl.wrapy << 4;
     const std::vector<BatchClass> cls(bl.cls, bl.cls + bl.nclass);
     const bool rebuild = !b->graph.x || b->graphSteps != bl.steps || b->graphThreads != bl.threads ||
@@ -3686,8 +3688,30 @@ static femmd_status batch_launch(femmd_batch *b, const BatchLaunch &bl) {
         b->graphMinBlocks = bl.minBlocks;
         b->graphCls = cls;
     }
+    return FEMMD_OK;
+}
+
+static femmd_status batch_launch(femmd_batch *b, const BatchLaunch &bl) {
+    femmd_status st;
+    if ((st = batch_graph(b, bl))) return st;
     BCK(cudaMemsetAsync(bl.queue, 0, 2 * kBatchMaxCluster * sizeof(int), b->stream));
     BCK(cudaGraphLaunch(b->graph.x, b->stream));
+    return FEMMD_OK;
+}
+
+// The time of a trial, launched as femmd_batch_run launches it (kernel after kernel
+// in a stream the cluster sizes would run one after another and their times add
+// up), without the graph's instantiation and upload.
+static femmd_status batch_trial(femmd_batch *b, const BatchLaunch &bl, cudaEvent_t e0, cudaEvent_t e1, float *ms) {
+    femmd_status st;
+    if ((st = batch_graph(b, bl))) return st;
+    BCK(cudaGraphUpload(b->graph.x, b->stream));
+    BCK(cudaMemsetAsync(bl.queue, 0, 2 * kBatchMaxCluster * sizeof(int), b->stream));
+    BCK(cudaEventRecord(e0, b->stream));
+    BCK(cudaGraphLaunch(b->graph.x, b->stream));
+    BCK(cudaEventRecord(e1, b->stream));
+    BCK(cudaStreamSynchronize(b->stream));
+    BCK(cudaEventElapsedTime(ms, e0, e1));
     return FEMMD_OK;
 }
 
@@ -3892,25 +3916,16 @@ femmd_status femmd_batch_autotune(femmd_batch *b, int trial_steps, int *threads_
         femmd_status st;
         if ((st = batch_prepare(b, trial_steps, bl, sys))) return st;
         if ((st = batch_checkpoint(b, false))) return st;
-        BCK(cudaMemsetAsync(bl.queue, 0, 2 * kBatchMaxCluster * sizeof(int), b->stream));
-        BCK(cudaEventRecord(e0, b->stream));
-        cudaError_t le = cudaSuccess;
-        {
-            Launch L;
-            L.stream = b->stream;
-            le = enqueue_batch(L, bl);
-        }
-        BCK(cudaEventRecord(e1, b->stream));
-        cudaError_t se = cudaStreamSynchronize(b->stream);
-        if (le == cudaSuccess && se == cudaSuccess) {
-            float ms = 0;
-            BCK(cudaEventElapsedTime(&ms, e0, e1));
+        float ms = 0;
+        if (batch_trial(b, bl, e0, e1, &ms) == FEMMD_OK) {
             if (ms < best) {
                 best = ms;
                 bt = cd[0];
                 bc = cd[1];
             }
         } else {
+            b->graph.release();
+            b->err.clear();
             cudaGetLastError();  // a shape the device cannot run: skip it
         }
         if ((st = batch_checkpoint(b, true))) return st;
@@ -3973,17 +3988,8 @@ femmd_status femmd_batch_autotune_lists(femmd_batch *b, int trial_steps, const d
             std::vector<DevSys> sys;
             if ((st = batch_prepare(b, trial_steps, bl, sys))) return st;
             if ((st = batch_checkpoint(b, false))) return st;
-            BCK(cudaMemsetAsync(bl.queue, 0, 2 * kBatchMaxCluster * sizeof(int), b->stream));
-            BCK(cudaEventRecord(e0, b->stream));
-            {
-                Launch L;
-                L.stream = b->stream;
-                BCK(enqueue_batch(L, bl));
-            }
-            BCK(cudaEventRecord(e1, b->stream));
-            BCK(cudaStreamSynchronize(b->stream));
             float ms = 0;
-            BCK(cudaEventElapsedTime(&ms, e0, e1));
+            if ((st = batch_trial(b, bl, e0, e1, &ms))) return st;
             if ((st = batch_read(b))) return st;
             bool over = false;
             for (femmd_ctx *c : b->reps) over = over || (!c->pos.empty() && c->hsc->overflow);

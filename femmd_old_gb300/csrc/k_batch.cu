@@ -433,8 +433,8 @@ __global__ void __launch_bounds__(1024, 1)
 
 namespace {
 
-// One kernel per class, side by side (parallel branches of a graph; one after
-// another in a stream), the largest clusters first.
+// One kernel per class, side by side (parallel branches of a graph), the largest
+// clusters first.
 template <bool MT, bool SG, bool WX, bool WY, bool SIG1>
 cudaError_t launch_batch(Launch &L, const BatchLaunch &b) {
     const std::vector<cudaGraphNode_t> before = L.deps;
@@ -442,7 +442,7 @@ cudaError_t launch_batch(Launch &L, const BatchLaunch &b) {
     for (int k = 0; k < b.nclass && !e; k++) {
         const BatchClass &c = b.cls[k];
         int *queue = b.queue + 2 * k;
-        if (L.graph) L.deps = before;
+        L.deps = before;
         if (c.cluster > 1)
             e = L.kernel_clusters(k_batch_gang<MT, SG, WX, WY, SIG1>, c.cluster, dim3(c.ctas), dim3(b.threads), b.smem,
                                   b.reps, b.order + c.first, c.count, queue, b.state, b.steps);

@@ -96,26 +96,15 @@ struct Launch {
         return cudaSuccess;
     }
 
-    // kernel() with the grid in clusters of n blocks.
+    // kernel() with the grid in clusters of n blocks.  Graph mode only.
     template <typename... KArgs, typename... Args>
     cudaError_t kernel_clusters(void (*k)(KArgs...), int n, dim3 g, dim3 b, size_t smem, Args &&...args) {
-        cudaLaunchAttribute at[1] = {};
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = n;
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-        if (graph) {
-            cudaError_t e = kernel(k, g, b, smem, std::forward<Args>(args)...);
-            return e ? e : cudaGraphKernelNodeSetAttribute(deps.back(), at[0].id, &at[0].val);
-        }
-        kernels++;
-        cudaLaunchConfig_t c = {};
-        c.gridDim = g;
-        c.blockDim = b;
-        c.dynamicSmemBytes = smem;
-        c.stream = stream;
-        c.attrs = at;
-        c.numAttrs = 1;
-        return cudaLaunchKernelEx(&c, k, std::forward<Args>(args)...);
+        if (!graph) return cudaErrorInvalidValue;
+        cudaLaunchAttributeValue v = {};
+        v.clusterDim.x = n;
+        v.clusterDim.y = v.clusterDim.z = 1;
+        const cudaError_t e = kernel(k, g, b, smem, std::forward<Args>(args)...);
+        return e ? e : cudaGraphKernelNodeSetAttribute(deps.back(), cudaLaunchAttributeClusterDimension, &v);
     }
 
   private:
