@@ -798,7 +798,7 @@ __device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &me
         if (SIG1 && !SG) {
             // the packed terms, with the images where a lane of the warp is
             // near an edge; the scalar ones where they do not stand
-            float far = 0.0f, close = 1.0f;
+            float far = 0.0f, close = 1.0f, w = 0.0f;
             auto packed = [&](auto edge) {
 #pragma unroll
                 for (int u = 0; u < kQuadPairs; u++) {
@@ -807,11 +807,12 @@ __device__ __forceinline__ void coop_particle(const DevSys &s, const CoopMem &me
                         tab + (MT ? ti * s.numTypes + ((unsigned)tag[u] >> kIdBits) : 0));
                     o[u] = lj_terms_x2<decltype(edge)::value, WX, WY>(s, pi, pj[u], make_float2(e.x, e.y), e.z, e.w,
                                                                      in, far, close);
+                    w += o[u].w;
                 }
             };
             if (near) packed(std::true_type{});
             else packed(std::false_type{});
-            done = !__any_sync(0xffffffffu, !lj_sums_ok<WX, WY>(s, far, close));
+            done = !__any_sync(0xffffffffu, !lj_sums_ok<WX, WY>(s, far, close, w));
         }
         if (!done) {
 #pragma unroll

@@ -358,7 +358,10 @@ __device__ __forceinline__ void lj_pair(const DevSys &s, const PairEntry *tab, c
 // Measured: the batched kernel 27.2 -> 23.5 ms (128 replicas, run(100)), the
 // large mixed system's run(50) 9.32 -> 8.84 ms.
 //   * outside the cutoff zeros are added: no branch per pair.  (A sum that
-//     starts at +0 never is -0, so +-0 added leaves it as it is.)
+//     starts at +0 never is -0, so +-0 added leaves it as it is.)  The zero force
+//     times an infinite or NaN difference is NaN, where lj_pair adds nothing; the
+//     virial (zero times r^2) is then NaN too, and with a virial sum that is not
+//     finite the caller works the particle again by lj_pair.
 constexpr float kPairClose = 1e-30f;
 
 // The pair's terms: force x and y, doubled energy and virial.  EDGE: the
@@ -415,11 +418,12 @@ __device__ __forceinline__ void lj_pair_x2(const DevSys &s, float2 pi, float2 pj
     a.UW = add2(a.UW, make_float2(t.z, t.w));
 }
 
-// Whether the terms stand: no pair crossed the boundary, none was too close.
+// Whether the terms stand: no pair crossed the boundary, none was too close, and
+// every position was finite (w: the sum of the virials).
 template <bool WX, bool WY>
-__device__ __forceinline__ bool lj_sums_ok(const DevSys &s, float far, float close) {
+__device__ __forceinline__ bool lj_sums_ok(const DevSys &s, float far, float close, float w) {
     const float h = WX && WY ? fminf(0.5f * s.Lx, 0.5f * s.Ly) : (WX ? 0.5f * s.Lx : 0.0f);
-    return (!(WX || WY) || far < h) && close >= kPairClose;
+    return (!(WX || WY) || far < h) && close >= kPairClose && isfinite(w);
 }
 
 // A particle at p within reach of a periodic edge (its listed pairs may cross it).
@@ -597,7 +601,7 @@ __device__ __forceinline__ void particle_step(const DevSys &s, const PairEntry *
                 lj_list_x2<MT, !RO, WX, WY, RO>(s, tab, i, cnt, pi, pin, a);
             else
                 lj_list_x2<MT, false, WX, WY, RO>(s, tab, i, cnt, pi, pin, a);
-            if (lj_sums_ok<WX, WY>(s, a.far, a.close)) {
+            if (lj_sums_ok<WX, WY>(s, a.far, a.close, a.UW.y)) {
                 fx = a.F.x;
                 fy = a.F.y;
                 ue = a.UW.x;
