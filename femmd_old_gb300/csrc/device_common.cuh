@@ -49,12 +49,15 @@ __device__ __forceinline__ float diff_shift(float a, float b, int k, float L) {
 // pbcCalc (femmd2D/src/def.h:112)
 __device__ __forceinline__ float wrap_coord(float r, float L) { return r - floorf(r / L) * L; }
 
-// wrap_coord without its division for -L <= r < 2 L, where floor(r / L) is
-// -1, 0 or 1 whatever the quotient's rounding (r < L gives a quotient of at
-// most 1 - 2^-24, r < 2 L one of at most 2 - 2^-23): the same single rounding.
+// wrap_coord without its division where one box length added or taken away
+// gives a value in [0, L): -L <= r < 2 L, where floor(r / L) is -1, 0 or 1 whatever
+// the quotient's rounding (r < L gives a quotient of at most 1 - 2^-24, r < 2 L one
+// of at most 2 - 2^-23): the same single rounding.  A negative r that L swallows
+// is left to wrap_coord: its quotient can round to -0, whose floor is no -1.
+// (r - 0 L is r + 0: +0 for r = -0.)
 __device__ __forceinline__ float wrap_near(float r, float L) {
-    const float w = r < 0.0f ? r + L : (r >= L ? r - L : r);
-    return (r >= -L && r < 2.0f * L) ? w : wrap_coord(r, L);
+    const float w = r < 0.0f ? r + L : (r >= L ? r - L : r + 0.0f);
+    return (w >= 0.0f && w < L) ? w : wrap_coord(r, L);
 }
 
 // cellId (femmd2D/src/nnCuda.cu:9-17): float multiply, IEEE divide, truncate;
