@@ -1250,7 +1250,7 @@ static CoopArgs coop_plan(femmd_ctx *ctx, const DevSys &s) {
 // Whether runs of the context go to one cooperative launch (k_coop.cu), its
 // buffers allocated on the first of them.
 static bool coop_ready(femmd_ctx *ctx) {
-    if (ctx->coopOff || !coop_size_ok((int)ctx->pos.size(), ctx->ncells)) return false;
+    if (ctx->coopOff || !coop_size_ok(make_sys(ctx))) return false;
     const size_t cells = ctx->ncells;
     if (ctx->runRec.ensure(kCoopRecWords) || ctx->cellFill.ensure(2 * cells) ||
         ctx->cellIds.ensure(cells * kCellCap) || ctx->cellCand.ensure(cells * kCellCap)) {

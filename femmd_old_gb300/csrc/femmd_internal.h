@@ -282,7 +282,7 @@ struct CoopArgs {
 // Whether a launch groups the particles' energies by storage slot, as the fast
 // mode's step kernels do (small systems of one type without bonded particles).
 bool coop_by_slot(const DevSys &s);
-bool coop_size_ok(int N, int ncells);
+bool coop_size_ok(const DevSys &s);
 bool coop_run_fits(const DevSys &s, const CoopArgs &plan);
 // The blocks of a system; with triangles by block, the block of a tile of 128 particles.
 int coop_grid(const DevSys &s);

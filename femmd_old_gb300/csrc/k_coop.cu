@@ -68,7 +68,7 @@ int coop_grid(const DevSys &s) {
 // every rebuild would cost them a scan of all cells per block).
 bool coop_by_slot(const DevSys &s) {
     return s.fast && s.numTypes <= 1 && s.nBonded == 0 && s.N <= 128 * kStepBlock &&
-           s.ncells <= coop_terms(true) * kTermComp;
+           s.ncells <= 2 * coop_terms(true) * kTermComp;
 }
 
 int coop_block(int ntiles, int grid, int tile) { return coop_pairs(ntiles, grid) ? tile / 2 : tile % grid; }
@@ -83,9 +83,14 @@ bool coop_run_fits(const DevSys &s, const CoopArgs &plan) {
     return resident >= grid;
 }
 
-// The sizes a whole-run launch is made for: its cell table has kCellCap slots
-// per cell, so that a nearly empty box is left to the plain kernels.
-bool coop_size_ok(int N, int ncells) { return N > 0 && N <= kCoopMaxN && ncells <= 4 * N + 4096; }
+// The sizes a whole-run launch is made for: its cell table has kCellCap slots of 20
+// bytes per cell (250 MB at most), so that a nearly empty box is left to the plain
+// kernels.  Not a small fluid's in the fast mode: 2000 particles in 25,281 cells
+// (density 0.01), run(100) 630 us against 1590 by the plain kernels; 64 in 8100,
+// 411 against 1487.
+bool coop_size_ok(const DevSys &s) {
+    return s.N > 0 && s.N <= kCoopMaxN && (s.ncells <= 4 * s.N + 4096 || coop_by_slot(s));
+}
 
 cudaError_t launch_coop_run(cudaStream_t st, const DevSys &s, const CoopArgs &a) {
     int grid;

@@ -405,20 +405,21 @@ __device__ __forceinline__ CoopRebuild coop_rebuild(const DevSys &s, CoopShared 
     // 2: ascending id inside each cell; the other counts cleared for the next
     // rebuild (their last readers were the lists before this rebuild)
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < s.ncells; c += gridDim.x * blockDim.x) other[c] = 0;
-    [[maybe_unused]] int *start = reinterpret_cast<int *>(mem.term);  // by slot: the cells' starts (no terms there now)
+    // by slot: the cells' starts (no terms there now; at most 16,384 particles)
+    [[maybe_unused]] unsigned short *start = reinterpret_cast<unsigned short *>(mem.term);
     if constexpr (SLOT) {
         const int chunk = (s.ncells + blockDim.x - 1) / blockDim.x;
         const int c0 = min((int)threadIdx.x * chunk, s.ncells), c1 = min(c0 + chunk, s.ncells);
         int sum = 0, tot;
         for (int c = c0; c < c1; c++) {
             const int n = min(__ldcg(cnt + c), kCellCap);
-            start[c] = n;
+            start[c] = (unsigned short)n;
             sum += n;
         }
         int at = block_scan(sh, sum, tot);
         for (int c = c0; c < c1; c++) {
             const int n = start[c];
-            start[c] = at;
+            start[c] = (unsigned short)at;
             at += n;
         }
         __syncthreads();
