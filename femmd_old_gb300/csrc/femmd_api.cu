@@ -217,6 +217,7 @@ struct femmd_ctx {
     DBuf<int> cellFill, cellIds;
     DBuf<float4> cellCand;
     bool runClean = false, coopOff = false;
+    int cellCap = kCellCap;
     int triGrid = 0, triMost = 0;  // coop_plan: made for this many blocks (0: not made), CoopArgs::triMost
     bool permIdent = false;  // fast mode: the storage order is the id order
     // profiling
@@ -508,6 +509,7 @@ static DevSys make_sys(femmd_ctx *c) {
     s.cellFill = c->cellFill.p;
     s.cellIds = c->cellIds.p;
     s.cellCand = c->coopOff ? nullptr : c->cellCand.p;
+    s.cellCap = c->cellCap;
     s.obs = c->obs.p;
     s.obsCap = c->obsCap;
     s.trace = c->tracing ? c->trace.p : nullptr;
@@ -830,6 +832,7 @@ static femmd_status upload_topology(femmd_ctx *ctx) {
     CK(ctx->blockSums.ensure(scan_blocks(ctx->ncells)));
     CK(ctx->sc.ensure(1));
     ctx->runClean = ctx->coopOff = false;
+    ctx->cellCap = kCellCap;
     ctx->triGrid = 0;
     cudaStream_t s = ctx->stream;
     if (N > 0) {
@@ -1183,11 +1186,20 @@ static femmd_status expired(femmd_ctx *ctx, const char *what) {
 
 // A whole-run launch was left at a rebuild that it could not make (overflow bit
 // 32): a non-finite position, for which the run is repeated by the plain kernels, or a
-// cell of more than kCellCap particles (bit 16), from which on all runs are theirs.
+// cell of more than cellCap particles (bit 16).  A small fluid in the fast mode gets a
+// larger table of cells then (its runs were one launch with cells of any size
+// before the table; 2000 particles with a cutoff of 6 sigma, 31 a cell on average,
+// run(100) 1330 us against 3580 by the plain kernels), up to 20 MB; all runs of
+// another system are the plain kernels' from there on.  True: the launch again.
 // The cell counts of the binning are cleared before the next launch.
-static void coop_left(femmd_ctx *ctx) {
+static bool coop_left(femmd_ctx *ctx) {
     ctx->runClean = false;
-    if (ctx->hsc->overflow & 16) ctx->coopOff = true;
+    if (!(ctx->hsc->overflow & 16)) return false;
+    const int cap = std::max(2 * ctx->cellCap, (ctx->hsc->maxCell + ctx->hsc->maxCell / 4 + 31) / 32 * 32);
+    const bool again = (size_t)cap * ctx->ncells <= (1u << 20) && coop_by_slot(make_sys(ctx));
+    if (again) ctx->cellCap = cap;
+    else ctx->coopOff = true;
+    return again;
 }
 
 // The triangles by block of the whole-run launch (CoopArgs), laid out once per
@@ -1253,7 +1265,7 @@ static bool coop_ready(femmd_ctx *ctx) {
     if (ctx->coopOff || !coop_size_ok(make_sys(ctx))) return false;
     const size_t cells = ctx->ncells;
     if (ctx->runRec.ensure(kCoopRecWords) || ctx->cellFill.ensure(2 * cells) ||
-        ctx->cellIds.ensure(cells * kCellCap) || ctx->cellCand.ensure(cells * kCellCap)) {
+        ctx->cellIds.ensure(cells * ctx->cellCap) || ctx->cellCand.ensure(cells * ctx->cellCap)) {
         cudaGetLastError();  // no memory for the cell table: the plain kernels
         ctx->coopOff = true;
         return false;
@@ -2468,8 +2480,8 @@ femmd_status femmd_run(femmd_ctx *ctx, int steps) {
         if (ctx->propAvg)
             CK(cudaMemcpyAsync(ctx->props.p, ctx->propsCk.p, sizeof(DevProps), cudaMemcpyDeviceToDevice, ctx->stream));
         if (ctx->hsc->overflow & 32) {
-            plain = true;
-            coop_left(ctx);
+            plain = !coop_left(ctx);
+            attempt--;  // (once more at most by the plain kernels, or with a table twice as large, up to its limit)
             if (!(ctx->hsc->overflow & 1)) continue;
         }
         int need = std::max(ctx->hsc->maxCount, ctx->nbrCap + ctx->nbrCap / 2);

@@ -83,6 +83,7 @@ struct DevScalars {
     // the whole-run launch (k_coop): the exchanges so far, and which of its two cell-count arrays the last rebuild used
     unsigned long long runTag;
     int runFill;
+    int maxCell;  // the most particles of a cell that a launch found too crowded
     int runStop;  // its last launch was cut short: the run's later ones return at once
 };
 
@@ -195,10 +196,11 @@ struct DevSys {
     int *blockWin;
     // the whole-run launch (k_coop): its exchange slots (grid_sync.cuh), then
     // four sets of energy sums and a word per block; its cells hold up to kCellCap particles
-    // each (ids, then the candidates in id order; two arrays of counts in turn)
+    // (coop_by_slot: cellCap) each (ids, then the candidates in id order; two arrays of counts in turn)
     unsigned long long *runRec;
     int *cellFill, *cellIds;
     float4 *cellCand;
+    int cellCap;
 };
 
 
@@ -258,7 +260,7 @@ cudaError_t kernel_setup(const void *fn, int threads, size_t smem, int *resident
 constexpr int kCoopMaxBlocks = 256;
 // exchange slots, four sets of sums, a word per block
 constexpr size_t kCoopRecWords = 4 * 16 + 4 * 4 + (size_t)kCoopMaxBlocks;
-constexpr int kCellCap = 32;  // particles of a cell at most (a fuller one: the plain kernels)
+constexpr int kCellCap = 32;  // particles of a cell at most (a fuller one: the plain kernels, or a larger table)
 struct CoopArgs {
     int parity;   // of the current positions
     int begin;    // the run start, forced rebuild and first step, and the checkpoint of the start state

@@ -84,7 +84,7 @@ namespace {
 
 constexpr int kCoopThreads = 512;
 constexpr int kCoopTimeout = 8;     // DevScalars::overflow bit: a bounded wait expired
-constexpr int kCoopCrowded = 16;    // DevScalars::overflow bit: a cell holds more than kCellCap particles
+constexpr int kCoopCrowded = 16;    // DevScalars::overflow bit: a cell holds more than cell_cap particles
 constexpr int kCoopLeft = 32;       // DevScalars::overflow bit: a rebuild could not be made (kRebuildLeft)
 constexpr int kCoopMaxTiles = 32;   // tiles of one block (one lane of a warp sums each)
 constexpr int kTriTile = 256;       // triangles per energy group (k_tri_forces' block)
@@ -279,6 +279,12 @@ __host__ __device__ inline int coop_tiles(int ntiles, int grid, int b, bool pair
     return pair ? (ntiles - first < 2 ? ntiles - first : 2) : (ntiles - 1 - first) / stride + 1;
 }
 
+// Particles that a cell of the launch's table holds (a multiple of 8).
+template <bool SLOT>
+__device__ __forceinline__ int cell_cap(const DevSys &s) {
+    return SLOT ? s.cellCap : kCellCap;
+}
+
 // The list of particle i (slot 'col' of the block's tile j) by kListLanes
 // lanes: the 3 x 3 cells in the reference's order (dx outer, dy inner, each
 // cell's particles by ascending id, cell indices wrapped as applyCellBC,
@@ -287,7 +293,7 @@ __host__ __device__ inline int coop_tiles(int ntiles, int grid, int b, bool pair
 // the minimum image per pair.  The first candidates of all nine cells are in
 // flight together.  Entries go to shared memory (from entry mem.rows on, to
 // the list itself; the others are copied there at the end of the launch).  All lanes of the warp call it; returns the list length.
-template <bool FAST>
+template <bool FAST, bool SLOT>
 __device__ __forceinline__ int coop_list(const DevSys &s, const CoopMem &mem, const int *cnt, const float2 *pos, int i,
                                          int j, int col, bool valid) {
     const int lane = threadIdx.x & 31, sub = lane & (kListLanes - 1), shift = lane & ~(kListLanes - 1);
@@ -302,13 +308,14 @@ __device__ __forceinline__ int coop_list(const DevSys &s, const CoopMem &mem, co
     const int cy[3] = {(iy == 0 ? ncy : iy) - 1, iy, iy == ncy - 1 ? 0 : iy + 1};
     const float sx[3] = {ix == 0 ? -Lx : 0.0f, 0.0f, ix == ncx - 1 ? Lx : 0.0f};
     const float sy[3] = {iy == 0 ? -Ly : 0.0f, 0.0f, iy == ncy - 1 ? Ly : 0.0f};
+    const int cells = cell_cap<SLOT>(s);
     int n[9];
     float4 c0[9];
 #pragma unroll
     for (int q = 0; q < 9; q++) {
         const int cell = cx[q / 3] * ncy + cy[q % 3];
         n[q] = ld_early(cnt + cell);
-        c0[q] = ld_early(s.cellCand + (size_t)cell * kCellCap + sub);
+        c0[q] = ld_early(s.cellCand + (size_t)cell * cells + sub);
     }
     int *lst = mem.list + (size_t)j * mem.rows * kListRow + col;
     int k = 0;
@@ -336,7 +343,7 @@ __device__ __forceinline__ int coop_list(const DevSys &s, const CoopMem &mem, co
     bool more = false;
 #pragma unroll
     for (int q = 0; q < 9; q++) {
-        n[q] = valid ? min(n[q], kCellCap) : 0;
+        n[q] = valid ? min(n[q], cells) : 0;
         more = more || n[q] > kListLanes;
     }
     if (!__any_sync(0xffffffffu, more)) {
@@ -350,7 +357,7 @@ __device__ __forceinline__ int coop_list(const DevSys &s, const CoopMem &mem, co
             const int cell = cx[q / 3] * ncy + cy[q % 3];
             for (int o = kListLanes; o < most; o += kListLanes) {
                 const bool on = o + sub < n[q];
-                test(s.cellCand[(size_t)cell * kCellCap + (on ? o + sub : 0)], on, q);
+                test(s.cellCand[(size_t)cell * cells + (on ? o + sub : 0)], on, q);
             }
         }
     }
@@ -362,7 +369,7 @@ __device__ __forceinline__ int coop_list(const DevSys &s, const CoopMem &mem, co
 }
 
 // NeighborList::update's taken branch for the positions of buffer p: cells of
-// at most kCellCap particles by counting atomics, the in-cell order by id,
+// at most cell_cap particles by counting atomics, the in-cell order by id,
 // and the lists of the block's own particles.  Two exchanges.  A non-finite
 // position or a crowded cell ends the launch here, on every block alike
 // (kRebuildLeft): there are no lists to go on with (before a run's first rebuild
@@ -380,6 +387,7 @@ __device__ __forceinline__ CoopRebuild coop_rebuild(const DevSys &s, CoopShared 
     r.dispHi = 0.0f;
     r.cnt ^= 1;
     int *cnt = s.cellFill + (size_t)r.cnt * s.ncells, *other = s.cellFill + (size_t)(r.cnt ^ 1) * s.ncells;
+    const int cap = cell_cap<SLOT>(s);
     // 1: cells, and the ids into them in any order
     for (int j = grp; j < mem.tiles; j += groups) {
         const int i = (mem.first + j * mem.stride) * kStepBlock + gt;
@@ -390,8 +398,12 @@ __device__ __forceinline__ CoopRebuild coop_rebuild(const DevSys &s, CoopShared 
         const int c = cell_col(x.x, x.y, s.ncx, s.ncy, s.Lx, s.Ly);
         s.cellOf[i] = c;
         const int k = atomicAdd(cnt + c, 1);
-        if (k < kCellCap) s.cellIds[(size_t)c * kCellCap + k] = i;
-        else atomicOr(&sc->overflow, kCoopCrowded);
+        if (k < cap) {
+            s.cellIds[(size_t)c * cap + k] = i;
+        } else {
+            atomicOr(&sc->overflow, kCoopCrowded);
+            atomicMax(&sc->maxCell, k + 1);
+        }
     }
     __syncthreads();
     if (!coop_exchange(s, sh, r, 0u, withhold)) return kRebuildLost;
@@ -412,7 +424,7 @@ __device__ __forceinline__ CoopRebuild coop_rebuild(const DevSys &s, CoopShared 
         const int c0 = min((int)threadIdx.x * chunk, s.ncells), c1 = min(c0 + chunk, s.ncells);
         int sum = 0, tot;
         for (int c = c0; c < c1; c++) {
-            const int n = min(__ldcg(cnt + c), kCellCap);
+            const int n = min(__ldcg(cnt + c), cap);
             start[c] = (unsigned short)n;
             sum += n;
         }
@@ -427,8 +439,8 @@ __device__ __forceinline__ CoopRebuild coop_rebuild(const DevSys &s, CoopShared 
     for (int j = grp; j < mem.tiles; j += groups) {
         const int i = (mem.first + j * mem.stride) * kStepBlock + gt;
         if (i >= s.N) continue;
-        const int c = s.cellOf[i], n = min(__ldcg(cnt + c), kCellCap);
-        const int4 *ids = reinterpret_cast<const int4 *>(s.cellIds + (size_t)c * kCellCap);
+        const int c = s.cellOf[i], n = min(__ldcg(cnt + c), cap);
+        const int4 *ids = reinterpret_cast<const int4 *>(s.cellIds + (size_t)c * cap);
         const float2 x = pos[i];
         const int tag = own_tag(s, i), gi = s.excl[i];
         int k = 0;
@@ -439,7 +451,7 @@ __device__ __forceinline__ CoopRebuild coop_rebuild(const DevSys &s, CoopShared 
             for (int u = 0; u < 8; u++) k += q + u < n && id[u] < i;
         }
         if constexpr (SLOT) mem.slot[j * kStepBlock + gt] = min(start[c] + k, s.N - 1);
-        s.cellCand[(size_t)c * kCellCap + k] = make_float4(x.x, x.y, __int_as_float(tag), __int_as_float(gi));
+        s.cellCand[(size_t)c * cap + k] = make_float4(x.x, x.y, __int_as_float(tag), __int_as_float(gi));
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         sc->nbrSum = 0ull;
@@ -457,8 +469,8 @@ __device__ __forceinline__ CoopRebuild coop_rebuild(const DevSys &s, CoopShared 
         for (int b = (threadIdx.x >> 5) * per; b < mem.tiles * kStepBlock; b += (blockDim.x >> 5) * per) {
             const int q = b + lane / kListLanes, j = q / kStepBlock, col = q % kStepBlock;
             const int i = (mem.first + j * mem.stride) * kStepBlock + col;
-            const int k = fast ? coop_list<true>(s, mem, cnt, pos, i, j, col, i < s.N)
-                               : coop_list<false>(s, mem, cnt, pos, i, j, col, i < s.N);
+            const int k = fast ? coop_list<true, SLOT>(s, mem, cnt, pos, i, j, col, i < s.N)
+                               : coop_list<false, SLOT>(s, mem, cnt, pos, i, j, col, i < s.N);
             if (i < s.N && (lane & (kListLanes - 1)) == 0) {
                 kmax = max(kmax, k);
                 ksum += k;
@@ -518,14 +530,16 @@ __device__ __forceinline__ void coop_write_lists(const DevSys &s, const CoopMem 
 // The cell arrays of the last rebuild as the plain kernels leave them:
 // cellStart (the exclusive scan of the counts, a contiguous chunk of cells per
 // block), sortedIds and cellSorted.
+template <bool SLOT>
 __device__ __forceinline__ bool coop_cells(const DevSys &s, CoopShared &sh, CoopRun &r) {
+    const int cap = cell_cap<SLOT>(s);
     const int *cnt = s.cellFill + (size_t)r.cnt * s.ncells;
     const int chunk = (s.ncells + gridDim.x - 1) / gridDim.x;
     const int c0 = min((int)blockIdx.x * chunk, s.ncells), c1 = min(c0 + chunk, s.ncells);
     int sum = 0, tot = 0;
     for (int cb = c0; cb < c1; cb += blockDim.x) {
         const int c = cb + threadIdx.x;
-        block_scan(sh, c < c1 ? min(__ldcg(cnt + c), kCellCap) : 0, tot);
+        block_scan(sh, c < c1 ? min(__ldcg(cnt + c), cap) : 0, tot);
         sum += tot;
     }
     unsigned long long *counts = coop_words(s);
@@ -542,12 +556,12 @@ __device__ __forceinline__ bool coop_cells(const DevSys &s, CoopShared &sh, Coop
     int carry = sh.before;
     for (int cb = c0; cb < c1; cb += blockDim.x) {
         const int c = cb + threadIdx.x;
-        const int n = c < c1 ? min(__ldcg(cnt + c), kCellCap) : 0;
+        const int n = c < c1 ? min(__ldcg(cnt + c), cap) : 0;
         const int at = carry + block_scan(sh, n, tot);
         carry += tot;
         if (c < c1) s.cellStart[c] = at;
         for (int q = 0; q < n && at + q < s.N; q++) {
-            const float4 e = __ldcg(s.cellCand + (size_t)c * kCellCap + q);
+            const float4 e = __ldcg(s.cellCand + (size_t)c * cap + q);
             s.cellSorted[at + q] = e;
             s.sortedIds[at + q] = __float_as_int(e.z) & kIdMask;
         }
@@ -1156,7 +1170,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
     // the cell arrays of the last rebuild; then the last sums
     if (ok && r.updates != updates0) {
         coop_write_lists<FAST>(s, mem);
-        ok = coop_cells(s, sh, r);
+        ok = coop_cells<SLOT>(s, sh, r);
     }
     __syncthreads();
     if (ok) ok = coop_exchange(s, sh, r, 0u, false, true);
