@@ -79,6 +79,13 @@ bool coop_run_fits(const DevSys &s, const CoopArgs &plan) {
     size_t smem;
     CoopArgs a = plan;
     if (!coop_shape(s, grid, smem, a)) return false;
+    // One type in the fast mode with long lists: from the fifth tile of a block on
+    // shared memory does not hold them all, and the step kernel's packed loop is
+    // faster.  LJ fluid, run(50), launch / plain kernels (us): capacity 56 (cutoff
+    // 3.5), 70,000 particles 1149 / 1322, 80,000 1422 / 1380; 96 (cutoff 5), 1862 /
+    // 1994 and 2293 / 2063; 48 (skin 1), 80,000 1063 / 1083, 98,000 1158 / 1140.
+    const int ntiles = (s.N + kStepBlock - 1) / kStepBlock;
+    if (s.fast && s.numTypes <= 1 && s.nBonded == 0 && ntiles > 4 * grid && s.nbrCap > 48) return false;
     if (kernel_setup(coop_kernel(s, a.eng), kCoopThreads, smem, &resident)) return false;
     return resident >= grid;
 }
