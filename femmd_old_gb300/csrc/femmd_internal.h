@@ -99,6 +99,7 @@ struct DevSys {
     float nnRadiusSq;
     int imageExact;
     int numTypes, sigmaByType, sigmaOne;  // sigmaOne: every sigma_ij^2 of the table is exactly 1
+    int cellCap;  // see cellCand
     const PairEntry *pair;
     float2 *pos0, *pos1;
     float2 *vel, *acc, *forceOut;
@@ -200,7 +201,6 @@ struct DevSys {
     unsigned long long *runRec;
     int *cellFill, *cellIds;
     float4 *cellCand;
-    int cellCap;
 };
 
 

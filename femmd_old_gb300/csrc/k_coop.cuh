@@ -315,7 +315,8 @@ __device__ __forceinline__ int coop_list(const DevSys &s, const CoopMem &mem, co
     for (int q = 0; q < 9; q++) {
         const int cell = cx[q / 3] * ncy + cy[q % 3];
         n[q] = ld_early(cnt + cell);
-        c0[q] = ld_early(s.cellCand + (size_t)cell * cells + sub);
+        if constexpr (SLOT) c0[q] = ld_early(s.cellCand + (size_t)cell * cells + sub);
+        else c0[q] = ld_early(s.cellCand + (size_t)cell * kCellCap + sub);  // (by 'cells' the kernel spills)
     }
     int *lst = mem.list + (size_t)j * mem.rows * kListRow + col;
     int k = 0;
@@ -398,12 +399,9 @@ __device__ __forceinline__ CoopRebuild coop_rebuild(const DevSys &s, CoopShared 
         const int c = cell_col(x.x, x.y, s.ncx, s.ncy, s.Lx, s.Ly);
         s.cellOf[i] = c;
         const int k = atomicAdd(cnt + c, 1);
-        if (k < cap) {
-            s.cellIds[(size_t)c * cap + k] = i;
-        } else {
-            atomicOr(&sc->overflow, kCoopCrowded);
-            atomicMax(&sc->maxCell, k + 1);
-        }
+        if (k < cap) s.cellIds[(size_t)c * cap + k] = i;
+        else atomicOr(&sc->overflow, kCoopCrowded);
+        if (SLOT && k >= cap) atomicMax(&sc->maxCell, k + 1);
     }
     __syncthreads();
     if (!coop_exchange(s, sh, r, 0u, withhold)) return kRebuildLost;
