@@ -121,7 +121,7 @@ __device__ __forceinline__ int ld_early(const int *p) {
     return v;
 }
 struct CoopDue {
-    unsigned long long x;  // the exchange after which the last of the step's sums were stored
+    unsigned x;  // the exchange (modulo 2^32) after which the last of the step's sums were stored
     unsigned set;  // their set
     int mode, row, reb;
     float vm, d;
@@ -141,8 +141,7 @@ struct CoopShared {
 
 // What every block carries through the launch (the same on each).
 struct CoopRun {
-    unsigned long long base;  // exchanges before this launch
-    unsigned xi;              // and of it
+    unsigned long long made;  // exchanges over the life of the context
     unsigned dueIn, dueOut;  // entries pushed to and taken from CoopShared::due (one per step)
     unsigned dueOk;          // entries whose sums are all stored
     float dispHi;
@@ -204,17 +203,17 @@ __device__ __forceinline__ bool coop_exchange(const DevSys &s, CoopShared &sh, C
     if (threadIdx.x == 0) {
         unsigned m = value, o = 0u;
         sh.ok = (gridDim.x == 1 && !withhold) ||
-                grid_exchange(s.runRec, r.base + r.xi, gridDim.x, value, 0u, withhold, m, o);
+                grid_exchange(s.runRec, r.made, gridDim.x, value, 0u, withhold, m, o);
         sh.maxBits = m;
     }
     // a step's sums are visible once the exchange after its own is complete
     while (r.dueOut != r.dueOk && !all) {
         const CoopDue &d = sh.due[r.dueOut & 3u];
-        if (r.base + r.xi < d.x + 2) break;
+        if ((int)((unsigned)r.made - d.x) < 2) break;
         if (blockIdx.x == 0 && threadIdx.x == 64) coop_totals(s, d);
         r.dueOut++;
     }
-    r.xi++;
+    r.made++;
     if (threadIdx.x >> 5 >= 3) meanwhile();
     __syncthreads();
     if (sh.ok) return true;
@@ -940,7 +939,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
     for (int q = threadIdx.x; q < nt; q += blockDim.x) sh.tab[q] = s.pair[q];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     CoopRun r = {};
-    r.base = sc->runTag;
+    r.made = sc->runTag;
     r.dispHi = a.begin ? 0.0f : sc->dispHi;
     r.row = a.begin ? 0 : sc->obsRow;
     r.stepNow = a.begin ? s.stepBase : sc->stepNow;
@@ -1041,8 +1040,9 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
         if (rebuild) {
             // (neither lists nor their lengths are read before a rebuild that was
             // made, or the lists of the launch before, loaded above)
-            if (!(ok = coop_rebuild<SLOT>(s, sh, mem, r, p, withhold) == kRebuildDone)) break;
+            ok = coop_rebuild<SLOT>(s, sh, mem, r, p, withhold) == kRebuildDone;
             withhold = false;
+            if (!ok) break;
         }
         if (u >= total) break;
         const int mode = (a.begin && u == 0) ? MODE_FIRST : ((a.end && u == total - 1) ? MODE_LAST : MODE_MID);
@@ -1099,7 +1099,6 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
             if (anybad) atomicOr(&sc->nonfinite, 1);
         }
         __syncthreads();
-        const unsigned long long x = r.base + r.xi;
         float mm = 0.0f;
         if (warp == 0) mm = warp_max(lane < kCoopThreads / 32 ? sh.vmax[lane] : 0.0f);
         if (!(ok = coop_exchange(s, sh, r, __float_as_uint(mm), withhold, false,
@@ -1123,7 +1122,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
                 atomicAdd(coop_sums(s, r.dueIn - 1), sh.accTri);
                 sh.accTri = 0ull;
             }
-            if (blockIdx.x == 0 && threadIdx.x == 0) sh.due[(r.dueIn - 1) & 3u].x = x;
+            if (blockIdx.x == 0 && threadIdx.x == 0) sh.due[(r.dueIn - 1) & 3u].x = (unsigned)r.made - 1u;
             r.dueOk = r.dueIn;
         }
         // the rebuild rule (md3dsystem.cpp:177, nn.cpp:118), the same on every block
@@ -1136,7 +1135,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
         }
         if (blockIdx.x == 0 && threadIdx.x == 0) {
             CoopDue &d = sh.due[r.dueIn & 3u];
-            d.x = x;
+            d.x = (unsigned)r.made - 1u;
             d.set = r.dueIn;
             d.mode = mode;
             d.row = r.row;
@@ -1179,7 +1178,7 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_coop(const __grid_constant_
         sc->obsRow = r.row;
         sc->stepNow = r.stepNow;
         sc->totalUpdates = r.updates;
-        sc->runTag = r.base + r.xi;
+        sc->runTag = r.made;
         sc->runFill = r.cnt;
         sc->runStop = !ok;
     }
