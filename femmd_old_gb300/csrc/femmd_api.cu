@@ -3298,7 +3298,8 @@ static femmd_status adj_recompute(femmd_ctx *ctx, int g, std::vector<int> &rebui
             }
         }
         if ((e = read_scalars(ctx))) return e;
-        if (ctx->hsc->overflow & 8) return expired(ctx, "a grid-wide exchange");
+        // (sweepLost: in the reverse sweep of the segment after this one)
+        if ((ctx->hsc->overflow & 8) || ctx->hsc->sweepLost) return expired(ctx, "a grid-wide exchange");
         if (!(ctx->hsc->overflow & 32)) break;
         coop_left(ctx);
     }
@@ -3378,8 +3379,8 @@ femmd_status femmd_adjoint_backward(femmd_ctx *ctx, double c_wall, double c_fea,
     if (sweep) {
         const DevSys s = make_sys(ctx);
         sweep = adj_sweep_fits(s, coop_plan(ctx, s));
-        CK(cudaMemsetAsync(&ctx->sc.p->sweepLost, 0, sizeof(int), sm));
     }
+    CK(cudaMemsetAsync(&ctx->sc.p->sweepLost, 0, sizeof(int), sm));
     for (int g = nseg - 1; g >= 0; g--) {
         if ((st = adj_recompute(ctx, g, rebuilt))) return st;
         const int K = a.segLen[g], s0 = a.segStart[g];
@@ -3415,6 +3416,8 @@ femmd_status femmd_adjoint_backward(femmd_ctx *ctx, double c_wall, double c_fea,
                 w.kLo = to;
                 w.segStart = s0;
                 w.start = a.segStart[0];
+                w.withhold = ctx->testExpire ? 1 : 0;
+                ctx->testExpire = false;
                 if ((st = coop_clean(ctx))) return st;
                 CK(launch_adj_sweep(sm, s, coop_plan(ctx, s), w));
                 if ((k - std::max(to, 1) + 1) & 1) std::swap(wc, wn);

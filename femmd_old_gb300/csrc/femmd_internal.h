@@ -323,6 +323,7 @@ struct AdjSweep {
     float2 *w0, *w1, *xbar, *vbar;
     double *gMu, *gLam, *epsAcc, *sigAcc;
     int kHi, kLo, segStart, start;    // step numbers of the segment's slot 0 and of the run's start
+    int withhold;                     // block 0 withholds its first exchange record (a test of the timeout)
     int rows, incStaged;              // shared memory (the launch sets them)
 };
 // plan: the triangles by block of the whole-run launch, whose grid it has.

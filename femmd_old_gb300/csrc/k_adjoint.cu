@@ -496,7 +496,8 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_adj_sweep(DevSys s, CoopArg
         __syncthreads();
         if (threadIdx.x == 0) {
             unsigned mv, ov;
-            okay = gridDim.x == 1 || grid_exchange(s.runRec, base + xi, gridDim.x, 0u, 0u, false, mv, ov);
+            okay = gridDim.x == 1 || grid_exchange(s.runRec, base + xi, gridDim.x, 0u, 0u,
+                                                       a.withhold && xi == 0 && blockIdx.x == 0, mv, ov);
             if (!okay) s.sc->sweepLost = 1;
         }
         xi++;

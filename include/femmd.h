@@ -249,10 +249,10 @@ femmd_status femmd_set_profiling(femmd_ctx *ctx, int profile);
 femmd_status femmd_get_profile(femmd_ctx *ctx, double *force_kernel_ms, long long *force_kernel_launches,
                                double *rebuild_ms, long long *rebuilds, long long *kernel_launches);
 /* For tests of the failure path: in the next run that is one cooperative
- * launch (small and medium systems, both force modes), block 0 withholds its record of
- * the first grid-wide exchange, so every block's bounded wait gives up
- * (about a second) and femmd_run returns FEMMD_TIMEOUT with the context
- * still usable.  No GPU fault, trap or endless wait is involved. */
+ * launch (small and medium systems, both force modes), or the next reverse sweep
+ * that is, block 0 withholds its record of the first grid-wide exchange, so every
+ * block's bounded wait gives up (about a second) and femmd_run or
+ * femmd_adjoint_backward returns FEMMD_TIMEOUT with the context still usable.  No GPU fault, trap or endless wait is involved. */
 femmd_status femmd_test_expire_next_exchange(femmd_ctx *ctx);
 /* For tests of long-lived contexts: from here on as if 'made' grid-wide
  * exchanges had been made (FEMMD_UNSUPPORTED where runs are not one
