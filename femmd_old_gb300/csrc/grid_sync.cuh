@@ -2,8 +2,8 @@
 // (k_coop in k_coop.cuh, k_adj_sweep in k_adjoint.cu).
 //
 // An exchange is a barrier over the grid that carries the maximum of one
-// unsigned value per block and the OR of another.  Each block's thread 0 adds
-// to one slot of memory {max, or, count} with reductions, the count last
+// unsigned value per block.  Each block's thread 0 adds
+// to one slot of memory {max, count} with reductions, the count last
 // behind an acquire-release fence, and polls the slot (one 16-byte acquire
 // load) until every block has counted.  Measured on 512-thread blocks that
 // have just stored 2 KB each (cycles): 2400 with 32 blocks, 2730 with 152; a
@@ -15,7 +15,7 @@
 // Four slots take turns, exchange X (counted over the life of the context, in 64
 // bits: a small system makes 2^32 of them in hours)
 // using slot X & 3; a slot's count grows by the grid size with every use, and
-// its max and or are cleared for exchange X + 2 by block 0 after exchange X:
+// its maximum is cleared for exchange X + 2 by block 0 after exchange X:
 // every block that used them last (X - 2) has read them before it counted in
 // X - 1, and none adds to them again before block 0 has counted in X + 1.
 #pragma once
@@ -37,13 +37,9 @@ __device__ __forceinline__ unsigned long long *grid_slot(unsigned long long *bas
 // barrier that follows it, every store made by any block before its call is
 // visible to the whole block.
 __device__ __forceinline__ bool grid_exchange(unsigned long long *base, unsigned long long x, int blocks,
-                                              unsigned value, unsigned flags, bool withhold, unsigned &maxv,
-                                              unsigned &orv) {
+                                              unsigned value, bool withhold, unsigned &maxv) {
     unsigned long long *slot = grid_slot(base, x);
     if (value) asm volatile("red.relaxed.gpu.global.max.u32 [%0], %1;" ::"l"(slot), "r"(value) : "memory");
-    if (flags)
-        asm volatile("red.relaxed.gpu.global.or.b32 [%0], %1;" ::"l"(reinterpret_cast<unsigned *>(slot) + 1), "r"(flags)
-                     : "memory");
     asm volatile("fence.acq_rel.gpu;" ::: "memory");
     if (!withhold) asm volatile("red.relaxed.gpu.global.add.u64 [%0], %1;" ::"l"(slot + 1), "l"(1ull) : "memory");
     const unsigned long long want = (x / kGridSlots + 1ull) * (unsigned long long)blocks;
@@ -56,7 +52,6 @@ __device__ __forceinline__ bool grid_exchange(unsigned long long *base, unsigned
                      : "memory");
     } while (hi < want && ++it < kGridPolls);
     maxv = (unsigned)lo;
-    orv = (unsigned)(lo >> 32);
     if (blockIdx.x == 0) *reinterpret_cast<volatile unsigned long long *>(grid_slot(base, x + 2)) = 0ull;
     return hi >= want;
 }

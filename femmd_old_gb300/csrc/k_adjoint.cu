@@ -495,9 +495,9 @@ __global__ void __launch_bounds__(kCoopThreads, 1) k_adj_sweep(DevSys s, CoopArg
         if (k == a.kLo) break;
         __syncthreads();
         if (threadIdx.x == 0) {
-            unsigned mv, ov;
-            okay = gridDim.x == 1 || grid_exchange(s.runRec, base + xi, gridDim.x, 0u, 0u,
-                                                       a.withhold && xi == 0 && blockIdx.x == 0, mv, ov);
+            unsigned mv;
+            okay = gridDim.x == 1 || grid_exchange(s.runRec, base + xi, gridDim.x, 0u,
+                                                       a.withhold && xi == 0 && blockIdx.x == 0, mv);
             if (!okay) s.sc->sweepLost = 1;
         }
         xi++;

@@ -3,7 +3,7 @@
 //
 // One graph unit of the plain path (step kernel, conditional rebuild) costs
 // 15-25 us whatever the system's size: launches, the IF node, and the drain
-// of each kernel.  Up to a few hundred thousand particles the arithmetic of a
+// of each kernel.  Up to about 100,000 particles the arithmetic of a
 // step takes less than that, so k_coop advances the run inside one launch:
 // every block owns fixed tiles of particles, a step is the triangle pass, the
 // particle pass and a grid-wide exchange, and every block takes the rebuild
@@ -201,9 +201,9 @@ template <class Work = Nothing>
 __device__ __forceinline__ bool coop_exchange(const DevSys &s, CoopShared &sh, CoopRun &r, unsigned value,
                                               bool withhold = false, bool all = false, Work meanwhile = {}) {
     if (threadIdx.x == 0) {
-        unsigned m = value, o = 0u;
+        unsigned m = value;
         sh.ok = (gridDim.x == 1 && !withhold) ||
-                grid_exchange(s.runRec, r.made, gridDim.x, value, 0u, withhold, m, o);
+                grid_exchange(s.runRec, r.made, gridDim.x, value, withhold, m);
         sh.maxBits = m;
     }
     // a step's sums are visible once the exchange after its own is complete

@@ -39,7 +39,6 @@
 #include "launch.h"
 #include "device_common.cuh"
 #include "fast_body.cuh"
-#include "grid_sync.cuh"
 #include "nn_body.cuh"
 #include "step_body.cuh"
 

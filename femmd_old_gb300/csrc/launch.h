@@ -78,24 +78,6 @@ struct Launch {
         return cudaSuccess;
     }
 
-    // Open a WHILE node (the body runs while the condition, set on the
-    // device, is nonzero); 'body' receives the body graph.  Graph mode only.
-    cudaError_t begin_while(cudaGraphConditionalHandle h, Launch &body) {
-        cudaGraphNodeParams p = {};
-        p.type = cudaGraphNodeTypeConditional;
-        p.conditional.handle = h;
-        p.conditional.type = cudaGraphCondTypeWhile;
-        p.conditional.size = 1;
-        cudaGraphNode_t n;
-        cudaError_t e = cudaGraphAddNode(&n, graph, deps.empty() ? nullptr : deps.data(), nullptr, deps.size(), &p);
-        if (e != cudaSuccess) return e;
-        deps.assign(1, n);
-        body.stream = stream;
-        body.graph = p.conditional.phGraph_out[0];
-        body.deps.clear();
-        return cudaSuccess;
-    }
-
     // kernel() with the grid in clusters of n blocks.  Graph mode only.
     template <typename... KArgs, typename... Args>
     cudaError_t kernel_clusters(void (*k)(KArgs...), int n, dim3 g, dim3 b, size_t smem, Args &&...args) {

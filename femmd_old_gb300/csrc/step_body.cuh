@@ -474,20 +474,19 @@ __device__ __forceinline__ void bonded_forces(const DevSys &s, int i, int mode, 
 // the doubled energy and virial, add the wall energy and the moving walls,
 // then the integration of the mode (kick, observables, next half kick and
 // drift into pout) and the outputs of MODE_FORCES / MODE_INIT / MODE_LAST.
-// m, v: its mass and velocity; stepIdx: the step the moving walls are at
-// (-1: DevScalars::stepNow).
+// m, v: its mass and velocity.
 template <bool WX, bool WY>
 __device__ __forceinline__ void finish_particle(const DevSys &s, int i, int mode, float2 pi, float2 *pout, float fx,
                                                 float fy, float ue, float we, float utri, float uwall, float m,
                                                 float2 v, float &ue_out, float &we_out, float &ke, float &vvm,
-                                                bool &bad, int stepIdx = -1) {
+                                                bool &bad) {
     const float Lx = s.Lx, Ly = s.Ly;
     ue *= 0.5f;
     we *= 0.5f;
     ue += uwall;
     if (s.wallOn) {
         // harmonic walls after the pair forces: top wall at y_w(n), bottom at 0
-        const float yw = wall_y(s, stepIdx >= 0 ? stepIdx : s.sc->stepNow);
+        const float yw = wall_y(s, s.sc->stepNow);
         const float dl = s.wallDelta[i];
         const float ht = (pi.y + dl) - yw;
         if (ht > 0.0f) {
