@@ -136,6 +136,16 @@ __device__ __forceinline__ float2 add2(float2 a, float2 b) {
     return unpack2(r);
 }
 
+// 1/x for 2^-100 <= x <= 2^100, correctly rounded as __frcp_rn gives it: the
+// approximate reciprocal and one Newton-Raphson step in fused multiply-adds
+// (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990).  tests/test_gpu_rcp.py compares every float of the range.
+__device__ __forceinline__ float rcp_newton(float x) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+    return __fmaf_rn(y, __fmaf_rn(-x, y, 1.0f), y);
+}
+
 __device__ __forceinline__ float warp_sum_f(float v) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);

@@ -348,11 +348,7 @@ __device__ __forceinline__ void lj_pair(const DevSys &s, const PairEntry *tab, c
 //     difference), no image test.  'far' keeps the largest |difference|: if it
 //     reaches half a box length, a pair crossed the boundary and the caller
 //     works the particle again by lj_pair.
-//   * 1/r^2 correctly rounded as __frcp_rn gives it: the approximate
-//     reciprocal and one Newton-Raphson step in fused multiply-adds
-//     (Markstein, "Computation of elementary functions on the IBM RISC
-//     System/6000 processor", 1990).  All floats of [2^-100, 2^100] were
-//     compared with __frcp_rn; 'close' keeps the smallest r^2, and below
+//   * 1/r^2 by rcp_newton; 'close' keeps the smallest r^2, and below
 //     kPairClose the caller works the particle again by lj_pair.
 //   * c s6 (s6 - 1/2) and 4 eps s6 (s6 - 1) as one packed product.
 // Measured: the batched kernel 27.2 -> 23.5 ms (128 replicas, run(100)), the
@@ -394,9 +390,7 @@ __device__ __forceinline__ float4 lj_terms_x2(const DevSys &s, float2 pi, float2
         if (!EDGE) far = fmaxf(far, fmaxf(fabsf(d.x), fabsf(d.y)));
         close = fminf(close, dr2);
     }
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(dr2));
-    const float dr2i = __fmaf_rn(y, __fmaf_rn(-dr2, y, 1.0f), y);
+    const float dr2i = rcp_newton(dr2);
     const float dr6i = dr2i * dr2i * dr2i;
     const float2 r6 = make_float2(dr6i, dr6i);
     const float2 g = mul2(mul2(ce, r6), add2(r6, make_float2(-0.5f, -1.0f)));
