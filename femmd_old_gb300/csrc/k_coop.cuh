@@ -408,7 +408,10 @@ __device__ __forceinline__ CoopRebuild coop_rebuild(const DevSys &s, CoopShared 
     // of the exchange above, and nothing sets it again before the next one, which no
     // block completes without this one
     if (__ldcg(&sc->nonfinite) != 0 || (__ldcg(&sc->overflow) & kCoopCrowded)) {
-        if (blockIdx.x == 0 && threadIdx.x == 0) atomicOr(&sc->overflow, kCoopLeft);
+        if (blockIdx.x == 0 && threadIdx.x == 0) {
+            atomicOr(&sc->overflow, kCoopLeft);
+            sc->builds -= (unsigned long long)(r.updates - 1);  // the run's lists are built again by its repeat
+        }
         return kRebuildLeft;
     }
     // 2: ascending id inside each cell; the other counts cleared for the next

@@ -53,7 +53,7 @@ def record(sc, mode, direct, runs, path=None, every=0):
     for n in runs:
         s.run(n)
         out += [*s.get_state(), s.forces(), s.step_observables(), *s.cells(), *s.neighbors(),
-                np.array([s.total_updates(), s.steps()])]
+                np.array([s.total_updates(), s.steps(), s.nn_stats()["builds"]])]
     s.set_profiling(False)
     if path:
         s.flush_trajectory()
@@ -137,6 +137,7 @@ def test_non_finite_inside_the_run():
         s.set_profiling(direct)
         with pytest.raises(F.FemmdError):
             s.run(60)
-        left.append([np.isnan(x) for x in s.get_state()] + [np.nan_to_num(x) for x in s.get_state()])
+        left.append([np.isnan(x) for x in s.get_state()] + [np.nan_to_num(x) for x in s.get_state()] +
+                    [np.array([s.nn_stats()["builds"]])])
         s.set_profiling(False)
     same_bytes(*left)
