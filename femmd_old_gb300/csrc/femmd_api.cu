@@ -1197,8 +1197,13 @@ static bool coop_left(femmd_ctx *ctx) {
     if (!(ctx->hsc->overflow & 16)) return false;
     const int cap = std::max(2 * ctx->cellCap, (ctx->hsc->maxCell + ctx->hsc->maxCell / 4 + 31) / 32 * 32);
     const bool again = (size_t)cap * ctx->ncells <= (1u << 20) && coop_by_slot(make_sys(ctx));
-    if (again) ctx->cellCap = cap;
-    else ctx->coopOff = true;
+    if (again) {
+        ctx->cellCap = cap;
+    } else {
+        ctx->coopOff = true;
+        ctx->cellIds.release();  // (the stream is idle: the scalars have just been read)
+        ctx->cellCand.release();
+    }
     return again;
 }
 
